@@ -233,6 +233,9 @@ spe::Ctx make_ctx(spe_engine* e, int first, int count) {
   c.ipp = e->ipp;
   c.tma = e->tma;
   c.err = e->dev_err;
+  c.At = e->At;
+  c.sp = e->sp;
+  c.odd = e->odd;
   return c;
 }
 
@@ -368,6 +371,10 @@ void free_population(spe_engine* e) {
   cudaFreeHost(e->red_host);
   cudaFree(e->sel_state);
   cudaFree(e->sel_hist);
+  cudaFree(e->sp);
+  cudaFree(e->odd);
+  e->sp = nullptr;
+  e->odd = nullptr;
   e->rho = nullptr;
   e->S = nullptr;
   e->T = e->T2 = nullptr;
@@ -508,6 +515,7 @@ int spe_create(int n, int device, spe_engine** out) {
   ops->fill_tw(tw.data(), n);
   err = cudaMalloc(&e->tw, tw.size() * sizeof(float2));
   if (err == cudaSuccess) err = cudaMalloc(&e->A, e->npix * sizeof(float));
+  if (err == cudaSuccess && ops->blocked_cols) err = cudaMalloc(&e->At, e->npix * sizeof(float));
   if (err == cudaSuccess) err = cudaMemcpy(e->tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice);
   if (err == cudaSuccess) err = cudaMalloc(&e->dev_err, sizeof(int));
   if (err == cudaSuccess) err = cudaMemset(e->dev_err, 0, sizeof(int));
@@ -518,6 +526,7 @@ int spe_create(int n, int device, spe_engine** out) {
   if (err != cudaSuccess) {
     cudaFree(e->tw);
     cudaFree(e->A);
+    cudaFree(e->At);
     cudaFree(e->dev_err);
     cudaStreamDestroy(e->own);
     delete e;
@@ -533,6 +542,7 @@ int spe_destroy(spe_engine* e) {
   cudaStreamSynchronize(e->st);
   free_population(e);
   cudaFree(e->A);
+  cudaFree(e->At);
   cudaFree(e->tw);
   cudaFree(e->dev_err);
   delete[] static_cast<unsigned char*>(e->tma);
@@ -573,6 +583,7 @@ int spe_set_amplitudes(spe_engine* e, const float* amp) {
   if (!e || !amp) return fail(SPE_ERR_INVALID, "null argument");
   CK(cudaSetDevice(e->dev), "cudaSetDevice");
   CK(cudaMemcpyAsync(e->A, amp, e->npix * sizeof(float), cudaMemcpyHostToDevice, e->st), "upload amplitudes");
+  if (e->At) CK(e->ops->block_amplitudes(e->A, e->At, 1, e->st), "amplitude order");
   CK(cudaStreamSynchronize(e->st), "synchronize");
   e->have_amp = true;
   e->ipp = 0;
@@ -587,14 +598,24 @@ int spe_set_amplitudes_batch(spe_engine* e, const float* amp, int npatterns, int
   CK(cudaSetDevice(e->dev), "cudaSetDevice");
   if (npatterns > e->a_cap) {
     CK(cudaStreamSynchronize(e->st), "synchronize");
-    float* a = nullptr;
+    float *a = nullptr, *at = nullptr;
     CK(cudaMalloc(&a, (size_t)npatterns * e->npix * sizeof(float)), "amplitude allocation");
+    if (e->At) {
+      const cudaError_t err = cudaMalloc(&at, (size_t)npatterns * e->npix * sizeof(float));
+      if (err != cudaSuccess) {
+        cudaFree(a);
+        return cuda_fail(err, "amplitude allocation");
+      }
+      cudaFree(e->At);
+      e->At = at;
+    }
     cudaFree(e->A);
     e->A = a;
     e->a_cap = npatterns;
   }
   CK(cudaMemcpyAsync(e->A, amp, (size_t)npatterns * e->npix * sizeof(float), cudaMemcpyHostToDevice, e->st),
      "upload amplitudes");
+  if (e->At) CK(e->ops->block_amplitudes(e->A, e->At, npatterns, e->st), "amplitude order");
   CK(cudaStreamSynchronize(e->st), "synchronize");
   e->npatterns = npatterns;
   e->ipp = npatterns > 1 ? individuals_per_pattern : 0;
@@ -630,6 +651,8 @@ int spe_reserve(spe_engine* e, int capacity) {
   t.partials = t.red = nullptr;
   t.red_host = nullptr;
   t.sel_state = t.sel_hist = nullptr;
+  t.sp = nullptr;
+  t.odd = nullptr;
   if (err == cudaSuccess) err = cudaMalloc(&t.rho, np * sizeof(float2));
   if (err == cudaSuccess) err = cudaMalloc(&t.S, np * sizeof(int));
   if (err == cudaSuccess) err = cudaMalloc(&t.T, np * sizeof(float2));
@@ -640,6 +663,8 @@ int spe_reserve(spe_engine* e, int capacity) {
   if (err == cudaSuccess) err = cudaMallocHost(&t.red_host, (size_t)capacity * 16 * sizeof(double));
   if (err == cudaSuccess) err = cudaMalloc(&t.sel_state, (size_t)capacity * 2 * sizeof(uint32_t));
   if (err == cudaSuccess) err = cudaMalloc(&t.sel_hist, (size_t)capacity * 256 * sizeof(uint32_t));
+  if (err == cudaSuccess && e->ops->sp_bytes) err = cudaMalloc(&t.sp, (size_t)capacity * e->ops->sp_bytes);
+  if (err == cudaSuccess && e->ops->sp_bytes) err = cudaMalloc(&t.odd, (size_t)capacity * e->n);
   if (err == cudaSuccess && e->cap > 0) {
     const size_t old = (size_t)e->cap * e->npix;
     err = cudaMemcpy(t.rho, e->rho, old * sizeof(float2), cudaMemcpyDeviceToDevice);
@@ -671,6 +696,8 @@ int spe_reserve(spe_engine* e, int capacity) {
   e->red_host = t.red_host;
   e->sel_state = t.sel_state;
   e->sel_hist = t.sel_hist;
+  e->sp = t.sp;
+  e->odd = t.odd;
   return SPE_OK;
 }
 
@@ -923,6 +950,10 @@ int spe_set_tiles(spe_engine* e, int cols, int rows) {
   };
   if (!ok(cols, e->ops->col_widths) || !ok(rows, e->ops->row_widths))
     return fail(SPE_ERR_INVALID, "tile widths %d/%d not compiled for size %d", cols, rows, e->n);
+  // the blocked-scratch passes hand T to each other in their own layout
+  const int bc = e->ops->blocked_cols, br = e->ops->blocked_rows;
+  if (bc && ((cols == bc && rows != 0 && rows != br) || (rows == br && cols != 0 && cols != bc)))
+    return fail(SPE_ERR_INVALID, "tile codes %d/%d: %d and %d go together", cols, rows, bc, br);
   e->tile_cols = cols;
   e->tile_rows = rows;
   return SPE_OK;
@@ -1123,15 +1154,22 @@ int spe_get_schedule(spe_engine* e, int* chunk, int* lanes) {
 
 int spe_get_tiles(spe_engine* e, int* cols, int* rows) {
   if (!e || !cols || !rows) return fail(SPE_ERR_INVALID, "null argument");
-  *cols = e->tile_cols != 0 ? e->tile_cols : e->ops->default_cols;
-  *rows = e->tile_rows > 0 ? e->tile_rows : e->ops->default_rows;
+  const spe::SizeOps* o = e->ops;
+  if (o->blocked_cols && (e->tile_cols == 0 || e->tile_cols == o->blocked_cols) &&
+      (e->tile_rows <= 0 || e->tile_rows == o->blocked_rows)) {
+    *cols = o->blocked_cols;
+    *rows = o->blocked_rows;
+    return SPE_OK;
+  }
+  *cols = e->tile_cols != 0 ? e->tile_cols : o->default_cols;
+  *rows = e->tile_rows > 0 ? e->tile_rows : o->default_rows;
   return SPE_OK;
 }
 
 // Times the compiled tile widths of the iteration kernels on the resident
 // population [first, first+count) (RAAR, `iterations` per trial, median of
-// three) -- first the column pass with the current row width, then every row
-// width with every schedule (whole range, or blocks on one or two lanes; a
+// three) -- first the row-major column passes with the current row width, then
+// every row width (the blocked-scratch pair among them) with every schedule (whole range, or blocks on one or two lanes; a
 // blocked schedule is kept only when 2% faster than the best whole-range
 // one, the two re-timed over three times the iterations when they are within
 // 5%) -- keeps the fastest and restores the densities.
@@ -1166,10 +1204,12 @@ int spe_autotune(spe_engine* e, int first, int count, int iterations, int* cols,
   auto trial = [&](int wc, int wr, float* ms) { return trial_s(wc, wr, 0, 1, ms); };
   int wcs[32], wrs[32];
   const int nc = e->ops->col_widths(wcs), nr = e->ops->row_widths(wrs);
-  int best_c = e->tile_cols != 0 ? e->tile_cols : e->ops->default_cols;
-  int best_r = e->tile_rows > 0 ? e->tile_rows : e->ops->default_rows;
+  const int blk_c = e->ops->blocked_cols, blk_w = e->ops->blocked_rows;
+  int best_c = e->tile_cols != 0 && e->tile_cols != blk_c ? e->tile_cols : e->ops->default_cols;
+  int best_r = e->tile_rows > 0 && e->tile_rows != blk_w ? e->tile_rows : e->ops->default_rows;
   float best = 1e30f;
   for (int i = 0; i < nc; ++i) {
+    if (blk_c && wcs[i] == blk_c) continue;
     float ms;
     if ((rc = trial(wcs[i], best_r, &ms))) break;
     if (ms < best) {
@@ -1190,13 +1230,15 @@ int spe_autotune(spe_engine* e, int first, int count, int iterations, int* cols,
       for (int k = 0; k < ns && !dup; ++k) dup = sched[k][0] == chunk && sched[k][1] == lanes;
       if (!dup && ns < 16) sched[ns][0] = chunk, sched[ns][1] = lanes, ++ns;
     }
-  // the fastest whole-range and the fastest blocked configuration
+  // the column code that goes with row code wr
+  auto col_of = [&](int wr) { return blk_w && wr == blk_w ? blk_c : best_c; };
+  // the fastest whole-range configuration and the fastest in blocks of individuals
   int whole_r = best_r, blk_r = 0, blk_chunk = 0, blk_lanes = 1;
   float whole = 1e30f, blocked = 1e30f;
   for (int i = 0; !rc && i < nr; ++i)
     for (int k = 0; !rc && k < ns; ++k) {
       float ms;
-      if ((rc = trial_s(best_c, wrs[i], sched[k][0], sched[k][1], &ms))) break;
+      if ((rc = trial_s(col_of(wrs[i]), wrs[i], sched[k][0], sched[k][1], &ms))) break;
       if (sched[k][0] == 0) {
         if (ms < whole) whole = ms, whole_r = wrs[i];
       } else if (ms < blocked) {
@@ -1213,7 +1255,8 @@ int spe_autotune(spe_engine* e, int first, int count, int iterations, int* cols,
       float tw = 0.f, tb = 0.f;
       const int it1 = iterations;
       iterations = 10 * it1;
-      if (!(rc = trial_s(best_c, whole_r, 0, 1, &tw))) rc = trial_s(best_c, blk_r, blk_chunk, blk_lanes, &tb);
+      if (!(rc = trial_s(col_of(whole_r), whole_r, 0, 1, &tw)))
+        rc = trial_s(col_of(blk_r), blk_r, blk_chunk, blk_lanes, &tb);
       iterations = it1;
       whole = tw, blocked = tb;
     }
@@ -1224,6 +1267,7 @@ int spe_autotune(spe_engine* e, int first, int count, int iterations, int* cols,
   if (rc) return rc;
   CK(cudaMemcpyAsync(e->rho + (size_t)first * e->npix, save, bytes, cudaMemcpyDeviceToDevice, e->st), "restore");
   CK(cudaStreamSynchronize(e->st), "synchronize");
+  best_c = col_of(best_r);
   e->tile_cols = best_c;
   e->tile_rows = best_r;
   e->chunk = best_chunk;

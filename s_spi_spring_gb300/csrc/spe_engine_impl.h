@@ -49,6 +49,10 @@ struct spe_engine {
   int a_cap = 1;  // patterns the A allocation holds
   void* tma = nullptr;     // tensor maps of the TMA row pass (null: not available)
   int* dev_err = nullptr;  // device flag of the kernels' bounded waits
+  // operands of the blocked-scratch kernels (null at sides without them)
+  float* At = nullptr;           // A in register order, as many patterns
+  void* sp = nullptr;            // packed support, cap * ops->sp_bytes
+  unsigned char* odd = nullptr;  // per row tile: support not 0 / 1, cap * n
   cudaStream_t lane2 = nullptr;          // second lane (created on first use)
   cudaEvent_t fork = nullptr, join = nullptr, phase = nullptr;
   // copy streams of spe_iterate_host and its per-block events (uploaded,

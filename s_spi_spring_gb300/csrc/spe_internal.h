@@ -63,6 +63,11 @@ struct Ctx {
   int ipp;              // individuals per pattern (slot p uses pattern p / ipp of A); 0: A is one pattern
   const void* tma;      // tensor maps of the TMA row pass (row_maps), or null
   int* err;             // device flag set by a bounded wait that gave up, or null
+  // operands of the blocked-scratch kernels (spe_blocked.cuh), or null: the
+  // amplitudes in register order, the packed support and its per-row-tile flags
+  const float* At;
+  void* sp;
+  unsigned char* odd;
 };
 
 // Tensor maps of the TMA row pass (spe_tma_maps.cu): row_maps_bytes() of
@@ -135,6 +140,12 @@ struct SizeOps {
   // place with moments m, v (see OpRowsGradAdam)
   cudaError_t (*adam_step)(const Ctx&, int loss, float eps, double* partials, float2* m, float2* v, float b1,
                            float b2, float step_size, float inv_sqrt_bc2, float adam_eps);
+  // blocked-scratch kernels of the iteration (0 / null: none at this side):
+  // the tile codes of the column and the row pass, the bytes of packed
+  // support per individual, and the amplitudes' reordering
+  int blocked_cols, blocked_rows;
+  size_t sp_bytes;
+  cudaError_t (*block_amplitudes)(const float* A, float* At, int npatterns, cudaStream_t st);
 };
 
 const SizeOps* size_ops(int n);

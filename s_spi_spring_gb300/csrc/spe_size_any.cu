@@ -926,7 +926,11 @@ const SizeOps* size_ops_any(int n) {
                     &SizeAny::known_power,
                     &SizeAny::loss_grad,
                     tiles,
-                    &SizeAny::adam_step};
+                    &SizeAny::adam_step,
+                    0,
+                    0,
+                    0,
+                    nullptr};
   const SizeOps* out = &en->ops;
   g_any.emplace(n, std::move(en));
   return out;

@@ -6,6 +6,7 @@
 #include "spe_internal.h"
 #include "spe_kernels.cuh"
 #include "spe_pipe.cuh"
+#include "spe_blocked.cuh"
 #include "spe_pairs.cuh"
 #include "spe_tma.cuh"
 
@@ -276,6 +277,65 @@ cudaError_t launch_rows_iterate1(const Ctx& c, float scale, float beta, Gate g) 
                     scale, beta, g, c.tw);
 }
 
+// ---- the blocked-scratch kernels (spe_blocked.cuh), tile codes 800 + W
+template <int N>
+constexpr int blocked_cols_code() {
+  return Blocked<N>::ok ? 800 + Blocked<N>::BC : 0;
+}
+template <int N>
+constexpr int blocked_rows_code() {
+  return Blocked<N>::ok ? 800 + Blocked<N>::WR : 0;
+}
+template <int N>
+cudaError_t launch_cols_blocked(const Ctx& c) {
+  using P = BlkCfg<N, Blocked<N>::BC, Blocked<N>::NXC>;
+  auto kern = k_cols_blocked<N>;
+  static std::atomic<unsigned long long> configured{0ull};
+  static std::atomic<int> resident[64] = {};
+  cudaError_t e = configure(kern, P::SMEM, configured);
+  if (e != cudaSuccess || c.count <= 0) return e;
+  const int tiles = c.count * (N / Blocked<N>::BC);
+  const int slots = share(resident_ctas(kern, P::NT, P::SMEM, resident), c.grid_div);
+  return launch_pdl(kern, tiles < slots ? tiles : slots, P::NT, P::SMEM, c.st, c.T, c.At, c.ipp, c.first, c.count,
+                    c.tw);
+}
+template <int N, int UPD>
+cudaError_t launch_rows_blocked(const Ctx& c, float scale, float beta, Gate g) {
+  using P = BlkRowCfg<N>;
+  static_assert(P::SMEM <= kMaxSmem, "row tile");
+  auto kern = k_rows_blocked<N, UPD>;
+  static std::atomic<unsigned long long> configured{0ull};
+  static std::atomic<int> resident[64] = {};
+  cudaError_t e = configure(kern, P::SMEM, configured);
+  if (e != cudaSuccess || c.count <= 0) return e;
+  const int tiles = c.count * (N / Blocked<N>::WR);
+  const int slots = share(resident_ctas(kern, P::NT, P::SMEM, resident), c.grid_div);
+  return launch_pdl(kern, tiles < slots ? tiles : slots, P::NT, P::SMEM, c.st, c.T, c.rho, static_cast<const int*>(c.S),
+                    static_cast<const SpBits<N>*>(c.sp), static_cast<const unsigned char*>(c.odd), c.first, c.count,
+                    scale, beta, g, c.tw);
+}
+template <int N>
+cudaError_t launch_rows_blocked_first(const Ctx& c) {
+  using P = BlkCfg<N, Blocked<N>::WR, 1>;
+  auto kern = k_rows_blocked_first<N>;
+  static std::atomic<unsigned long long> configured{0ull};
+  cudaError_t e = configure(kern, P::SMEM, configured);
+  if (e != cudaSuccess || c.count <= 0) return e;
+  kern<<<(unsigned)c.count * (N / Blocked<N>::WR), P::NT, P::SMEM, c.st>>>(
+      c.rho, c.S, c.T, static_cast<SpBits<N>*>(c.sp), c.odd, c.first, c.tw);
+  return cudaGetLastError();
+}
+template <int N>
+cudaError_t launch_rows_blocked_last(const Ctx& c, float scale) {
+  using P = BlkCfg<N, Blocked<N>::WR, 1>;
+  auto kern = k_rows_blocked_last<N>;
+  static std::atomic<unsigned long long> configured{0ull};
+  cudaError_t e = configure(kern, P::SMEM, configured);
+  if (e != cudaSuccess || c.count <= 0) return e;
+  kern<<<(unsigned)c.count * (N / Blocked<N>::WR), P::NT, P::SMEM, c.st>>>(c.T, c.rho, c.first, scale, c.tw);
+  return cudaGetLastError();
+}
+
 template <int N, int WP>
 cudaError_t launch_cols_pairs_st(const Ctx& c) {
   using P = PairColStCfg<N, WP>;
@@ -495,8 +555,35 @@ struct SizeImpl {
     return launch_pass<N, AX_ROWS>(fin, c.count, c.st, c.tw);
   }
 
-  // wc / wr: tile widths of the column / row pass (<= 0: defaults)
+  // the same sequence on the blocked scratch
+  template <int UPD>
+  static cudaError_t iterate_blocked(const Ctx& c, int iters, float beta, Gate g) {
+    SPE_TRY(launch_rows_blocked_first<N>(c));
+    for (int i = 0; i < iters; ++i) {
+      SPE_TRY(launch_cols_blocked<N>(c));
+      if (i == 0 && c.mark) SPE_TRY(cudaEventRecord(c.mark, c.st));
+      SPE_TRY((launch_rows_blocked<N, UPD>(c, scale(), beta, g)));
+    }
+    SPE_TRY(launch_cols_blocked<N>(c));
+    if (iters == 0 && c.mark) SPE_TRY(cudaEventRecord(c.mark, c.st));
+    return launch_rows_blocked_last<N>(c, scale());
+  }
+
+  // wc / wr: tile codes of the column / row pass (<= 0: defaults).  The
+  // defaults are the blocked-scratch kernels where the side has them and the
+  // caller holds their operands (an engine does, the allocation-free entry
+  // point does not)
   static cudaError_t iterate(const Ctx& c, int upd, int iters, float beta, Gate g, int wc, int wr) {
+    if constexpr (Blocked<N>::ok) {
+      const bool cols = wc == 0 || wc == blocked_cols_code<N>(), rows = wr <= 0 || wr == blocked_rows_code<N>();
+      if (cols && rows && c.At && c.sp && c.odd) {
+        switch (upd) {
+          case 0: return iterate_blocked<UPD_HIO>(c, iters, beta, g);
+          case 1: return iterate_blocked<UPD_RAAR>(c, iters, beta, g);
+          default: return iterate_blocked<UPD_ER>(c, iters, beta, g);
+        }
+      }
+    }
     if (wc == 0) wc = DefaultTiles<N>::cols;
     if (wr <= 0) wr = DefaultTiles<N>::rows;
     switch (upd) {
@@ -508,6 +595,7 @@ struct SizeImpl {
 
   static int col_widths(int* out) {
     int k = 0;
+    if constexpr (Blocked<N>::ok) out[k++] = blocked_cols_code<N>();
     if constexpr (paircolst_ok<N, 4>()) out[k++] = 608;
     if constexpr (paircolst_ok<N, 8>()) out[k++] = 616;
     if constexpr (warpcol_ok<N, 4>()) out[k++] = 104;
@@ -527,6 +615,7 @@ struct SizeImpl {
   }
   static int row_widths(int* out) {
     int k = 0;
+    if constexpr (Blocked<N>::ok) out[k++] = blocked_rows_code<N>();
     if constexpr (tmarow_ok<N, 2, LayPad<N, 2>>()) out[k++] = 502;
     if constexpr (tmarow_ok<N, 4, LayPad<N, 4>>()) out[k++] = 504;
     if constexpr (tmarow_ok<N, 8, LayPad<N, 8>>()) out[k++] = 508;
@@ -818,6 +907,15 @@ struct SizeImpl {
                                 : loss_grad_t<LOSS_AMPLITUDE>(c, eps, partials, grad, scale, stage);
   }
 
+  static cudaError_t block_amplitudes(const float* A, float* At, int npatterns, cudaStream_t st) {
+    if constexpr (Blocked<N>::ok) {
+      k_block_amplitudes<N><<<152 * 8, 256, 0, st>>>(A, At, npatterns);
+      return cudaGetLastError();
+    } else {
+      return cudaSuccess;
+    }
+  }
+
   static const SizeOps* table() {
     static const SizeOps t = {N,
                               N / TileW<N>::rows,
@@ -840,7 +938,11 @@ struct SizeImpl {
                               &SizeImpl<N>::known_power,
                               &SizeImpl<N>::loss_grad,
                               N / DefaultTiles<N>::cols,
-                              &SizeImpl<N>::adam_step};
+                              &SizeImpl<N>::adam_step,
+                              blocked_cols_code<N>(),
+                              blocked_rows_code<N>(),
+                              Blocked<N>::ok ? (size_t)N * Plan<N>::TPT * sizeof(SpBits<N>) : 0,
+                              &SizeImpl<N>::block_amplitudes};
     return &t;
   }
 };
