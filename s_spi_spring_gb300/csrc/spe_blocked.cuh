@@ -423,10 +423,75 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, BlkCfg<N, Blocked<N>::WR, 1>
   for (int e = 0; e < E; ++e) gr[C::step(e)] = make_float2(v[e].x * scale, v[e].y * scale);
 }
 
+// Any op (spe_kernels.cuh) on the blocked scratch: one tile per CTA, W = WR
+// rows or BC columns, elements straight between memory and registers.  Row
+// passes read and write the row-major arrays in runs of 32 / WR pixels.  An
+// op's per-pixel operand comes in the order of k_block_amplitudes.
+template <int N, int AXIS, class Op>
+struct BlkPassCfg : BlkCfg<N, AXIS == AX_ROWS ? Blocked<N>::WR : Blocked<N>::BC, 1> {
+  static constexpr int W = AXIS == AX_ROWS ? Blocked<N>::WR : Blocked<N>::BC;
+  using C = BlkCfg<N, W, 1>;
+  // registers a thread: 64 (a pair of arrays: 80) per 8 elements
+  static constexpr int REGS = C::E <= 8 ? (Op::PAIR ? 80 : 64) : 128;
+  static constexpr int MINB = 65536 / (C::NT * REGS) < 1 ? 1 : 65536 / (C::NT * REGS);
+};
+template <int N, int AXIS, class Op>
+__global__ void __launch_bounds__(BlkPassCfg<N, AXIS, Op>::NT, BlkPassCfg<N, AXIS, Op>::MINB)
+    k_blocked_pass(const Op op, const float2* __restrict__ twg) {
+  using B = Blocked<N>;
+  using C = BlkPassCfg<N, AXIS, Op>;
+  using Lay = typename C::Lay;
+  constexpr int NT = C::NT, E = C::E, W = C::W, TPI = N / W;
+  static_assert(!Op::AMP || (AXIS == AX_COLS && E % 4 == 0), "operands are in column order");
+  extern __shared__ __align__(128) unsigned char sm[];
+  float2* tw = reinterpret_cast<float2*>(sm);
+  float2* xb = reinterpret_cast<float2*>(sm + C::TWB);
+  pdl_enter();
+  load_twiddles<N>(tw, twg, NT);
+  const int t = threadIdx.x;
+  const int c = t % W, j = t / W;
+  const int p = op.first + blockIdx.x / TPI;
+  const int fixed = (blockIdx.x % TPI) * W + c;
+  const int y0 = AXIS == AX_ROWS ? fixed : j, x0 = AXIS == AX_ROWS ? j : fixed;
+  const size_t g0 = (size_t)p * N * N + (size_t)y0 * N + x0, t0 = (size_t)p * N * N + B::at(y0, x0);
+  typename Op::Acc acc;
+  pdl_wait();
+  __syncthreads();
+  float4 a[Op::AMP ? E / 4 : 1];
+  if constexpr (Op::AMP) {
+    const float4* A4 = reinterpret_cast<const float4*>(op.amp(p, N)) + (size_t)((blockIdx.x % TPI) * NT + t) * (E / 4);
+#pragma unroll
+    for (int i = 0; i < E / 4; ++i) a[i] = __ldg(A4 + i);
+  }
+  auto px = [&](int e) {
+    const int d = C::step(e);
+    Px q;
+    q.p = p;
+    q.y = AXIS == AX_ROWS ? y0 : y0 + d;
+    q.x = AXIS == AX_ROWS ? x0 + d : x0;
+    q.gi = g0 + (AXIS == AX_ROWS ? (size_t)d : (size_t)d * N);
+    q.ti = t0 + (AXIS == AX_ROWS ? (size_t)(d / B::BC) * B::XS : (size_t)d * B::YS);
+    q.a = 0.f;
+    if constexpr (Op::AMP) q.a = e % 4 == 0 ? a[e / 4].x : e % 4 == 1 ? a[e / 4].y : e % 4 == 2 ? a[e / 4].z : a[e / 4].w;
+    return q;
+  };
+  pass_elements<N, E, Lay, Op>(op, px, acc, [&](float2* v, auto sign) {
+    fft_x<N, Lay, decltype(sign)::value, 1, 0>(v, xb, tw, c, j);
+  });
+  if constexpr (Op::NSUM + Op::NMAX > 0) {
+    double r[NRED];
+    acc.values(r);
+    block_reduce_store<NT, Op::NSUM, Op::NMAX>(op.partials, r);
+  }
+  if constexpr (Op::PEAK) block_argmax_store<NT>(op.partials, acc.mx, acc.idx);
+}
+
 // amplitudes in the order of the column pass's registers: At[(tile of BC
-// columns) * NT + thread][e]
-template <int N>
-__global__ void k_block_amplitudes(const float* __restrict__ A, float* __restrict__ At, int npatterns) {
+// columns) * NT + thread][e]; with BAND, the correlation ops' weights
+// (band_weight) of the band [minr, maxr] instead
+template <int N, bool BAND>
+__global__ void k_block_amplitudes(const float* __restrict__ A, float* __restrict__ At, int npatterns, float minr,
+                                   float maxr) {
   using C = BlkCfg<N, Blocked<N>::BC, 1>;
   constexpr int W = Blocked<N>::BC, NT = C::NT, E = C::E;
   const size_t total = (size_t)npatterns * N * N;
@@ -434,7 +499,9 @@ __global__ void k_block_amplitudes(const float* __restrict__ A, float* __restric
     const size_t pat = i / ((size_t)N * N);
     const int q = (int)(i % ((size_t)N * N));
     const int e = q % E, t = (q / E) % NT, tile = q / (E * NT);
-    At[i] = A[pat * N * N + (size_t)elem_pos<N>(e, t / W) * N + tile * W + t % W];
+    const int y = elem_pos<N>(e, t / W), x = tile * W + t % W;
+    const float a = A[pat * N * N + (size_t)y * N + x];
+    At[i] = BAND ? band_weight(a, x, y, N, minr, maxr) : a;
   }
 }
 

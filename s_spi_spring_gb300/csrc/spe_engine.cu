@@ -4,6 +4,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -45,34 +46,53 @@ constexpr int NRED = 4;
 // helper kernels
 // ---------------------------------------------------------------------------
 
-// out[i*ostride + oslot] = sum / max over the tpi partials of individual i
-__global__ void k_reduce(const double* __restrict__ part, int count, int tpi, int k, int is_max, double* out,
-                         int ostride, int oslot) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const double* p = part + (size_t)i * tpi * NRED + k;
-  double a = p[0];
-  for (int t = 1; t < tpi; ++t) a = is_max ? fmax(a, p[(size_t)t * NRED]) : a + p[(size_t)t * NRED];
-  out[(size_t)i * ostride + oslot] = a;
-}
-
-// per-individual argmax over the per-CTA (value, index) pairs
-__global__ void k_reduce_peak(const double* __restrict__ part, int count, int tpi, double* out, int ostride,
-                              int oslot) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const double* p = part + (size_t)i * tpi * NRED;
-  double m = p[0], idx = p[1];
-  for (int t = 1; t < tpi; ++t) {
-    const double v = p[(size_t)t * NRED], j = p[(size_t)t * NRED + 1];
-    if (v > m || (v == m && j < idx)) {
-      m = v;
-      idx = j;
+// Reductions over the tpi per-CTA partials of every individual, one block per
+// individual and job: kind 0 the sum of component k, 1 its maximum, 2 the
+// argmax over the (value, index) pairs.  The partials come through shared
+// memory and one thread folds them in tile order (a fixed order, the sums in
+// double); one thread per individual reading them from memory one after the
+// other took 10-18 us a job at 64 individuals of 512^2, and a call has up to
+// eight.
+__global__ void k_reduce(const RedJobs jobs, double* out, int ostride) {
+  const RedJob jb = jobs.job[blockIdx.y];
+  const int i = blockIdx.x;
+  constexpr int CH = 128;
+  __shared__ double a[CH], b[CH];
+  const double* p = jb.part + (size_t)i * jb.tpi * NRED + jb.k;
+  double m = 0.0, idx = 0.0;
+  for (int t0 = 0; t0 < jb.tpi; t0 += CH) {
+    const int nt = min(CH, jb.tpi - t0);
+    if ((int)threadIdx.x < nt) {
+      a[threadIdx.x] = p[(size_t)(t0 + threadIdx.x) * NRED];
+      if (jb.kind == 2) b[threadIdx.x] = p[(size_t)(t0 + threadIdx.x) * NRED + 1];
     }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int t = 0;
+      if (t0 == 0) {
+        m = a[0];
+        idx = b[0];
+        t = 1;
+      }
+      if (jb.kind == 0) {
+        for (; t < nt; ++t) m += a[t];
+      } else if (jb.kind == 1) {
+        for (; t < nt; ++t) m = fmax(m, a[t]);
+      } else {
+        for (; t < nt; ++t)
+          if (a[t] > m || (a[t] == m && b[t] < idx)) {
+            m = a[t];
+            idx = b[t];
+          }
+      }
+    }
+    __syncthreads();
   }
-  if (!(m > 0.0)) idx = 0.0;  // no value above 0: the reference keeps index 0
-  out[(size_t)i * ostride + oslot] = m;
-  out[(size_t)i * ostride + oslot + 1] = idx;
+  if (threadIdx.x == 0) {
+    double* o = out + (size_t)i * ostride + jb.slot;
+    o[0] = m;
+    if (jb.kind == 2) o[1] = m > 0.0 ? idx : 0.0;  // no value above 0: the reference keeps index 0
+  }
 }
 
 // support <- M >= max * thr (cut_support, gpu_context.cu:466-481)
@@ -234,6 +254,7 @@ spe::Ctx make_ctx(spe_engine* e, int first, int count) {
   c.tma = e->tma;
   c.err = e->dev_err;
   c.At = e->At;
+  c.band = e->band;
   c.sp = e->sp;
   c.odd = e->odd;
   return c;
@@ -268,6 +289,8 @@ int pattern_of_range(spe_engine* e, int first, int count, const float** A) {
 
 spe::Ctx item_ctx(spe_engine* e, int count, const float* A) {
   spe::Ctx c = make_ctx(e, 0, count);
+  if (e->At) c.At = e->At + (A - e->A);
+  c.band = e->band + (A - e->A);
   c.A = A;
   c.ipp = 0;
   return c;
@@ -339,17 +362,20 @@ size_t max_tiles(const spe::SizeOps* o) {
 }
 size_t region(spe_engine* e) { return (size_t)e->cap * max_tiles(e->ops) * spe::NRED; }
 
-// tpi: CTAs per individual of the pass that wrote the partials
-int reduce(spe_engine* e, const double* part, int count, int tpi, int k, int is_max, int slot) {
-  spe::k_reduce<<<(count + 127) / 128, 128, 0, e->st>>>(part, count, tpi, k, is_max, e->red, 16, slot);
+int reduce(spe_engine* e, int count, std::initializer_list<spe::RedJob> jobs, double* out, int ostride) {
+  spe::RedJobs j;
+  int k = 0;
+  for (const spe::RedJob& job : jobs) j.job[k++] = job;
+  spe::k_reduce<<<dim3((unsigned)count, (unsigned)k), 128, 0, e->st>>>(j, out, ostride);
   CK(cudaGetLastError(), "reduce launch");
   return SPE_OK;
 }
 
-int reduce_peak(spe_engine* e, const double* part, int count, int slot) {
-  const int tpi = e->ops->tiles_rows;
-  spe::k_reduce_peak<<<(count + 127) / 128, 128, 0, e->st>>>(part, count, tpi, e->red, 16, slot);
-  CK(cudaGetLastError(), "peak reduce launch");
+// band-pass weights of the patterns that slots [first, first+count) use
+int band_weights(spe_engine* e, int first, int count, float minr, float maxr) {
+  const int p0 = e->ipp > 0 ? first / e->ipp : 0, p1 = e->ipp > 0 ? (first + count - 1) / e->ipp : 0;
+  const size_t off = (size_t)p0 * e->npix;
+  CK(e->ops->band_table(e->A + off, e->band + off, e->n, p1 - p0 + 1, minr, maxr, e->st), "band weights");
   return SPE_OK;
 }
 
@@ -409,7 +435,7 @@ int do_shrinkwrap(spe_engine* e, int first, int count, float sigma, bool absolut
   CK(e->ops->blur_magnitude(c, sft), "shrink-wrap kernels");
   const unsigned grid = 152 * 8;
   if (!absolute) {
-    if ((rc = reduce(e, e->partials, count, e->ops->tiles_rows, 0, 1, 0))) return rc;
+    if ((rc = reduce(e, count, {{e->partials, e->ops->tiles_rows, 0, 1, 0}}, e->red, 16))) return rc;
     spe::k_threshold_rel<<<grid, 256, 0, e->st>>>(e->M, e->S, e->red, 16, threshold, e->npix, first, count);
     CK(cudaGetLastError(), "threshold launch");
     return SPE_OK;
@@ -515,6 +541,7 @@ int spe_create(int n, int device, spe_engine** out) {
   ops->fill_tw(tw.data(), n);
   err = cudaMalloc(&e->tw, tw.size() * sizeof(float2));
   if (err == cudaSuccess) err = cudaMalloc(&e->A, e->npix * sizeof(float));
+  if (err == cudaSuccess) err = cudaMalloc(&e->band, e->npix * sizeof(float));
   if (err == cudaSuccess && ops->blocked_cols) err = cudaMalloc(&e->At, e->npix * sizeof(float));
   if (err == cudaSuccess) err = cudaMemcpy(e->tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice);
   if (err == cudaSuccess) err = cudaMalloc(&e->dev_err, sizeof(int));
@@ -527,6 +554,7 @@ int spe_create(int n, int device, spe_engine** out) {
     cudaFree(e->tw);
     cudaFree(e->A);
     cudaFree(e->At);
+    cudaFree(e->band);
     cudaFree(e->dev_err);
     cudaStreamDestroy(e->own);
     delete e;
@@ -543,6 +571,7 @@ int spe_destroy(spe_engine* e) {
   free_population(e);
   cudaFree(e->A);
   cudaFree(e->At);
+  cudaFree(e->band);
   cudaFree(e->tw);
   cudaFree(e->dev_err);
   delete[] static_cast<unsigned char*>(e->tma);
@@ -598,19 +627,20 @@ int spe_set_amplitudes_batch(spe_engine* e, const float* amp, int npatterns, int
   CK(cudaSetDevice(e->dev), "cudaSetDevice");
   if (npatterns > e->a_cap) {
     CK(cudaStreamSynchronize(e->st), "synchronize");
-    float *a = nullptr, *at = nullptr;
-    CK(cudaMalloc(&a, (size_t)npatterns * e->npix * sizeof(float)), "amplitude allocation");
-    if (e->At) {
-      const cudaError_t err = cudaMalloc(&at, (size_t)npatterns * e->npix * sizeof(float));
-      if (err != cudaSuccess) {
-        cudaFree(a);
-        return cuda_fail(err, "amplitude allocation");
-      }
-      cudaFree(e->At);
-      e->At = at;
+    const size_t bytes = (size_t)npatterns * e->npix * sizeof(float);
+    float *a = nullptr, *at = nullptr, *band = nullptr;
+    cudaError_t err = cudaMalloc(&a, bytes);
+    if (err == cudaSuccess) err = cudaMalloc(&band, bytes);
+    if (err == cudaSuccess && e->At) err = cudaMalloc(&at, bytes);
+    if (err != cudaSuccess) {
+      cudaFree(a);
+      cudaFree(band);
+      return cuda_fail(err, "amplitude allocation");
     }
-    cudaFree(e->A);
+    for (float* old : {e->A, e->band, e->At}) cudaFree(old);
     e->A = a;
+    e->band = band;
+    e->At = at;
     e->a_cap = npatterns;
   }
   CK(cudaMemcpyAsync(e->A, amp, (size_t)npatterns * e->npix * sizeof(float), cudaMemcpyHostToDevice, e->st),
@@ -881,22 +911,19 @@ int spe_evaluate(spe_engine* e, int first, int count, float reality, float realp
   const size_t R = region(e);
   double *p1 = e->partials, *p2 = p1 + R, *p3 = p2 + R, *p4 = p3 + R, *p5 = p4 + R;
   CK(e->ops->error_terms(c, gate_er(reality), p1, p2, p3), "error kernels");
-  // red slots: 0 modulesum, 1 err_f, 2 norm_f, 3 max|F|, 4 err_r, 5 norm_r,
-  //            6/7 peak1 (value, index), 8/9 peak2
-  const int tr = e->ops->tiles_rows, tc = e->ops->tiles_cols;
-  if ((rc = reduce(e, p1, count, tr, 0, 0, 0))) return rc;
-  if ((rc = reduce(e, p2, count, tc, 0, 0, 1))) return rc;
-  if ((rc = reduce(e, p2, count, tc, 1, 0, 2))) return rc;
-  if ((rc = reduce(e, p2, count, tc, 2, 1, 3))) return rc;
-  if ((rc = reduce(e, p3, count, tr, 0, 0, 4))) return rc;
-  if ((rc = reduce(e, p3, count, tr, 1, 0, 5))) return rc;
   // get_symmetry (gpu_context.cu:1378-1463): D = FFT+(|rho|) normalised,
-  // peaks of |FFT-(conj(D) D w)|^2 and |FFT-(D D w)|^2, band 0..1
-  CK(e->ops->abs_spectrum(c, e->T2), "symmetry spectrum");
-  CK(e->ops->corr_peak(c, e->T2, e->T2, e->npix, first, -1, 0.f, 1.f, 1, 1, p4), "symmetry correlation");
-  if ((rc = reduce_peak(e, p4, count, 6))) return rc;
-  CK(e->ops->corr_peak(c, e->T2, e->T2, e->npix, first, +1, 0.f, 1.f, 1, 1, p5), "symmetry correlation");
-  if ((rc = reduce_peak(e, p5, count, 8))) return rc;
+  // peaks of |FFT-(conj(D) D w)|^2 (the square of the sum in p4) and of
+  // |FFT-(D D w)|^2, band 0..1
+  if ((rc = band_weights(e, first, count, 0.f, 1.f))) return rc;
+  CK(e->ops->symmetry(c, p4, p5), "symmetry correlation");
+  // red slots: 0 modulesum, 1 err_f, 2 norm_f, 3 max|F|, 4 err_r, 5 norm_r,
+  //            6 root of peak1, 8/9 peak2 (value, index)
+  const int tr = e->ops->tiles_rows, tc = e->ops->tiles_cols;
+  if ((rc = reduce(e, count,
+                   {{p1, tr, 0, 0, 0}, {p2, tc, 0, 0, 1}, {p2, tc, 1, 0, 2}, {p2, tc, 2, 1, 3}, {p3, tr, 0, 0, 4},
+                    {p3, tr, 1, 0, 5}, {p4, tc, 0, 0, 6}, {p5, tr, 0, 2, 8}},
+                   e->red, 16)))
+    return rc;
   if ((rc = fetch_red(e, count))) return rc;
   for (int i = 0; i < count; ++i) {
     const double* r = e->red_host + (size_t)i * 16;
@@ -907,7 +934,9 @@ int spe_evaluate(spe_engine* e, int first, int count, float reality, float realp
     o.error_real = (float)std::pow((double)(er / nr), 0.5);
     o.complexsum = (float)r[3];
     o.modulesum = (float)r[0];
-    o.symmetry = std::sqrt((float)r[8] / (float)r[6]);
+    // (a sum that is not finite makes the whole correlation NaN: no peak)
+    const float s1 = (float)r[6];
+    o.symmetry = std::sqrt((float)r[8] / (std::isfinite(s1) ? s1 * s1 : 0.f));
     // Solver::Evaluate (src/solver.cpp:552-554)
     o.reality = (float)(1. - (double)(o.complexsum / o.modulesum));
     o.error = (float)((double)o.error_fourier * (1. + (double)(realpen * o.reality)));
@@ -986,7 +1015,7 @@ static int loss_args(spe_engine* e, const void* density, const int32_t* support,
 
 // per-item losses from the column-pass partials into loss_out
 static int loss_sums(spe_engine* e, int count, double* loss_out) {
-  int rc = reduce(e, e->partials, count, e->ops->loss_tiles, 0, 0, 0);
+  int rc = reduce(e, count, {{e->partials, e->ops->loss_tiles, 0, 0, 0}}, e->red, 16);
   if (rc) return rc;
   CK(cudaMemcpy2DAsync(loss_out, sizeof(double), e->red, 16 * sizeof(double), sizeof(double), count,
                        cudaMemcpyDeviceToDevice, e->st),
@@ -1129,7 +1158,7 @@ int spe_adam_step(spe_engine* e, void* density, const int32_t* support, void* ex
                        beta1, beta2, (float)(lr / bc1), (float)(1.0 / std::sqrt(bc2)), adam_eps),
      "refinement kernels");
   if (loss_out) {
-    if ((rc = reduce(e, e->partials, count, e->ops->loss_tiles, 0, 0, 0))) return rc;
+    if ((rc = reduce(e, count, {{e->partials, e->ops->loss_tiles, 0, 0, 0}}, e->red, 16))) return rc;
     CK(cudaMemcpy2DAsync(loss_out, sizeof(double), e->red, 16 * sizeof(double), sizeof(double), count,
                          cudaMemcpyDeviceToDevice, e->st),
        "loss copy");

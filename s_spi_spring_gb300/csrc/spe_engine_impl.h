@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <random>
 #include <vector>
 
@@ -51,6 +52,7 @@ struct spe_engine {
   int* dev_err = nullptr;  // device flag of the kernels' bounded waits
   // operands of the blocked-scratch kernels (null at sides without them)
   float* At = nullptr;           // A in register order, as many patterns
+  float* band = nullptr;         // weights of the correlation ops, as many patterns
   void* sp = nullptr;            // packed support, cap * ops->sp_bytes
   unsigned char* odd = nullptr;  // per row tile: support not 0 / 1, cap * n
   cudaStream_t lane2 = nullptr;          // second lane (created on first use)
@@ -77,8 +79,9 @@ int pattern_of_range(spe_engine* e, int first, int count, const float** A);
 spe::Ctx item_ctx(spe_engine* e, int count, const float* A);
 size_t max_tiles(const spe::SizeOps* o);
 size_t region(spe_engine* e);
-int reduce(spe_engine* e, const double* part, int count, int tpi, int k, int is_max, int slot);
-int reduce_peak(spe_engine* e, const double* part, int count, int slot);
+// k_reduce over `count` individuals: results of individual i at out[i * ostride + slot]
+int reduce(spe_engine* e, int count, std::initializer_list<spe::RedJob> jobs, double* out, int ostride);
+int band_weights(spe_engine* e, int first, int count, float minr, float maxr);
 int fetch_red(spe_engine* e, int count);
 int ensure_lanes(spe_engine* e);
 int have_patterns(spe_engine* e, int first, int count);

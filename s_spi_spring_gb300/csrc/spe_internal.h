@@ -66,6 +66,7 @@ struct Ctx {
   // operands of the blocked-scratch kernels (spe_blocked.cuh), or null: the
   // amplitudes in register order, the packed support and its per-row-tile flags
   const float* At;
+  const float* band;  // weights of the correlation ops (SizeOps::band_table)
   void* sp;
   unsigned char* odd;
 };
@@ -80,6 +81,16 @@ size_t row_maps_bytes();
 // its wait gives up
 cudaError_t launch_wait_selftest(int* err, cudaStream_t st);
 bool build_row_maps(void* out, int n, int cap, const float2* T, const float2* rho, const int* S);
+
+// One reduction over per-CTA partials (k_reduce): component k of every tile's
+// partial, kind 0 sum, 1 maximum, 2 argmax of (value, index)
+struct RedJob {
+  const double* part;
+  int tpi, k, kind, slot;
+};
+struct RedJobs {
+  RedJob job[8];
+};
 
 // Phase gate (see phase_out in spe_kernels.cuh): float thresholds of
 // arg > hi / arg < -lo and the cos / sin of each threshold.
@@ -104,23 +115,27 @@ struct SizeOps {
   // error terms: stage 1 -> partials (modulesum), stage 2 -> partials+P1
   // (err, norm, max), stage 3 -> partials+P2 (err_r, norm_r)
   cudaError_t (*error_terms)(const Ctx&, Gate g, double* p1, double* p2, double* p3);
-  // |rho| -> D = FFT+(|rho|) into dst (2D)
-  cudaError_t (*abs_spectrum)(const Ctx&, float2* dst);
-  // cross-correlation peak of D (per individual) against Dref:
-  // sign -1: conj(D) Dref, +1: D Dref; peaks into partials (value, index)
-  cudaError_t (*corr_peak)(const Ctx&, const float2* D, const float2* Dref, size_t ref_stride, int ref_first,
-                           int sign, float minr, float maxr, int norm_d, int norm_ref, double* partials);
+  // the two peaks of the symmetry metric (get_symmetry), through Ctx::T with
+  // the weights Ctx::band: column-pass partials (the sum whose square is the
+  // first peak) and row-pass partials (value, index of the second)
+  cudaError_t (*symmetry)(const Ctx&, double* psum, double* ppeak);
   // generic transforms over Ctx::count items starting at the given arrays
   // in-place 2D transform; sign +1: FFT+ unnormalised, -1: FFT- then /N^2
   cudaError_t (*fft2)(const Ctx&, float2* data, int sign);
   // M = |FFT+(src)| (tmp: scratch items)
   cudaError_t (*ft_magnitude)(const Ctx&, const float2* src, float2* tmp, float* M);
-  // dst = FFT+(|src|)
-  cudaError_t (*abs_spectrum_items)(const Ctx&, const float2* src, float2* dst);
+  // dst = FFT+(|src|) (in the passes' own order), the complex sums of src in
+  // row-pass partials
+  cudaError_t (*abs_spectrum_items)(const Ctx&, const float2* src, float2* dst, double* psum);
   // peaks (value, index) of |FFT-(cross power of D[xi[p]], Dref[ri[p]])|^2
-  cudaError_t (*corr_peak_idx)(const Ctx&, const float2* D, const float2* Dref, const int* xi, const int* ri,
-                               int sign, float minr, float maxr, int norm_d, int norm_ref, float2* scratch,
-                               double* partials);
+  // with the weights Ctx::band: conj(D) Dref in part1, D Dref in part2.  D and
+  // Dref come from abs_spectrum_items; scratch1, scratch2: count items each
+  cudaError_t (*corr_peaks)(const Ctx&, const float2* D, const float2* Dref, const int* xi, const int* ri,
+                            int norm_d, int norm_ref, float2* scratch1, float2* scratch2, double* part1,
+                            double* part2);
+  // band-pass weights of the correlation ops for `npatterns` patterns
+  cudaError_t (*band_table)(const float* A, float* band, int n, int npatterns, float minr, float maxr,
+                            cudaStream_t st);
   // tile widths compiled for this size
   int (*col_widths)(int* out);
   int (*row_widths)(int* out);

@@ -52,7 +52,10 @@ __device__ __forceinline__ bool phase_out(float2 v, const GateK& g) {
   const float band = 4e-6f * (fabsf(v.x) + ay);
   if (D > band) return true;
   if (D < -band) return false;
-  const float ph = atan2f(v.y, v.x);
+  // zeros (most of a density outside its object) without the arc tangent's
+  // slow path: arg = +-0 for x = +0, +-pi for x = -0
+  const float ph = v.x == 0.f && ay == 0.f ? copysignf(signbit(v.x) ? 3.14159265358979f : 0.f, v.y)
+                                           : atan2f(v.y, v.x);
   return (ph > g.hi) || (ph < -g.lo);
 }
 
@@ -83,7 +86,13 @@ __device__ __forceinline__ float2 project(float2 F, float a) {
   return F;
 }
 
-__device__ __forceinline__ float cabsf2(float2 v) { return sqrtf(v.y * v.y + v.x * v.x); }
+// (sqrtf takes its slow path for an argument of 0, which most pixels outside
+// an object are)
+__device__ __forceinline__ float cabsf2(float2 v) {
+  const float m2 = v.y * v.y + v.x * v.x;
+  const float m = sqrtf(m2 == 0.f ? 1.f : m2);
+  return m2 == 0.f ? 0.f : m;
+}
 
 // ---------------------------------------------------------------------------
 // block reduction of NRED values per CTA into partials[blockIdx.x*NRED + k]
@@ -157,6 +166,17 @@ __device__ __forceinline__ void block_argmax_store(double* __restrict__ partials
   }
 }
 
+// Programmatic dependent launch: a kernel launched with the programmatic
+// stream serialisation attribute may start while the previous kernel of the
+// stream drains.  It lets its own dependents start early, loads what no
+// kernel writes (the twiddle tables), then waits until the previous grid has
+// completed and its writes are visible before touching the population.
+// Without the attribute both instructions are no-ops.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // the pass kernel
 //
@@ -183,6 +203,47 @@ struct PassCfg {
   static constexpr int MINB = MINB_RAW < 1 ? 1 : (MINB_RAW > 4 ? 4 : MINB_RAW);
 };
 
+// A pixel as an op sees it: gi, its offset in the row-major arrays (density,
+// support, magnitudes); ti, its offset in the scratch arrays that only
+// passes touch (equal to gi, or in the blocked order of spe_blocked.cuh); a,
+// the per-pixel operand of an op with AMP (amplitude, or band weight),
+// which the pass loads.
+struct Px {
+  size_t gi, ti;
+  float a;
+  int p, y, x;
+};
+
+// An op over a thread's E elements held in registers: load, transform,
+// pointwise step, transform, store.  px(e): the pixel of element e; fft(v,
+// sign): the transform of the CTA's sequences (std::integral_constant sign).
+template <int N, int E, class Lay, class Op, class PxF, class Fft>
+__device__ __forceinline__ void pass_elements(const Op& op, const PxF& px, typename Op::Acc& acc, const Fft& fft) {
+  float2 v[E];
+  if constexpr (Op::PAIR) {
+    float2 u[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) op.load_pair(px(e), v[e], u[e]);
+    fft(v, std::integral_constant<int, Op::FFT1>());
+#pragma unroll
+    for (int e = 0; e < E; ++e) op.store_pair(v[e], px(e), 0);
+    fft(u, std::integral_constant<int, Op::FFT1>());
+#pragma unroll
+    for (int e = 0; e < E; ++e) op.store_pair(u[e], px(e), 1);
+  } else {
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = op.load(px(e), acc);
+    if constexpr (Op::FFT1 != 0) fft(v, std::integral_constant<int, Op::FFT1>());
+    if constexpr (Op::FFT2 != 0) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) v[e] = op.mid(v[e], px(e), acc);
+      fft(v, std::integral_constant<int, Op::FFT2>());
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) op.store(v[e], px(e), acc);
+  }
+}
+
 template <int N, int AXIS, class Op>
 __global__ void __launch_bounds__(PassCfg<N, AXIS>::NT, PassCfg<N, AXIS>::MINB)
     pass_kernel(const Op op, const float2* __restrict__ twg) {
@@ -192,6 +253,7 @@ __global__ void __launch_bounds__(PassCfg<N, AXIS>::NT, PassCfg<N, AXIS>::MINB)
   float2* tw = smem;
   float2* buf = smem + C::TWN;
   constexpr int TWS = TwiddleTable<N>::size();
+  pdl_enter();
   for (int i = threadIdx.x; i < TWS; i += NT) tw[i] = twg[i];
 
   const int t = threadIdx.x;
@@ -202,33 +264,20 @@ __global__ void __launch_bounds__(PassCfg<N, AXIS>::NT, PassCfg<N, AXIS>::MINB)
   const int fixed = (blockIdx.x % TPI) * W + c;  // row (row pass) or column (column pass)
   const size_t base = (size_t)p * N * N;
   typename Op::Acc acc;
-
-  float2 v[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
+  pdl_wait();
+  auto px = [&](int e) {
     const int l = elem_pos<N>(e, j);
-    const int y = (AXIS == AX_ROWS) ? fixed : l;
-    const int x = (AXIS == AX_ROWS) ? l : fixed;
-    v[e] = op.load(base + (size_t)y * N + x, p, y, x, acc);
-  }
-  if constexpr (Op::FFT1 != 0) fft_reg<N, typename C::Lay, Op::FFT1>(v, buf, tw, c, j);
-  if constexpr (Op::FFT2 != 0) {
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int l = elem_pos<N>(e, j);
-      const int y = (AXIS == AX_ROWS) ? fixed : l;
-      const int x = (AXIS == AX_ROWS) ? l : fixed;
-      v[e] = op.mid(v[e], base + (size_t)y * N + x, p, y, x, acc);
-    }
-    fft_reg<N, typename C::Lay, Op::FFT2>(v, buf, tw, c, j);
-  }
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int l = elem_pos<N>(e, j);
-    const int y = (AXIS == AX_ROWS) ? fixed : l;
-    const int x = (AXIS == AX_ROWS) ? l : fixed;
-    op.store(v[e], base + (size_t)y * N + x, p, y, x, acc);
-  }
+    Px q;
+    q.p = p;
+    q.y = (AXIS == AX_ROWS) ? fixed : l;
+    q.x = (AXIS == AX_ROWS) ? l : fixed;
+    q.gi = q.ti = base + (size_t)q.y * N + q.x;
+    q.a = Op::AMP ? __ldg(op.amp(p, N) + (size_t)q.y * N + q.x) : 0.f;
+    return q;
+  };
+  pass_elements<N, E, typename C::Lay, Op>(op, px, acc, [&](float2* v, auto sign) {
+    fft_reg<N, typename C::Lay, decltype(sign)::value>(v, buf, tw, c, j);
+  });
   if constexpr (Op::NSUM + Op::NMAX > 0) {
     double r[NRED];
     acc.values(r);
@@ -249,64 +298,76 @@ struct NoAcc {
 // ---------------------------------------------------------------------------
 struct OpBase {
   static constexpr int NSUM = 0, NMAX = 0, PEAK = 0;
+  static constexpr bool AMP = false;   // reads amp(): A, one n x n array per pattern
+  static constexpr bool PAIR = false;  // two arrays through the pass (load_pair, store_pair)
   int first = 0;
   double* partials = nullptr;
+  const float* A = nullptr;
   // individuals per pattern when the engine holds several patterns (slot p
   // uses pattern p / ipp); 0: one pattern shared by all
   int ipp = 0;
-  __device__ __forceinline__ const float* amp(const float* A, int p, int n) const {
+  __device__ __forceinline__ const float* amp(int p, int n) const {
     return ipp > 0 ? A + (size_t)(p / ipp) * n * n : A;
+  }
+};
+// most ops keep the value between two transforms
+struct OpKeep : OpBase {
+  template <class Acc>
+  __device__ float2 mid(float2 v, const Px&, Acc&) const {
+    return v;
   }
 };
 
 // Source transforms of the first row pass: rho itself, rho gated by the
-// support (apply_support_er on a copy), or its modulus.
-enum { SRC_RHO = 0, SRC_GATED = 1, SRC_ABS = 2 };
+// support (apply_support_er on a copy), its modulus, or its modulus with the
+// complex sum of rho in the partials.
+enum { SRC_RHO = 0, SRC_GATED = 1, SRC_ABS = 2, SRC_ABS_SUM = 3 };
 
 // row pass: load rho (optionally gated / modulus) -> FFT+ (x) -> T.
 // SRC_GATED accumulates sum |rho_s| (get_module_sum, gpu_context.cu:219-246).
 template <int SRC>
-struct OpRowsForward : OpBase {
+struct OpRowsForward : OpKeep {
   static constexpr int FFT1 = +1, FFT2 = 0;
-  static constexpr int NSUM = (SRC == SRC_GATED) ? 1 : 0, NMAX = 0;
+  static constexpr int NSUM = SRC == SRC_GATED ? 1 : (SRC == SRC_ABS_SUM ? 2 : 0), NMAX = 0;
   const float2* rho;
   const int* S;
   float2* T;
   GateK g;
   struct Acc {
-    float s = 0.f;
+    float s = 0.f, t = 0.f;
     __device__ void values(double (&v)[NRED]) const {
       v[0] = s;
-      v[1] = v[2] = v[3] = 0.0;
+      v[1] = t;
+      v[2] = v[3] = 0.0;
     }
   };
-  __device__ float2 load(size_t gi, int, int, int, Acc& a) const {
-    float2 v = rho[gi];
+  __device__ float2 load(const Px& q, Acc& acc) const {
+    float2 v = rho[q.gi];
     if (SRC == SRC_GATED) {
-      const float t = phase_out(v, g) ? 0.f : (float)S[gi];
+      const float t = phase_out(v, g) ? 0.f : (float)S[q.gi];
       v = make_float2(v.x * t, v.y * t);
-      a.s += cabsf2(v);
-    } else if (SRC == SRC_ABS) {
+      acc.s += cabsf2(v);
+    } else if (SRC == SRC_ABS || SRC == SRC_ABS_SUM) {
+      if (SRC == SRC_ABS_SUM) {
+        acc.s += v.x;
+        acc.t += v.y;
+      }
       v = make_float2(cabsf2(v), 0.f);
     }
     return v;
   }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { T[gi] = v; }
+  __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
 // column pass: T -> FFT+ (y) -> P_M -> FFT- (y) -> T
 struct OpColsProject : OpBase {
-  static constexpr int FFT1 = +1, FFT2 = -1, NSUM = 0, NMAX = 0;
+  static constexpr int FFT1 = +1, FFT2 = -1;
+  static constexpr bool AMP = true;
   float2* T;
-  const float* A;
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  int n;
-  __device__ float2 mid(float2 v, size_t, int p, int y, int x, Acc&) const {
-    return project(v, __ldg(amp(A, p, n) + (size_t)y * n + x));
-  }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { T[gi] = v; }
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ float2 mid(float2 v, const Px& q, Acc&) const { return project(v, q.a); }
+  __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
 // Support updates (reference apply_support_{hio,raar,er},
@@ -337,36 +398,35 @@ __device__ __forceinline__ float2 update(float2 rp, float2 prev, int s, float be
 // row pass of an iteration: T -> FFT- (x) -> /N^2 -> update -> rho -> FFT+ (x) -> T
 template <int UPD>
 struct OpRowsIterate : OpBase {
-  static constexpr int FFT1 = -1, FFT2 = +1, NSUM = 0, NMAX = 0;
+  static constexpr int FFT1 = -1, FFT2 = +1;
   float2* T;
   float2* rho;
   const int* S;
   float scale, beta;
   GateK g;
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t gi, int, int, int, Acc&) const {
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ float2 mid(float2 v, const Px& q, Acc&) const {
     const float2 rp = make_float2(v.x * scale, v.y * scale);
-    const float2 prev = (UPD == UPD_ER) ? make_float2(0.f, 0.f) : rho[gi];
-    const float2 r = update<UPD>(rp, prev, S[gi], beta, g);
-    rho[gi] = r;
+    const float2 prev = (UPD == UPD_ER) ? make_float2(0.f, 0.f) : rho[q.gi];
+    const float2 r = update<UPD>(rp, prev, S[q.gi], beta, g);
+    rho[q.gi] = r;
     return r;
   }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { T[gi] = v; }
+  __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
 // last row pass of a call: T -> FFT- (x) -> /N^2 -> rho (the trailing
 // modulus projection of GPU_context::HIO/RAAR/ER, gpu_context.cu:803-812)
-struct OpRowsFinal : OpBase {
-  static constexpr int FFT1 = -1, FFT2 = 0, NSUM = 0, NMAX = 0;
+struct OpRowsFinal : OpKeep {
+  static constexpr int FFT1 = -1, FFT2 = 0;
   float2* T;
   float2* out;
   float scale;
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const {
-    out[gi] = make_float2(v.x * scale, v.y * scale);
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ void store(float2 v, const Px& q, Acc&) const {
+    out[q.gi] = make_float2(v.x * scale, v.y * scale);
   }
 };
 
@@ -374,38 +434,38 @@ struct OpRowsFinal : OpBase {
 
 // row pass: T -> FFT- (x) -> |./N^2| (get_module) -> FFT+ (x) -> T
 struct OpRowsModulusForward : OpBase {
-  static constexpr int FFT1 = -1, FFT2 = +1, NSUM = 0, NMAX = 0;
+  static constexpr int FFT1 = -1, FFT2 = +1;
   float2* T;
   float scale;
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const {
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ float2 mid(float2 v, const Px&, Acc&) const {
     return make_float2(cabsf2(make_float2(v.x * scale, v.y * scale)), 0.f);
   }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { T[gi] = v; }
+  __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
 // column pass: T -> FFT+ (y) -> * exp(-r^2/sigma_ft^2) (smooth_intensities,
 // r measured from the corner origin) -> FFT- (y) -> T
 struct OpColsBlur : OpBase {
-  static constexpr int FFT1 = +1, FFT2 = -1, NSUM = 0, NMAX = 0;
+  static constexpr int FFT1 = +1, FFT2 = -1;
   float2* T;
   int n;
   float sig2;  // sigma_ft^2
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int y, int x, Acc&) const {
-    const int xx = (x >= n / 2) ? x - n : x;
-    const int yy = (y >= n / 2) ? y - n : y;
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ float2 mid(float2 v, const Px& q, Acc&) const {
+    const int xx = (q.x >= n / 2) ? q.x - n : q.x;
+    const int yy = (q.y >= n / 2) ? q.y - n : q.y;
     const float r2 = (float)(xx * xx + yy * yy);
     const float k = expf(-__fdiv_rn(r2, sig2));
     return make_float2(v.x * k, v.y * k);
   }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { T[gi] = v; }
+  __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
 // row pass: T -> FFT- (x) -> M = |.| (float), per-CTA max (get_max_module)
-struct OpRowsMagnitude : OpBase {
+struct OpRowsMagnitude : OpKeep {
   static constexpr int FFT1 = -1, FFT2 = 0, NSUM = 0, NMAX = 1;
   const float2* T;
   float* M;
@@ -416,12 +476,11 @@ struct OpRowsMagnitude : OpBase {
       v[1] = v[2] = v[3] = 0.0;
     }
   };
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc& a) const {
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ void store(float2 v, const Px& q, Acc& acc) const {
     const float m = cabsf2(v);
-    M[gi] = m;
-    a.mx = fmaxf(a.mx, m);
+    M[q.gi] = m;
+    acc.mx = fmaxf(acc.mx, m);
   }
 };
 
@@ -432,9 +491,8 @@ struct OpRowsMagnitude : OpBase {
 // (get_error_gpu, get_max_module); then P_M -> FFT- (y) -> T
 struct OpColsError : OpBase {
   static constexpr int FFT1 = +1, FFT2 = -1, NSUM = 2, NMAX = 1;
+  static constexpr bool AMP = true;
   float2* T;
-  const float* A;
-  int n;
   struct Acc {
     float e = 0.f, a2 = 0.f, mx = 0.f;
     __device__ void values(double (&v)[NRED]) const {
@@ -444,28 +502,26 @@ struct OpColsError : OpBase {
       v[3] = 0.0;
     }
   };
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int p, int y, int x, Acc& acc) const {
-    const float a = __ldg(amp(A, p, n) + (size_t)y * n + x);
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ float2 mid(float2 v, const Px& q, Acc& acc) const {
     const float m = cabsf2(v);
     acc.mx = fmaxf(acc.mx, m);
-    if (a >= 0.f) {
-      acc.a2 += a * a;
-      acc.e += (a - m) * (a - m);
+    if (q.a >= 0.f) {
+      acc.a2 += q.a * q.a;
+      acc.e += (q.a - m) * (q.a - m);
     }
-    return project(v, a);
+    return project(v, q.a);
   }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { T[gi] = v; }
+  __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
 // row pass: T -> FFT- (x) -> /N^2 -> real-space error terms of
 // get_real_error_gpu (gpu_context.cu:386-434), including its x*xs term
-struct OpRowsRealError : OpBase {
+struct OpRowsRealError : OpKeep {
   static constexpr int FFT1 = -1, FFT2 = 0, NSUM = 2, NMAX = 0;
   const float2* T;
   const int* S;
   float scale;
-  GateK g;
   struct Acc {
     float err = 0.f, nrm = 0.f;
     __device__ void values(double (&v)[NRED]) const {
@@ -474,30 +530,20 @@ struct OpRowsRealError : OpBase {
       v[2] = v[3] = 0.0;
     }
   };
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc& a) const {
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ void store(float2 v, const Px& q, Acc& acc) const {
     const float2 r = make_float2(v.x * scale, v.y * scale);
-    const int s = S[gi];
-    const float t = phase_out(r, g) ? 0.f : (float)s;
-    const float xs = r.x * t, ys = r.y * t;
-    a.nrm += r.y * r.y + r.x * r.x;
-    if (s == 0) a.err += (r.y - ys) * (r.y - ys) + (r.x * xs) * (r.x * xs);
+    const int s = S[q.gi];
+    acc.nrm += r.y * r.y + r.x * r.x;
+    // (the gated support counts where it is 0, gate or not)
+    if (s == 0) {
+      const float xs = r.x * 0.f, ys = r.y * 0.f;
+      acc.err += (r.y - ys) * (r.y - ys) + (r.x * xs) * (r.x * xs);
+    }
   }
 };
 
 // ---- cross-correlations (get_symmetry / get_shift, gpu_context.cu:1157-1463)
-
-// column pass: T -> FFT+ (y) -> T (finishes D = FFT(|rho|))
-struct OpColsForward : OpBase {
-  static constexpr int FFT1 = +1, FFT2 = 0, NSUM = 0, NMAX = 0;
-  const float2* src;
-  float2* dst;
-  using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return src[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { dst[gi] = v; }
-};
 
 // Band-pass weight of multiply() (gpu_context.cu:1157-1200), squared.
 __device__ __forceinline__ float bandpass2(int x, int y, int n, float minr, float maxr) {
@@ -516,55 +562,77 @@ __device__ __forceinline__ float bandpass2(int x, int y, int n, float minr, floa
   return coeff * coeff;
 }
 
+// The operand of the correlation ops: the weight above, or -1 where A < 0
+// (those pixels are left out).  One table per pattern and call: evaluated per
+// pixel of every individual, the two exponentials and four divisions made the
+// cross-power pass 2.4 times as long as its transform (154 against 65 us at
+// 512^2 x 64).
+__device__ __forceinline__ float band_weight(float a, int x, int y, int n, float minr, float maxr) {
+  return a < 0.f ? -1.f : bandpass2(x, y, n, minr, maxr);
+}
+__device__ __forceinline__ float2 weighted(float2 c, float w) {
+  return w < 0.f ? make_float2(0.f, 0.f) : make_float2(c.x * w, c.y * w);
+}
+
 // normalize_ft_shift with exponent 1 (gpu_context.cu:37-50): identity, NaN
-// where |D| == 0.
+// where |D| == 0 (the float root of a sum of squares is 0 only where the sum is).
 __device__ __forceinline__ float2 ft_shift_norm(float2 d) {
-  const float m = cabsf2(d);
-  if (m == 0.f) {
+  if (d.y * d.y + d.x * d.x == 0.f) {
     const float q = __int_as_float(0x7fffffff);
     return make_float2(q, q);
   }
   return d;
 }
 
-// column pass: form the band-passed cross-power spectrum of D (individual
-// spectrum) with Dref (reference spectrum, one per individual or shared),
-// conj(D) Dref (SIGN=-1) or D Dref (SIGN=+1), masked where A < 0; then
-// FFT- (y) -> dst.
-template <int SIGN>
-struct OpColsCrossPower : OpBase {
-  static constexpr int FFT1 = -1, FFT2 = 0, NSUM = 0, NMAX = 0;
-  const float2* D;
-  const float2* Dref;
-  size_t ref_stride;  // elements between references of consecutive individuals (0: shared)
-  int ref_first;
-  float2* dst;
-  const float* A;
-  int n;
-  float minr, maxr;
-  int norm_d, norm_ref;  // apply normalize_ft_shift
-  using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int p, int y, int x, Acc&) const {
-    float2 d = D[gi];
-    const size_t pix = (size_t)y * n + x;
-    float2 r = Dref[(size_t)(p - first + ref_first) * ref_stride + pix];
-    if (norm_d) d = ft_shift_norm(d);
-    if (norm_ref) r = ft_shift_norm(r);
-    const float sd = (float)SIGN * d.y;
-    float2 c = make_float2(d.x * r.x - sd * r.y, d.x * r.y + sd * r.x);
-    const float w = bandpass2(x, y, n, minr, maxr);
-    c = make_float2(c.x * w, c.y * w);
-    if (__ldg(amp(A, p, n) + pix) < 0.f) c = make_float2(0.f, 0.f);
-    return c;
+// band[pattern][y][x] = band_weight of A, row-major
+static __global__ void k_band_table(const float* __restrict__ A, float* __restrict__ band, int n, size_t total,
+                                    float minr, float maxr) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const int pix = (int)(i % ((size_t)n * n));
+    band[i] = band_weight(A[i], pix % n, pix / n, n, minr, maxr);
   }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { dst[gi] = v; }
+}
+static cudaError_t launch_band_table(const float* A, float* band, int n, int npatterns, float minr, float maxr,
+                                     cudaStream_t st) {
+  k_band_table<<<152 * 8, 256, 0, st>>>(A, band, n, (size_t)npatterns * n * n, minr, maxr);
+  return cudaGetLastError();
+}
+
+// conj(d) r (SIGN = -1) or d r (SIGN = +1)
+template <int SIGN>
+__device__ __forceinline__ float2 cross_power(float2 d, float2 r) {
+  const float sd = (float)SIGN * d.y;
+  return make_float2(d.x * r.x - sd * r.y, d.x * r.y + sd * r.x);
+}
+
+// column pass of the symmetry metric: T = FFT(|rho|) along x -> FFT+ (y) = D
+// -> D D w -> FFT- (y) -> T, and the sum of |D|^2 w in the partials.  The
+// peak of |FFT-(conj(D) D w)|^2 needs no transform: its input is real and not
+// negative, so the largest value is the one at the origin, the squared sum.
+struct OpColsSymmetry : OpBase {
+  static constexpr int FFT1 = +1, FFT2 = -1, NSUM = 1;
+  static constexpr bool AMP = true;
+  float2* T;
+  struct Acc {
+    float s = 0.f;
+    __device__ void values(double (&v)[NRED]) const {
+      v[0] = s;
+      v[1] = v[2] = v[3] = 0.0;
+    }
+  };
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ float2 mid(float2 v, const Px& q, Acc& acc) const {
+    const float2 d = ft_shift_norm(v);
+    acc.s += weighted(make_float2(d.y * d.y + d.x * d.x, 0.f), q.a).x;
+    return weighted(cross_power<+1>(d, d), q.a);
+  }
+  __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
 // row pass: T -> FFT- (x) -> |.|^2; per-CTA max and the raster index of its
 // first occurrence (encoded as a double-precision pair: value, index)
-struct OpRowsPeak : OpBase {
-  static constexpr int FFT1 = -1, FFT2 = 0, NSUM = 0, NMAX = 0, PEAK = 1;
+struct OpRowsPeak : OpKeep {
+  static constexpr int FFT1 = -1, FFT2 = 0, PEAK = 1;
   const float2* T;
   int n;
   struct Acc {
@@ -574,11 +642,10 @@ struct OpRowsPeak : OpBase {
       v[0] = v[1] = v[2] = v[3] = 0.0;
     }
   };
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t, int, int y, int x, Acc& a) const {
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ void store(float2 v, const Px& q, Acc& a) const {
     const float val = v.x * v.x + v.y * v.y;
-    const int i = y * n + x;
+    const int i = q.y * n + q.x;
     // strict '>' in raster order keeps the first maximum; NaN never wins
     if (val > a.mx || (val == a.mx && val > 0.f && i < a.idx)) {
       a.mx = val;
@@ -590,11 +657,10 @@ struct OpRowsPeak : OpBase {
 // column pass on the row-transformed starting density: FFT+ (y) gives F;
 // sum over known pixels of |F|^2 and of A^2 (Initialize_rec's scaling,
 // src/solver.cpp:938-947); nothing is stored
-struct OpColsKnownPower : OpBase {
+struct OpColsKnownPower : OpKeep {
   static constexpr int FFT1 = +1, FFT2 = 0, NSUM = 2, NMAX = 0;
+  static constexpr bool AMP = true;
   const float2* T;
-  const float* A;
-  int n;
   struct Acc {
     float f2 = 0.f, a2 = 0.f;
     __device__ void values(double (&v)[NRED]) const {
@@ -603,13 +669,11 @@ struct OpColsKnownPower : OpBase {
       v[2] = v[3] = 0.0;
     }
   };
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t, int p, int y, int x, Acc& acc) const {
-    const float a = __ldg(amp(A, p, n) + (size_t)y * n + x);
-    if (a >= 0.f) {
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ void store(float2 v, const Px& q, Acc& acc) const {
+    if (q.a >= 0.f) {
       acc.f2 += v.x * v.x + v.y * v.y;
-      acc.a2 += a * a;
+      acc.a2 += q.a * q.a;
     }
   }
 };
@@ -624,40 +688,42 @@ struct OpColsKnownPower : OpBase {
 // adjoint of FFT+; no normalisation).
 enum { LOSS_AMPLITUDE = 0, LOSS_POISSON = 1 };
 
+// (roundings spelled out, so that every kernel's loss terms have the same bits;
+// add them with loss_add)
 template <int LOSS>
 __device__ __forceinline__ float loss_term(float2 F, float a, float eps, float2* g) {
-  const float m2 = F.x * F.x + F.y * F.y;
+  const float m2 = fmaf(F.x, F.x, __fmul_rn(F.y, F.y));
   if (LOSS == LOSS_AMPLITUDE) {
     const float m = sqrtf(m2);
     const float d = m - a;
     const float f = m > 0.f ? 2.f * d / m : 0.f;
     if (g) *g = make_float2(f * F.x, f * F.y);
-    return d * d;
+    return __fmul_rn(d, d);
   } else {
     // the hardware logarithm and reciprocal (a few ulp) instead of the
     // IEEE-rounded logf and division: the loss and the gradient stay within
     // the errors stated against the FP64 oracle, at a third of the
     // instructions of this term
-    const float i = a * a;
-    const float den = m2 + eps;
+    const float i = __fmul_rn(a, a);
+    const float den = __fadd_rn(m2, eps);
     const float f = 2.f * (1.f - __fdividef(i, den));
     if (g) *g = make_float2(f * F.x, f * F.y);
-    return m2 - i * __logf(den);
+    return fmaf(-i, __logf(den), m2);
   }
 }
+__device__ __forceinline__ void loss_add(float& sum, float term) { sum = __fadd_rn(sum, term); }
 
 // row pass: S rho -> FFT+ (x) -> T
-struct OpRowsSupportForward : OpBase {
-  static constexpr int FFT1 = +1, FFT2 = 0, NSUM = 0, NMAX = 0;
+struct OpRowsSupportForward : OpKeep {
+  static constexpr int FFT1 = +1, FFT2 = 0;
   const float2* rho;
   const int* S;
   float2* T;
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const {
-    return S[gi] > 0 ? rho[gi] : make_float2(0.f, 0.f);
+  __device__ float2 load(const Px& q, Acc&) const {
+    return S[q.gi] > 0 ? rho[q.gi] : make_float2(0.f, 0.f);
   }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { T[gi] = v; }
+  __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
 // column pass: T -> FFT+ (y) = F -> loss terms; with GRAD, -> 2 dL/dconj(F)
@@ -665,9 +731,8 @@ struct OpRowsSupportForward : OpBase {
 template <int LOSS, bool GRAD>
 struct OpColsLoss : OpBase {
   static constexpr int FFT1 = +1, FFT2 = GRAD ? -1 : 0, NSUM = 1, NMAX = 0;
+  static constexpr bool AMP = true;
   float2* T;
-  const float* A;
-  int n;
   float eps;
   struct Acc {
     float l = 0.f;
@@ -676,36 +741,33 @@ struct OpColsLoss : OpBase {
       v[1] = v[2] = v[3] = 0.0;
     }
   };
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int p, int y, int x, Acc& acc) const {
-    const float a = __ldg(amp(A, p, n) + (size_t)y * n + x);
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ float2 mid(float2 v, const Px& q, Acc& acc) const {
     float2 g = make_float2(0.f, 0.f);
-    if (a >= 0.f) acc.l += loss_term<LOSS>(v, a, eps, &g);
+    if (q.a >= 0.f) loss_add(acc.l, loss_term<LOSS>(v, q.a, eps, &g));
     return g;
   }
-  __device__ void store(float2 v, size_t gi, int p, int y, int x, Acc& acc) const {
+  __device__ void store(float2 v, const Px& q, Acc& acc) const {
     if (GRAD) {
-      T[gi] = v;
-    } else {
-      const float a = __ldg(amp(A, p, n) + (size_t)y * n + x);
-      if (a >= 0.f) acc.l += loss_term<LOSS>(v, a, eps, nullptr);
+      T[q.ti] = v;
+    } else if (q.a >= 0.f) {
+      loss_add(acc.l, loss_term<LOSS>(v, q.a, eps, nullptr));
     }
   }
 };
 
 // row pass: T -> FFT- (x) -> G = scale[p] * S * (.)
-struct OpRowsGradOut : OpBase {
-  static constexpr int FFT1 = -1, FFT2 = 0, NSUM = 0, NMAX = 0;
+struct OpRowsGradOut : OpKeep {
+  static constexpr int FFT1 = -1, FFT2 = 0;
   const float2* T;
   const int* S;
   float2* G;
   const float* scale;  // per item (upstream gradient), or null for 1
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int p, int, int, Acc&) const {
-    const float f = S[gi] > 0 ? (scale ? scale[p - first] : 1.f) : 0.f;
-    G[gi] = make_float2(v.x * f, v.y * f);
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ void store(float2 v, const Px& q, Acc&) const {
+    const float f = S[q.gi] > 0 ? (scale ? scale[q.p - first] : 1.f) : 0.f;
+    G[q.gi] = make_float2(v.x * f, v.y * f);
   }
 };
 
@@ -732,8 +794,8 @@ struct AdamParams {
   }
 };
 
-struct OpRowsGradAdam : OpBase {
-  static constexpr int FFT1 = -1, FFT2 = 0, NSUM = 0, NMAX = 0;
+struct OpRowsGradAdam : OpKeep {
+  static constexpr int FFT1 = -1, FFT2 = 0;
   const float2* T;
   const int* S;
   float2* rho;
@@ -741,14 +803,13 @@ struct OpRowsGradAdam : OpBase {
   float2* v;
   AdamParams ap;
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return T[gi]; }
-  __device__ float2 mid(float2 x, size_t, int, int, int, Acc&) const { return x; }
-  __device__ void store(float2 g, size_t gi, int, int, int, Acc&) const {
-    float2 mm = m[gi], vv = v[gi], p = rho[gi];
-    ap.step(g, S[gi], mm, vv, p);
-    m[gi] = mm;
-    v[gi] = vv;
-    rho[gi] = p;
+  __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
+  __device__ void store(float2 g, const Px& q, Acc&) const {
+    float2 mm = m[q.gi], vv = v[q.gi], p = rho[q.gi];
+    ap.step(g, S[q.gi], mm, vv, p);
+    m[q.gi] = mm;
+    v[q.gi] = vv;
+    rho[q.gi] = p;
   }
 };
 
@@ -756,60 +817,52 @@ struct OpRowsGradAdam : OpBase {
 
 // column pass: src -> FFT(S) (y) -> dst
 template <int S>
-struct OpColsTransform : OpBase {
+struct OpColsTransform : OpKeep {
   static constexpr int FFT1 = S, FFT2 = 0;
   const float2* src;
   float2* dst;
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return src[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { dst[gi] = v; }
+  __device__ float2 load(const Px& q, Acc&) const { return src[q.ti]; }
+  __device__ void store(float2 v, const Px& q, Acc&) const { dst[q.ti] = v; }
 };
 
 // column pass: src -> FFT+ (y) -> |.| -> M (float)
-struct OpColsMagnitude : OpBase {
+struct OpColsMagnitude : OpKeep {
   static constexpr int FFT1 = +1, FFT2 = 0;
   const float2* src;
   float* M;
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int, int, int, Acc&) const { return src[gi]; }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { M[gi] = cabsf2(v); }
+  __device__ float2 load(const Px& q, Acc&) const { return src[q.ti]; }
+  __device__ void store(float2 v, const Px& q, Acc&) const { M[q.gi] = cabsf2(v); }
 };
 
-// column pass over pairs: item p forms the band-passed cross-power spectrum
-// of D[xi[p]] with Dref[ri[p]] (conj(D) Dref for SIGN=-1, D Dref for +1;
-// multiply() of gpu_context.cu:1157-1200), masked where A < 0, then
-// FFT- (y) -> dst[p].  Items are numbered from 0 (first == 0).
-template <int SIGN>
-struct OpColsCrossPowerIdx : OpBase {
+// column pass over pairs: item p forms the band-passed cross-power spectra of
+// D[xi[p]] with Dref[ri[p]] -- conj(D) Dref and D Dref (multiply() of
+// gpu_context.cu:1157-1200), zero where A < 0 -- then FFT- (y) -> dst[p] and
+// dst2[p].  Items are numbered from 0 (first == 0).  Both products are formed
+// from one read of the spectra.
+struct OpColsCrossPower : OpBase {
   static constexpr int FFT1 = -1, FFT2 = 0;
+  static constexpr bool AMP = true, PAIR = true;
   const float2* D;
   const float2* Dref;
   const int* xi;
   const int* ri;
   float2* dst;
-  const float* A;
-  int n;
-  float minr, maxr;
-  int norm_d, norm_ref;
+  float2* dst2;
+  size_t npix;
+  int norm_d, norm_ref;  // apply normalize_ft_shift
   using Acc = NoAcc;
-  __device__ float2 load(size_t gi, int p, int y, int x, Acc&) const {
-    const size_t npix = (size_t)n * n;
-    const size_t pix = (size_t)y * n + x;
-    float2 d = D[(size_t)__ldg(xi + p) * npix + pix];
-    float2 r = Dref[(size_t)__ldg(ri + p) * npix + pix];
+  __device__ void load_pair(const Px& q, float2& c1, float2& c2) const {
+    const size_t pix = q.ti - (size_t)q.p * npix;
+    float2 d = D[(size_t)__ldg(xi + q.p) * npix + pix];
+    float2 r = Dref[(size_t)__ldg(ri + q.p) * npix + pix];
     if (norm_d) d = ft_shift_norm(d);
     if (norm_ref) r = ft_shift_norm(r);
-    const float sd = (float)SIGN * d.y;
-    float2 c = make_float2(d.x * r.x - sd * r.y, d.x * r.y + sd * r.x);
-    const float w = bandpass2(x, y, n, minr, maxr);
-    c = make_float2(c.x * w, c.y * w);
-    if (__ldg(A + pix) < 0.f) c = make_float2(0.f, 0.f);
-    return c;
+    c1 = weighted(cross_power<-1>(d, r), q.a);
+    c2 = weighted(cross_power<+1>(d, r), q.a);
   }
-  __device__ float2 mid(float2 v, size_t, int, int, int, Acc&) const { return v; }
-  __device__ void store(float2 v, size_t gi, int, int, int, Acc&) const { dst[gi] = v; }
+  __device__ void store_pair(float2 v, const Px& q, int second) const { (second ? dst2 : dst)[q.ti] = v; }
 };
 
 }  // namespace spe

@@ -132,17 +132,6 @@ __device__ __forceinline__ void load_twiddles(float2* tw, const float2* __restri
   for (int i = threadIdx.x; i < TWS; i += nt) tw[i] = twg[i];
 }
 
-// Programmatic dependent launch: a kernel launched with the programmatic
-// stream serialisation attribute may start while the previous kernel of the
-// stream drains.  It lets its own dependents start early, loads what no
-// kernel writes (the twiddle tables), then waits until the previous grid has
-// completed and its writes are visible before touching the population.
-// Without the attribute both instructions are no-ops.
-__device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Stage one column tile: W columns of T (16-byte chunks of two columns) in
 // the exchange layout, and the matching W amplitude columns.  When the
 // chunks divide evenly over the threads, each thread copies the same column
@@ -294,7 +283,7 @@ __global__ void __launch_bounds__(ColCfg<N, W>::NT, ColCfg<N, W>::MINB)
     for (int e = 0; e < E; ++e) {
       const float a = sA[elem_pos<N>(e, j) * W + c];
       float2 g = make_float2(0.f, 0.f);
-      if (a >= 0.f) acc += loss_term<LOSS>(v[e], a, eps, GRAD ? &g : nullptr);
+      if (a >= 0.f) loss_add(acc, loss_term<LOSS>(v[e], a, eps, GRAD ? &g : nullptr));
       v[e] = g;
     }
     if (GRAD) {

@@ -22,48 +22,6 @@ using namespace spe_detail;
 
 namespace spe {
 
-__global__ void k_reduce_peak(const double* __restrict__ part, int count, int tpi, double* out, int ostride, int oslot);
-__global__ void k_reduce(const double* __restrict__ part, int count, int tpi, int k, int is_max, double* out,
-                         int ostride, int oslot);
-
-// complex sum of item idx[p] (or p) per block, double accumulation
-__global__ void k_complex_sum(const float2* __restrict__ src, size_t npix, const int* __restrict__ idx,
-                              double* __restrict__ out) {
-  const int p = blockIdx.x;
-  const float2* a = src + (size_t)(idx ? idx[p] : p) * npix;
-  double sx = 0.0, sy = 0.0;
-  for (size_t i0 = (size_t)threadIdx.x * 16; i0 < npix; i0 += (size_t)blockDim.x * 16) {
-    float fx = 0.f, fy = 0.f;
-    const size_t end = (i0 + 16 < npix) ? i0 + 16 : npix;
-    for (size_t i = i0; i < end; ++i) {
-      const float2 v = a[i];
-      fx += v.x;
-      fy += v.y;
-    }
-    sx += fx;
-    sy += fy;
-  }
-  __shared__ double rx[32], ry[32];
-  for (int off = 16; off > 0; off >>= 1) {
-    sx += __shfl_down_sync(0xffffffffu, sx, off);
-    sy += __shfl_down_sync(0xffffffffu, sy, off);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    rx[threadIdx.x >> 5] = sx;
-    ry[threadIdx.x >> 5] = sy;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double ax = 0.0, ay = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      ax += rx[w];
-      ay += ry[w];
-    }
-    out[2 * p] = ax;
-    out[2 * p + 1] = ay;
-  }
-}
-
 __global__ void k_int_sum(const int* __restrict__ s, size_t npix, long long* __restrict__ out) {
   long long acc = 0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < npix; i += (size_t)gridDim.x * blockDim.x)
@@ -461,13 +419,16 @@ int spe_reshift(spe_engine* e, int first, int count, int ref_slot, const float* 
   const size_t npix = e->npix;
   const int tr = e->ops->tiles_rows;
   const size_t need = ((size_t)(count + 1) * npix + (size_t)count * npix) * sizeof(float2) +
-                      (size_t)count * tr * spe::NRED * sizeof(double) * 2 + (size_t)(count + 1) * 2 * sizeof(double) +
+                      (size_t)(3 * count + 1) * tr * spe::NRED * sizeof(double) +
+                      (size_t)(count + 1) * 2 * sizeof(double) +
                       (size_t)count * (sizeof(spe::ShiftItem) + 2 * sizeof(int) + 8 * sizeof(double)) + 64 * 256;
   if ((rc = ensure_work(e, need))) return rc;
   Carve cv{(char*)e->work};
   float2* D = cv.take<float2>((size_t)(count + 1) * npix);  // [0,count) members, count: reference
   float2* scratch = cv.take<float2>((size_t)count * npix);
   double* part = cv.take<double>((size_t)count * tr * spe::NRED);
+  double* part2 = cv.take<double>((size_t)count * tr * spe::NRED);
+  double* psum = cv.take<double>((size_t)(count + 1) * tr * spe::NRED);
   double* sums = cv.take<double>((size_t)(count + 1) * 2);
   int* xi = cv.take<int>(count);
   int* ri = cv.take<int>(count);
@@ -482,22 +443,19 @@ int spe_reshift(spe_engine* e, int first, int count, int ref_slot, const float* 
   else
     CK(cudaMemcpyAsync(e->ref, ref_density, npix * sizeof(float2), cudaMemcpyHostToDevice, e->st), "reference upload");
   spe::Ctx c = item_ctx(e, count, Apat);
-  CK(e->ops->abs_spectrum_items(c, e->rho + (size_t)first * npix, D), "spectra");
+  CK(e->ops->abs_spectrum_items(c, e->rho + (size_t)first * npix, D, psum), "spectra");
   spe::Ctx c1 = item_ctx(e, 1, Apat);
-  CK(e->ops->abs_spectrum_items(c1, e->ref, D + (size_t)count * npix), "reference spectrum");
-  spe::k_complex_sum<<<count, 256, 0, e->st>>>(e->rho + (size_t)first * npix, npix, nullptr, sums);
-  spe::k_complex_sum<<<1, 256, 0, e->st>>>(e->ref, npix, nullptr, sums + 2 * count);
-  CK(cudaGetLastError(), "complex sums");
+  CK(e->ops->abs_spectrum_items(c1, e->ref, D + (size_t)count * npix, psum + (size_t)count * tr * spe::NRED),
+     "reference spectrum");
+  if ((rc = reduce(e, count + 1, {{psum, tr, 0, 0, 0}, {psum, tr, 1, 0, 1}}, sums, 2))) return rc;
+  if ((rc = band_weights(e, first, count, minr, maxr))) return rc;
   std::vector<int> hx(count), hr(count, count);
   std::iota(hx.begin(), hx.end(), 0);
   CK(cudaMemcpyAsync(xi, hx.data(), count * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
   CK(cudaMemcpyAsync(ri, hr.data(), count * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
   // get_shift (gpu_context.cu:1226-1326): both spectra normalised
-  for (int s = 0; s < 2; ++s) {
-    CK(e->ops->corr_peak_idx(c, D, D, xi, ri, s == 0 ? -1 : +1, minr, maxr, 1, 1, scratch, part), "correlation");
-    spe::k_reduce_peak<<<(count + 127) / 128, 128, 0, e->st>>>(part, count, tr, peaks, 4, 2 * s);
-    CK(cudaGetLastError(), "peak reduce");
-  }
+  CK(e->ops->corr_peaks(c, D, D, xi, ri, 1, 1, scratch, e->T, part, part2), "correlation");
+  if ((rc = reduce(e, count, {{part, tr, 0, 2, 0}, {part2, tr, 0, 2, 2}}, peaks, 4))) return rc;
   std::vector<double> hp((size_t)count * 4), hs((size_t)(count + 1) * 2);
   CK(cudaMemcpyAsync(hp.data(), peaks, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "peaks");
   CK(cudaMemcpyAsync(hs.data(), sums, hs.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "sums");
@@ -609,9 +567,7 @@ int spe_initialize_pop(spe_engine* e, int first, int count, int support_size, fl
   spe::k_init_objects<<<grid, 256, 0, e->st>>>(e->rho, e->S, dinds, ditems, first, e->n, support_size);
   CK(cudaGetLastError(), "object synthesis");
   CK(e->ops->known_power(make_ctx(e, first, count), part), "power transform");
-  spe::k_reduce<<<(count + 127) / 128, 128, 0, e->st>>>(part, count, tc, 0, 0, sums, 2, 0);
-  spe::k_reduce<<<(count + 127) / 128, 128, 0, e->st>>>(part, count, tc, 1, 0, sums, 2, 1);
-  CK(cudaGetLastError(), "power reduce");
+  if ((rc = reduce(e, count, {{part, tc, 0, 0, 0}, {part, tc, 1, 0, 1}}, sums, 2))) return rc;
   std::vector<double> hs((size_t)count * 2);
   CK(cudaMemcpyAsync(hs.data(), sums, hs.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "sums");
   CK(cudaStreamSynchronize(e->st), "synchronize");
@@ -710,7 +666,7 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
                 + (size_t)5 * P * npix * sizeof(float2)        // parents per child
                 + (size_t)P * npix * sizeof(float2)            // children
                 + (size_t)3 * P * npix * sizeof(int)           // supports per child
-                + (size_t)items * tr * spe::NRED * sizeof(double) + (size_t)items * 4 * sizeof(double) +
+                + (size_t)(2 * items + P + 1) * tr * spe::NRED * sizeof(double) + (size_t)items * 4 * sizeof(double) +
                 (size_t)(P + 1) * 2 * sizeof(double) + (size_t)items * (2 * sizeof(int) + sizeof(spe::ShiftItem)) +
                 (size_t)P * (sizeof(spe::CrossChild) + 2 * sizeof(int)) + 64 * 256;
   const size_t mod_need = (size_t)P * npix * (sizeof(float) + sizeof(float2)) + P * sizeof(int) + 1024;
@@ -777,6 +733,8 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
     float2* C = cv2.take<float2>((size_t)P * npix);
     int* Ws = cv2.take<int>((size_t)3 * P * npix);
     double* part = cv2.take<double>((size_t)items * tr * spe::NRED);
+    double* part2 = cv2.take<double>((size_t)items * tr * spe::NRED);
+    double* psum = cv2.take<double>((size_t)(P + 1) * tr * spe::NRED);
     double* peaks = cv2.take<double>((size_t)items * 4);
     double* sums = cv2.take<double>((size_t)(P + 1) * 2);
     int* xi = cv2.take<int>(items);
@@ -791,12 +749,12 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
     // (prepare_parents / reshift_parent, gpu_context.cu:1536-1694; spectra
     // not normalised on this path).  Spectra of the members and the average.
     spe::Ctx c = item_ctx(e, P, Apat);
-    CK(e->ops->abs_spectrum_items(c, e->rho + (size_t)first * npix, D), "spectra");
-    CK(e->ops->abs_spectrum_items(item_ctx(e, 1, Apat), e->rho + (size_t)avg_slot * npix, D + (size_t)P * npix),
+    CK(e->ops->abs_spectrum_items(c, e->rho + (size_t)first * npix, D, psum), "spectra");
+    CK(e->ops->abs_spectrum_items(item_ctx(e, 1, Apat), e->rho + (size_t)avg_slot * npix, D + (size_t)P * npix,
+                                  psum + (size_t)P * tr * spe::NRED),
        "average spectrum");
-    spe::k_complex_sum<<<P, 256, 0, e->st>>>(e->rho + (size_t)first * npix, npix, nullptr, sums);
-    spe::k_complex_sum<<<1, 256, 0, e->st>>>(e->rho + (size_t)avg_slot * npix, npix, nullptr, sums + 2 * P);
-    CK(cudaGetLastError(), "complex sums");
+    if ((rc = reduce(e, P + 1, {{psum, tr, 0, 0, 0}, {psum, tr, 1, 0, 1}}, sums, 2))) return rc;
+    if ((rc = band_weights(e, first, P, minr, maxr))) return rc;
     std::vector<int> hx(items), hr(items);
     for (int i = 0; i < P; ++i) {
       hx[4 * i + 0] = i;
@@ -808,11 +766,9 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
     CK(cudaMemcpyAsync(xi, hx.data(), items * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
     CK(cudaMemcpyAsync(ri, hr.data(), items * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
     spe::Ctx ci = item_ctx(e, items, Apat);
-    for (int s = 0; s < 2; ++s) {
-      CK(e->ops->corr_peak_idx(ci, D, D, xi, ri, s == 0 ? -1 : +1, minr, maxr, 0, 0, scratch, part), "correlation");
-      spe::k_reduce_peak<<<(items + 127) / 128, 128, 0, e->st>>>(part, items, tr, peaks, 4, 2 * s);
-      CK(cudaGetLastError(), "peak reduce");
-    }
+    // (W holds nothing yet: scratch of the second product)
+    CK(e->ops->corr_peaks(ci, D, D, xi, ri, 0, 0, scratch, W, part, part2), "correlation");
+    if ((rc = reduce(e, items, {{part, tr, 0, 2, 0}, {part2, tr, 0, 2, 2}}, peaks, 4))) return rc;
     std::vector<double> hp((size_t)items * 4), hs((size_t)(P + 1) * 2);
     CK(cudaMemcpyAsync(hp.data(), peaks, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "peaks");
     CK(cudaMemcpyAsync(hs.data(), sums, hs.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "sums");

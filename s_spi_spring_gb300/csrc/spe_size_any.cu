@@ -387,6 +387,7 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, BIG ? 2 : 
   float2* cur = sm_any;
   float2* oth = sm_any + (size_t)W * LS;
   float2* tws = sm_any + (size_t)2 * W * LS;  // the twiddle table, n entries
+  pdl_enter();
   for (int i = threadIdx.x; i < n; i += NT) tws[i] = __ldg(tw + i);
   const int tpi = (n + W - 1) / W;
   const int p = op.first + blockIdx.x / tpi;
@@ -398,39 +399,63 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, BIG ? 2 : 
   typename Op::Acc acc;
   // element i of the tile: row passes walk along x (whole rows), column
   // passes across the tile's columns first (row segments of nl elements)
-  auto coords = [&](int i, int& c, int& l, int& y, int& x) {
+  auto px = [&](int i, int& c, int& l) {
     if (AXIS == AX_ROWS) {
       c = fdiv(i, pl.inv_n);
       l = i - c * n;
-      y = l0 + c;
-      x = l;
     } else {
       l = fdiv(i, inv_nl);
       c = i - l * nl;
-      y = l;
-      x = l0 + c;
     }
+    Px q;
+    q.p = p;
+    q.y = AXIS == AX_ROWS ? l0 + c : l;
+    q.x = AXIS == AX_ROWS ? l : l0 + c;
+    q.gi = q.ti = base + (size_t)q.y * n + q.x;
+    q.a = Op::AMP ? __ldg(op.amp(p, n) + (size_t)q.y * n + q.x) : 0.f;
+    return q;
   };
-  for (int i = threadIdx.x; i < tot; i += NT) {
-    int c, l, y, x;
-    coords(i, c, l, y, x);
-    cur[c * LS + l] = op.load(base + (size_t)y * n + x, p, y, x, acc);
-  }
-  __syncthreads();
-  if constexpr (Op::FFT1 != 0) fft_any<Op::FFT1, BIG>(cur, oth, pl, tws, nl);
-  if constexpr (Op::FFT2 != 0) {
+  pdl_wait();
+  if constexpr (Op::PAIR) {
+    for (int second = 0; second < 2; ++second) {
+      for (int i = threadIdx.x; i < tot; i += NT) {
+        int c, l;
+        const Px q = px(i, c, l);
+        float2 v1, v2;
+        op.load_pair(q, v1, v2);
+        cur[c * LS + l] = second ? v2 : v1;
+      }
+      __syncthreads();
+      fft_any<Op::FFT1, BIG>(cur, oth, pl, tws, nl);
+      for (int i = threadIdx.x; i < tot; i += NT) {
+        int c, l;
+        const Px q = px(i, c, l);
+        op.store_pair(cur[c * LS + l], q, second);
+      }
+      __syncthreads();
+    }
+  } else {
     for (int i = threadIdx.x; i < tot; i += NT) {
-      int c, l, y, x;
-      coords(i, c, l, y, x);
-      cur[c * LS + l] = op.mid(cur[c * LS + l], base + (size_t)y * n + x, p, y, x, acc);
+      int c, l;
+      const Px q = px(i, c, l);
+      cur[c * LS + l] = op.load(q, acc);
     }
     __syncthreads();
-    fft_any<Op::FFT2, BIG>(cur, oth, pl, tws, nl);
-  }
-  for (int i = threadIdx.x; i < tot; i += NT) {
-    int c, l, y, x;
-    coords(i, c, l, y, x);
-    op.store(cur[c * LS + l], base + (size_t)y * n + x, p, y, x, acc);
+    if constexpr (Op::FFT1 != 0) fft_any<Op::FFT1, BIG>(cur, oth, pl, tws, nl);
+    if constexpr (Op::FFT2 != 0) {
+      for (int i = threadIdx.x; i < tot; i += NT) {
+        int c, l;
+        const Px q = px(i, c, l);
+        cur[c * LS + l] = op.mid(cur[c * LS + l], q, acc);
+      }
+      __syncthreads();
+      fft_any<Op::FFT2, BIG>(cur, oth, pl, tws, nl);
+    }
+    for (int i = threadIdx.x; i < tot; i += NT) {
+      int c, l;
+      const Px q = px(i, c, l);
+      op.store(cur[c * LS + l], q, acc);
+    }
   }
   if constexpr (Op::NSUM + Op::NMAX > 0) {
     double r[NRED];
@@ -512,7 +537,12 @@ cudaError_t launch_any_k(const Op& op, const AnyPlan& pl, int count, cudaStream_
   cudaError_t e = configure(kern, kAnySmem, configured);
   if (e != cudaSuccess || count <= 0) return e;
   const int tpi = (pl.n + pl.W - 1) / pl.W;
-  kern<<<(unsigned)count * tpi, BIG ? kAnyThreadsBig : kAnyThreads, smem, st>>>(op, pl, tw);
+  const int grid = (int)((unsigned)count * tpi), threads = BIG ? kAnyThreadsBig : kAnyThreads;
+  // the early launch pays where a pass is a few waves of CTAs (a prologue
+  // beside the previous pass's drain: 111 -> 82 us for an evaluation of one
+  // small pattern); over many waves it measured 0.6% slower (1054^2 x 16)
+  if (grid <= 4 * sm_count()) return launch_pdl(kern, grid, threads, smem, st, op, pl, tw);
+  kern<<<grid, threads, smem, st>>>(op, pl, tw);
   return cudaGetLastError();
 }
 template <int AXIS, class Op>
@@ -542,10 +572,8 @@ struct SizeAny {
   static OpColsProject cols_project(const Ctx& c) {
     OpColsProject op;
     op.first = c.first;
-    op.partials = nullptr;
     op.T = c.T;
     op.A = c.A;
-    op.n = c.n;
     op.ipp = c.ipp;
     return op;
   }
@@ -557,7 +585,6 @@ struct SizeAny {
     const OpColsProject proj = cols_project(c);
     OpRowsIterate<UPD> it;
     it.first = c.first;
-    it.partials = nullptr;
     it.T = c.T;
     it.rho = c.rho;
     it.S = c.S;
@@ -573,7 +600,6 @@ struct SizeAny {
     if (iters == 0 && c.mark) SPE_TRY(cudaEventRecord(c.mark, c.st));
     OpRowsFinal fin;
     fin.first = c.first;
-    fin.partials = nullptr;
     fin.T = c.T;
     fin.out = c.rho;
     fin.scale = scale(c.n);
@@ -601,13 +627,11 @@ struct SizeAny {
     SPE_TRY((launch_any<AX_COLS>(cols_project(c), pl, c.count, c.st, c.tw)));
     OpRowsModulusForward mf;
     mf.first = c.first;
-    mf.partials = nullptr;
     mf.T = c.T;
     mf.scale = scale(c.n);
     SPE_TRY((launch_any<AX_ROWS>(mf, pl, c.count, c.st, c.tw)));
     OpColsBlur bl;
     bl.first = c.first;
-    bl.partials = nullptr;
     bl.T = c.T;
     bl.n = c.n;
     bl.sig2 = sigma_ft * sigma_ft;
@@ -628,7 +652,6 @@ struct SizeAny {
     ce.partials = p2;
     ce.T = c.T;
     ce.A = c.A;
-    ce.n = c.n;
     ce.ipp = c.ipp;
     SPE_TRY((launch_any<AX_COLS>(ce, pl, c.count, c.st, c.tw)));
     OpRowsRealError re;
@@ -637,54 +660,29 @@ struct SizeAny {
     re.T = c.T;
     re.S = c.S;
     re.scale = scale(c.n);
-    re.g = g;
     return launch_any<AX_ROWS>(re, pl, c.count, c.st, c.tw);
   }
 
-  static cudaError_t abs_spectrum(const Ctx& c, float2* dst) {
+  static cudaError_t symmetry(const Ctx& c, double* psum, double* ppeak) {
     const AnyPlan& pl = plan_of(c.n);
-    const Gate g{};
-    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_ABS>(c, c.rho, dst, g, nullptr), pl, c.count, c.st, c.tw)));
-    OpColsForward cf;
-    cf.first = c.first;
-    cf.partials = nullptr;
-    cf.src = dst;
-    cf.dst = dst;
-    return launch_any<AX_COLS>(cf, pl, c.count, c.st, c.tw);
+    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_ABS>(c, c.rho, c.T, Gate{}, nullptr), pl, c.count, c.st, c.tw)));
+    OpColsSymmetry sy;
+    sy.first = c.first;
+    sy.partials = psum;
+    sy.T = c.T;
+    sy.A = c.band;
+    sy.ipp = c.ipp;
+    SPE_TRY((launch_any<AX_COLS>(sy, pl, c.count, c.st, c.tw)));
+    return rows_peak(c, pl, c.T, ppeak);
   }
 
-  template <int SIGN>
-  static cudaError_t corr_peak_t(const Ctx& c, const float2* D, const float2* Dref, size_t ref_stride, int ref_first,
-                                 float minr, float maxr, int norm_d, int norm_ref, double* partials) {
-    const AnyPlan& pl = plan_of(c.n);
-    OpColsCrossPower<SIGN> cp;
-    cp.first = c.first;
-    cp.partials = nullptr;
-    cp.D = D;
-    cp.Dref = Dref;
-    cp.ref_stride = ref_stride;
-    cp.ref_first = ref_first;
-    cp.dst = c.T;
-    cp.A = c.A;
-    cp.n = c.n;
-    cp.ipp = c.ipp;
-    cp.minr = minr;
-    cp.maxr = maxr;
-    cp.norm_d = norm_d;
-    cp.norm_ref = norm_ref;
-    SPE_TRY((launch_any<AX_COLS>(cp, pl, c.count, c.st, c.tw)));
+  static cudaError_t rows_peak(const Ctx& c, const AnyPlan& pl, const float2* T, double* partials) {
     OpRowsPeak pk;
     pk.first = c.first;
     pk.partials = partials;
-    pk.T = c.T;
+    pk.T = T;
     pk.n = c.n;
     return launch_any<AX_ROWS>(pk, pl, c.count, c.st, c.tw);
-  }
-
-  static cudaError_t corr_peak(const Ctx& c, const float2* D, const float2* Dref, size_t ref_stride, int ref_first,
-                               int sign, float minr, float maxr, int norm_d, int norm_ref, double* partials) {
-    if (sign < 0) return corr_peak_t<-1>(c, D, Dref, ref_stride, ref_first, minr, maxr, norm_d, norm_ref, partials);
-    return corr_peak_t<+1>(c, D, Dref, ref_stride, ref_first, minr, maxr, norm_d, norm_ref, partials);
   }
 
   // ---- generic transforms over `c.count` items starting at `data` (c.first ignored)
@@ -696,20 +694,17 @@ struct SizeAny {
       SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(z, data, data, Gate{}, nullptr), pl, c.count, c.st, c.tw)));
       OpColsTransform<+1> ct;
       ct.first = 0;
-      ct.partials = nullptr;
       ct.src = data;
       ct.dst = data;
       return launch_any<AX_COLS>(ct, pl, c.count, c.st, c.tw);
     }
     OpColsTransform<-1> ct;
     ct.first = 0;
-    ct.partials = nullptr;
     ct.src = data;
     ct.dst = data;
     SPE_TRY((launch_any<AX_COLS>(ct, pl, c.count, c.st, c.tw)));
     OpRowsFinal fin;
     fin.first = 0;
-    fin.partials = nullptr;
     fin.T = data;
     fin.out = data;
     fin.scale = scale(c.n);
@@ -723,58 +718,42 @@ struct SizeAny {
     SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(z, src, tmp, Gate{}, nullptr), pl, c.count, c.st, c.tw)));
     OpColsMagnitude cm;
     cm.first = 0;
-    cm.partials = nullptr;
     cm.src = tmp;
     cm.M = M;
     return launch_any<AX_COLS>(cm, pl, c.count, c.st, c.tw);
   }
 
-  static cudaError_t abs_spectrum_items(const Ctx& c, const float2* src, float2* dst) {
+  static cudaError_t abs_spectrum_items(const Ctx& c, const float2* src, float2* dst, double* psum) {
     const AnyPlan& pl = plan_of(c.n);
     Ctx z = c;
     z.first = 0;
-    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_ABS>(z, src, dst, Gate{}, nullptr), pl, c.count, c.st, c.tw)));
+    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_ABS_SUM>(z, src, dst, Gate{}, psum), pl, c.count, c.st, c.tw)));
     OpColsTransform<+1> ct;
-    ct.first = 0;
-    ct.partials = nullptr;
     ct.src = dst;
     ct.dst = dst;
     return launch_any<AX_COLS>(ct, pl, c.count, c.st, c.tw);
   }
 
-  template <int SIGN>
-  static cudaError_t corr_peak_idx_t(const Ctx& c, const float2* D, const float2* Dref, const int* xi, const int* ri,
-                                     float minr, float maxr, int norm_d, int norm_ref, float2* scratch,
-                                     double* partials) {
+  static cudaError_t corr_peaks(const Ctx& c, const float2* D, const float2* Dref, const int* xi, const int* ri,
+                                int norm_d, int norm_ref, float2* scratch1, float2* scratch2, double* part1,
+                                double* part2) {
     const AnyPlan& pl = plan_of(c.n);
-    OpColsCrossPowerIdx<SIGN> cp;
-    cp.first = 0;
-    cp.partials = nullptr;
+    OpColsCrossPower cp;
+    cp.A = c.band;
     cp.D = D;
     cp.Dref = Dref;
     cp.xi = xi;
     cp.ri = ri;
-    cp.dst = scratch;
-    cp.A = c.A;
-    cp.n = c.n;
-    cp.minr = minr;
-    cp.maxr = maxr;
+    cp.dst = scratch1;
+    cp.dst2 = scratch2;
+    cp.npix = (size_t)c.n * c.n;
     cp.norm_d = norm_d;
     cp.norm_ref = norm_ref;
     SPE_TRY((launch_any<AX_COLS>(cp, pl, c.count, c.st, c.tw)));
-    OpRowsPeak pk;
-    pk.first = 0;
-    pk.partials = partials;
-    pk.T = scratch;
-    pk.n = c.n;
-    return launch_any<AX_ROWS>(pk, pl, c.count, c.st, c.tw);
-  }
-
-  static cudaError_t corr_peak_idx(const Ctx& c, const float2* D, const float2* Dref, const int* xi, const int* ri,
-                                   int sign, float minr, float maxr, int norm_d, int norm_ref, float2* scratch,
-                                   double* partials) {
-    if (sign < 0) return corr_peak_idx_t<-1>(c, D, Dref, xi, ri, minr, maxr, norm_d, norm_ref, scratch, partials);
-    return corr_peak_idx_t<+1>(c, D, Dref, xi, ri, minr, maxr, norm_d, norm_ref, scratch, partials);
+    Ctx z = c;
+    z.first = 0;
+    SPE_TRY(rows_peak(z, pl, scratch1, part1));
+    return rows_peak(z, pl, scratch2, part2);
   }
 
   static cudaError_t known_power(const Ctx& c, double* partials) {
@@ -785,7 +764,6 @@ struct SizeAny {
     kp.partials = partials;
     kp.T = c.T;
     kp.A = c.A;
-    kp.n = c.n;
     kp.ipp = c.ipp;
     return launch_any<AX_COLS>(kp, pl, c.count, c.st, c.tw);
   }
@@ -794,7 +772,6 @@ struct SizeAny {
   static cudaError_t grad_rows(const Ctx& c, const AnyPlan& pl, float2* grad, const float* scale) {
     OpRowsGradOut go;
     go.first = c.first;
-    go.partials = nullptr;
     go.T = c.T;
     go.S = c.S;
     go.G = grad;
@@ -808,7 +785,6 @@ struct SizeAny {
     if (stage == GRAD_ROWS) return grad_rows(c, pl, grad, scale);
     OpRowsSupportForward rf;
     rf.first = c.first;
-    rf.partials = nullptr;
     rf.rho = c.rho;
     rf.S = c.S;
     rf.T = c.T;
@@ -819,7 +795,6 @@ struct SizeAny {
       cl.partials = partials;
       cl.T = c.T;
       cl.A = c.A;
-      cl.n = c.n;
       cl.ipp = c.ipp;
       cl.eps = eps;
       return launch_any<AX_COLS>(cl, pl, c.count, c.st, c.tw);
@@ -829,7 +804,6 @@ struct SizeAny {
     cl.partials = partials;
     cl.T = c.T;
     cl.A = c.A;
-    cl.n = c.n;
     cl.ipp = c.ipp;
     cl.eps = eps;
     SPE_TRY((launch_any<AX_COLS>(cl, pl, c.count, c.st, c.tw)));
@@ -849,7 +823,6 @@ struct SizeAny {
     const AnyPlan& pl = plan_of(c.n);
     OpRowsSupportForward rf;
     rf.first = c.first;
-    rf.partials = nullptr;
     rf.rho = c.rho;
     rf.S = c.S;
     rf.T = c.T;
@@ -859,13 +832,11 @@ struct SizeAny {
     cl.partials = partials;
     cl.T = c.T;
     cl.A = c.A;
-    cl.n = c.n;
     cl.ipp = c.ipp;
     cl.eps = eps;
     SPE_TRY((launch_any<AX_COLS>(cl, pl, c.count, c.st, c.tw)));
     OpRowsGradAdam ad;
     ad.first = c.first;
-    ad.partials = nullptr;
     ad.T = c.T;
     ad.S = c.S;
     ad.rho = c.rho;
@@ -913,12 +884,12 @@ const SizeOps* size_ops_any(int n) {
                     &SizeAny::iterate,
                     &SizeAny::blur_magnitude,
                     &SizeAny::error_terms,
-                    &SizeAny::abs_spectrum,
-                    &SizeAny::corr_peak,
+                    &SizeAny::symmetry,
                     &SizeAny::fft2,
                     &SizeAny::ft_magnitude,
                     &SizeAny::abs_spectrum_items,
-                    &SizeAny::corr_peak_idx,
+                    &SizeAny::corr_peaks,
+                    &launch_band_table,
                     &SizeAny::one_width,
                     &SizeAny::one_width,
                     0,

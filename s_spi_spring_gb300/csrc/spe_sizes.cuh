@@ -52,6 +52,23 @@ cudaError_t configure(K kern, size_t smem, std::atomic<unsigned long long>& conf
   return cudaSuccess;
 }
 
+// launch with programmatic stream serialisation (the kernel's prologue
+// overlaps the previous kernel's drain; see pdl_wait)
+template <class K, class... Args>
+cudaError_t launch_pdl(K kern, int grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 template <int N, int AXIS, class Op>
 cudaError_t launch_pass(const Op& op, int count, cudaStream_t st, const float2* tw) {
   using C = PassCfg<N, AXIS>;
@@ -66,8 +83,22 @@ cudaError_t launch_pass(const Op& op, int count, cudaStream_t st, const float2* 
   cudaError_t e = configure(kern, smem, configured);
   if (e != cudaSuccess) return e;
   if (count <= 0) return cudaSuccess;
-  kern<<<(unsigned)count * (N / W), NT, smem, st>>>(op, tw);
-  return cudaGetLastError();
+  return launch_pdl(kern, (int)((unsigned)count * (N / W)), NT, smem, st, op, tw);
+}
+
+// an op on the blocked scratch where the side has one, else row-major
+template <int N, int AXIS, class Op>
+cudaError_t run_pass(const Op& op, int count, cudaStream_t st, const float2* tw) {
+  if constexpr (Blocked<N>::ok) {
+    using C = BlkPassCfg<N, AXIS, Op>;
+    auto kern = k_blocked_pass<N, AXIS, Op>;
+    static std::atomic<unsigned long long> configured{0ull};
+    cudaError_t e = configure(kern, C::SMEM, configured);
+    if (e != cudaSuccess || count <= 0) return e;
+    return launch_pdl(kern, (int)((unsigned)count * (N / C::W)), C::NT, C::SMEM, st, op, tw);
+  } else {
+    return launch_pass<N, AXIS>(op, count, st, tw);
+  }
 }
 
 // tile-width variants compiled per size: those whose tile fits in shared
@@ -179,23 +210,6 @@ int resident_ctas(K kern, int threads, size_t smem, std::atomic<int>* cache) {
     cache[dev].store(r, std::memory_order_release);
   }
   return r;
-}
-
-// launch with programmatic stream serialisation (the kernel's prologue
-// overlaps the previous kernel's drain; see pdl_wait)
-template <class K, class... Args>
-cudaError_t launch_pdl(K kern, int grid, int threads, size_t smem, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 // the resident CTAs a persistent launch takes when `div` kernels share the GPU
@@ -515,13 +529,14 @@ struct SizeImpl {
     return op;
   }
 
+  // amplitudes in the order of run_pass's column passes
+  static const float* amps(const Ctx& c) { return Blocked<N>::ok ? c.At : c.A; }
+
   static OpColsProject cols_project(const Ctx& c) {
     OpColsProject op;
     op.first = c.first;
-    op.partials = nullptr;
     op.T = c.T;
-    op.A = c.A;
-    op.n = N;
+    op.A = amps(c);
     op.ipp = c.ipp;
     return op;
   }
@@ -529,16 +544,6 @@ struct SizeImpl {
   template <int UPD>
   static cudaError_t iterate_t(const Ctx& c, int iters, float beta, Gate g, int wc, int wr) {
     SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, g, nullptr), c.count, c.st, c.tw)));
-    const OpColsProject proj = cols_project(c);
-    OpRowsIterate<UPD> it;
-    it.first = c.first;
-    it.partials = nullptr;
-    it.T = c.T;
-    it.rho = c.rho;
-    it.S = c.S;
-    it.scale = scale();
-    it.beta = beta;
-    it.g = g;
     for (int i = 0; i < iters; ++i) {
       SPE_TRY(launch_cols_w<N>(c, wc));
       if (i == 0 && c.mark) SPE_TRY(cudaEventRecord(c.mark, c.st));
@@ -548,7 +553,6 @@ struct SizeImpl {
     if (iters == 0 && c.mark) SPE_TRY(cudaEventRecord(c.mark, c.st));
     OpRowsFinal fin;
     fin.first = c.first;
-    fin.partials = nullptr;
     fin.T = c.T;
     fin.out = c.rho;
     fin.scale = scale();
@@ -642,93 +646,65 @@ struct SizeImpl {
 
   static cudaError_t blur_magnitude(const Ctx& c, float sigma_ft) {
     const Gate g{};
-    SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, g, nullptr), c.count, c.st, c.tw)));
-    SPE_TRY((launch_pass<N, AX_COLS>(cols_project(c), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, g, nullptr), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_COLS>(cols_project(c), c.count, c.st, c.tw)));
     OpRowsModulusForward mf;
     mf.first = c.first;
-    mf.partials = nullptr;
     mf.T = c.T;
     mf.scale = scale();
-    SPE_TRY((launch_pass<N, AX_ROWS>(mf, c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(mf, c.count, c.st, c.tw)));
     OpColsBlur bl;
     bl.first = c.first;
-    bl.partials = nullptr;
     bl.T = c.T;
     bl.n = N;
     bl.sig2 = sigma_ft * sigma_ft;
-    SPE_TRY((launch_pass<N, AX_COLS>(bl, c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_COLS>(bl, c.count, c.st, c.tw)));
     OpRowsMagnitude mg;
     mg.first = c.first;
     mg.partials = c.partials;
     mg.T = c.T;
     mg.M = c.M;
-    return launch_pass<N, AX_ROWS>(mg, c.count, c.st, c.tw);
+    return run_pass<N, AX_ROWS>(mg, c.count, c.st, c.tw);
   }
 
   static cudaError_t error_terms(const Ctx& c, Gate g, double* p1, double* p2, double* p3) {
-    SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_GATED>(c, c.rho, c.T, g, p1), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_GATED>(c, c.rho, c.T, g, p1), c.count, c.st, c.tw)));
     OpColsError ce;
     ce.first = c.first;
     ce.partials = p2;
     ce.T = c.T;
-    ce.A = c.A;
-    ce.n = N;
+    ce.A = amps(c);
     ce.ipp = c.ipp;
-    SPE_TRY((launch_pass<N, AX_COLS>(ce, c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_COLS>(ce, c.count, c.st, c.tw)));
     OpRowsRealError re;
     re.first = c.first;
     re.partials = p3;
     re.T = c.T;
     re.S = c.S;
     re.scale = scale();
-    re.g = g;
-    return launch_pass<N, AX_ROWS>(re, c.count, c.st, c.tw);
+    return run_pass<N, AX_ROWS>(re, c.count, c.st, c.tw);
   }
 
-  static cudaError_t abs_spectrum(const Ctx& c, float2* dst) {
-    const Gate g{};
-    SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_ABS>(c, c.rho, dst, g, nullptr), c.count, c.st, c.tw)));
-    OpColsForward cf;
-    cf.first = c.first;
-    cf.partials = nullptr;
-    cf.src = dst;
-    cf.dst = dst;
-    return launch_pass<N, AX_COLS>(cf, c.count, c.st, c.tw);
+  static cudaError_t symmetry(const Ctx& c, double* psum, double* ppeak) {
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_ABS>(c, c.rho, c.T, Gate{}, nullptr), c.count, c.st, c.tw)));
+    OpColsSymmetry sy;
+    sy.first = c.first;
+    sy.partials = psum;
+    sy.T = c.T;
+    sy.A = c.band;
+    sy.ipp = c.ipp;
+    SPE_TRY((run_pass<N, AX_COLS>(sy, c.count, c.st, c.tw)));
+    return rows_peak(c, c.T, ppeak);
   }
 
-  template <int SIGN>
-  static cudaError_t corr_peak_t(const Ctx& c, const float2* D, const float2* Dref, size_t ref_stride, int ref_first,
-                                 float minr, float maxr, int norm_d, int norm_ref, double* partials) {
-    OpColsCrossPower<SIGN> cp;
-    cp.first = c.first;
-    cp.partials = nullptr;
-    cp.D = D;
-    cp.Dref = Dref;
-    cp.ref_stride = ref_stride;
-    cp.ref_first = ref_first;
-    cp.dst = c.T;
-    cp.A = c.A;
-    cp.n = N;
-    cp.ipp = c.ipp;
-    cp.minr = minr;
-    cp.maxr = maxr;
-    cp.norm_d = norm_d;
-    cp.norm_ref = norm_ref;
-    SPE_TRY((launch_pass<N, AX_COLS>(cp, c.count, c.st, c.tw)));
+  static cudaError_t rows_peak(const Ctx& c, const float2* T, double* partials) {
     OpRowsPeak pk;
     pk.first = c.first;
     pk.partials = partials;
-    pk.T = c.T;
+    pk.T = T;
     pk.n = N;
-    return launch_pass<N, AX_ROWS>(pk, c.count, c.st, c.tw);
+    return run_pass<N, AX_ROWS>(pk, c.count, c.st, c.tw);
   }
-
-  static cudaError_t corr_peak(const Ctx& c, const float2* D, const float2* Dref, size_t ref_stride, int ref_first,
-                               int sign, float minr, float maxr, int norm_d, int norm_ref, double* partials) {
-    if (sign < 0) return corr_peak_t<-1>(c, D, Dref, ref_stride, ref_first, minr, maxr, norm_d, norm_ref, partials);
-    return corr_peak_t<+1>(c, D, Dref, ref_stride, ref_first, minr, maxr, norm_d, norm_ref, partials);
-  }
-
 
   // ---- generic transforms over `c.count` items starting at `data` (c.first ignored)
   static cudaError_t fft2(const Ctx& c, float2* data, int sign) {
@@ -738,20 +714,17 @@ struct SizeImpl {
       SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, data, data, Gate{}, nullptr), c.count, c.st, c.tw)));
       OpColsTransform<+1> ct;
       ct.first = 0;
-      ct.partials = nullptr;
-      ct.src = data;
+        ct.src = data;
       ct.dst = data;
       return launch_pass<N, AX_COLS>(ct, c.count, c.st, c.tw);
     }
     OpColsTransform<-1> ct;
     ct.first = 0;
-    ct.partials = nullptr;
     ct.src = data;
     ct.dst = data;
     SPE_TRY((launch_pass<N, AX_COLS>(ct, c.count, c.st, c.tw)));
     OpRowsFinal fin;
     fin.first = 0;
-    fin.partials = nullptr;
     fin.T = data;
     fin.out = data;
     fin.scale = scale();
@@ -762,74 +735,55 @@ struct SizeImpl {
   static cudaError_t ft_magnitude(const Ctx& c, const float2* src, float2* tmp, float* M) {
     Ctx z = c;
     z.first = 0;
-    SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, src, tmp, Gate{}, nullptr), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, src, tmp, Gate{}, nullptr), c.count, c.st, c.tw)));
     OpColsMagnitude cm;
-    cm.first = 0;
-    cm.partials = nullptr;
     cm.src = tmp;
     cm.M = M;
-    return launch_pass<N, AX_COLS>(cm, c.count, c.st, c.tw);
+    return run_pass<N, AX_COLS>(cm, c.count, c.st, c.tw);
   }
 
   // dst[p] = FFT+(|src[p]|) (2D)
-  static cudaError_t abs_spectrum_items(const Ctx& c, const float2* src, float2* dst) {
+  static cudaError_t abs_spectrum_items(const Ctx& c, const float2* src, float2* dst, double* psum) {
     Ctx z = c;
     z.first = 0;
-    SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_ABS>(z, src, dst, Gate{}, nullptr), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_ABS_SUM>(z, src, dst, Gate{}, psum), c.count, c.st, c.tw)));
     OpColsTransform<+1> ct;
-    ct.first = 0;
-    ct.partials = nullptr;
     ct.src = dst;
     ct.dst = dst;
-    return launch_pass<N, AX_COLS>(ct, c.count, c.st, c.tw);
+    return run_pass<N, AX_COLS>(ct, c.count, c.st, c.tw);
   }
 
-  template <int SIGN>
-  static cudaError_t corr_peak_idx_t(const Ctx& c, const float2* D, const float2* Dref, const int* xi, const int* ri,
-                                     float minr, float maxr, int norm_d, int norm_ref, float2* scratch,
-                                     double* partials) {
-    OpColsCrossPowerIdx<SIGN> cp;
-    cp.first = 0;
-    cp.partials = nullptr;
+  static cudaError_t corr_peaks(const Ctx& c, const float2* D, const float2* Dref, const int* xi, const int* ri,
+                                int norm_d, int norm_ref, float2* scratch1, float2* scratch2, double* part1,
+                                double* part2) {
+    OpColsCrossPower cp;
+    cp.A = c.band;
     cp.D = D;
     cp.Dref = Dref;
     cp.xi = xi;
     cp.ri = ri;
-    cp.dst = scratch;
-    cp.A = c.A;
-    cp.n = N;
-    cp.minr = minr;
-    cp.maxr = maxr;
+    cp.dst = scratch1;
+    cp.dst2 = scratch2;
+    cp.npix = (size_t)N * N;
     cp.norm_d = norm_d;
     cp.norm_ref = norm_ref;
-    SPE_TRY((launch_pass<N, AX_COLS>(cp, c.count, c.st, c.tw)));
-    OpRowsPeak pk;
-    pk.first = 0;
-    pk.partials = partials;
-    pk.T = scratch;
-    pk.n = N;
-    return launch_pass<N, AX_ROWS>(pk, c.count, c.st, c.tw);
-  }
-
-  // peaks of item p: correlation of D[xi[p]] with Dref[ri[p]], c.count items
-  static cudaError_t corr_peak_idx(const Ctx& c, const float2* D, const float2* Dref, const int* xi, const int* ri,
-                                   int sign, float minr, float maxr, int norm_d, int norm_ref, float2* scratch,
-                                   double* partials) {
-    if (sign < 0) return corr_peak_idx_t<-1>(c, D, Dref, xi, ri, minr, maxr, norm_d, norm_ref, scratch, partials);
-    return corr_peak_idx_t<+1>(c, D, Dref, xi, ri, minr, maxr, norm_d, norm_ref, scratch, partials);
+    SPE_TRY((run_pass<N, AX_COLS>(cp, c.count, c.st, c.tw)));
+    Ctx z = c;
+    z.first = 0;
+    SPE_TRY(rows_peak(z, scratch1, part1));
+    return rows_peak(z, scratch2, part2);
   }
 
   // partials (rows of the column pass): sum_{A>=0} |FFT+(rho)|^2, sum_{A>=0} A^2
   static cudaError_t known_power(const Ctx& c, double* partials) {
-    SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, Gate{}, nullptr), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, Gate{}, nullptr), c.count, c.st, c.tw)));
     OpColsKnownPower kp;
     kp.first = c.first;
     kp.partials = partials;
     kp.T = c.T;
-    kp.A = c.A;
-    kp.n = N;
+    kp.A = amps(c);
     kp.ipp = c.ipp;
-    return launch_pass<N, AX_COLS>(kp, c.count, c.st, c.tw);
+    return run_pass<N, AX_COLS>(kp, c.count, c.st, c.tw);
   }
 
   // far-field loss per item into partials (column-pass tiles); with grad,
@@ -842,7 +796,6 @@ struct SizeImpl {
     } else {
       OpRowsSupportForward rf;
       rf.first = c.first;
-      rf.partials = nullptr;
       rf.rho = c.rho;
       rf.S = c.S;
       rf.T = c.T;
@@ -857,7 +810,6 @@ struct SizeImpl {
     } else {
       OpRowsGradOut go;
       go.first = c.first;
-      go.partials = nullptr;
       go.T = c.T;
       go.S = c.S;
       go.G = grad;
@@ -885,7 +837,6 @@ struct SizeImpl {
     SPE_TRY((launch_cols_loss<N, WL, LOSS, true>(c, eps, partials)));
     OpRowsGradAdam ad;
     ad.first = c.first;
-    ad.partials = nullptr;
     ad.T = c.T;
     ad.S = c.S;
     ad.rho = c.rho;
@@ -909,28 +860,37 @@ struct SizeImpl {
 
   static cudaError_t block_amplitudes(const float* A, float* At, int npatterns, cudaStream_t st) {
     if constexpr (Blocked<N>::ok) {
-      k_block_amplitudes<N><<<152 * 8, 256, 0, st>>>(A, At, npatterns);
+      k_block_amplitudes<N, false><<<152 * 8, 256, 0, st>>>(A, At, npatterns, 0.f, 0.f);
       return cudaGetLastError();
     } else {
       return cudaSuccess;
     }
   }
+  static cudaError_t band_table(const float* A, float* band, int n, int npatterns, float minr, float maxr,
+                                cudaStream_t st) {
+    if constexpr (Blocked<N>::ok) {
+      k_block_amplitudes<N, true><<<152 * 8, 256, 0, st>>>(A, band, npatterns, minr, maxr);
+      return cudaGetLastError();
+    } else {
+      return launch_band_table(A, band, n, npatterns, minr, maxr, st);
+    }
+  }
 
   static const SizeOps* table() {
     static const SizeOps t = {N,
-                              N / TileW<N>::rows,
-                              N / TileW<N>::cols,
+                              Blocked<N>::ok ? N / Blocked<N>::WR : N / TileW<N>::rows,
+                              Blocked<N>::ok ? N / Blocked<N>::BC : N / TileW<N>::cols,
                               TwiddleTable<N>::size(),
                               &fill_twiddles_n<N>,
                               &SizeImpl<N>::iterate,
                               &SizeImpl<N>::blur_magnitude,
                               &SizeImpl<N>::error_terms,
-                              &SizeImpl<N>::abs_spectrum,
-                              &SizeImpl<N>::corr_peak,
+                              &SizeImpl<N>::symmetry,
                               &SizeImpl<N>::fft2,
                               &SizeImpl<N>::ft_magnitude,
                               &SizeImpl<N>::abs_spectrum_items,
-                              &SizeImpl<N>::corr_peak_idx,
+                              &SizeImpl<N>::corr_peaks,
+                              &SizeImpl<N>::band_table,
                               &SizeImpl<N>::col_widths,
                               &SizeImpl<N>::row_widths,
                               DefaultTiles<N>::cols,
