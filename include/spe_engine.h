@@ -302,8 +302,9 @@ int spe_loss_grad(spe_engine* e, const void* density, const int32_t* support, in
  * reference counterpart).  spe_loss_grad_cols computes the loss into
  * loss_out (may be NULL) and the adjoint up to its column pass, leaving the
  * column-transformed gradient in `half` (device, complex64 count*n*n,
- * caller-owned, not the density; it also holds the forward transform, so no
- * engine scratch is used).  spe_grad_rows then runs the adjoint's last pass
+ * caller-owned, not the density; it also holds the forward transform).  Its
+ * order in memory is the engine's own, and parts that the support multiplies
+ * by zero may be left as they were.  spe_grad_rows then runs the adjoint's last pass
  * from `half` into grad_out times grad_scale (as in spe_loss_grad); grad_out
  * may be `half` itself.  `half` must be left unchanged between the calls.
  * The gradient equals spe_loss_grad's bit for bit.  density, support and
@@ -346,6 +347,15 @@ int spe_graph_destroy(spe_graph* g);
 int spe_adam_step(spe_engine* e, void* density, const int32_t* support, void* exp_avg, void* exp_avg_sq, int count,
                   int loss, float eps, float lr, float beta1, float beta2, float adam_eps, int step,
                   double* loss_out);
+
+/* `steps` steps of spe_adam_step from zero moments (steps 1 .. steps), the
+ * losses of step t at losses_out + (t - 1) * count.  exp_avg and exp_avg_sq
+ * are working memory: they need not be set before the call, and afterwards
+ * they hold the moments of the pixels inside the support (those of the others
+ * are 0 and need not be stored). */
+int spe_adam_run(spe_engine* e, void* density, const int32_t* support, void* exp_avg, void* exp_avg_sq, int count,
+                 int loss, float eps, float lr, float beta1, float beta2, float adam_eps, int steps,
+                 double* losses_out);
 
 /* Detector-image preprocessing (the spring_core.pattern module,
  * src/pattern/pattern.cpp, bindings src/wrapper.cpp:318-449), on the GPU.

@@ -89,6 +89,7 @@ SIGNATURES = {
     "spe_grad_rows": (_i, [_vp, _vp, _vp, _i, _vp, _vp]),
     "spe_set_amplitudes_batch": (_i, [_vp, _fp, _i, _i]),
     "spe_adam_step": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _f, _f, _f, _f, _f, _i, _vp]),
+    "spe_adam_run": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _f, _f, _f, _f, _f, _i, _vp]),
     "spe_get_rng_state": (_i, [_vp, C.c_char_p, _i, C.POINTER(_i)]),
     "spe_set_rng_state": (_i, [_vp, C.c_char_p]),
     "spe_pattern_resample": (_i, [_i, _vp, _vp, _i, _i, C.c_double, C.c_double, C.c_double, C.c_double, _i, _i,
@@ -413,6 +414,13 @@ class Engine:
         call("spe_adam_step", self.h, _vp(density_ptr), _vp(support_ptr), _vp(m_ptr), _vp(v_ptr), int(count),
              int(loss), float(eps), float(lr), float(beta1), float(beta2), float(adam_eps), int(step),
              _vp(loss_ptr or 0))
+
+    def adam_run(self, density_ptr, support_ptr, m_ptr, v_ptr, count, loss=1, eps=0.0, lr=1e-3, beta1=0.9,
+                 beta2=0.999, adam_eps=1e-8, steps=1, losses_ptr=0):
+        """`steps` fused Adam steps from zero moments (m, v: working memory)."""
+        call("spe_adam_run", self.h, _vp(density_ptr), _vp(support_ptr), _vp(m_ptr), _vp(v_ptr), int(count),
+             int(loss), float(eps), float(lr), float(beta1), float(beta2), float(adam_eps), int(steps),
+             _vp(losses_ptr or 0))
 
     def population_arrays(self, first, count):
         """Device addresses of slots [first, first+count): (density, support)."""

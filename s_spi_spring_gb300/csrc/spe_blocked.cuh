@@ -479,9 +479,9 @@ __global__ void __launch_bounds__(BlkPassCfg<N, AXIS, Op>::NT, BlkPassCfg<N, AXI
     fft_x<N, Lay, decltype(sign)::value, 1, 0>(v, xb, tw, c, j);
   });
   if constexpr (Op::NSUM + Op::NMAX > 0) {
-    double r[NRED];
+    float r[NRED];
     acc.values(r);
-    block_reduce_store<NT, Op::NSUM, Op::NMAX>(op.partials, r);
+    block_reduce_store<NT, Op::NSUM, Op::NMAX>(op.partials, blockIdx.x, r);
   }
   if constexpr (Op::PEAK) block_argmax_store<NT>(op.partials, acc.mx, acc.idx);
 }

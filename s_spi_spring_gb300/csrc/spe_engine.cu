@@ -47,74 +47,66 @@ constexpr int NRED = 4;
 // ---------------------------------------------------------------------------
 
 // Reductions over the tpi per-CTA partials of every individual, one block per
-// individual and job: kind 0 the sum of component k, 1 its maximum, 2 the
-// argmax over the (value, index) pairs.  The partials come through shared
-// memory and one thread folds them in tile order (a fixed order, the sums in
-// double); one thread per individual reading them from memory one after the
-// other took 10-18 us a job at 64 individuals of 512^2, and a call has up to
-// eight.
+// individual and job: kind 0 the sum of component k (in a fixed order), 1 its
+// maximum, 2 the argmax over the (value, index) pairs, ties to the lower
+// index.  One thread per individual, reading partials one after the other,
+// took 10-18 us a job at 64 individuals of 512^2, and a call has up to eight.
+__device__ __forceinline__ void reduce_step(int kind, double& m, double& idx, double v, double j) {
+  if (kind == 0) {
+    m += v;
+  } else if (kind == 1) {
+    m = fmax(m, v);
+  } else if (v > m || (v == m && j < idx)) {
+    m = v;
+    idx = j;
+  }
+}
 __global__ void k_reduce(const RedJobs jobs, double* out, int ostride) {
   const RedJob jb = jobs.job[blockIdx.y];
-  const int i = blockIdx.x;
-  constexpr int CH = 128;
-  __shared__ double a[CH], b[CH];
+  const int i = blockIdx.x, t = threadIdx.x;
   const double* p = jb.part + (size_t)i * jb.tpi * NRED + jb.k;
-  double m = 0.0, idx = 0.0;
-  for (int t0 = 0; t0 < jb.tpi; t0 += CH) {
-    const int nt = min(CH, jb.tpi - t0);
-    if ((int)threadIdx.x < nt) {
-      a[threadIdx.x] = p[(size_t)(t0 + threadIdx.x) * NRED];
-      if (jb.kind == 2) b[threadIdx.x] = p[(size_t)(t0 + threadIdx.x) * NRED + 1];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int t = 0;
-      if (t0 == 0) {
-        m = a[0];
-        idx = b[0];
-        t = 1;
-      }
-      if (jb.kind == 0) {
-        for (; t < nt; ++t) m += a[t];
-      } else if (jb.kind == 1) {
-        for (; t < nt; ++t) m = fmax(m, a[t]);
-      } else {
-        for (; t < nt; ++t)
-          if (a[t] > m || (a[t] == m && b[t] < idx)) {
-            m = a[t];
-            idx = b[t];
-          }
-      }
-    }
-    __syncthreads();
+  // (a thread without a partial repeats the first, or adds nothing)
+  double m = jb.kind == 0 ? 0.0 : p[0], idx = jb.kind == 2 ? p[1] : 0.0;
+  for (int k = t; k < jb.tpi; k += blockDim.x)
+    reduce_step(jb.kind, m, idx, p[(size_t)k * NRED], jb.kind == 2 ? p[(size_t)k * NRED + 1] : 0.0);
+  for (int off = 16; off > 0; off >>= 1) {
+    const double v = __shfl_down_sync(0xffffffffu, m, off), j = __shfl_down_sync(0xffffffffu, idx, off);
+    reduce_step(jb.kind, m, idx, v, j);
   }
-  if (threadIdx.x == 0) {
+  __shared__ double rm[4], ri[4];
+  if ((t & 31) == 0) {
+    rm[t >> 5] = m;
+    ri[t >> 5] = idx;
+  }
+  __syncthreads();
+  if (t == 0) {
+    for (int w = 1; w < 4; ++w) reduce_step(jb.kind, m, idx, rm[w], ri[w]);
     double* o = out + (size_t)i * ostride + jb.slot;
     o[0] = m;
     if (jb.kind == 2) o[1] = m > 0.0 ? idx : 0.0;  // no value above 0: the reference keeps index 0
   }
 }
 
-// support <- M >= max * thr (cut_support, gpu_context.cu:466-481)
-__global__ void k_threshold_rel(const float* __restrict__ M, int* __restrict__ S, const double* __restrict__ mx,
-                                int mstride, float thr, size_t npix, int first, int count) {
-  const size_t total = npix * (size_t)count;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int p = (int)(i / npix);
-    const size_t gi = (size_t)first * npix + i;
-    const float t = (float)mx[(size_t)p * mstride] * thr;
-    S[gi] = (M[gi] >= t) ? 1 : 0;
-  }
-}
-
-// support <- M >= thr_p (cut_support with an absolute threshold, gpu_context.cu:484-499)
-__global__ void k_threshold_abs(const float* __restrict__ M, int* __restrict__ S, const uint32_t* __restrict__ state,
-                                size_t npix, int first, int count) {
-  const size_t total = npix * (size_t)count;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int p = (int)(i / npix);
-    const size_t gi = (size_t)first * npix + i;
-    S[gi] = (M[gi] >= __uint_as_float(state[2 * p])) ? 1 : 0;
+// support <- M >= threshold of the individual (blockIdx.x): max * thr
+// (cut_support, gpu_context.cu:466-481) or, with `state`, the selected
+// magnitude itself (gpu_context.cu:484-499).  Four pixels a thread where the
+// arrays allow 16-byte accesses (an odd side's individuals do not): 44 -> 24 us
+// at 512^2 x 64.
+__global__ void k_threshold(const float* __restrict__ M, int* __restrict__ S, const double* __restrict__ mx,
+                            int mstride, float thr, const uint32_t* __restrict__ state, size_t npix, int first) {
+  const int p = blockIdx.x;
+  const float t = state ? __uint_as_float(state[2 * p]) : (float)mx[(size_t)p * mstride] * thr;
+  const size_t base = (size_t)(first + p) * npix, stride = (size_t)gridDim.y * blockDim.x;
+  const size_t i0 = blockIdx.y * (size_t)blockDim.x + threadIdx.x;
+  if (npix % 4 == 0) {
+    const float4* m4 = reinterpret_cast<const float4*>(M + base);
+    int4* s4 = reinterpret_cast<int4*>(S + base);
+    for (size_t i = i0; i < npix / 4; i += stride) {
+      const float4 m = m4[i];
+      s4[i] = make_int4(m.x >= t, m.y >= t, m.z >= t, m.w >= t);
+    }
+  } else {
+    for (size_t i = i0; i < npix; i += stride) S[base + i] = (M[base + i] >= t) ? 1 : 0;
   }
 }
 
@@ -257,6 +249,7 @@ spe::Ctx make_ctx(spe_engine* e, int first, int count) {
   c.band = e->band;
   c.sp = e->sp;
   c.odd = e->odd;
+  c.bad = e->sel_state;
   return c;
 }
 
@@ -433,10 +426,10 @@ int do_shrinkwrap(spe_engine* e, int first, int count, float sigma, bool absolut
   const float sft = (float)((double)((float)e->n / sigma) / M_PI);
   spe::Ctx c = make_ctx(e, first, count);
   CK(e->ops->blur_magnitude(c, sft), "shrink-wrap kernels");
-  const unsigned grid = 152 * 8;
+  const dim3 grid((unsigned)count, (unsigned)std::min<size_t>((e->npix + 1023) / 1024, 152));
   if (!absolute) {
     if ((rc = reduce(e, count, {{e->partials, e->ops->tiles_rows, 0, 1, 0}}, e->red, 16))) return rc;
-    spe::k_threshold_rel<<<grid, 256, 0, e->st>>>(e->M, e->S, e->red, 16, threshold, e->npix, first, count);
+    spe::k_threshold<<<grid, 256, 0, e->st>>>(e->M, e->S, e->red, 16, threshold, nullptr, e->npix, first);
     CK(cudaGetLastError(), "threshold launch");
     return SPE_OK;
   }
@@ -454,7 +447,7 @@ int do_shrinkwrap(spe_engine* e, int first, int count, float sigma, bool absolut
     spe::k_select_pick<<<(count + 127) / 128, 128, 0, e->st>>>(e->sel_state, e->sel_hist, count, shift);
     CK(cudaGetLastError(), "select pick");
   }
-  spe::k_threshold_abs<<<grid, 256, 0, e->st>>>(e->M, e->S, e->sel_state, e->npix, first, count);
+  spe::k_threshold<<<grid, 256, 0, e->st>>>(e->M, e->S, nullptr, 0, 0.f, e->sel_state, e->npix, first);
   CK(cudaGetLastError(), "threshold launch");
   return SPE_OK;
 }
@@ -1015,12 +1008,7 @@ static int loss_args(spe_engine* e, const void* density, const int32_t* support,
 
 // per-item losses from the column-pass partials into loss_out
 static int loss_sums(spe_engine* e, int count, double* loss_out) {
-  int rc = reduce(e, count, {{e->partials, e->ops->loss_tiles, 0, 0, 0}}, e->red, 16);
-  if (rc) return rc;
-  CK(cudaMemcpy2DAsync(loss_out, sizeof(double), e->red, 16 * sizeof(double), sizeof(double), count,
-                       cudaMemcpyDeviceToDevice, e->st),
-     "loss copy");
-  return SPE_OK;
+  return reduce(e, count, {{e->partials, e->ops->loss_tiles, 0, 0, 0}}, loss_out, 1);
 }
 
 int spe_loss_grad(spe_engine* e, const void* density, const int32_t* support, int count, int loss, float eps,
@@ -1132,36 +1120,79 @@ int spe_graph_destroy(spe_graph* g) {
   return SPE_OK;
 }
 
+// checks shared by the refinement entry points; 1 when there is nothing to do
+static int adam_args(spe_engine* e, const void* density, const int32_t* support, const void* m, const void* v,
+                     int count, int loss, float eps, float lr, float beta1, float beta2, float adam_eps, int step,
+                     int* rc) {
+  *rc = SPE_OK;
+  if (!e) return (*rc = fail(SPE_ERR_INVALID, "null engine")), 1;
+  if ((*rc = need_amp(e))) return 1;
+  if (count < 0 || step < 1) return (*rc = fail(SPE_ERR_INVALID, "negative count or step < 1")), 1;
+  if (loss != SPE_LOSS_AMPLITUDE && loss != SPE_LOSS_POISSON)
+    return (*rc = fail(SPE_ERR_INVALID, "unknown loss %d", loss)), 1;
+  if (!(eps >= 0.f) || !(lr >= 0.f) || !(beta1 >= 0.f && beta1 < 1.f) || !(beta2 >= 0.f && beta2 < 1.f) ||
+      !(adam_eps > 0.f))
+    return (*rc = fail(SPE_ERR_INVALID, "invalid optimiser parameters")), 1;
+  if (count == 0) return 1;
+  if (!density || !support || !m || !v) return (*rc = fail(SPE_ERR_INVALID, "null device array")), 1;
+  if (misaligned16(e, density) || misaligned16(e, support) || misaligned16(e, m) || misaligned16(e, v))
+    return (*rc = fail(SPE_ERR_INVALID, "density, support and moments must start on a 16-byte boundary")), 1;
+  return 0;
+}
+
+// torch.optim.Adam's bias corrections of step t, in double
+static spe::AdamStep adam_params(float lr, float beta1, float beta2, float adam_eps, int t) {
+  const double bc1 = 1.0 - std::pow((double)beta1, t), bc2 = 1.0 - std::pow((double)beta2, t);
+  return spe::AdamStep{beta1, beta2, (float)(lr / bc1), (float)(1.0 / std::sqrt(bc2)), adam_eps, 0, 0, 0, 0};
+}
+
 int spe_adam_step(spe_engine* e, void* density, const int32_t* support, void* exp_avg, void* exp_avg_sq, int count,
                   int loss, float eps, float lr, float beta1, float beta2, float adam_eps, int step,
                   double* loss_out) {
-  if (!e) return fail(SPE_ERR_INVALID, "null engine");
-  int rc = need_amp(e);
-  if (rc) return rc;
-  if (count < 0 || step < 1) return fail(SPE_ERR_INVALID, "negative count or step < 1");
-  if (loss != SPE_LOSS_AMPLITUDE && loss != SPE_LOSS_POISSON) return fail(SPE_ERR_INVALID, "unknown loss %d", loss);
-  if (!(eps >= 0.f) || !(lr >= 0.f) || !(beta1 >= 0.f && beta1 < 1.f) || !(beta2 >= 0.f && beta2 < 1.f) ||
-      !(adam_eps > 0.f))
-    return fail(SPE_ERR_INVALID, "invalid optimiser parameters");
-  if (count == 0) return SPE_OK;
-  if (!density || !support || !exp_avg || !exp_avg_sq) return fail(SPE_ERR_INVALID, "null device array");
-  if (misaligned16(e, density) || misaligned16(e, support) || misaligned16(e, exp_avg) || misaligned16(e, exp_avg_sq))
-    return fail(SPE_ERR_INVALID, "density, support and moments must start on a 16-byte boundary");
+  int rc;
+  if (adam_args(e, density, support, exp_avg, exp_avg_sq, count, loss, eps, lr, beta1, beta2, adam_eps, step, &rc))
+    return rc;
   if ((rc = spe_reserve(e, count))) return rc;
   CK(cudaSetDevice(e->dev), "cudaSetDevice");
-  // torch.optim.Adam's bias corrections, in double
-  const double bc1 = 1.0 - std::pow((double)beta1, step), bc2 = 1.0 - std::pow((double)beta2, step);
   spe::Ctx c = make_ctx(e, 0, count);
   c.rho = static_cast<float2*>(density);
   c.S = const_cast<int*>(support);
   CK(e->ops->adam_step(c, loss, eps, e->partials, static_cast<float2*>(exp_avg), static_cast<float2*>(exp_avg_sq),
-                       beta1, beta2, (float)(lr / bc1), (float)(1.0 / std::sqrt(bc2)), adam_eps),
+                       adam_params(lr, beta1, beta2, adam_eps, step)),
      "refinement kernels");
-  if (loss_out) {
-    if ((rc = reduce(e, count, {{e->partials, e->ops->loss_tiles, 0, 0, 0}}, e->red, 16))) return rc;
-    CK(cudaMemcpy2DAsync(loss_out, sizeof(double), e->red, 16 * sizeof(double), sizeof(double), count,
-                         cudaMemcpyDeviceToDevice, e->st),
-       "loss copy");
+  return loss_out ? loss_sums(e, count, loss_out) : SPE_OK;
+}
+
+int spe_adam_run(spe_engine* e, void* density, const int32_t* support, void* exp_avg, void* exp_avg_sq, int count,
+                 int loss, float eps, float lr, float beta1, float beta2, float adam_eps, int steps,
+                 double* losses_out) {
+  int rc;
+  if (steps < 0) return fail(SPE_ERR_INVALID, "negative step count");
+  if (adam_args(e, density, support, exp_avg, exp_avg_sq, count, loss, eps, lr, beta1, beta2, adam_eps, 1, &rc))
+    return rc;
+  if ((rc = spe_reserve(e, count))) return rc;
+  CK(cudaSetDevice(e->dev), "cudaSetDevice");
+  spe::Ctx c = make_ctx(e, 0, count);
+  c.rho = static_cast<float2*>(density);
+  c.S = const_cast<int*>(support);
+  const bool inside = e->ops->blocked_cols != 0;
+  if (!inside) {
+    const size_t bytes = (size_t)count * e->npix * sizeof(float2);
+    CK(cudaMemsetAsync(exp_avg, 0, bytes, e->st), "moments");
+    CK(cudaMemsetAsync(exp_avg_sq, 0, bytes, e->st), "moments");
+  }
+  for (int t = 1; t <= steps; ++t) {
+    spe::AdamStep a = adam_params(lr, beta1, beta2, adam_eps, t);
+    if (inside) {
+      a.prepared = t > 1;
+      a.fresh = t == 1;
+      a.inside = 1;
+      a.next = t < steps;
+    }
+    CK(e->ops->adam_step(c, loss, eps, e->partials, static_cast<float2*>(exp_avg), static_cast<float2*>(exp_avg_sq),
+                         a),
+       "refinement kernels");
+    if (losses_out && (rc = loss_sums(e, count, losses_out + (size_t)(t - 1) * count))) return rc;
   }
   return SPE_OK;
 }

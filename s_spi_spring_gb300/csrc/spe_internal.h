@@ -68,7 +68,18 @@ struct Ctx {
   const float* At;
   const float* band;  // weights of the correlation ops (SizeOps::band_table)
   void* sp;
-  unsigned char* odd;
+  unsigned char* odd;  // (the loss passes: row tiles with support)
+  unsigned* bad;       // per individual: a gradient that is not finite
+};
+
+// One Adam step (SizeOps::adam_step).  On sides with blocked passes a run of
+// steps may leave out what it knows: prepared (Ctx::T holds the forward row
+// pass: the step before had `next`), fresh (the moments are 0 and not read),
+// inside (the moments outside the support are 0 and stay 0), next (leave the
+// updated densities' forward row pass in Ctx::T).
+struct AdamStep {
+  float b1, b2, step_size, inv_sqrt_bc2, eps;
+  int prepared, fresh, inside, next;
 };
 
 // Tensor maps of the TMA row pass (spe_tma_maps.cu): row_maps_bytes() of
@@ -112,11 +123,11 @@ struct SizeOps {
   cudaError_t (*iterate)(const Ctx&, int upd, int iterations, float beta, Gate g, int wc, int wr);
   // blurred modulus into M, per-CTA max into partials
   cudaError_t (*blur_magnitude)(const Ctx&, float sigma_ft);
-  // error terms: stage 1 -> partials (modulesum), stage 2 -> partials+P1
-  // (err, norm, max), stage 3 -> partials+P2 (err_r, norm_r)
+  // error terms: stage 1 -> p1 (modulesum), stage 2 -> p2 (err, norm, max),
+  // stage 3 -> p3 (err_r, norm_r); leaves |rho|'s row transforms in Ctx::T2
   cudaError_t (*error_terms)(const Ctx&, Gate g, double* p1, double* p2, double* p3);
-  // the two peaks of the symmetry metric (get_symmetry), through Ctx::T with
-  // the weights Ctx::band: column-pass partials (the sum whose square is the
+  // the two peaks of the symmetry metric (get_symmetry), after error_terms and
+  // from what it left in Ctx::T2, with the weights Ctx::band: column-pass partials (the sum whose square is the
   // first peak) and row-pass partials (value, index of the second)
   cudaError_t (*symmetry)(const Ctx&, double* psum, double* ppeak);
   // generic transforms over Ctx::count items starting at the given arrays
@@ -153,8 +164,8 @@ struct SizeOps {
   int loss_tiles;  // loss partials per item
   // loss at the current densities into partials, then one Adam step in
   // place with moments m, v (see OpRowsGradAdam)
-  cudaError_t (*adam_step)(const Ctx&, int loss, float eps, double* partials, float2* m, float2* v, float b1,
-                           float b2, float step_size, float inv_sqrt_bc2, float adam_eps);
+  cudaError_t (*adam_step)(const Ctx&, int loss, float eps, double* partials, float2* m, float2* v,
+                           const AdamStep& a);
   // blocked-scratch kernels of the iteration (0 / null: none at this side):
   // the tile codes of the column and the row pass, the bytes of packed
   // support per individual, and the amplitudes' reordering

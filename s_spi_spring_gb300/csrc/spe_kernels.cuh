@@ -45,6 +45,12 @@ using GateK = Gate;  // hi, lo: float thresholds; chi/shi, clo/slo: their cos an
 
 __device__ __forceinline__ bool phase_out(float2 v, const GateK& g) {
   const float ay = fabsf(v.y);
+  // zeros (most of a density outside its object): arg = +-0 for x = +0, +-pi
+  // for x = -0, without the arc tangent's slow path
+  if (v.x == 0.f && ay == 0.f) {
+    const float ph = copysignf(signbit(v.x) ? 3.14159265358979f : 0.f, v.y);
+    return (ph > g.hi) || (ph < -g.lo);
+  }
   const bool up = !(v.y < 0.f);  // y = +0 belongs to the upper half plane (atan2(+0, x) >= 0)
   const float c = up ? g.chi : g.clo;
   const float s = up ? g.shi : g.slo;
@@ -52,10 +58,7 @@ __device__ __forceinline__ bool phase_out(float2 v, const GateK& g) {
   const float band = 4e-6f * (fabsf(v.x) + ay);
   if (D > band) return true;
   if (D < -band) return false;
-  // zeros (most of a density outside its object) without the arc tangent's
-  // slow path: arg = +-0 for x = +0, +-pi for x = -0
-  const float ph = v.x == 0.f && ay == 0.f ? copysignf(signbit(v.x) ? 3.14159265358979f : 0.f, v.y)
-                                           : atan2f(v.y, v.x);
+  const float ph = atan2f(v.y, v.x);
   return (ph > g.hi) || (ph < -g.lo);
 }
 
@@ -95,38 +98,58 @@ __device__ __forceinline__ float cabsf2(float2 v) {
 }
 
 // ---------------------------------------------------------------------------
-// block reduction of NRED values per CTA into partials[blockIdx.x*NRED + k]
+// block reduction of NRED values per CTA into partials[slot*NRED + k]
 // (k < NSUM: sums, k >= NSUM: maxima)
+//
+// The threads' float sums are added as pairs of floats (high part and rounding
+// error, Knuth's two-sum: about 48 bits), in full-rate instructions; a double
+// add takes the SM 16 cycles a warp, and five per value and warp of a shuffle
+// tree were a third of the loss's column pass (104 us at 512^2 x 64, 70 of
+// them the pass itself) and 40% of the error metrics'.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void add_pair(float2& a, float2 b) {
+  const float s = __fadd_rn(a.x, b.x);
+  const float t = __fsub_rn(s, a.x);
+  const float e = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, t)), __fsub_rn(b.x, t));
+  a = make_float2(s, __fadd_rn(__fadd_rn(a.y, b.y), e));
+}
 template <int NT, int NSUM, int NMAX>
-__device__ __forceinline__ void block_reduce_store(double* __restrict__ partials, const double (&v)[NRED]) {
+__device__ __forceinline__ void block_reduce_store(double* __restrict__ partials, size_t slot, const float (&v)[NRED]) {
   static_assert(NSUM + NMAX <= NRED, "too many reduction values");
   constexpr int NW = NT / 32;
-  __shared__ double red[NRED][NW > 0 ? NW : 1];
-  double x[NRED];
+  __shared__ float2 red[NRED][NW > 0 ? NW : 1];
+  float2 x[NRED];
 #pragma unroll
-  for (int k = 0; k < NRED; ++k) x[k] = v[k];
+  for (int k = 0; k < NRED; ++k) x[k] = make_float2(v[k], 0.f);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
     for (int k = 0; k < NSUM + NMAX; ++k) {
-      const double o = __shfl_down_sync(0xffffffffu, x[k], off);
-      x[k] = (k < NSUM) ? x[k] + o : fmax(x[k], o);
+      float2 o;
+      o.x = __shfl_down_sync(0xffffffffu, x[k].x, off);
+      if (k < NSUM) {
+        o.y = __shfl_down_sync(0xffffffffu, x[k].y, off);
+        add_pair(x[k], o);
+      } else {
+        x[k].x = fmaxf(x[k].x, o.x);
+      }
     }
   }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) {
 #pragma unroll
-    for (int k = 0; k < NRED; ++k) red[k][wid] = x[k];
+    for (int k = 0; k < NSUM + NMAX; ++k) red[k][wid] = x[k];
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < NSUM + NMAX; ++k) {
-      double a = red[k][0];
-      for (int w = 1; w < NW; ++w) a = (k < NSUM) ? a + red[k][w] : fmax(a, red[k][w]);
-      partials[(size_t)blockIdx.x * NRED + k] = a;
+  if ((int)threadIdx.x < NSUM + NMAX) {
+    const int k = threadIdx.x;
+    float2 a = red[k][0];
+    for (int w = 1; w < NW; ++w) {
+      if (k < NSUM) add_pair(a, red[k][w]);
+      else a.x = fmaxf(a.x, red[k][w].x);
     }
+    // (the error of an overflowed sum is not a number)
+    partials[slot * NRED + k] = isfinite(a.x) ? (double)a.x + (double)a.y : (double)a.x;
   }
 }
 
@@ -222,8 +245,16 @@ __device__ __forceinline__ void pass_elements(const Op& op, const PxF& px, typen
   float2 v[E];
   if constexpr (Op::PAIR) {
     float2 u[E];
+    if constexpr (Op::FETCH) {
+      typename Op::Raw r[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) op.load_pair(px(e), v[e], u[e]);
+      for (int e = 0; e < E; ++e) r[e] = op.fetch(px(e));
+#pragma unroll
+      for (int e = 0; e < E; ++e) op.form_pair(r[e], v[e], u[e], acc);
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) op.load_pair(px(e), v[e], u[e], acc);
+    }
     fft(v, std::integral_constant<int, Op::FFT1>());
 #pragma unroll
     for (int e = 0; e < E; ++e) op.store_pair(v[e], px(e), 0);
@@ -231,8 +262,16 @@ __device__ __forceinline__ void pass_elements(const Op& op, const PxF& px, typen
 #pragma unroll
     for (int e = 0; e < E; ++e) op.store_pair(u[e], px(e), 1);
   } else {
+    if constexpr (Op::FETCH) {
+      typename Op::Raw r[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) v[e] = op.load(px(e), acc);
+      for (int e = 0; e < E; ++e) r[e] = op.fetch(px(e));
+#pragma unroll
+      for (int e = 0; e < E; ++e) v[e] = op.form(r[e], acc);
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) v[e] = op.load(px(e), acc);
+    }
     if constexpr (Op::FFT1 != 0) fft(v, std::integral_constant<int, Op::FFT1>());
     if constexpr (Op::FFT2 != 0) {
 #pragma unroll
@@ -279,17 +318,17 @@ __global__ void __launch_bounds__(PassCfg<N, AXIS>::NT, PassCfg<N, AXIS>::MINB)
     fft_reg<N, typename C::Lay, decltype(sign)::value>(v, buf, tw, c, j);
   });
   if constexpr (Op::NSUM + Op::NMAX > 0) {
-    double r[NRED];
+    float r[NRED];
     acc.values(r);
-    block_reduce_store<NT, Op::NSUM, Op::NMAX>(op.partials, r);
+    block_reduce_store<NT, Op::NSUM, Op::NMAX>(op.partials, blockIdx.x, r);
   }
   if constexpr (Op::PEAK) block_argmax_store<NT>(op.partials, acc.mx, acc.idx);
 }
 
 struct NoAcc {
-  __device__ void values(double (&v)[NRED]) const {
+  __device__ void values(float (&v)[NRED]) const {
 #pragma unroll
-    for (int k = 0; k < NRED; ++k) v[k] = 0.0;
+    for (int k = 0; k < NRED; ++k) v[k] = 0.f;
   }
 };
 
@@ -300,6 +339,10 @@ struct OpBase {
   static constexpr int NSUM = 0, NMAX = 0, PEAK = 0;
   static constexpr bool AMP = false;   // reads amp(): A, one n x n array per pattern
   static constexpr bool PAIR = false;  // two arrays through the pass (load_pair, store_pair)
+  // load in two steps, fetch and form: for a load that computes with branches
+  // (roots, the phase gate), across which a thread's memory reads are not
+  // reordered -- all are issued before the first value is formed
+  static constexpr bool FETCH = false;
   int first = 0;
   double* partials = nullptr;
   const float* A = nullptr;
@@ -318,45 +361,71 @@ struct OpKeep : OpBase {
   }
 };
 
-// Source transforms of the first row pass: rho itself, rho gated by the
-// support (apply_support_er on a copy), its modulus, or its modulus with the
-// complex sum of rho in the partials.
-enum { SRC_RHO = 0, SRC_GATED = 1, SRC_ABS = 2, SRC_ABS_SUM = 3 };
+// Source transforms of the first row pass: rho itself, or its modulus with
+// the complex sum of rho in the partials.
+enum { SRC_RHO = 0, SRC_ABS_SUM = 1 };
 
-// row pass: load rho (optionally gated / modulus) -> FFT+ (x) -> T.
-// SRC_GATED accumulates sum |rho_s| (get_module_sum, gpu_context.cu:219-246).
+// row pass: load rho (or its modulus) -> FFT+ (x) -> T
 template <int SRC>
 struct OpRowsForward : OpKeep {
   static constexpr int FFT1 = +1, FFT2 = 0;
-  static constexpr int NSUM = SRC == SRC_GATED ? 1 : (SRC == SRC_ABS_SUM ? 2 : 0), NMAX = 0;
+  static constexpr int NSUM = SRC == SRC_ABS_SUM ? 2 : 0, NMAX = 0;
   const float2* rho;
-  const int* S;
   float2* T;
-  GateK g;
   struct Acc {
     float s = 0.f, t = 0.f;
-    __device__ void values(double (&v)[NRED]) const {
+    __device__ void values(float (&v)[NRED]) const {
       v[0] = s;
       v[1] = t;
-      v[2] = v[3] = 0.0;
+      v[2] = v[3] = 0.f;
     }
   };
-  __device__ float2 load(const Px& q, Acc& acc) const {
-    float2 v = rho[q.gi];
-    if (SRC == SRC_GATED) {
-      const float t = phase_out(v, g) ? 0.f : (float)S[q.gi];
-      v = make_float2(v.x * t, v.y * t);
-      acc.s += cabsf2(v);
-    } else if (SRC == SRC_ABS || SRC == SRC_ABS_SUM) {
-      if (SRC == SRC_ABS_SUM) {
-        acc.s += v.x;
-        acc.t += v.y;
-      }
+  static constexpr bool FETCH = SRC == SRC_ABS_SUM;
+  using Raw = float2;
+  __device__ float2 fetch(const Px& q) const { return rho[q.gi]; }
+  __device__ float2 form(float2 v, Acc& acc) const {
+    if (SRC == SRC_ABS_SUM) {
+      acc.s += v.x;
+      acc.t += v.y;
       v = make_float2(cabsf2(v), 0.f);
     }
     return v;
   }
+  __device__ float2 load(const Px& q, Acc& acc) const { return form(fetch(q), acc); }
   __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
+};
+
+// row pass of the evaluation: rho gated by the support (apply_support_er on a
+// copy) -> FFT+ (x) -> T, its summed modulus in the partials (get_module_sum,
+// gpu_context.cu:219-246), and |rho| -> FFT+ (x) -> T2, from one read of rho
+struct OpRowsEvaluate : OpBase {
+  static constexpr int FFT1 = +1, FFT2 = 0, NSUM = 1;
+  static constexpr bool PAIR = true;
+  const float2* rho;
+  const int* S;
+  float2 *T, *T2;
+  GateK g;
+  struct Acc {
+    float s = 0.f;
+    __device__ void values(float (&v)[NRED]) const {
+      v[0] = s;
+      v[1] = v[2] = v[3] = 0.f;
+    }
+  };
+  static constexpr bool FETCH = true;
+  struct Raw {
+    float2 v;
+    int s;
+  };
+  __device__ Raw fetch(const Px& q) const { return {rho[q.gi], S[q.gi]}; }
+  __device__ void form_pair(const Raw& r, float2& v, float2& u, Acc& acc) const {
+    u = make_float2(cabsf2(r.v), 0.f);
+    const float t = r.s == 0 || phase_out(r.v, g) ? 0.f : (float)r.s;
+    v = make_float2(r.v.x * t, r.v.y * t);
+    acc.s += r.s == 0 || r.s == 1 ? u.x * t : cabsf2(v);
+  }
+  __device__ void load_pair(const Px& q, float2& v, float2& u, Acc& acc) const { form_pair(fetch(q), v, u, acc); }
+  __device__ void store_pair(float2 v, const Px& q, int second) const { (second ? T2 : T)[q.ti] = v; }
 };
 
 // column pass: T -> FFT+ (y) -> P_M -> FFT- (y) -> T
@@ -471,9 +540,9 @@ struct OpRowsMagnitude : OpKeep {
   float* M;
   struct Acc {
     float mx = 0.f;
-    __device__ void values(double (&v)[NRED]) const {
+    __device__ void values(float (&v)[NRED]) const {
       v[0] = mx;
-      v[1] = v[2] = v[3] = 0.0;
+      v[1] = v[2] = v[3] = 0.f;
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
@@ -495,11 +564,11 @@ struct OpColsError : OpBase {
   float2* T;
   struct Acc {
     float e = 0.f, a2 = 0.f, mx = 0.f;
-    __device__ void values(double (&v)[NRED]) const {
+    __device__ void values(float (&v)[NRED]) const {
       v[0] = e;
       v[1] = a2;
       v[2] = mx;
-      v[3] = 0.0;
+      v[3] = 0.f;
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
@@ -524,10 +593,10 @@ struct OpRowsRealError : OpKeep {
   float scale;
   struct Acc {
     float err = 0.f, nrm = 0.f;
-    __device__ void values(double (&v)[NRED]) const {
+    __device__ void values(float (&v)[NRED]) const {
       v[0] = err;
       v[1] = nrm;
-      v[2] = v[3] = 0.0;
+      v[2] = v[3] = 0.f;
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
@@ -615,9 +684,9 @@ struct OpColsSymmetry : OpBase {
   float2* T;
   struct Acc {
     float s = 0.f;
-    __device__ void values(double (&v)[NRED]) const {
+    __device__ void values(float (&v)[NRED]) const {
       v[0] = s;
-      v[1] = v[2] = v[3] = 0.0;
+      v[1] = v[2] = v[3] = 0.f;
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
@@ -638,8 +707,8 @@ struct OpRowsPeak : OpKeep {
   struct Acc {
     float mx = 0.f;
     int idx = 0x7fffffff;
-    __device__ void values(double (&v)[NRED]) const {
-      v[0] = v[1] = v[2] = v[3] = 0.0;
+    __device__ void values(float (&v)[NRED]) const {
+      v[0] = v[1] = v[2] = v[3] = 0.f;
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
@@ -663,10 +732,10 @@ struct OpColsKnownPower : OpKeep {
   const float2* T;
   struct Acc {
     float f2 = 0.f, a2 = 0.f;
-    __device__ void values(double (&v)[NRED]) const {
+    __device__ void values(float (&v)[NRED]) const {
       v[0] = f2;
       v[1] = a2;
-      v[2] = v[3] = 0.0;
+      v[2] = v[3] = 0.f;
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
@@ -736,9 +805,9 @@ struct OpColsLoss : OpBase {
   float eps;
   struct Acc {
     float l = 0.f;
-    __device__ void values(double (&v)[NRED]) const {
+    __device__ void values(float (&v)[NRED]) const {
       v[0] = l;
-      v[1] = v[2] = v[3] = 0.0;
+      v[1] = v[2] = v[3] = 0.f;
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
@@ -853,7 +922,7 @@ struct OpColsCrossPower : OpBase {
   size_t npix;
   int norm_d, norm_ref;  // apply normalize_ft_shift
   using Acc = NoAcc;
-  __device__ void load_pair(const Px& q, float2& c1, float2& c2) const {
+  __device__ void load_pair(const Px& q, float2& c1, float2& c2, Acc&) const {
     const size_t pix = q.ti - (size_t)q.p * npix;
     float2 d = D[(size_t)__ldg(xi + q.p) * npix + pix];
     float2 r = Dref[(size_t)__ldg(ri + q.p) * npix + pix];

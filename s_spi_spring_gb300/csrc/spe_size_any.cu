@@ -422,7 +422,8 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, BIG ? 2 : 
         int c, l;
         const Px q = px(i, c, l);
         float2 v1, v2;
-        op.load_pair(q, v1, v2);
+        typename Op::Acc once;
+        op.load_pair(q, v1, v2, second ? once : acc);
         cur[c * LS + l] = second ? v2 : v1;
       }
       __syncthreads();
@@ -458,9 +459,9 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, BIG ? 2 : 
     }
   }
   if constexpr (Op::NSUM + Op::NMAX > 0) {
-    double r[NRED];
+    float r[NRED];
     acc.values(r);
-    block_reduce_store<NT, Op::NSUM, Op::NMAX>(op.partials, r);
+    block_reduce_store<NT, Op::NSUM, Op::NMAX>(op.partials, blockIdx.x, r);
   }
   if constexpr (Op::PEAK) block_argmax_store<NT>(op.partials, acc.mx, acc.idx);
 }
@@ -558,14 +559,12 @@ struct SizeAny {
   static float scale(int n) { return (float)(1.0 / ((double)n * (double)n)); }
 
   template <int SRC>
-  static OpRowsForward<SRC> rows_forward(const Ctx& c, const float2* src, float2* dst, Gate g, double* partials) {
+  static OpRowsForward<SRC> rows_forward(const Ctx& c, const float2* src, float2* dst, double* partials) {
     OpRowsForward<SRC> op;
     op.first = c.first;
     op.partials = partials;
     op.rho = src;
-    op.S = c.S;
     op.T = dst;
-    op.g = g;
     return op;
   }
 
@@ -581,7 +580,7 @@ struct SizeAny {
   template <int UPD>
   static cudaError_t iterate_t(const Ctx& c, int iters, float beta, Gate g) {
     const AnyPlan& pl = plan_of(c.n);
-    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, g, nullptr), pl, c.count, c.st, c.tw)));
+    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, nullptr), pl, c.count, c.st, c.tw)));
     const OpColsProject proj = cols_project(c);
     OpRowsIterate<UPD> it;
     it.first = c.first;
@@ -622,8 +621,7 @@ struct SizeAny {
 
   static cudaError_t blur_magnitude(const Ctx& c, float sigma_ft) {
     const AnyPlan& pl = plan_of(c.n);
-    const Gate g{};
-    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, g, nullptr), pl, c.count, c.st, c.tw)));
+    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, nullptr), pl, c.count, c.st, c.tw)));
     SPE_TRY((launch_any<AX_COLS>(cols_project(c), pl, c.count, c.st, c.tw)));
     OpRowsModulusForward mf;
     mf.first = c.first;
@@ -646,7 +644,15 @@ struct SizeAny {
 
   static cudaError_t error_terms(const Ctx& c, Gate g, double* p1, double* p2, double* p3) {
     const AnyPlan& pl = plan_of(c.n);
-    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_GATED>(c, c.rho, c.T, g, p1), pl, c.count, c.st, c.tw)));
+    OpRowsEvaluate ev;
+    ev.first = c.first;
+    ev.partials = p1;
+    ev.rho = c.rho;
+    ev.S = c.S;
+    ev.T = c.T;
+    ev.T2 = c.T2;
+    ev.g = g;
+    SPE_TRY((launch_any<AX_ROWS>(ev, pl, c.count, c.st, c.tw)));
     OpColsError ce;
     ce.first = c.first;
     ce.partials = p2;
@@ -665,15 +671,14 @@ struct SizeAny {
 
   static cudaError_t symmetry(const Ctx& c, double* psum, double* ppeak) {
     const AnyPlan& pl = plan_of(c.n);
-    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_ABS>(c, c.rho, c.T, Gate{}, nullptr), pl, c.count, c.st, c.tw)));
     OpColsSymmetry sy;
     sy.first = c.first;
     sy.partials = psum;
-    sy.T = c.T;
+    sy.T = c.T2;
     sy.A = c.band;
     sy.ipp = c.ipp;
     SPE_TRY((launch_any<AX_COLS>(sy, pl, c.count, c.st, c.tw)));
-    return rows_peak(c, pl, c.T, ppeak);
+    return rows_peak(c, pl, c.T2, ppeak);
   }
 
   static cudaError_t rows_peak(const Ctx& c, const AnyPlan& pl, const float2* T, double* partials) {
@@ -691,7 +696,7 @@ struct SizeAny {
     if (sign > 0) {
       Ctx z = c;
       z.first = 0;
-      SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(z, data, data, Gate{}, nullptr), pl, c.count, c.st, c.tw)));
+      SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(z, data, data, nullptr), pl, c.count, c.st, c.tw)));
       OpColsTransform<+1> ct;
       ct.first = 0;
       ct.src = data;
@@ -715,7 +720,7 @@ struct SizeAny {
     const AnyPlan& pl = plan_of(c.n);
     Ctx z = c;
     z.first = 0;
-    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(z, src, tmp, Gate{}, nullptr), pl, c.count, c.st, c.tw)));
+    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(z, src, tmp, nullptr), pl, c.count, c.st, c.tw)));
     OpColsMagnitude cm;
     cm.first = 0;
     cm.src = tmp;
@@ -727,7 +732,7 @@ struct SizeAny {
     const AnyPlan& pl = plan_of(c.n);
     Ctx z = c;
     z.first = 0;
-    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_ABS_SUM>(z, src, dst, Gate{}, psum), pl, c.count, c.st, c.tw)));
+    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_ABS_SUM>(z, src, dst, psum), pl, c.count, c.st, c.tw)));
     OpColsTransform<+1> ct;
     ct.src = dst;
     ct.dst = dst;
@@ -758,7 +763,7 @@ struct SizeAny {
 
   static cudaError_t known_power(const Ctx& c, double* partials) {
     const AnyPlan& pl = plan_of(c.n);
-    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, Gate{}, nullptr), pl, c.count, c.st, c.tw)));
+    SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, nullptr), pl, c.count, c.st, c.tw)));
     OpColsKnownPower kp;
     kp.first = c.first;
     kp.partials = partials;
@@ -818,8 +823,8 @@ struct SizeAny {
   }
 
   template <int LOSS>
-  static cudaError_t adam_step_t(const Ctx& c, float eps, double* partials, float2* m, float2* v, float b1, float b2,
-                                 float step_size, float inv_sqrt_bc2, float adam_eps) {
+  static cudaError_t adam_step_t(const Ctx& c, float eps, double* partials, float2* m, float2* v,
+                                 const AdamStep& a) {
     const AnyPlan& pl = plan_of(c.n);
     OpRowsSupportForward rf;
     rf.first = c.first;
@@ -842,15 +847,14 @@ struct SizeAny {
     ad.rho = c.rho;
     ad.m = m;
     ad.v = v;
-    ad.ap = {b1, b2, step_size, inv_sqrt_bc2, adam_eps};
+    ad.ap = {a.b1, a.b2, a.step_size, a.inv_sqrt_bc2, a.eps};
     return launch_any<AX_ROWS>(ad, pl, c.count, c.st, c.tw);
   }
 
-  static cudaError_t adam_step(const Ctx& c, int loss, float eps, double* partials, float2* m, float2* v, float b1,
-                               float b2, float step_size, float inv_sqrt_bc2, float adam_eps) {
-    return loss == LOSS_POISSON
-               ? adam_step_t<LOSS_POISSON>(c, eps, partials, m, v, b1, b2, step_size, inv_sqrt_bc2, adam_eps)
-               : adam_step_t<LOSS_AMPLITUDE>(c, eps, partials, m, v, b1, b2, step_size, inv_sqrt_bc2, adam_eps);
+  static cudaError_t adam_step(const Ctx& c, int loss, float eps, double* partials, float2* m, float2* v,
+                               const AdamStep& a) {
+    return loss == LOSS_POISSON ? adam_step_t<LOSS_POISSON>(c, eps, partials, m, v, a)
+                                : adam_step_t<LOSS_AMPLITUDE>(c, eps, partials, m, v, a);
   }
 };
 

@@ -7,6 +7,7 @@
 #include "spe_kernels.cuh"
 #include "spe_pipe.cuh"
 #include "spe_blocked.cuh"
+#include "spe_support.cuh"
 #include "spe_pairs.cuh"
 #include "spe_tma.cuh"
 
@@ -218,35 +219,6 @@ inline int share(int slots, int div) {
   return s < 1 ? 1 : s;
 }
 
-// persistent staged row passes of the loss (k_rows_io): sides from 256, the
-// default row-tile width
-template <int N>
-constexpr int rowsio_w() {
-  return DefaultTiles<N>::rows;
-}
-template <int N>
-constexpr bool rowsio_ok() {
-  constexpr int W = rowsio_w<N>();
-  return N >= 256 && N % W == 0 && RowsIoCfg<N, W>::NT % 32 == 0 && RowsIoCfg<N, W>::NT <= 1024 &&
-         RowsIoCfg<N, W>::SMEM <= kMaxSmem;
-}
-template <int N, int MODE>
-cudaError_t launch_rows_io(const Ctx& c, const float2* src, float2* dst, const float* scale) {
-  constexpr int W = rowsio_w<N>();
-  using P = RowsIoCfg<N, W>;
-  auto kern = k_rows_io<N, W, MODE>;
-  static std::atomic<unsigned long long> configured{0ull};
-  static std::atomic<int> resident[64] = {};
-  cudaError_t e = configure(kern, P::SMEM, configured);
-  if (e != cudaSuccess || c.count <= 0) return e;
-  const int tiles = c.count * (N / W);
-  const int slots = resident_ctas(kern, P::NT, P::SMEM, resident);
-  const int grid = tiles < slots ? tiles : slots;
-  return launch_pdl(kern, grid, P::NT, P::SMEM, c.st, src, static_cast<const int*>(c.S), dst, scale, c.first,
-                    c.count, c.tw);
-}
-
-
 template <int N, int W, class Lay = LayCol<N, W>>
 cudaError_t launch_cols_project(const Ctx& c) {
   using P = ColCfg<N, W, Lay>;
@@ -425,18 +397,62 @@ cudaError_t launch_cols_warp(const Ctx& c) {
   return launch_pdl(kern, grid, P::NT, P::SMEM, c.st, c.T, c.A, c.ipp, c.first, c.count, c.tw);
 }
 
-template <int N, int W, int LOSS, bool GRAD>
-cudaError_t launch_cols_loss(const Ctx& c, float eps, double* partials) {
-  using P = ColCfg<N, W>;
-  auto kern = k_cols_loss<N, W, LOSS, GRAD>;
+// ---- the loss passes (spe_support.cuh): one row tile or BC columns per CTA
+template <class K, class... Args>
+cudaError_t launch_loss(K kern, size_t smem, std::atomic<unsigned long long>& configured, int grid, int threads,
+                        cudaStream_t st, Args... args) {
+  cudaError_t e = configure(kern, smem, configured);
+  if (e != cudaSuccess || grid <= 0) return e;
+  return launch_pdl(kern, grid, threads, smem, st, args...);
+}
+template <int N>
+cudaError_t launch_loss_rows_in(const Ctx& c) {
+  using P = LossRows<N>;
+  static std::atomic<unsigned long long> configured{0ull};
+  return launch_loss(k_loss_rows_in<N>, P::SMEM, configured, c.count * (N / Blocked<N>::WR), P::NT, c.st,
+                     static_cast<const float2*>(c.rho), static_cast<const int*>(c.S), c.T, c.odd, c.first, c.tw);
+}
+template <int N, int LOSS, bool GRAD>
+cudaError_t launch_loss_cols(const Ctx& c, float eps, double* partials) {
+  using P = LossCols<N>;
+  auto kern = k_loss_cols<N, LOSS, GRAD>;
   static std::atomic<unsigned long long> configured{0ull};
   static std::atomic<int> resident[64] = {};
   cudaError_t e = configure(kern, P::SMEM, configured);
   if (e != cudaSuccess || c.count <= 0) return e;
-  const int tiles = c.count * (N / W);
-  const int slots = share(resident_ctas(kern, P::NT, P::SMEM, resident), c.grid_div);
-  const int grid = tiles < slots ? tiles : slots;
-  return launch_pdl(kern, grid, P::NT, P::SMEM, c.st, c.T, c.A, c.ipp, c.first, c.count, eps, partials, c.tw);
+  const int tiles = c.count * (N / Blocked<N>::BC);
+  const int slots = resident_ctas(kern, P::NT, P::SMEM, resident);
+  return launch_pdl(kern, tiles < slots ? tiles : slots, P::NT, P::SMEM, c.st, c.T, c.At, c.ipp,
+                    static_cast<const unsigned char*>(c.odd), c.first, c.count, eps, partials, c.tw);
+}
+template <int N>
+cudaError_t launch_loss_rows_out(const Ctx& c, float2* grad, const float* scale) {
+  using P = LossRows<N>;
+  static std::atomic<unsigned long long> configured{0ull};
+  cudaError_t e = cudaMemsetAsync(c.bad + c.first, 0, (size_t)c.count * sizeof(unsigned), c.st);
+  if (e != cudaSuccess) return e;
+  e = launch_loss(k_loss_rows_out<N>, P::SMEM, configured, c.count * (N / Blocked<N>::WR), P::NT, c.st,
+                  static_cast<const float2*>(c.T), static_cast<const int*>(c.S), grad, scale, c.bad, c.first, c.tw);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)c.count, 8);
+  cfg.blockDim = dim3(256);
+  cfg.stream = c.st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_loss_rows_bad, static_cast<const int*>(c.S), grad, N, Blocked<N>::WR, c.first,
+                            static_cast<const unsigned*>(c.bad));
+}
+template <int N, bool OUTSIDE>
+cudaError_t launch_adam_rows(const Ctx& c, float2* m, float2* v, const AdamParams& ap, int fresh, int next) {
+  using P = LossRows<N>;
+  static std::atomic<unsigned long long> configured{0ull};
+  return launch_loss(k_adam_rows<N, OUTSIDE>, P::SMEM, configured, c.count * (N / Blocked<N>::WR), P::NT, c.st, c.T,
+                     static_cast<const unsigned char*>(c.odd), static_cast<const int*>(c.S), c.rho, m, v, ap, fresh,
+                     next, c.first, c.tw);
 }
 
 // column-pass variant code: W > 0 one column per thread, W columns per tile;
@@ -518,14 +534,12 @@ struct SizeImpl {
   static float scale() { return (float)(1.0 / ((double)N * (double)N)); }
 
   template <int SRC>
-  static OpRowsForward<SRC> rows_forward(const Ctx& c, const float2* src, float2* dst, Gate g, double* partials) {
+  static OpRowsForward<SRC> rows_forward(const Ctx& c, const float2* src, float2* dst, double* partials) {
     OpRowsForward<SRC> op;
     op.first = c.first;
     op.partials = partials;
     op.rho = src;
-    op.S = c.S;
     op.T = dst;
-    op.g = g;
     return op;
   }
 
@@ -543,7 +557,7 @@ struct SizeImpl {
 
   template <int UPD>
   static cudaError_t iterate_t(const Ctx& c, int iters, float beta, Gate g, int wc, int wr) {
-    SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, g, nullptr), c.count, c.st, c.tw)));
+    SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, nullptr), c.count, c.st, c.tw)));
     for (int i = 0; i < iters; ++i) {
       SPE_TRY(launch_cols_w<N>(c, wc));
       if (i == 0 && c.mark) SPE_TRY(cudaEventRecord(c.mark, c.st));
@@ -645,8 +659,7 @@ struct SizeImpl {
   }
 
   static cudaError_t blur_magnitude(const Ctx& c, float sigma_ft) {
-    const Gate g{};
-    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, g, nullptr), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, nullptr), c.count, c.st, c.tw)));
     SPE_TRY((run_pass<N, AX_COLS>(cols_project(c), c.count, c.st, c.tw)));
     OpRowsModulusForward mf;
     mf.first = c.first;
@@ -668,7 +681,15 @@ struct SizeImpl {
   }
 
   static cudaError_t error_terms(const Ctx& c, Gate g, double* p1, double* p2, double* p3) {
-    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_GATED>(c, c.rho, c.T, g, p1), c.count, c.st, c.tw)));
+    OpRowsEvaluate ev;
+    ev.first = c.first;
+    ev.partials = p1;
+    ev.rho = c.rho;
+    ev.S = c.S;
+    ev.T = c.T;
+    ev.T2 = c.T2;
+    ev.g = g;
+    SPE_TRY((run_pass<N, AX_ROWS>(ev, c.count, c.st, c.tw)));
     OpColsError ce;
     ce.first = c.first;
     ce.partials = p2;
@@ -686,15 +707,14 @@ struct SizeImpl {
   }
 
   static cudaError_t symmetry(const Ctx& c, double* psum, double* ppeak) {
-    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_ABS>(c, c.rho, c.T, Gate{}, nullptr), c.count, c.st, c.tw)));
     OpColsSymmetry sy;
     sy.first = c.first;
     sy.partials = psum;
-    sy.T = c.T;
+    sy.T = c.T2;
     sy.A = c.band;
     sy.ipp = c.ipp;
     SPE_TRY((run_pass<N, AX_COLS>(sy, c.count, c.st, c.tw)));
-    return rows_peak(c, c.T, ppeak);
+    return rows_peak(c, c.T2, ppeak);
   }
 
   static cudaError_t rows_peak(const Ctx& c, const float2* T, double* partials) {
@@ -711,7 +731,7 @@ struct SizeImpl {
     if (sign > 0) {
       Ctx z = c;
       z.first = 0;
-      SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, data, data, Gate{}, nullptr), c.count, c.st, c.tw)));
+      SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, data, data, nullptr), c.count, c.st, c.tw)));
       OpColsTransform<+1> ct;
       ct.first = 0;
         ct.src = data;
@@ -735,7 +755,7 @@ struct SizeImpl {
   static cudaError_t ft_magnitude(const Ctx& c, const float2* src, float2* tmp, float* M) {
     Ctx z = c;
     z.first = 0;
-    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, src, tmp, Gate{}, nullptr), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, src, tmp, nullptr), c.count, c.st, c.tw)));
     OpColsMagnitude cm;
     cm.src = tmp;
     cm.M = M;
@@ -746,7 +766,7 @@ struct SizeImpl {
   static cudaError_t abs_spectrum_items(const Ctx& c, const float2* src, float2* dst, double* psum) {
     Ctx z = c;
     z.first = 0;
-    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_ABS_SUM>(z, src, dst, Gate{}, psum), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_ABS_SUM>(z, src, dst, psum), c.count, c.st, c.tw)));
     OpColsTransform<+1> ct;
     ct.src = dst;
     ct.dst = dst;
@@ -776,7 +796,7 @@ struct SizeImpl {
 
   // partials (rows of the column pass): sum_{A>=0} |FFT+(rho)|^2, sum_{A>=0} A^2
   static cudaError_t known_power(const Ctx& c, double* partials) {
-    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, Gate{}, nullptr), c.count, c.st, c.tw)));
+    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, nullptr), c.count, c.st, c.tw)));
     OpColsKnownPower kp;
     kp.first = c.first;
     kp.partials = partials;
@@ -788,11 +808,12 @@ struct SizeImpl {
 
   // far-field loss per item into partials (column-pass tiles); with grad,
   // grad = scale[p] * 2 S FFT-(dL/dconj F) for items [first, first+count)
-  // of c.rho / c.S (c.T is scratch)
-  // S * rho -> FFT+ (x) -> T: the staged persistent pass where compiled
+  // of c.rho / c.S (c.T is scratch).  Through the support's row tiles where
+  // the side has blocked passes (spe_support.cuh), else row-major.
+  // S * rho -> FFT+ (x) -> T
   static cudaError_t support_forward(const Ctx& c) {
-    if constexpr (rowsio_ok<N>()) {
-      return launch_rows_io<N, ROWS_SUPPORT_FORWARD>(c, c.rho, c.T, nullptr);
+    if constexpr (Blocked<N>::ok) {
+      return launch_loss_rows_in<N>(c);
     } else {
       OpRowsSupportForward rf;
       rf.first = c.first;
@@ -802,11 +823,25 @@ struct SizeImpl {
       return launch_pass<N, AX_ROWS>(rf, c.count, c.st, c.tw);
     }
   }
-
+  template <int LOSS, bool GRAD>
+  static cudaError_t loss_cols(const Ctx& c, float eps, double* partials) {
+    if constexpr (Blocked<N>::ok) {
+      return launch_loss_cols<N, LOSS, GRAD>(c, eps, partials);
+    } else {
+      OpColsLoss<LOSS, GRAD> cl;
+      cl.first = c.first;
+      cl.partials = partials;
+      cl.T = c.T;
+      cl.A = c.A;
+      cl.ipp = c.ipp;
+      cl.eps = eps;
+      return launch_pass<N, AX_COLS>(cl, c.count, c.st, c.tw);
+    }
+  }
   // the last pass of the adjoint: T -> FFT- (x) -> grad = scale[p] * S * .
   static cudaError_t grad_rows(const Ctx& c, float2* grad, const float* scale) {
-    if constexpr (rowsio_ok<N>()) {
-      return launch_rows_io<N, ROWS_GRAD_OUT>(c, c.T, grad, scale);
+    if constexpr (Blocked<N>::ok) {
+      return launch_loss_rows_out<N>(c, grad, scale);
     } else {
       OpRowsGradOut go;
       go.first = c.first;
@@ -822,34 +857,37 @@ struct SizeImpl {
                                  int stage) {
     if (stage == GRAD_ROWS) return grad_rows(c, grad, scale);
     SPE_TRY(support_forward(c));
-    constexpr int WL = DefaultTiles<N>::cols;  // loss partials: N / WL per item
-    if (!grad && stage == GRAD_ALL) return launch_cols_loss<N, WL, LOSS, false>(c, eps, partials);
-    SPE_TRY((launch_cols_loss<N, WL, LOSS, true>(c, eps, partials)));
+    if (!grad && stage == GRAD_ALL) return loss_cols<LOSS, false>(c, eps, partials);
+    SPE_TRY((loss_cols<LOSS, true>(c, eps, partials)));
     if (stage == GRAD_COLS) return cudaSuccess;
     return grad_rows(c, grad, scale);
   }
   // loss (partials) at the current densities, then one Adam step in place
   template <int LOSS>
-  static cudaError_t adam_step_t(const Ctx& c, float eps, double* partials, float2* m, float2* v, float b1, float b2,
-                                 float step_size, float inv_sqrt_bc2, float adam_eps) {
-    SPE_TRY(support_forward(c));
-    constexpr int WL = DefaultTiles<N>::cols;
-    SPE_TRY((launch_cols_loss<N, WL, LOSS, true>(c, eps, partials)));
-    OpRowsGradAdam ad;
-    ad.first = c.first;
-    ad.T = c.T;
-    ad.S = c.S;
-    ad.rho = c.rho;
-    ad.m = m;
-    ad.v = v;
-    ad.ap = {b1, b2, step_size, inv_sqrt_bc2, adam_eps};
-    return launch_pass<N, AX_ROWS>(ad, c.count, c.st, c.tw);
+  static cudaError_t adam_step_t(const Ctx& c, float eps, double* partials, float2* m, float2* v,
+                                 const AdamStep& a) {
+    const AdamParams ap = {a.b1, a.b2, a.step_size, a.inv_sqrt_bc2, a.eps};
+    if (!a.prepared) SPE_TRY(support_forward(c));
+    SPE_TRY((loss_cols<LOSS, true>(c, eps, partials)));
+    if constexpr (Blocked<N>::ok) {
+      return a.inside ? launch_adam_rows<N, false>(c, m, v, ap, a.fresh, a.next)
+                      : launch_adam_rows<N, true>(c, m, v, ap, a.fresh, a.next);
+    } else {
+      OpRowsGradAdam ad;
+      ad.first = c.first;
+      ad.T = c.T;
+      ad.S = c.S;
+      ad.rho = c.rho;
+      ad.m = m;
+      ad.v = v;
+      ad.ap = ap;
+      return launch_pass<N, AX_ROWS>(ad, c.count, c.st, c.tw);
+    }
   }
-  static cudaError_t adam_step(const Ctx& c, int loss, float eps, double* partials, float2* m, float2* v, float b1,
-                               float b2, float step_size, float inv_sqrt_bc2, float adam_eps) {
-    return loss == LOSS_POISSON
-               ? adam_step_t<LOSS_POISSON>(c, eps, partials, m, v, b1, b2, step_size, inv_sqrt_bc2, adam_eps)
-               : adam_step_t<LOSS_AMPLITUDE>(c, eps, partials, m, v, b1, b2, step_size, inv_sqrt_bc2, adam_eps);
+  static cudaError_t adam_step(const Ctx& c, int loss, float eps, double* partials, float2* m, float2* v,
+                               const AdamStep& a) {
+    return loss == LOSS_POISSON ? adam_step_t<LOSS_POISSON>(c, eps, partials, m, v, a)
+                                : adam_step_t<LOSS_AMPLITUDE>(c, eps, partials, m, v, a);
   }
 
   static cudaError_t loss_grad(const Ctx& c, int loss, float eps, double* partials, float2* grad,
@@ -897,7 +935,7 @@ struct SizeImpl {
                               DefaultTiles<N>::rows,
                               &SizeImpl<N>::known_power,
                               &SizeImpl<N>::loss_grad,
-                              N / DefaultTiles<N>::cols,
+                              Blocked<N>::ok ? N / Blocked<N>::BC : N / TileW<N>::cols,
                               &SizeImpl<N>::adam_step,
                               blocked_cols_code<N>(),
                               blocked_rows_code<N>(),

@@ -12,8 +12,9 @@ the per-individual loss sums are FP64.
 ``refine`` runs Adam on individuals that stay in the engine's population
 slots: the optimiser works on a tensor that aliases the engine's device
 memory, so refinement and iteration share the data without copies.  By
-default each step is fused on the device (``spe_adam_step``: loss, adjoint,
-and the Adam update inside the adjoint's last pass); the autograd path
+default the steps are fused on the device (``spe_adam_run``: loss, adjoint,
+and the Adam update inside the adjoint's last pass, which also starts the next
+step's transform); the autograd path
 (``fused=False``) runs the same arithmetic through torch.optim.Adam.
 """
 from __future__ import annotations
@@ -124,8 +125,8 @@ def refine(engine, first, count, steps=50, lr=1e-3, loss="poisson", eps=1e-6, de
     place: `steps` steps on the summed per-individual loss.  Returns the
     per-step loss sums (on the host at the end).
 
-    fused=True runs each step as three passes on the device (loss, adjoint,
-    and the Adam update applied by the adjoint's last pass: spe_adam_step);
+    fused=True runs the steps on the device (loss, adjoint, and the Adam update
+    applied by the adjoint's last pass: spe_adam_run);
     fused=False runs FarFieldLoss through torch autograd and
     torch.optim.Adam -- the same arithmetic, the gradient going through
     memory and the optimiser's own kernels."""
@@ -134,12 +135,11 @@ def refine(engine, first, count, steps=50, lr=1e-3, loss="poisson", eps=1e-6, de
     history = []
     if fused:
         _bind_stream(engine, device)
-        m = torch.zeros_like(dens)
-        v = torch.zeros_like(dens)
+        m = torch.empty_like(dens)  # working memory of the run
+        v = torch.empty_like(dens)
         losses = torch.empty((steps, count), dtype=torch.float64, device=device)
-        for t in range(steps):
-            engine.adam_step(dens.data_ptr(), supp.data_ptr(), m.data_ptr(), v.data_ptr(), count, LOSSES[loss], eps,
-                             lr, betas[0], betas[1], adam_eps, t + 1, losses[t].data_ptr())
+        engine.adam_run(dens.data_ptr(), supp.data_ptr(), m.data_ptr(), v.data_ptr(), count, LOSSES[loss], eps, lr,
+                        betas[0], betas[1], adam_eps, steps, losses.data_ptr())
         torch.cuda.synchronize(device)
         return losses.sum(dim=1).tolist()
     param = torch.nn.Parameter(dens)  # shares the engine's memory
