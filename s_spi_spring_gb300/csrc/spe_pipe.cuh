@@ -32,40 +32,46 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Column exchange layout that keeps the element pairs of a 16-byte copy
 // adjacent (columns are never permuted, only rows).  W = 16: plain rows of
-// 128 bytes (a warp covers whole rows).  W = 8 / 4: rows of 64 / 32 bytes;
-// row l moves to l ^ ((l >> 3) & (16/W - 1)), so the rows a warp touches in
-// a Stockham store (l = 8j+q, consecutive j) fall into different bank groups.
+// 128 bytes (a warp covers whole rows).  Narrower: rows of 8 W bytes; row l
+// moves to l ^ ((l >> SH) & (16/W - 1)), with 2^SH the first radix, so that
+// the rows a half-warp touches in the first pass's stores (l = R0 j + q,
+// consecutive j) fall into different banks, as those of every other access do
+// (consecutive rows).  A shift of 3 for every plan left the first stores of
+// the sides with first radix 4 and 16 two-way conflicts (an iteration of 17 M
+// pixels at 384 190 -> 179 us, at 768 196 -> 192, at 2048 222 -> 212).
 // (A layout with a padding row after every 8, whose addresses are all
 // base + constant, measured about 3% slower at 512.)
 template <int L, int W>
 struct LayCol {
   static constexpr int SIZE = L * W;
   static constexpr int M = (W >= 16) ? 0 : 16 / W - 1;  // row swizzle mask
+  static constexpr int R0 = Plan<L>::R::value[0];
+  static constexpr int SH = R0 == 16 ? 4 : (R0 == 4 ? 2 : 3);
   static __device__ __forceinline__ int idx(int l, int c) {
     if (W >= 16) return l * W + c;
-    return (l ^ ((l >> 3) & M)) * W + c;
+    return (l ^ ((l >> SH) & M)) * W + c;
   }
-  // split addressing: the swizzle only changes bits 0..2 of l and reads bits
-  // 3..5, so a step that is a multiple of 8(M+1) passes through it; the
-  // radix-8 stores of the first two passes swizzle by a per-thread (b & M)
-  // or a compile-time (q & M) value
+  // split addressing: the swizzle only changes bits 0..2 of l and reads the
+  // bits of M from SH on, so a step that is a multiple of (M+1) << SH passes
+  // through it; the stores of the first two passes swizzle by a per-thread
+  // (b & M) or a compile-time (q & M) value
   static constexpr bool kFastAddr = true;
   template <int STEP>
   static __device__ __forceinline__ int load_addr(int b, int r, int c) {
-    if constexpr (STEP % (8 * (M + 1)) == 0) return idx(b, c) + r * STEP * W;
+    if constexpr (STEP % ((M + 1) << SH) == 0) return idx(b, c) + r * STEP * W;
     else return idx(b + r * STEP, c);
   }
   template <int NS, int R>
   static __device__ __forceinline__ int store_addr(int base, int q, int c) {
     if constexpr (M == 0) {
       return (base + q * NS) * W + c;
-    } else if constexpr (NS % (8 * (M + 1)) == 0) {
+    } else if constexpr (NS % ((M + 1) << SH) == 0) {
       return idx(base, c) + q * NS * W;
-    } else if constexpr (NS == 1 && R == 8) {  // base = 8b, position 8b + q
-      const int s = (base >> 3) & M;
+    } else if constexpr (NS == 1 && R == (1 << SH) && R > M) {  // base = R b, position R b + q
+      const int s = (base >> SH) & M;
       return (base + ((q & M) ^ s)) * W + c + (q & ~M) * W;
-    } else if constexpr (NS == 8 && R == 8) {  // base = 64(b/8) + b%8, position base + 8q
-      return (base ^ (q & M)) * W + c + 8 * q * W;
+    } else if constexpr (NS == (1 << SH) && R % (M + 1) == 0 && NS > M) {  // base = NS R (b/NS) + b%NS
+      return (base ^ (q & M)) * W + c + NS * q * W;
     } else {
       return idx(base + q * NS, c);
     }
