@@ -113,7 +113,8 @@ __device__ __forceinline__ void add_pair(float2& a, float2 b) {
   const float e = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, t)), __fsub_rn(b.x, t));
   a = make_float2(s, __fadd_rn(__fadd_rn(a.y, b.y), e));
 }
-template <int NT, int NSUM, int NMAX>
+// NT: threads of the CTA (with ANY at most that many, whole warps)
+template <int NT, int NSUM, int NMAX, bool ANY = false>
 __device__ __forceinline__ void block_reduce_store(double* __restrict__ partials, size_t slot, const float (&v)[NRED]) {
   static_assert(NSUM + NMAX <= NRED, "too many reduction values");
   constexpr int NW = NT / 32;
@@ -144,7 +145,7 @@ __device__ __forceinline__ void block_reduce_store(double* __restrict__ partials
   if ((int)threadIdx.x < NSUM + NMAX) {
     const int k = threadIdx.x;
     float2 a = red[k][0];
-    for (int w = 1; w < NW; ++w) {
+    for (int w = 1; w < (ANY ? (int)blockDim.x / 32 : NW); ++w) {
       if (k < NSUM) add_pair(a, red[k][w]);
       else a.x = fmaxf(a.x, red[k][w].x);
     }
@@ -155,7 +156,7 @@ __device__ __forceinline__ void block_reduce_store(double* __restrict__ partials
 
 // block argmax of (value, raster index): larger value wins, ties go to the
 // lower index; writes partials[blockIdx.x*NRED + {0,1}] = {value, index}
-template <int NT>
+template <int NT, bool ANY = false>
 __device__ __forceinline__ void block_argmax_store(double* __restrict__ partials, float mx, int idx) {
   constexpr int NW = NT / 32;
   __shared__ float rv[NW > 0 ? NW : 1];
@@ -178,7 +179,7 @@ __device__ __forceinline__ void block_argmax_store(double* __restrict__ partials
   if (threadIdx.x == 0) {
     float m = rv[0];
     int i = ri[0];
-    for (int w = 1; w < NW; ++w) {
+    for (int w = 1; w < (ANY ? (int)blockDim.x / 32 : NW); ++w) {
       if (rv[w] > m || (rv[w] == m && ri[w] < i)) {
         m = rv[w];
         i = ri[w];
@@ -275,7 +276,7 @@ __device__ __forceinline__ void pass_elements(const Op& op, const PxF& px, typen
     if constexpr (Op::FFT1 != 0) fft(v, std::integral_constant<int, Op::FFT1>());
     if constexpr (Op::FFT2 != 0) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) v[e] = op.mid(v[e], px(e), acc);
+      for (int e = 0; e < E; ++e) v[e] = op.mid(v[e], px(e), op.fetch_mid(px(e)), acc);
       fft(v, std::integral_constant<int, Op::FFT2>());
     }
 #pragma unroll
@@ -343,6 +344,12 @@ struct OpBase {
   // (roots, the phase gate), across which a thread's memory reads are not
   // reordered -- all are issued before the first value is formed
   static constexpr bool FETCH = false;
+  // likewise the operands of the pointwise step: fetch_mid, then mid
+  struct Mid {};
+  template <class Q>
+  __device__ Mid fetch_mid(const Q&) const {
+    return {};
+  }
   int first = 0;
   double* partials = nullptr;
   const float* A = nullptr;
@@ -356,7 +363,7 @@ struct OpBase {
 // most ops keep the value between two transforms
 struct OpKeep : OpBase {
   template <class Acc>
-  __device__ float2 mid(float2 v, const Px&, Acc&) const {
+  __device__ float2 mid(float2 v, const Px&, const Mid&, Acc&) const {
     return v;
   }
 };
@@ -435,7 +442,7 @@ struct OpColsProject : OpBase {
   float2* T;
   using Acc = NoAcc;
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
-  __device__ float2 mid(float2 v, const Px& q, Acc&) const { return project(v, q.a); }
+  __device__ float2 mid(float2 v, const Px& q, const Mid&, Acc&) const { return project(v, q.a); }
   __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
@@ -475,10 +482,16 @@ struct OpRowsIterate : OpBase {
   GateK g;
   using Acc = NoAcc;
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
-  __device__ float2 mid(float2 v, const Px& q, Acc&) const {
+  struct Mid {
+    float2 prev;
+    int s;
+  };
+  __device__ Mid fetch_mid(const Px& q) const {
+    return {(UPD == UPD_ER) ? make_float2(0.f, 0.f) : rho[q.gi], S[q.gi]};
+  }
+  __device__ float2 mid(float2 v, const Px& q, const Mid& m, Acc&) const {
     const float2 rp = make_float2(v.x * scale, v.y * scale);
-    const float2 prev = (UPD == UPD_ER) ? make_float2(0.f, 0.f) : rho[q.gi];
-    const float2 r = update<UPD>(rp, prev, S[q.gi], beta, g);
+    const float2 r = update<UPD>(rp, m.prev, m.s, beta, g);
     rho[q.gi] = r;
     return r;
   }
@@ -508,7 +521,7 @@ struct OpRowsModulusForward : OpBase {
   float scale;
   using Acc = NoAcc;
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
-  __device__ float2 mid(float2 v, const Px&, Acc&) const {
+  __device__ float2 mid(float2 v, const Px&, const Mid&, Acc&) const {
     return make_float2(cabsf2(make_float2(v.x * scale, v.y * scale)), 0.f);
   }
   __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
@@ -523,7 +536,7 @@ struct OpColsBlur : OpBase {
   float sig2;  // sigma_ft^2
   using Acc = NoAcc;
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
-  __device__ float2 mid(float2 v, const Px& q, Acc&) const {
+  __device__ float2 mid(float2 v, const Px& q, const Mid&, Acc&) const {
     const int xx = (q.x >= n / 2) ? q.x - n : q.x;
     const int yy = (q.y >= n / 2) ? q.y - n : q.y;
     const float r2 = (float)(xx * xx + yy * yy);
@@ -572,7 +585,7 @@ struct OpColsError : OpBase {
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
-  __device__ float2 mid(float2 v, const Px& q, Acc& acc) const {
+  __device__ float2 mid(float2 v, const Px& q, const Mid&, Acc& acc) const {
     const float m = cabsf2(v);
     acc.mx = fmaxf(acc.mx, m);
     if (q.a >= 0.f) {
@@ -690,7 +703,7 @@ struct OpColsSymmetry : OpBase {
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
-  __device__ float2 mid(float2 v, const Px& q, Acc& acc) const {
+  __device__ float2 mid(float2 v, const Px& q, const Mid&, Acc& acc) const {
     const float2 d = ft_shift_norm(v);
     acc.s += weighted(make_float2(d.y * d.y + d.x * d.x, 0.f), q.a).x;
     return weighted(cross_power<+1>(d, d), q.a);
@@ -811,7 +824,7 @@ struct OpColsLoss : OpBase {
     }
   };
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
-  __device__ float2 mid(float2 v, const Px& q, Acc& acc) const {
+  __device__ float2 mid(float2 v, const Px& q, const Mid&, Acc& acc) const {
     float2 g = make_float2(0.f, 0.f);
     if (q.a >= 0.f) loss_add(acc.l, loss_term<LOSS>(v, q.a, eps, &g));
     return g;

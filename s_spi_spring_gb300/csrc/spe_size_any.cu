@@ -13,15 +13,16 @@
 // columns) of one individual in shared memory, applies the operation's load,
 // transforms, pointwise step and store (the same op functors as the
 // compiled passes), and reduces its partial sums.  The 1D transform is a
-// self-sorting Stockham FFT over the factors of the side (radix 8, then 4,
-// then the primes), with the twiddles of a table exp(2 pi i m / n) computed
-// in double and held in shared memory.  Radices 2, 3, 4, 5, 7 and 8 run as
-// butterflies in registers (a thread reads the R inputs of one butterfly,
+// self-sorting Stockham FFT over the factors of the side (2 .. 10, as few as
+// make up the side, then the larger primes), with the twiddles of a table
+// exp(2 pi i m / n) computed in double and held in shared memory.  Radices 2
+// to 10 run as butterflies in registers (a thread reads the R inputs of one butterfly,
 // applies its twiddles and the radix-R DFT, writes R outputs), and so do the
 // primes 11 .. 31, with the symmetric form of the prime DFT; a larger prime
 // radix, up to the side itself, runs the same symmetric form with run-time
 // R over shared memory (about R real multiply-adds per point).  Sides are
 // limited only by their lines fitting in shared memory (n <= 9386).
+#include <algorithm>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -31,7 +32,7 @@
 namespace spe {
 namespace {
 
-constexpr int kAnyThreads = 512;     // threads of a pass CTA
+constexpr int kAnyThreads = 512;     // most threads of a pass CTA
 constexpr int kAnyThreadsBig = 256;  // the same for plans with a prime radix of 11 or more (128 registers each)
 constexpr int kMaxRadices = 24;
 constexpr size_t kAnySmem = 220 * 1024;  // shared-memory budget of one CTA (two line buffers)
@@ -42,6 +43,7 @@ struct AnyPlan {
   int LS;                 // shared-memory stride of a line (odd: conflict-free 8-byte columns)
   int nrad;               // radix passes
   int rad[kMaxRadices];   // radices in pass order
+  int threads;            // of a CTA
   int big;                // a prime radix of 11 or more (any_pass_prime, any_pass_sym: the BIG kernels)
   // divisors of the index arithmetic as fast-division constants (fdiv):
   // the side, and per pass the butterflies per line n / R, the stride NS of
@@ -103,23 +105,55 @@ template <int R, int S>
 __device__ __forceinline__ void small_dft(float2* v) {
   if constexpr (R == 5 || R == 7) {
     dft_odd_sym<R, S>(v);
+  } else if constexpr (R == 10) {  // 2 x 5 (dft has no factor 5)
+    float2 y[10];
+#pragma unroll
+    for (int n2 = 0; n2 < 5; ++n2) {
+      y[2 * n2] = cadd(v[n2], v[5 + n2]);
+      y[2 * n2 + 1] = csub(v[n2], v[5 + n2]);
+    }
+    twiddle_block<10, 2, 5, S, 1>(y);
+#pragma unroll
+    for (int k1 = 0; k1 < 2; ++k1) {
+      float2 t[5];
+#pragma unroll
+      for (int n2 = 0; n2 < 5; ++n2) t[n2] = y[n2 * 2 + k1];
+      dft_odd_sym<5, S>(t);
+#pragma unroll
+      for (int k2 = 0; k2 < 5; ++k2) v[k1 + 2 * k2] = t[k2];
+    }
   } else {
     dft<R, S>(v);
   }
 }
 
+// The dynamic shared memory of pass_any: two line buffers and the side's
+// twiddle table.  The pass functions below are not inlined (one copy of each
+// serves every operation's kernel) and take offsets into it, not pointers, so
+// that their accesses are shared-memory accesses, and the plan's values they
+// need by value.
+extern __shared__ float2 sm_any[];
+
+struct PassArgs {  // one pass of the plan
+  int cur, oth, tw;  // offsets of the line buffers and the table in sm_any
+  int nl, n, LS, NS;
+  unsigned inv_m, inv_ns;
+};
+
 // One Stockham pass of radix R as butterflies: each thread reads the R
 // inputs x[b + r n/R] of a butterfly, multiplies them by w_{NS R}^{k r}
 // (k = b mod NS), runs the radix-R DFT in registers and writes its R
 // outputs at (b/NS) NS R + k + q NS.
-template <int R, int S, int NT>
-__device__ __forceinline__ void any_pass_r(const float2* cur, float2* oth, const AnyPlan& pl, const float2* tw, int nl,
-                                           int ps) {
-  const int n = pl.n, LS = pl.LS, m = n / R, NS = pl.ns[ps], tstep = n / (NS * R);
-  const unsigned inv_m = pl.inv_m[ps], inv_ns = pl.inv_ns[ps];
-  for (int i = threadIdx.x; i < nl * m; i += NT) {
-    const int c = fdiv(i, inv_m), b = i - c * m;
-    const int bq = fdiv(b, inv_ns), k = b - bq * NS;
+template <int R, int S, bool BIG>
+__device__ __noinline__ void any_pass_r(const PassArgs a) {
+  const float2* cur = sm_any + a.cur;
+  float2* oth = sm_any + a.oth;
+  const float2* tw = sm_any + a.tw;
+  const int n = a.n, LS = a.LS, m = n / R, NS = a.NS, tstep = n / (NS * R);
+  const int total = a.nl * m;
+  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+    const int c = fdiv(i, a.inv_m), b = i - c * m;
+    const int bq = fdiv(b, a.inv_ns), k = b - bq * NS;
     const float2* src = cur + c * LS + b;
     float2 v[R];
 #pragma unroll
@@ -162,18 +196,6 @@ __device__ __forceinline__ void odd_sym_outputs(const float2* a, const float2* b
   }
 }
 
-// The dynamic shared memory of pass_any: two line buffers and the side's
-// twiddle table.  The non-inlined pass functions below take offsets into it
-// (not pointers), so that their accesses are shared-memory accesses, and
-// the plan's values they need by value.
-extern __shared__ float2 sm_any[];
-
-struct PassArgs {  // one pass of the plan, for the non-inlined pass functions
-  int cur, oth, tw;  // offsets of the line buffers and the table in sm_any
-  int nl, n, LS, NS;
-  unsigned inv_m, inv_ns;
-};
-
 // One Stockham pass of an odd prime radix R (11 .. 31) as butterflies: the
 // inputs and twiddles of any_pass_r, the symmetric DFT above.  Not inlined:
 // one copy per (R, S) serves every operation's pass kernel.
@@ -185,7 +207,7 @@ __device__ __noinline__ void any_pass_prime(const PassArgs a) {
   const float2* tw = sm_any + a.tw;
   const int nl = a.nl, n = a.n, LS = a.LS, m = n / R, NS = a.NS, tstep = n / (NS * R);
   const unsigned inv_m = a.inv_m, inv_ns = a.inv_ns;
-  for (int i = threadIdx.x; i < nl * m; i += kAnyThreadsBig) {
+  for (int i = threadIdx.x; i < nl * m; i += blockDim.x) {
     const int c = fdiv(i, inv_m), b = i - c * m;
     const int bq = fdiv(b, inv_ns), k = b - bq * NS;
     const float2* src = cur + c * LS + b;
@@ -217,91 +239,56 @@ __device__ __noinline__ void any_pass_prime(const PassArgs a) {
   }
 }
 
-// One pass of an odd prime radix above 31, in the symmetric form of the
-// prime DFT with run-time R (H = (R-1)/2), in two steps over shared memory:
-//   1. per butterfly and pair (r, R-r), r = 1 .. H: y_r = x_r w^{k r},
-//      y_{R-r} = x_{R-r} w^{k (R-r)} (the inter-pass twiddles), then
-//      a_r = y_r + y_{R-r} into slot r and b_r = y_r - y_{R-r} into slot R-r,
-//      in place (each element is read and written by one thread);
-//   2. per butterfly and q = 0 .. H: X_0 = y_0 + sum a_r, and for q >= 1
-//      X_q, X_{R-q} = A_q +- i B_q with A_q = y_0 + sum_r a_r cos(2 pi r q / R),
-//      B_q = sum_r b_r S sin(2 pi r q / R), the cosines and sines read from
-//      the side's table (exp(2 pi i t m / n) = exp(2 pi i t / R), m = n / R).
-// About 2 real multiply-adds per input and output pair instead of 4 per
-// input and output.
-template <int S, int NT>
-__device__ __noinline__ void any_pass_sym(const PassArgs a, int R) {
-  float2* cur = sm_any + a.cur;
+// Outputs of a symmetric pass (step 2 of any_pass_sym): kSymQ values of q for
+// BB butterflies per thread, so that each a_r, b_r read serves kSymQ pairs and
+// each table read BB butterflies; the multiply-adds of a pair's x and y are one
+// packed instruction.  Consecutive threads take consecutive butterflies of one
+// group of q: their table reads coincide and their inputs are contiguous.
+// q = 0 takes the table's exp(0) = 1 exactly: X_0 = y_0 + sum a_r.
+constexpr int kSymQ = 4;
+template <int S, int BB>
+__device__ __forceinline__ void any_sym_outputs(const PassArgs& a, int R) {
+  constexpr int QB = kSymQ;
+  const float2* cur = sm_any + a.cur;
   float2* oth = sm_any + a.oth;
   const float2* tw = sm_any + a.tw;
-  const int nl = a.nl, n = a.n, LS = a.LS, NS = a.NS, H = (R - 1) / 2;
-  const int m = n / R, tstep = n / (NS * R);
-  const unsigned inv_m = a.inv_m, inv_ns = a.inv_ns;
-  const unsigned inv_h = fdiv_inv(H), inv_h1 = fdiv_inv(H + 1);
-  // 1. twiddles and pairs, in place
-  for (int i = threadIdx.x; i < nl * m * H; i += NT) {
-    const int u = fdiv(i, inv_h), r = 1 + (i - u * H);  // u: butterfly of the tile
-    const int c = fdiv(u, inv_m), b = u - c * m;
-    const int k = b - fdiv(b, inv_ns) * NS;
-    float2* src = cur + c * LS + b;
-    float2 x = src[r * m], y = src[(R - r) * m];
-    if (NS > 1) {
-      const int e = k * tstep;  // w^{k r} = table[e r]; e < n / R, so e r < n
-      float2 w1 = tw[e * r], w2 = tw[e * (R - r)];
-      if (S < 0) {
-        w1.y = -w1.y;
-        w2.y = -w2.y;
-      }
-      x = cmul(x, w1);
-      y = cmul(y, w2);
-    }
-    src[r * m] = cadd(x, y);
-    src[(R - r) * m] = csub(x, y);
-  }
-  __syncthreads();
-  // 2. output pairs: QB values of q for BB butterflies per thread (each
-  // a_r, b_r load serves QB pairs, each table lookup BB butterflies); q = 0
-  // takes the table's exp(0) = 1 exactly: X_0 = y_0 + sum a_r
-  constexpr int QB = 4, BB = 2;
-  const int G = (H + QB) / QB;  // groups of q in [0, H]
-  const int nb = nl * m;        // butterflies of the tile
-  const unsigned inv_g = fdiv_inv(G);
-  for (int i = threadIdx.x; i < ((nb + BB - 1) / BB) * G; i += NT) {
-    const int up = fdiv(i, inv_g), g = i - up * G;
+  const int n = a.n, LS = a.LS, NS = a.NS, H = (R - 1) / 2, m = n / R;
+  const int G = (H + QB) / QB, nb = a.nl * m, ng = (nb + BB - 1) / BB;
+  const unsigned inv_ng = fdiv_inv(ng);
+  for (int i = threadIdx.x; i < ng * G; i += blockDim.x) {
+    const int g = fdiv(i, inv_ng), up = i - g * ng;
     const float2* src[BB];
     float2* dst[BB];
-    float2 y0[BB];
+    float2 A[BB][QB], B[BB][QB];
     bool live[BB];
 #pragma unroll
     for (int v = 0; v < BB; ++v) {
-      const int u0 = up * BB + v;
+      const int u0 = up + v * ng;
       live[v] = u0 < nb;
-      const int u = live[v] ? u0 : up * BB;  // a tail slot repeats the first butterfly, unstored
-      const int c = fdiv(u, inv_m), b = u - c * m;
-      const int bq = fdiv(b, inv_ns), k = b - bq * NS;
+      const int u = live[v] ? u0 : up;  // a tail slot repeats the first butterfly, unstored
+      const int c = fdiv(u, a.inv_m), b = u - c * m;
+      const int bq = fdiv(b, a.inv_ns), k = b - bq * NS;
       src[v] = cur + c * LS + b;
       dst[v] = oth + c * LS + bq * NS * R + k;
-      y0[v] = src[v][0];
+#pragma unroll
+      for (int t = 0; t < QB; ++t) {
+        A[v][t] = src[v][0];
+        B[v][t] = make_float2(0.f, 0.f);
+      }
     }
-    float2 A[BB][QB], B[BB][QB];
     int idx[QB], step[QB];
 #pragma unroll
     for (int t = 0; t < QB; ++t) {
       const int q = g * QB + t;
       idx[t] = 0;
       step[t] = q <= H ? q * m : 0;  // table index of exp(2 pi i r q / R) advances by q m mod n
-#pragma unroll
-      for (int v = 0; v < BB; ++v) {
-        A[v][t] = y0[v];
-        B[v][t] = make_float2(0.f, 0.f);
-      }
     }
     for (int r = 1; r <= H; ++r) {
-      float2 a[BB], bb[BB];
+      float2 x[BB], y[BB];
 #pragma unroll
       for (int v = 0; v < BB; ++v) {
-        a[v] = src[v][r * m];
-        bb[v] = src[v][(R - r) * m];
+        x[v] = src[v][r * m];
+        y[v] = src[v][(R - r) * m];
       }
 #pragma unroll
       for (int t = 0; t < QB; ++t) {
@@ -309,12 +296,11 @@ __device__ __noinline__ void any_pass_sym(const PassArgs a, int R) {
         if (idx[t] >= n) idx[t] -= n;
         const float2 w = tw[idx[t]];
         const float ws = S < 0 ? -w.y : w.y;
+        const float2 cc = make_float2(w.x, w.x), ss = make_float2(ws, ws);
 #pragma unroll
         for (int v = 0; v < BB; ++v) {
-          A[v][t].x = fmaf(a[v].x, w.x, A[v][t].x);
-          A[v][t].y = fmaf(a[v].y, w.x, A[v][t].y);
-          B[v][t].x = fmaf(bb[v].x, ws, B[v][t].x);
-          B[v][t].y = fmaf(bb[v].y, ws, B[v][t].y);
+          A[v][t] = __ffma2_rn(x[v], cc, A[v][t]);
+          B[v][t] = __ffma2_rn(y[v], ss, B[v][t]);
         }
       }
     }
@@ -335,26 +321,78 @@ __device__ __noinline__ void any_pass_sym(const PassArgs a, int R) {
   }
 }
 
+// One pass of an odd prime radix above 31, in the symmetric form of the
+// prime DFT with run-time R (H = (R-1)/2), in two steps over shared memory:
+//   1. per butterfly and pair (r, R-r), r = 1 .. H: y_r = x_r w^{k r},
+//      y_{R-r} = x_{R-r} w^{k (R-r)} (the inter-pass twiddles), then
+//      a_r = y_r + y_{R-r} into slot r and b_r = y_r - y_{R-r} into slot R-r,
+//      in place (each element is read and written by one thread);
+//   2. per butterfly and q = 0 .. H: X_0 = y_0 + sum a_r, and for q >= 1
+//      X_q, X_{R-q} = A_q +- i B_q with A_q = y_0 + sum_r a_r cos(2 pi r q / R),
+//      B_q = sum_r b_r S sin(2 pi r q / R), the cosines and sines read from
+//      the side's table (exp(2 pi i t m / n) = exp(2 pi i t / R), m = n / R).
+// About 2 real multiply-adds per input and output pair instead of 4 per
+// input and output.
+template <int S>
+__device__ __noinline__ void any_pass_sym(const PassArgs a, int R) {
+  float2* cur = sm_any + a.cur;
+  const float2* tw = sm_any + a.tw;
+  const int nl = a.nl, n = a.n, LS = a.LS, NS = a.NS, H = (R - 1) / 2;
+  const int m = n / R, tstep = n / (NS * R);
+  const unsigned inv_m = a.inv_m, inv_ns = a.inv_ns;
+  const unsigned inv_h = fdiv_inv(H);
+  // 1. twiddles and pairs, in place
+  for (int i = threadIdx.x; i < nl * m * H; i += blockDim.x) {
+    const int u = fdiv(i, inv_h), r = 1 + (i - u * H);  // u: butterfly of the tile
+    const int c = fdiv(u, inv_m), b = u - c * m;
+    const int k = b - fdiv(b, inv_ns) * NS;
+    float2* src = cur + c * LS + b;
+    float2 x = src[r * m], y = src[(R - r) * m];
+    if (NS > 1) {
+      const int e = k * tstep;  // w^{k r} = table[e r]; e < n / R, so e r < n
+      float2 w1 = tw[e * r], w2 = tw[e * (R - r)];
+      if (S < 0) {
+        w1.y = -w1.y;
+        w2.y = -w2.y;
+      }
+      x = cmul(x, w1);
+      y = cmul(y, w2);
+    }
+    src[r * m] = cadd(x, y);
+    src[(R - r) * m] = csub(x, y);
+  }
+  __syncthreads();
+  // 2. output pairs, as many butterflies per thread as leave every thread work
+  const int G = (H + kSymQ) / kSymQ;  // groups of q in [0, H]
+  const int NT = blockDim.x;
+  if (((nl * m + 3) / 4) * G >= NT) any_sym_outputs<S, 4>(a, R);
+  else if (((nl * m + 1) / 2) * G >= NT) any_sym_outputs<S, 2>(a, R);
+  else any_sym_outputs<S, 1>(a, R);
+}
+
 // The transform of the tile's nl lines: one pass per radix of the plan,
 // ping-ponging between the two line buffers; on return `cur` holds it.
 // BIG: the plan has a prime radix of 11 or more, whose pass functions need
 // more registers than the rest; kernels without them are compiled
 // separately so that the other sides keep their occupancy.
-template <int S, bool BIG, int NT = BIG ? kAnyThreadsBig : kAnyThreads>
+template <int S, bool BIG>
 __device__ __forceinline__ void fft_any(float2*& cur, float2*& oth, const AnyPlan& pl, const float2* tw, int nl) {
   for (int ps = 0; ps < pl.nrad; ++ps) {
     const int R = pl.rad[ps];
+    const PassArgs a{(int)(cur - sm_any), (int)(oth - sm_any), (int)(tw - sm_any), nl, pl.n, pl.LS, pl.ns[ps],
+                     pl.inv_m[ps], pl.inv_ns[ps]};
     switch (R) {
-      case 2: any_pass_r<2, S, NT>(cur, oth, pl, tw, nl, ps); break;
-      case 3: any_pass_r<3, S, NT>(cur, oth, pl, tw, nl, ps); break;
-      case 4: any_pass_r<4, S, NT>(cur, oth, pl, tw, nl, ps); break;
-      case 5: any_pass_r<5, S, NT>(cur, oth, pl, tw, nl, ps); break;
-      case 7: any_pass_r<7, S, NT>(cur, oth, pl, tw, nl, ps); break;
-      case 8: any_pass_r<8, S, NT>(cur, oth, pl, tw, nl, ps); break;
+      case 2: any_pass_r<2, S, BIG>(a); break;
+      case 3: any_pass_r<3, S, BIG>(a); break;
+      case 4: any_pass_r<4, S, BIG>(a); break;
+      case 5: any_pass_r<5, S, BIG>(a); break;
+      case 6: any_pass_r<6, S, BIG>(a); break;
+      case 7: any_pass_r<7, S, BIG>(a); break;
+      case 8: any_pass_r<8, S, BIG>(a); break;
+      case 9: any_pass_r<9, S, BIG>(a); break;
+      case 10: any_pass_r<10, S, BIG>(a); break;
       default:
         if constexpr (BIG) {
-          const PassArgs a{(int)(cur - sm_any), (int)(oth - sm_any), (int)(tw - sm_any), nl, pl.n, pl.LS, pl.ns[ps],
-                           pl.inv_m[ps], pl.inv_ns[ps]};
           switch (R) {
             case 11: any_pass_prime<11, S>(a); break;
             case 13: any_pass_prime<13, S>(a); break;
@@ -363,7 +401,7 @@ __device__ __forceinline__ void fft_any(float2*& cur, float2*& oth, const AnyPla
             case 23: any_pass_prime<23, S>(a); break;
             case 29: any_pass_prime<29, S>(a); break;
             case 31: any_pass_prime<31, S>(a); break;
-            default: any_pass_sym<S, NT>(a, R); break;
+            default: any_pass_sym<S>(a, R); break;
           }
         }
         // (kernels without BIG never see a radix of 11 or more: make_plan
@@ -380,15 +418,15 @@ __device__ __forceinline__ void fft_any(float2*& cur, float2*& oth, const AnyPla
 template <int AXIS, class Op, bool BIG>
 // BIG kernels: two 256-thread CTAs per SM, 128 registers a thread (a few
 // spilled bytes; one CTA per SM without the cap ran 30% slower at side 1054)
-__global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, BIG ? 2 : 0)
+__global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
     pass_any(const Op op, const AnyPlan pl, const float2* __restrict__ tw) {
-  constexpr int NT = BIG ? kAnyThreadsBig : kAnyThreads;
+  const int NT = blockDim.x;
   const int n = pl.n, W = pl.W, LS = pl.LS;
   float2* cur = sm_any;
   float2* oth = sm_any + (size_t)W * LS;
   float2* tws = sm_any + (size_t)2 * W * LS;  // the twiddle table, n entries
   pdl_enter();
-  for (int i = threadIdx.x; i < n; i += NT) tws[i] = __ldg(tw + i);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) tws[i] = __ldg(tw + i);
   const int tpi = (n + W - 1) / W;
   const int p = op.first + blockIdx.x / tpi;
   const int l0 = (blockIdx.x % tpi) * W;
@@ -399,7 +437,9 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, BIG ? 2 : 
   typename Op::Acc acc;
   // element i of the tile: row passes walk along x (whole rows), column
   // passes across the tile's columns first (row segments of nl elements)
-  auto px = [&](int i, int& c, int& l) {
+  const float* amp = Op::AMP ? op.amp(p, n) : nullptr;
+  auto px = [&](int i, int& at) {
+    int c, l;
     if (AXIS == AX_ROWS) {
       c = fdiv(i, pl.inv_n);
       l = i - c * n;
@@ -407,87 +447,178 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, BIG ? 2 : 
       l = fdiv(i, inv_nl);
       c = i - l * nl;
     }
+    at = c * LS + l;
     Px q;
     q.p = p;
     q.y = AXIS == AX_ROWS ? l0 + c : l;
     q.x = AXIS == AX_ROWS ? l : l0 + c;
-    q.gi = q.ti = base + (size_t)q.y * n + q.x;
-    q.a = Op::AMP ? __ldg(op.amp(p, n) + (size_t)q.y * n + q.x) : 0.f;
+    const int off = q.y * n + q.x;
+    q.gi = q.ti = base + off;
+    q.a = Op::AMP ? __ldg(amp + off) : 0.f;
     return q;
+  };
+  // a thread's elements in batches of U: the batch's memory reads are issued
+  // before the first of them is used (one at a time, the waits for them were
+  // 35-45% of the iteration's passes)
+  constexpr int U = 8;
+  auto batches = [&](auto&& body) {
+    for (int i0 = threadIdx.x; i0 < tot; i0 += NT * U) body(i0);
   };
   pdl_wait();
   if constexpr (Op::PAIR) {
     for (int second = 0; second < 2; ++second) {
-      for (int i = threadIdx.x; i < tot; i += NT) {
-        int c, l;
-        const Px q = px(i, c, l);
+      for (int i = threadIdx.x; i < tot; i += blockDim.x) {
+        int at;
+        const Px q = px(i, at);
         float2 v1, v2;
         typename Op::Acc once;
         op.load_pair(q, v1, v2, second ? once : acc);
-        cur[c * LS + l] = second ? v2 : v1;
+        cur[at] = second ? v2 : v1;
       }
       __syncthreads();
       fft_any<Op::FFT1, BIG>(cur, oth, pl, tws, nl);
-      for (int i = threadIdx.x; i < tot; i += NT) {
-        int c, l;
-        const Px q = px(i, c, l);
-        op.store_pair(cur[c * LS + l], q, second);
+      for (int i = threadIdx.x; i < tot; i += blockDim.x) {
+        int at;
+        const Px q = px(i, at);
+        op.store_pair(cur[at], q, second);
       }
       __syncthreads();
     }
   } else {
-    for (int i = threadIdx.x; i < tot; i += NT) {
-      int c, l;
-      const Px q = px(i, c, l);
-      cur[c * LS + l] = op.load(q, acc);
-    }
+    batches([&](int i0) {
+      int at[U];
+      if constexpr (Op::FETCH) {
+        typename Op::Raw r[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) if (i0 + u * NT < tot) r[u] = op.fetch(px(i0 + u * NT, at[u]));
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 + u * NT < tot) cur[at[u]] = op.form(r[u], acc);
+      } else {
+        float2 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) if (i0 + u * NT < tot) v[u] = op.load(px(i0 + u * NT, at[u]), acc);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 + u * NT < tot) cur[at[u]] = v[u];
+      }
+    });
     __syncthreads();
     if constexpr (Op::FFT1 != 0) fft_any<Op::FFT1, BIG>(cur, oth, pl, tws, nl);
     if constexpr (Op::FFT2 != 0) {
-      for (int i = threadIdx.x; i < tot; i += NT) {
-        int c, l;
-        const Px q = px(i, c, l);
-        cur[c * LS + l] = op.mid(cur[c * LS + l], q, acc);
-      }
+      batches([&](int i0) {
+        Px q[U];
+        int at[U];
+        typename Op::Mid m[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 + u * NT < tot) {
+            q[u] = px(i0 + u * NT, at[u]);
+            m[u] = op.fetch_mid(q[u]);
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 + u * NT < tot) cur[at[u]] = op.mid(cur[at[u]], q[u], m[u], acc);
+      });
       __syncthreads();
       fft_any<Op::FFT2, BIG>(cur, oth, pl, tws, nl);
     }
-    for (int i = threadIdx.x; i < tot; i += NT) {
-      int c, l;
-      const Px q = px(i, c, l);
-      op.store(cur[c * LS + l], q, acc);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < tot; i += blockDim.x) {
+      int at;
+      const Px q = px(i, at);
+      op.store(cur[at], q, acc);
     }
   }
   if constexpr (Op::NSUM + Op::NMAX > 0) {
     float r[NRED];
     acc.values(r);
-    block_reduce_store<NT, Op::NSUM, Op::NMAX>(op.partials, blockIdx.x, r);
+    block_reduce_store<BIG ? kAnyThreadsBig : kAnyThreads, Op::NSUM, Op::NMAX, true>(op.partials, blockIdx.x, r);
   }
-  if constexpr (Op::PEAK) block_argmax_store<NT>(op.partials, acc.mx, acc.idx);
+  if constexpr (Op::PEAK) block_argmax_store<BIG ? kAnyThreadsBig : kAnyThreads, true>(op.partials, acc.mx, acc.idx);
 }
 
 // ---------------------------------------------------------------------------
 // plans
 // ---------------------------------------------------------------------------
-bool make_plan(int n, AnyPlan& pl) {
+// n (primes up to 7) as a product of the fewest factors in [2, 10], the
+// largest first; fewest factors, then the smallest sum (equal factors).
+int fewest_radices(int n, int* rad) {
+  int best = kMaxRadices + 1, best_sum = 0, cur[kMaxRadices];
+  auto search = [&](auto&& self, int rest, int top, int k, int sum) -> void {
+    if (rest == 1) {
+      if (k < best || (k == best && sum < best_sum)) {
+        best = k;
+        best_sum = sum;
+        std::copy(cur, cur + k, rad);
+      }
+      return;
+    }
+    if (k + 1 > best || k >= kMaxRadices) return;
+    for (int f = top; f >= 2; --f)
+      if (rest % f == 0) {
+        cur[k] = f;
+        self(self, rest / f, f, k + 1, sum + f);
+      }
+  };
+  search(search, n, 10, 0, 0);
+  return best > kMaxRadices ? 0 : best;
+}
+
+size_t smem_of(const AnyPlan& pl) { return (2 * (size_t)pl.W * pl.LS + pl.n) * sizeof(float2); }
+
+// Threads of a pass CTA: those that keep the most threads of an SM (as many
+// CTAs as its shared memory and registers hold) busy in the pass with the
+// fewest butterflies (the largest radix), the larger of equals, as they have
+// more reads in flight.  A run-time prime pass spreads over its outputs too
+// and takes them all.  512 threads at every side left five of six idle at 100
+// (935 -> 487 us for 8 iterations of 200 individuals).
+int best_threads(const AnyPlan& pl) {
+  const int top = pl.big ? kAnyThreadsBig : kAnyThreads, regs = pl.big ? 512 : 1024;
+  int rmax = 1, best = top;
+  for (int i = 0; i < pl.nrad; ++i) rmax = std::max(rmax, pl.rad[i]);
+  if (rmax > 31) return top;
+  const int fly = pl.W * (pl.n / rmax), ctas = (int)(kAnySmem / smem_of(pl));
+  double most = 0.0;
+  for (int t = 64; t <= top; t += 32) {
+    const int rounds = (fly + t - 1) / t;
+    const double busy = (double)std::min(ctas, regs / t) * fly / rounds;
+    if (busy >= most) {
+      most = busy;
+      best = t;
+    }
+  }
+  return best;
+}
+
+// plain: the radices of the operations whose results are compared digit by
+// digit.  A far-field loss is a 64-bit sum that a few bright pixels dominate,
+// and a shrink-wrap's support is a threshold: other radices round differently,
+// which moves a loss in its ninth digit and may flip a pixel.
+bool make_plan(int n, AnyPlan& pl, bool plain) {
   if (n < 2) return false;
   pl.n = n;
   pl.nrad = 0;
-  int m = n;
-  while (m % 8 == 0 && pl.nrad < kMaxRadices) {
-    pl.rad[pl.nrad++] = 8;
-    m /= 8;
+  // the part of the side without prime factors above 7: in as few passes of
+  // radix 2 .. 10 as it can be, or (`plain`) by 8, 4 and its primes; then the
+  // larger primes
+  int smooth = 1, m = n;
+  for (int f : {2, 3, 5, 7})
+    for (; m % f == 0; m /= f) smooth *= f;
+  if (plain) {
+    for (int f : {8, 4, 2, 3, 5, 7})
+      for (; smooth % f == 0; smooth /= f) pl.rad[pl.nrad++] = f;
+  } else {
+    pl.nrad = fewest_radices(smooth, pl.rad);
   }
-  while (m % 4 == 0 && pl.nrad < kMaxRadices) {
-    pl.rad[pl.nrad++] = 4;
-    m /= 4;
-  }
-  for (int f = 2; f <= m && pl.nrad < kMaxRadices;) {
+  for (int f = 11; m > 1 && pl.nrad < kMaxRadices;) {
     if (m % f == 0) {
       pl.rad[pl.nrad++] = f;
       m /= f;
+    } else if (f * f > m) {
+      f = m;
     } else {
-      f += (f == 2) ? 1 : 2;
+      f += 2;
     }
   }
   if (m != 1) return false;
@@ -508,6 +639,7 @@ bool make_plan(int n, AnyPlan& pl) {
   const size_t budget = (table + 2 * per_line <= kAnySmem / 2) ? kAnySmem / 2 : kAnySmem;
   const size_t w = (budget - table) / per_line;
   pl.W = (int)(w < 8 ? w : 8);
+  pl.threads = best_threads(pl);
   // the bounds of fdiv: indices below W n < 2^17, divisors below 2^15
   if (n >= (1 << 15)) return false;
   while (pl.W > 1 && (size_t)pl.W * n >= (1u << 17)) --pl.W;
@@ -515,7 +647,7 @@ bool make_plan(int n, AnyPlan& pl) {
 }
 
 struct AnyEntry {
-  AnyPlan plan;
+  AnyPlan plan, plain;  // the same tiles
   SizeOps ops;
 };
 
@@ -526,19 +658,25 @@ const AnyPlan& plan_of(int n) {
   std::lock_guard<std::mutex> lock(g_any_mutex);
   return g_any.at(n)->plan;
 }
-
-size_t smem_of(const AnyPlan& pl) { return (2 * (size_t)pl.W * pl.LS + pl.n) * sizeof(float2); }
+const AnyPlan& plain_of(int n) {
+  std::lock_guard<std::mutex> lock(g_any_mutex);
+  return g_any.at(n)->plain;
+}
 
 template <int AXIS, class Op, bool BIG>
-cudaError_t launch_any_k(const Op& op, const AnyPlan& pl, int count, cudaStream_t st, const float2* tw) {
+cudaError_t launch_any_k(const Op& op, AnyPlan pl, int count, cudaStream_t st, const float2* tw) {
   auto kern = pass_any<AXIS, Op, BIG>;
   static std::atomic<unsigned long long> configured{0ull};
-  const size_t smem = smem_of(pl);
   // the attribute is set to the largest budget once: it is an upper bound
   cudaError_t e = configure(kern, kAnySmem, configured);
   if (e != cudaSuccess || count <= 0) return e;
+  // narrower tiles where the plan's leave SMs without a CTA (not where the op
+  // reduces: its partials are one per tile of the plan)
+  if (Op::NSUM + Op::NMAX == 0 && !Op::PEAK)
+    while (pl.W > 2 && (size_t)count * ((pl.n + pl.W - 1) / pl.W) < (size_t)sm_count()) pl.W /= 2;
   const int tpi = (pl.n + pl.W - 1) / pl.W;
-  const int grid = (int)((unsigned)count * tpi), threads = BIG ? kAnyThreadsBig : kAnyThreads;
+  const int grid = (int)((unsigned)count * tpi), threads = pl.threads;
+  const size_t smem = smem_of(pl);
   // the early launch pays where a pass is a few waves of CTAs (a prologue
   // beside the previous pass's drain: 111 -> 82 us for an evaluation of one
   // small pattern); over many waves it measured 0.6% slower (1054^2 x 16)
@@ -620,7 +758,7 @@ struct SizeAny {
   }
 
   static cudaError_t blur_magnitude(const Ctx& c, float sigma_ft) {
-    const AnyPlan& pl = plan_of(c.n);
+    const AnyPlan& pl = plain_of(c.n);
     SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, nullptr), pl, c.count, c.st, c.tw)));
     SPE_TRY((launch_any<AX_COLS>(cols_project(c), pl, c.count, c.st, c.tw)));
     OpRowsModulusForward mf;
@@ -786,7 +924,7 @@ struct SizeAny {
   template <int LOSS>
   static cudaError_t loss_grad_t(const Ctx& c, float eps, double* partials, float2* grad, const float* scale,
                                  int stage) {
-    const AnyPlan& pl = plan_of(c.n);
+    const AnyPlan& pl = plain_of(c.n);
     if (stage == GRAD_ROWS) return grad_rows(c, pl, grad, scale);
     OpRowsSupportForward rf;
     rf.first = c.first;
@@ -825,7 +963,7 @@ struct SizeAny {
   template <int LOSS>
   static cudaError_t adam_step_t(const Ctx& c, float eps, double* partials, float2* m, float2* v,
                                  const AdamStep& a) {
-    const AnyPlan& pl = plan_of(c.n);
+    const AnyPlan& pl = plain_of(c.n);
     OpRowsSupportForward rf;
     rf.first = c.first;
     rf.rho = c.rho;
@@ -870,7 +1008,7 @@ void fill_any(float2* out, int n) {
 
 bool any_side_supported(int n) {
   AnyPlan pl;
-  return make_plan(n, pl);
+  return make_plan(n, pl, false);
 }
 
 const SizeOps* size_ops_any(int n) {
@@ -878,7 +1016,7 @@ const SizeOps* size_ops_any(int n) {
   auto it = g_any.find(n);
   if (it != g_any.end()) return &it->second->ops;
   std::unique_ptr<AnyEntry> en(new AnyEntry());
-  if (!make_plan(n, en->plan)) return nullptr;
+  if (!make_plan(n, en->plan, false) || !make_plan(n, en->plain, true)) return nullptr;
   const int tiles = (n + en->plan.W - 1) / en->plan.W;
   en->ops = SizeOps{n,
                     tiles,
