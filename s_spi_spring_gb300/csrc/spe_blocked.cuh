@@ -486,6 +486,139 @@ __global__ void __launch_bounds__(BlkPassCfg<N, AXIS, Op>::NT, BlkPassCfg<N, AXI
   if constexpr (Op::PEAK) block_argmax_store<NT>(op.partials, acc.mx, acc.idx);
 }
 
+// ---- the column pass of the Fourier-space crossover
+// The pixels that child w takes from the crossed parents, as a bit per element
+// of the column pass's threads (SpBits): the polar coordinates of a pixel cost
+// more than its share of the pass, and here one thread has nothing else to
+// hold.
+template <int N>
+__global__ void k_cross_bits(const CrossArgs a) {
+  constexpr int W = Blocked<N>::BC, TPT = Plan<N>::TPT, NT = W * TPT, E = Elems<N>::value;
+  const CrossChild c = a.children[blockIdx.y];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // (tile, thread)
+  if (i >= N * TPT) return;
+  const int tile = i / NT, t = i % NT;
+  unsigned bits = 0;
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    bits |= cross_pixel(tile * W + t % W, elem_pos<N>(e, t / W), N, c, a.crosssym, a.cmaps, a.cmap_total) ? 1u << e : 0u;
+  reinterpret_cast<SpBits<N>*>(a.bits)[(size_t)blockIdx.y * N * TPT + i] = (SpBits<N>)bits;
+}
+
+// row pass of the children's parents: gathered copy of item blockIdx / TPI ->
+// FFT+ (x) -> W; the shifted supports of self, p2 and p3 into Ws.  (450 us at
+// 512^2 x 64, four parents a child: the reads at any shift and the int32
+// supports take twice the L1 line requests of the plain forward pass.)
+template <int N>
+__global__ void __launch_bounds__(BlkCfg<N, Blocked<N>::WR, 1>::NT,
+                                  BlkCfg<N, Blocked<N>::WR, 1>::E <= 8 ? 1024 / BlkCfg<N, Blocked<N>::WR, 1>::NT : 2)
+    k_cross_rows(const CrossArgs a, Gate g, const float2* __restrict__ twg) {
+  using B = Blocked<N>;
+  constexpr int W = B::WR;
+  using C = BlkCfg<N, W, 1>;
+  constexpr int E = C::E, TPI = N / W;
+  constexpr size_t npix = (size_t)N * N;
+  extern __shared__ __align__(128) unsigned char sm[];
+  float2* tw = reinterpret_cast<float2*>(sm);
+  float2* xb = reinterpret_cast<float2*>(sm + C::TWB);
+  pdl_enter();
+  load_twiddles<N>(tw, twg, C::NT);
+  const int c = threadIdx.x % W, j = threadIdx.x / W;
+  const int p = blockIdx.x / TPI, y = (blockIdx.x % TPI) * W + c;
+  pdl_wait();
+  __syncthreads();
+  const ShiftItem it = load_item(a.items + p);
+  const int row = shift_source(it, j, y, N) / N;  // of the source: the same for the whole row
+  const int x0 = (it.flip ? N - 1 - j : j) - it.sx, dir = it.flip ? -1 : 1;
+  const float2* src = a.rho + (size_t)it.src * npix + (size_t)row * N;
+  // (an item without a support of its own is gated with gsrc, unshifted: only
+  // the plain copy, whose shift is 0)
+  const int ss = it.ssrc >= 0 ? it.ssrc : it.gsrc;
+  const int* sup = a.S + (size_t)max(ss, 0) * npix + (size_t)row * N;
+  float2 v[E];
+  int s[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    int x = x0 + dir * C::step(e);
+    x += x < 0 ? N : (x >= N ? -N : 0);
+    v[e] = __ldcg(src + x);
+    s[e] = ss >= 0 ? __ldcg(sup + x) : 0;
+  }
+  if (it.sdst >= 0) {
+    int* ws = a.Ws + (size_t)it.sdst * npix + (size_t)y * N + j;
+#pragma unroll
+    for (int e = 0; e < E; ++e) ws[C::step(e)] = s[e];
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    v[e] = shift_value(it, v[e]);
+    if (it.gate) {
+      const float t = s[e] == 0 || phase_out(v[e], g) ? 0.f : (float)s[e];
+      v[e] = make_float2(v[e].x * t, v[e].y * t);
+    }
+  }
+  fft_x<N, typename C::Lay, +1, 1, 0>(v, xb, tw, c, j);
+  float2* o = a.W + (size_t)p * npix + B::at(y, j);
+#pragma unroll
+  for (int e = 0; e < E; ++e) o[(size_t)(C::step(e) / B::BC) * B::XS] = v[e];
+}
+
+// W[per w + k] (row transforms) -> FFT+ (y) -> crossed child -> FFT- (y) -> C[w].
+// Each parent is transformed in turn and only its share kept, so the parents'
+// spectra never reach memory (they were written once and read twice).
+template <int N, bool AVG>
+__global__ void __launch_bounds__(BlkCfg<N, Blocked<N>::BC, 1>::NT,
+                                  BlkCfg<N, Blocked<N>::BC, 1>::E <= 8 ? 768 / BlkCfg<N, Blocked<N>::BC, 1>::NT : 1)
+    k_cross_cols(const CrossArgs a, const float* __restrict__ At, const float2* __restrict__ twg) {
+  using B = Blocked<N>;
+  constexpr int W = B::BC;
+  using C = BlkCfg<N, W, 1>;
+  using Lay = typename C::Lay;
+  constexpr int NT = C::NT, E = C::E, TPI = N / W;
+  extern __shared__ __align__(128) unsigned char sm[];
+  float2* tw = reinterpret_cast<float2*>(sm);
+  float2* xb = reinterpret_cast<float2*>(sm + C::TWB);
+  pdl_enter();
+  load_twiddles<N>(tw, twg, NT);
+  const int t = threadIdx.x, c = t % W, j = t / W;
+  const int w = blockIdx.x / TPI, tile = blockIdx.x % TPI;
+  constexpr size_t npix = (size_t)N * N;
+  const size_t t0 = B::at(j, tile * W + c);
+  pdl_wait();
+  __syncthreads();
+  const unsigned bits = reinterpret_cast<const SpBits<N>*>(a.bits)[((size_t)w * TPI + tile) * NT + t];
+  auto spectrum = [&](float2* v, int k) {
+    const float2* g = a.W + ((size_t)a.per * w + k) * npix + t0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = __ldcg(g + (size_t)C::step(e) * B::YS);
+    fft_x<N, Lay, +1, 1, 0>(v, xb, tw, c, j);
+  };
+  float2 out[E], d[E], v[E];
+  spectrum(out, 0);
+  spectrum(d, 2);
+  spectrum(v, 3);
+#pragma unroll
+  for (int e = 0; e < E; ++e) d[e] = make_float2(d[e].x - v[e].x, d[e].y - v[e].y);
+  float amod[AVG ? E : 1];
+  if (AVG) {
+    spectrum(v, 4);
+#pragma unroll
+    for (int e = 0; e < E; ++e) amod[AVG ? e : 0] = sqrtf(v[e].x * v[e].x + v[e].y * v[e].y);
+  }
+  spectrum(v, 1);
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    float2 d1 = v[e];
+    if (AVG && ((bits >> e) & 1u) && At[((size_t)tile * NT + t) * E + e] < 0.f)
+      d1 = cross_average(d1, a.avg_mod[(size_t)(j + C::step(e)) * N + tile * W + c], amod[AVG ? e : 0], a.use_average);
+    if ((bits >> e) & 1u) out[e] = make_float2(d1.x + a.crossdiff * d[e].x, d1.y + a.crossdiff * d[e].y);
+  }
+  fft_x<N, Lay, -1, 1, 0>(out, xb, tw, c, j);
+  float2* o = a.C + (size_t)w * npix + t0;
+#pragma unroll
+  for (int e = 0; e < E; ++e) o[(size_t)C::step(e) * B::YS] = out[e];
+}
+
 // amplitudes in the order of the column pass's registers: At[(tile of BC
 // columns) * NT + thread][e]; with BAND, the correlation ops' weights
 // (band_weight) of the band [minr, maxr] instead

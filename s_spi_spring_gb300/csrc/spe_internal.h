@@ -72,6 +72,59 @@ struct Ctx {
   unsigned* bad;       // per individual: a gradient that is not finite
 };
 
+// One gathered, shifted copy of an individual (reference shift kernel,
+// gpu_context.cu:1329-1357, as a gather: destination pixel d reads the source
+// pixel that the reference's scatter writes to d), optionally gated by
+// apply_support_er with the shifted support (gpu_context.cu:519-537).
+struct ShiftItem {
+  int src;       // source density slot (in the source pool)
+  int dst;       // destination density slot
+  int ssrc;      // source support slot or -1
+  int sdst;      // destination support slot or -1
+  int sx, sy;    // shift
+  float pc, ps;  // cosine and sine of the added phase
+  int flip;      // point reflection (twin image)
+  int polar;     // 0: plain copy (no shift, flip or phase)
+  int gate;      // apply the phase/support gate with the (shifted) support
+  int gsrc;      // gate with support slot gsrc of the source support pool when no ssrc (-1: none)
+};
+
+// One child of the crossover (reference cross_density / cross_density_real /
+// cross_support, gpu_context.cu:1699-1883)
+struct CrossChild {
+  int cft;           // Fourier-space crossover
+  int csx, csy;      // crossmap cells
+  int ssx, ssy;      // cell sizes
+  int ox, oy;        // offsets
+  float rot;         // rotation angle
+  int cmap;          // offset of the crossmap in the crossmap pool
+  int w;             // work index
+  int p1;            // slot of parent 1 (its support is S1)
+  int self, dst;     // slots of the child's own parent and of the child
+};
+
+// Operands of the crossover's kernels.  Work arrays of child w: W[per w + k],
+// k = 0 self', 1 p1, 2 p2', 3 p3', 4 avg' (per = 5; 4 where the average is not
+// used); Ws[3 w + k], k = 0 S', 1 S2', 2 S3'; C[w] the child.
+struct CrossArgs {
+  const float2* rho;   // source pool
+  const int* S;
+  float2* rho_out;     // the population that the children join
+  int* S_out;
+  const ShiftItem* items;    // per w + k
+  const CrossChild* children;  // in work order
+  float2* W;
+  int* Ws;
+  float2* C;
+  unsigned char* bits;  // crossed pixels in column-pass order, one byte or 16-bit word per thread
+  const int* cmaps;
+  int cmap_total;
+  const float* avg_mod;
+  int per, count;       // count children from work index 0
+  float crossdiff, use_average;
+  int crosssym, update_support;
+};
+
 // One Adam step (SizeOps::adam_step).  On sides with blocked passes a run of
 // steps may leave out what it knows: prepared (Ctx::T holds the forward row
 // pass: the step before had `next`), fresh (the moments are 0 and not read),
@@ -144,6 +197,10 @@ struct SizeOps {
   cudaError_t (*corr_peaks)(const Ctx&, const float2* D, const float2* Dref, const int* xi, const int* ri,
                             int norm_d, int norm_ref, float2* scratch1, float2* scratch2, double* part1,
                             double* part2);
+  // Fourier-space children from gathered parents to population slots
+  // (CrossArgs; the amplitudes of Ctx), or null where the side has no blocked
+  // passes
+  cudaError_t (*cross_fourier)(const Ctx&, const CrossArgs&, Gate g);
   // band-pass weights of the correlation ops for `npatterns` patterns
   cudaError_t (*band_table)(const float* A, float* band, int n, int npatterns, float minr, float maxr,
                             cudaStream_t st);

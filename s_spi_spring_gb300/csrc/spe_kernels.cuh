@@ -268,7 +268,7 @@ __device__ __forceinline__ void pass_elements(const Op& op, const PxF& px, typen
 #pragma unroll
       for (int e = 0; e < E; ++e) r[e] = op.fetch(px(e));
 #pragma unroll
-      for (int e = 0; e < E; ++e) v[e] = op.form(r[e], acc);
+      for (int e = 0; e < E; ++e) v[e] = op.form(r[e], px(e), acc);
     } else {
 #pragma unroll
       for (int e = 0; e < E; ++e) v[e] = op.load(px(e), acc);
@@ -279,8 +279,16 @@ __device__ __forceinline__ void pass_elements(const Op& op, const PxF& px, typen
       for (int e = 0; e < E; ++e) v[e] = op.mid(v[e], px(e), op.fetch_mid(px(e)), acc);
       fft(v, std::integral_constant<int, Op::FFT2>());
     }
+    if constexpr (Op::FETCH_STORE) {
+      typename Op::Raw r[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) op.store(v[e], px(e), acc);
+      for (int e = 0; e < E; ++e) r[e] = op.fetch_store(px(e));
+#pragma unroll
+      for (int e = 0; e < E; ++e) op.store(v[e], px(e), r[e]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) op.store(v[e], px(e), acc);
+    }
   }
 }
 
@@ -344,6 +352,7 @@ struct OpBase {
   // (roots, the phase gate), across which a thread's memory reads are not
   // reordered -- all are issued before the first value is formed
   static constexpr bool FETCH = false;
+  static constexpr bool FETCH_STORE = false;  // likewise fetch_store, then store
   // likewise the operands of the pointwise step: fetch_mid, then mid
   struct Mid {};
   template <class Q>
@@ -390,7 +399,7 @@ struct OpRowsForward : OpKeep {
   static constexpr bool FETCH = SRC == SRC_ABS_SUM;
   using Raw = float2;
   __device__ float2 fetch(const Px& q) const { return rho[q.gi]; }
-  __device__ float2 form(float2 v, Acc& acc) const {
+  __device__ float2 form(float2 v, const Px&, Acc& acc) const {
     if (SRC == SRC_ABS_SUM) {
       acc.s += v.x;
       acc.t += v.y;
@@ -398,7 +407,7 @@ struct OpRowsForward : OpKeep {
     }
     return v;
   }
-  __device__ float2 load(const Px& q, Acc& acc) const { return form(fetch(q), acc); }
+  __device__ float2 load(const Px& q, Acc& acc) const { return form(fetch(q), q, acc); }
   __device__ void store(float2 v, const Px& q, Acc&) const { T[q.ti] = v; }
 };
 
@@ -945,6 +954,126 @@ struct OpColsCrossPower : OpBase {
     c2 = weighted(cross_power<+1>(d, r), q.a);
   }
   __device__ void store_pair(float2 v, const Px& q, int second) const { (second ? dst2 : dst)[q.ti] = v; }
+};
+
+// ---- crossover (reference cross_density / cross_density_real /
+// cross_support, gpu_context.cu:1699-1883; the gathered parents of
+// prepare_parents / reshift_parent, 1536-1694)
+
+// (read-only loads: one read of the item serves a thread's pixels, whatever is
+// stored in between)
+__device__ __forceinline__ ShiftItem load_item(const ShiftItem* p) {
+  static_assert(sizeof(ShiftItem) == 48, "three 16-byte reads");
+  union {
+    int4 v[3];
+    ShiftItem it;
+  } u;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) u.v[i] = __ldg(reinterpret_cast<const int4*>(p) + i);
+  return u.it;
+}
+
+// source pixel (row-major offset) of destination pixel (x, y)
+__device__ __forceinline__ int shift_source(const ShiftItem& it, int x, int y, int n) {
+  if (!it.polar) return y * n + x;
+  int ix = (it.flip ? n - 1 - x : x) - it.sx, iy = (it.flip ? n - 1 - y : y) - it.sy;
+  if (ix < 0) ix += n;
+  if (ix >= n) ix -= n;
+  if (iy < 0) iy += n;
+  if (iy >= n) iy -= n;
+  return iy * n + ix;
+}
+// modulus kept, phase (mirrored by the flip) + the item's: a rotation
+__device__ __forceinline__ float2 shift_value(const ShiftItem& it, float2 v) {
+  if (!it.polar) return v;
+  const float y = it.flip ? -v.y : v.y;
+  return make_float2(fmaf(v.x, it.pc, -y * it.ps), fmaf(v.x, it.ps, y * it.pc));
+}
+
+// whether pixel (ix, iy) of child c comes from the crossed parents
+__device__ __forceinline__ bool cross_pixel(int ix, int iy, int n, const CrossChild& c, int crosssym,
+                                            const int* __restrict__ cmaps, int cmap_total) {
+  int x = ix, y = iy;
+  if (x >= n / 2) x -= n;
+  if (y >= n / 2) y -= n;
+  float radius = sqrtf((float)(x * x + y * y));
+  if ((double)radius >= n / 2.) radius = (float)(n / 2 - 1);
+  float angle = atan2f((float)y, (float)x);
+  if (crosssym && angle < 0.f) angle = (float)((double)angle + 3.14159265358979323846);
+  angle += c.rot;
+  float sn, cs;
+  sincosf(angle, &sn, &cs);
+  x = (int)(cs * radius) + n / 2;
+  y = (int)(sn * radius) + n / 2;
+  const int cx = (x + c.ox) / c.ssx;
+  const int cy = (y + c.oy) / c.ssy;
+  const int cell = cx + cy * c.csx;
+  const bool inside = cx >= 0 && cy >= 0 && cx < c.csx && cy < c.csy && c.cmap + cell < cmap_total;
+  return inside && cmaps[c.cmap + cell] == 1;
+}
+
+// parent 1 at an unmeasured pixel of Fourier space, pulled towards the average
+// (avgmod: the averaged modulus, amod: the modulus of the averaged density)
+__device__ __forceinline__ float2 cross_average(float2 d1, float avgmod, float amod, float use_average) {
+  const float mod1 = sqrtf(d1.x * d1.x + d1.y * d1.y);
+  if (use_average > 0.f) {
+    const float avg = (float)((double)(avgmod + amod) * 0.5);
+    const float newmod = (float)((double)(avg * use_average) + (1. - (double)use_average) * (double)mod1);
+    if (mod1 > 0.f) {
+      const float r = newmod / mod1;
+      d1 = make_float2(d1.x * r, d1.y * r);
+    }
+  } else if (use_average < 0.f && mod1 > 0.f) {
+    const float loc = fabsf(use_average);
+    const float maxmod = avgmod, minmod = amod;
+    float newmod = mod1;
+    if (newmod < minmod)
+      newmod = (float)((double)(minmod * loc) + (double)newmod * (1. - (double)loc));
+    else if (newmod > maxmod)
+      newmod = (float)((double)(maxmod * loc) + (double)newmod * (1. - (double)loc));
+    const float r = newmod / mod1;
+    d1 = make_float2(d1.x * r, d1.y * r);
+  }
+  return d1;
+}
+
+// a child's new support S_new = [S1 + S2' S3' S' > 0.5] and its operands
+struct ChildSupport {
+  int s1, a, b, c, self;
+};
+__device__ __forceinline__ ChildSupport child_support(const CrossArgs& a, const CrossChild* c, size_t npix, size_t i) {
+  const int* ws = a.Ws + (size_t)__ldg(&c->w) * 3 * npix + i;
+  return {a.S[(size_t)__ldg(&c->p1) * npix + i], ws[0], ws[npix], ws[2 * npix],
+          a.update_support ? 0 : a.S[(size_t)__ldg(&c->self) * npix + i]};
+}
+// child -> its population slot: apply_support_er with the new support
+// (gpu_context.cu:2114); the support from the crossover or the parent's own
+__device__ __forceinline__ void child_store(const CrossArgs& a, const CrossChild* c, size_t npix, size_t i, float2 v,
+                                            const ChildSupport& r, const GateK& g) {
+  const int s = r.s1 + r.b * r.c * r.a > 0 ? 1 : 0;
+  const float t = s == 0 || phase_out(v, g) ? 0.f : 1.f;
+  const size_t d = (size_t)__ldg(&c->dst) * npix + i;
+  a.rho_out[d] = make_float2(v.x * t, v.y * t);
+  a.S_out[d] = a.update_support ? s : r.self;
+}
+
+// last row pass of a Fourier-space child: C[w] -> FFT- (x) -> /N^2 -> slot
+struct OpRowsChild : OpKeep {
+  static constexpr int FFT1 = -1, FFT2 = 0;
+  static constexpr bool FETCH_STORE = true;
+  CrossArgs a;
+  size_t npix;
+  float scale;
+  GateK g;
+  using Acc = NoAcc;
+  using Raw = ChildSupport;
+  __device__ float2 load(const Px& q, Acc&) const { return a.C[q.ti]; }
+  __device__ Raw fetch_store(const Px& q) const {
+    return child_support(a, a.children + q.p, npix, q.gi - (size_t)q.p * npix);
+  }
+  __device__ void store(float2 v, const Px& q, const Raw& r) const {
+    child_store(a, a.children + q.p, npix, q.gi - (size_t)q.p * npix, make_float2(v.x * scale, v.y * scale), r, g);
+  }
 };
 
 }  // namespace spe

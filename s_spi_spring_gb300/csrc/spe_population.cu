@@ -30,58 +30,23 @@ __global__ void k_int_sum(const int* __restrict__ s, size_t npix, long long* __r
   if ((threadIdx.x & 31) == 0) atomicAdd((unsigned long long*)out, (unsigned long long)acc);
 }
 
-// One gathered, shifted copy (reference shift kernel, gpu_context.cu:1329-1357,
-// as a gather: destination pixel d reads the source pixel that the
-// reference's scatter writes to d), optionally gated by apply_support_er
-// with the shifted support (gpu_context.cu:519-537).
-struct ShiftItem {
-  int src;       // source density slot (in the source pool)
-  int dst;       // destination density slot
-  int ssrc;      // source support slot or -1
-  int sdst;      // destination support slot or -1
-  int sx, sy;    // shift
-  float phase;   // added phase
-  int flip;      // point reflection (twin image)
-  int polar;     // 0: plain copy (no shift), 1: modulus/phase rewrite
-  int gate;      // apply the phase/support gate with the (shifted) support
-  int gsrc;      // gate with support slot gsrc of the source support pool when no sdst (-1: none)
-};
-
+// The gathered copies of `items` (ShiftItem)
 __global__ void k_shift_gather(const float2* __restrict__ srcpool, const int* __restrict__ ssrcpool,
                                float2* __restrict__ dstpool, int* __restrict__ sdstpool,
                                const ShiftItem* __restrict__ items, int n, Gate g) {
   const ShiftItem it = items[blockIdx.y];
-  const size_t npix = (size_t)n * n;
-  const size_t d = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const unsigned npix = (unsigned)n * n;
+  const unsigned d = blockIdx.x * blockDim.x + threadIdx.x;
   if (d >= npix) return;
-  size_t old = d;
-  if (it.polar) {
-    const size_t dd = it.flip ? npix - 1 - d : d;
-    int nx = (int)(dd % n), ny = (int)(dd / n);
-    int ix = nx - it.sx, iy = ny - it.sy;
-    if (ix < 0) ix += n;
-    if (ix >= n) ix -= n;
-    if (iy < 0) iy += n;
-    if (iy >= n) iy -= n;
-    old = (size_t)ix + (size_t)iy * n;
-  }
+  const unsigned y = d / (unsigned)n, x = d - y * n;
+  const int old = shift_source(it, (int)x, (int)y, n);
   const float2 v = srcpool[(size_t)it.src * npix + old];
-  float2 out = v;
-  if (it.polar) {
-    const float mod = sqrtf(v.x * v.x + v.y * v.y);
-    float ph = atan2f(v.y, v.x);
-    if (it.flip) ph = -ph;
-    ph += it.phase;
-    float sn, cs;
-    sincosf(ph, &sn, &cs);
-    out = make_float2(mod * cs, mod * sn);
-  }
-  int sval = 0;
-  if (it.ssrc >= 0) sval = ssrcpool[(size_t)it.ssrc * npix + old];
+  const int ss = it.ssrc >= 0 ? it.ssrc : it.gsrc;
+  const int sval = ss >= 0 ? ssrcpool[(size_t)ss * npix + (it.ssrc >= 0 ? old : (int)d)] : 0;
+  float2 out = shift_value(it, v);
   if (it.sdst >= 0) sdstpool[(size_t)it.sdst * npix + d] = sval;
   if (it.gate) {
-    const int gs = (it.ssrc >= 0) ? sval : ssrcpool[(size_t)it.gsrc * npix + d];
-    const float t = phase_out(out, g) ? 0.f : (float)gs;
+    const float t = sval == 0 || phase_out(out, g) ? 0.f : (float)sval;
     out = make_float2(out.x * t, out.y * t);
   }
   dstpool[(size_t)it.dst * npix + d] = out;
@@ -123,105 +88,33 @@ __global__ void k_abs(const float2* __restrict__ src, float* __restrict__ M, siz
   }
 }
 
-// ---- crossover (reference cross_density / cross_density_real /
-// cross_support, gpu_context.cu:1699-1883)
-struct CrossChild {
-  int cft;           // Fourier-space crossover
-  int csx, csy;      // crossmap cells
-  int ssx, ssy;      // cell sizes
-  int ox, oy;        // offsets
-  float rot;         // rotation angle
-  int cmap;          // offset of the crossmap in the crossmap pool
-  int w;             // work index
-  int p1;            // slot of parent 1 (its support is S1)
-};
-
-// W[5w+k]: k=0 self', 1 p1, 2 p2', 3 p3', 4 avg' ; result -> C[w]
-__global__ void k_cross(const float2* __restrict__ W, float2* __restrict__ C, const CrossChild* __restrict__ ch,
-                        const int* __restrict__ cmaps, int cmap_total, const float* __restrict__ A,
-                        const float* __restrict__ avg_mod, int n, float crossdiff, float use_average, int crosssym) {
-  const CrossChild c = ch[blockIdx.y];
-  const size_t npix = (size_t)n * n;
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+// ---- crossover of the children from work index `from` on whose parents W
+// holds whole (spatial ones, and Fourier-space ones of sides without blocked
+// passes)
+__global__ void k_cross(const CrossArgs a, int from, const float* __restrict__ A, int n) {
+  const CrossChild c = a.children[from + blockIdx.y];
+  const unsigned npix = (unsigned)n * n;
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= npix) return;
-  const int ix = (int)(i % n), iy = (int)(i / n);
-  int x = ix, y = iy;
-  if (x >= n / 2) x -= n;
-  if (y >= n / 2) y -= n;
-  float radius = sqrtf((float)(x * x + y * y));
-  if ((double)radius >= n / 2.) radius = (float)(n / 2 - 1);
-  float angle = atan2f((float)y, (float)x);
-  if (crosssym && angle < 0.f) angle = (float)((double)angle + 3.14159265358979323846);
-  angle += c.rot;
-  float sn, cs;
-  sincosf(angle, &sn, &cs);
-  x = (int)(cs * radius) + n / 2;
-  y = (int)(sn * radius) + n / 2;
-  const int cx = (x + c.ox) / c.ssx;
-  const int cy = (y + c.oy) / c.ssy;
-  const int cell = cx + cy * c.csx;
-  const bool inside = cx >= 0 && cy >= 0 && cx < c.csx && cy < c.csy && c.cmap + cell < cmap_total;
-  const bool docross = inside && cmaps[c.cmap + cell] == 1;
-  const float2* w = W + (size_t)c.w * 5 * npix;
+  const float2* w = a.W + (size_t)c.w * a.per * npix;
   float2 out = w[i];
-  if (docross) {
+  if (cross_pixel((int)(i % (unsigned)n), (int)(i / (unsigned)n), n, c, a.crosssym, a.cmaps, a.cmap_total)) {
     float2 d1 = w[npix + i];
-    const float2 d2 = w[2 * npix + i], d3 = w[3 * npix + i];
-    if (c.cft && A[i] < 0.f) {
-      const float mod1 = sqrtf(d1.x * d1.x + d1.y * d1.y);
-      const float2 da = w[4 * npix + i];
-      const float amod = sqrtf(da.x * da.x + da.y * da.y);
-      if (use_average > 0.f) {
-        const float avgmod = (float)((double)(avg_mod[i] + amod) * 0.5);
-        const float newmod = (float)((double)(avgmod * use_average) + (1. - (double)use_average) * (double)mod1);
-        if (mod1 > 0.f) {
-          const float r = newmod / mod1;
-          d1 = make_float2(d1.x * r, d1.y * r);
-        }
-      } else if (use_average < 0.f && mod1 > 0.f) {
-        const float loc = fabsf(use_average);
-        const float maxmod = avg_mod[i], minmod = amod;
-        float newmod = mod1;
-        if (newmod < minmod)
-          newmod = (float)((double)(minmod * loc) + (double)newmod * (1. - (double)loc));
-        else if (newmod > maxmod)
-          newmod = (float)((double)(maxmod * loc) + (double)newmod * (1. - (double)loc));
-        const float r = newmod / mod1;
-        d1 = make_float2(d1.x * r, d1.y * r);
-      }
+    const float2 d2 = w[2 * (size_t)npix + i], d3 = w[3 * (size_t)npix + i];
+    if (a.per == 5 && c.cft && A[i] < 0.f) {
+      const float2 da = w[4 * (size_t)npix + i];
+      d1 = cross_average(d1, a.avg_mod[i], sqrtf(da.x * da.x + da.y * da.y), a.use_average);
     }
-    out = make_float2(d1.x + crossdiff * (d2.x - d3.x), d1.y + crossdiff * (d2.y - d3.y));
+    out = make_float2(d1.x + a.crossdiff * (d2.x - d3.x), d1.y + a.crossdiff * (d2.y - d3.y));
   }
-  C[(size_t)c.w * npix + i] = out;
+  a.C[(size_t)c.w * npix + i] = out;
 }
 
-// S_new = [S1 + S2'*S3'*S' > 0.5] into Ws[3w]
-__global__ void k_cross_support(int* __restrict__ Ws, const int* __restrict__ S, const CrossChild* __restrict__ ch,
-                                size_t npix) {
-  const CrossChild c = ch[blockIdx.y];
+__global__ void k_cross_finish(const CrossArgs a, int from, size_t npix, Gate g) {
+  const CrossChild* c = a.children + from + blockIdx.y;
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= npix) return;
-  int* ws = Ws + (size_t)c.w * 3 * npix;
-  const int s = S[(size_t)c.p1 * npix + i] + ws[npix + i] * ws[2 * npix + i] * ws[i];
-  ws[i] = (s > 0.5) ? 1 : 0;
-}
-
-// child -> population slot: apply_support_er with the new support
-// (gpu_context.cu:2114); support from the crossover or the parent's own
-__global__ void k_cross_finish(const float2* __restrict__ C, const int* __restrict__ Ws,
-                               const CrossChild* __restrict__ ch, const int* __restrict__ self_slot,
-                               const int* __restrict__ dst_slot, float2* __restrict__ rho, int* __restrict__ S,
-                               size_t npix, int update_support, Gate g) {
-  const int k = blockIdx.y;
-  const CrossChild c = ch[k];
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= npix) return;
-  const int s = Ws[(size_t)c.w * 3 * npix + i];
-  const float2 v = C[(size_t)c.w * npix + i];
-  const float t = phase_out(v, g) ? 0.f : (float)s;
-  const size_t d = (size_t)dst_slot[k] * npix + i;
-  rho[d] = make_float2(v.x * t, v.y * t);
-  S[d] = update_support ? s : S[(size_t)self_slot[k] * npix + i];
+  child_store(a, c, npix, i, a.C[(size_t)c->w * npix + i], child_support(a, c, npix, i), g);
 }
 
 // ---- starting population (Solver::Initialize_rec, src/solver.cpp:880-957):
@@ -335,18 +228,21 @@ int navg_of(float fraction, int count) {
 // gpu_context.cu:1309-1321)
 void decide_shift(int n, double m1, double i1, double m2, double i2, float ph, float ph_ref, spe::ShiftItem& it) {
   const int a = (int)i1, b = (int)i2;
+  float phase;
   it.polar = 1;
   if ((float)m1 >= (float)m2) {
     it.sx = a % n;
     it.sy = a / n;
-    it.phase = ph_ref - ph;
+    phase = ph_ref - ph;
     it.flip = 0;
   } else {
     it.sx = -b % n;
     it.sy = -b / n;
-    it.phase = ph_ref + ph;
+    phase = ph_ref + ph;
     it.flip = 1;
   }
+  it.pc = (float)std::cos((double)phase);
+  it.ps = (float)std::sin((double)phase);
 }
 
 float phase_of(const double* sums, int k) { return std::atan2((float)sums[2 * k + 1], (float)sums[2 * k]); }
@@ -657,18 +553,22 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
   const size_t npix = e->npix;
   const int tr = e->ops->tiles_rows;
   const int P = count;
-  const int items = 4 * P;
+  // without an averaging weight the averaged density and modulus reach no
+  // child: neither is aligned, gathered or transformed
+  const bool averaged = use_average != 0.f;
+  const int pairs = averaged ? 4 : 3, per = averaged ? 5 : 4;
+  const int items = pairs * P;
 
   // ---- host: order, support size, average module, draws (solver.cpp:716-801)
   const std::vector<int> order = sorted_order(errors, P);
   size_t need = (size_t)(P + 1) * npix * sizeof(float2)        // spectra
                 + (size_t)items * npix * sizeof(float2)        // correlation scratch
-                + (size_t)5 * P * npix * sizeof(float2)        // parents per child
+                + (size_t)5 * P * npix * sizeof(float2)        // parents per child (and correlation scratch)
                 + (size_t)P * npix * sizeof(float2)            // children
                 + (size_t)3 * P * npix * sizeof(int)           // supports per child
                 + (size_t)(2 * items + P + 1) * tr * spe::NRED * sizeof(double) + (size_t)items * 4 * sizeof(double) +
                 (size_t)(P + 1) * 2 * sizeof(double) + (size_t)items * (2 * sizeof(int) + sizeof(spe::ShiftItem)) +
-                (size_t)P * (sizeof(spe::CrossChild) + 2 * sizeof(int)) + 64 * 256;
+                (size_t)P * (sizeof(spe::CrossChild) + npix / 4 + 2 * sizeof(int)) + 64 * 256;
   const size_t mod_need = (size_t)P * npix * (sizeof(float) + sizeof(float2)) + P * sizeof(int) + 1024;
   if ((rc = ensure_work(e, std::max(need, mod_need)))) return rc;
   if (!e->avg_mod) CK(cudaMalloc(&e->avg_mod, npix * sizeof(float)), "average module buffer");
@@ -685,13 +585,13 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
     CK(cudaStreamSynchronize(e->st), "synchronize");
     // GetAverageModule(rec_array, true, 0.66) (solver.cpp:731)
     Carve cm{(char*)e->work};
-    if ((rc = average_module_dev(e, first, P, order, true, 0.66f, e->avg_mod, cm))) return rc;
+    if (averaged && (rc = average_module_dev(e, first, P, order, true, 0.66f, e->avg_mod, cm))) return rc;
     // suppdim (solver.cpp:724-729)
     float suppdim = (float)(2. * std::sqrt((double)float(hb) / M_PI));
     if (suppdim < 4.) suppdim = 4;
     if (suppdim > n / 4.) suppdim = n / 4.;
     bsum = nullptr;
-    CK(cudaStreamSynchronize(e->st), "synchronize");
+    if (averaged) CK(cudaStreamSynchronize(e->st), "synchronize");
 
     // draws, child by child, in the reference's order
     std::vector<spe::ChildDraw> dr;
@@ -715,6 +615,8 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
       c.rot = dr[i].rot;
       c.cmap = dr[i].cmap;
       c.p1 = first + p1[i];
+      c.self = first + i;
+      c.dst = dst_first + i;
     }
     // work order: Fourier-space children first (one contiguous transform batch)
     int ncft = 0;
@@ -741,8 +643,7 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
     int* ri = cv2.take<int>(items);
     spe::ShiftItem* sitems = cv2.take<spe::ShiftItem>(5 * P);
     spe::CrossChild* dch = cv2.take<spe::CrossChild>(P);
-    int* dself = cv2.take<int>(P);
-    int* ddst = cv2.take<int>(P);
+    unsigned char* bits = cv2.take<unsigned char>((size_t)P * npix / 4);
     int* dcm = cv2.take<int>(cmaps.size() + 1);
 
     // ---- alignment of self, p2, p3 and the average to p1
@@ -750,18 +651,19 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
     // not normalised on this path).  Spectra of the members and the average.
     spe::Ctx c = item_ctx(e, P, Apat);
     CK(e->ops->abs_spectrum_items(c, e->rho + (size_t)first * npix, D, psum), "spectra");
-    CK(e->ops->abs_spectrum_items(item_ctx(e, 1, Apat), e->rho + (size_t)avg_slot * npix, D + (size_t)P * npix,
-                                  psum + (size_t)P * tr * spe::NRED),
-       "average spectrum");
-    if ((rc = reduce(e, P + 1, {{psum, tr, 0, 0, 0}, {psum, tr, 1, 0, 1}}, sums, 2))) return rc;
+    if (averaged)
+      CK(e->ops->abs_spectrum_items(item_ctx(e, 1, Apat), e->rho + (size_t)avg_slot * npix, D + (size_t)P * npix,
+                                    psum + (size_t)P * tr * spe::NRED),
+         "average spectrum");
+    if ((rc = reduce(e, averaged ? P + 1 : P, {{psum, tr, 0, 0, 0}, {psum, tr, 1, 0, 1}}, sums, 2))) return rc;
     if ((rc = band_weights(e, first, P, minr, maxr))) return rc;
     std::vector<int> hx(items), hr(items);
     for (int i = 0; i < P; ++i) {
-      hx[4 * i + 0] = i;
-      hx[4 * i + 1] = p2[i];
-      hx[4 * i + 2] = p3[i];
-      hx[4 * i + 3] = P;  // average
-      for (int k = 0; k < 4; ++k) hr[4 * i + k] = p1[i];
+      const int src[4] = {i, p2[i], p3[i], P};  // (P: the average)
+      for (int k = 0; k < pairs; ++k) {
+        hx[pairs * i + k] = src[k];
+        hr[pairs * i + k] = p1[i];
+      }
     }
     CK(cudaMemcpyAsync(xi, hx.data(), items * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
     CK(cudaMemcpyAsync(ri, hr.data(), items * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
@@ -769,73 +671,62 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
     // (W holds nothing yet: scratch of the second product)
     CK(e->ops->corr_peaks(ci, D, D, xi, ri, 0, 0, scratch, W, part, part2), "correlation");
     if ((rc = reduce(e, items, {{part, tr, 0, 2, 0}, {part2, tr, 0, 2, 2}}, peaks, 4))) return rc;
-    std::vector<double> hp((size_t)items * 4), hs((size_t)(P + 1) * 2);
+    std::vector<double> hp((size_t)items * 4), hs((size_t)(averaged ? P + 1 : P) * 2);
     CK(cudaMemcpyAsync(hp.data(), peaks, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "peaks");
     CK(cudaMemcpyAsync(hs.data(), sums, hs.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "sums");
     CK(cudaStreamSynchronize(e->st), "synchronize");
 
-    // ---- gathered parents per child: W[5w+k], supports Ws[3w+k]
-    // (source pool: the population, slots absolute)
-    std::vector<spe::ShiftItem> hi(5 * P);
+    // ---- gathered parents per child (source pool: the population, slots absolute)
+    std::vector<spe::ShiftItem> hi(per * P);
+    std::vector<spe::CrossChild> hc(P);
     for (int i = 0; i < P; ++i) {
       const int w = ch[i].w;
+      hc[w] = ch[i];
       const float ph_ref = phase_of(hs.data(), p1[i]);
       const int srcs[4] = {first + i, first + p2[i], first + p3[i], avg_slot};
       const int sidx[4] = {i, p2[i], p3[i], P};
-      for (int k = 0; k < 4; ++k) {
-        spe::ShiftItem& it = hi[5 * i + (k == 0 ? 0 : k + 1)];
-        const int pi = 4 * i + k;
+      for (int k = 0; k < pairs; ++k) {
+        const int at = per * w + (k == 0 ? 0 : k + 1);
+        spe::ShiftItem& it = hi[at];
+        const int pi = pairs * i + k;
         decide_shift(n, hp[4 * pi], hp[4 * pi + 1], hp[4 * pi + 2], hp[4 * pi + 3], phase_of(hs.data(), sidx[k]),
                      ph_ref, it);
         it.src = srcs[k];
-        it.dst = 5 * w + (k == 0 ? 0 : k + 1);
+        it.dst = at;
         it.ssrc = (k == 3) ? -1 : srcs[k];
         it.sdst = (k == 0) ? 3 * w : (k == 1 ? 3 * w + 1 : (k == 2 ? 3 * w + 2 : -1));
         it.gate = (k == 3) ? 0 : 1;  // apply_support_er on self, p2, p3 (not the average)
         it.gsrc = -1;
       }
       // p1 itself: unshifted copy gated with its own support
-      spe::ShiftItem& it = hi[5 * i + 1];
-      it.src = first + p1[i];
-      it.dst = 5 * w + 1;
-      it.ssrc = -1;
-      it.sdst = -1;
-      it.sx = it.sy = 0;
-      it.phase = 0.f;
-      it.flip = 0;
-      it.polar = 0;
-      it.gate = 1;
-      it.gsrc = first + p1[i];
+      spe::ShiftItem& it = hi[per * w + 1];
+      it = spe::ShiftItem{first + p1[i], per * w + 1, -1, -1, 0, 0, 1.f, 0.f, 0, 0, 1, first + p1[i]};
     }
-    // k_shift_gather writes supports into Ws through sdst (pool Ws)
     CK(cudaMemcpyAsync(sitems, hi.data(), hi.size() * sizeof(spe::ShiftItem), cudaMemcpyHostToDevice, e->st),
        "items");
-    const spe::Gate g = gate_er(reality);
-    dim3 grid5((unsigned)((npix + 255) / 256), (unsigned)(5 * P));
-    spe::k_shift_gather<<<grid5, 256, 0, e->st>>>(e->rho, e->S, W, Ws, sitems, n, g);
-    CK(cudaGetLastError(), "parent gather");
-
-    // ---- Fourier-space children: transform their five parents
-    if (ncft > 0) CK(e->ops->fft2(item_ctx(e, 5 * ncft, Apat), W, +1), "parent transforms");
-    CK(cudaMemcpyAsync(dch, ch.data(), P * sizeof(spe::CrossChild), cudaMemcpyHostToDevice, e->st), "children");
+    CK(cudaMemcpyAsync(dch, hc.data(), P * sizeof(spe::CrossChild), cudaMemcpyHostToDevice, e->st), "children");
     CK(cudaMemcpyAsync(dcm, cmaps.data(), cmaps.size() * sizeof(int), cudaMemcpyHostToDevice, e->st), "crossmaps");
-    dim3 gridc((unsigned)((npix + 255) / 256), (unsigned)P);
-    spe::k_cross<<<gridc, 256, 0, e->st>>>(W, C, dch, dcm, (int)cmaps.size(), Apat, e->avg_mod, n, crossdiff,
-                                           use_average, crosssym);
-    CK(cudaGetLastError(), "crossover");
-    spe::k_cross_support<<<gridc, 256, 0, e->st>>>(Ws, e->S, dch, npix);
-    CK(cudaGetLastError(), "crossover support");
-    if (ncft > 0) CK(e->ops->fft2(item_ctx(e, ncft, Apat), C, -1), "child transforms");
-    std::vector<int> hself(P), hdst(P);
-    for (int i = 0; i < P; ++i) {
-      hself[i] = first + i;
-      hdst[i] = dst_first + i;
+    const spe::Gate g = gate_er(reality);
+    // (the children's slots are no parent's: the population is read and written)
+    const spe::CrossArgs a{e->rho, e->S, e->rho, e->S, sitems, dch, W, Ws, C, bits, dcm, (int)cmaps.size(),
+                           e->avg_mod, per, ncft, crossdiff, use_average, crosssym, update_support};
+    // Fourier-space children: their parents' transforms stay in the passes
+    // where the side has blocked ones; the others' go through W
+    const bool fused = e->ops->cross_fourier != nullptr;
+    const int from = fused ? ncft : 0;
+    if (fused && ncft > 0) CK(e->ops->cross_fourier(item_ctx(e, ncft, Apat), a, g), "Fourier-space children");
+    if (from < P) {
+      const unsigned px = (unsigned)((npix + 255) / 256);
+      spe::k_shift_gather<<<dim3(px, (unsigned)(per * (P - from))), 256, 0, e->st>>>(e->rho, e->S, W, Ws,
+                                                                                  sitems + per * from, n, g);
+      CK(cudaGetLastError(), "parent gather");
+      if (!fused && ncft > 0) CK(e->ops->fft2(item_ctx(e, per * ncft, Apat), W, +1), "parent transforms");
+      spe::k_cross<<<dim3(px, (unsigned)(P - from)), 256, 0, e->st>>>(a, from, Apat, n);
+      CK(cudaGetLastError(), "crossover");
+      if (!fused && ncft > 0) CK(e->ops->fft2(item_ctx(e, ncft, Apat), C, -1), "child transforms");
+      spe::k_cross_finish<<<dim3(px, (unsigned)(P - from)), 256, 0, e->st>>>(a, from, npix, g);
+      CK(cudaGetLastError(), "crossover finish");
     }
-    CK(cudaMemcpyAsync(dself, hself.data(), P * sizeof(int), cudaMemcpyHostToDevice, e->st), "slots");
-    CK(cudaMemcpyAsync(ddst, hdst.data(), P * sizeof(int), cudaMemcpyHostToDevice, e->st), "slots");
-    spe::k_cross_finish<<<gridc, 256, 0, e->st>>>(C, Ws, dch, dself, ddst, e->rho, e->S, npix, update_support,
-                                                  g);
-    CK(cudaGetLastError(), "crossover finish");
     CK(cudaStreamSynchronize(e->st), "synchronize");
   }
   return SPE_OK;

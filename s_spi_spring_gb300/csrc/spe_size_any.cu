@@ -493,7 +493,10 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
         for (int u = 0; u < U; ++u) if (i0 + u * NT < tot) r[u] = op.fetch(px(i0 + u * NT, at[u]));
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          if (i0 + u * NT < tot) cur[at[u]] = op.form(r[u], acc);
+          if (i0 + u * NT < tot) {
+            int x;
+            cur[at[u]] = op.form(r[u], px(i0 + u * NT, x), acc);
+          }
       } else {
         float2 v[U];
 #pragma unroll
@@ -1031,6 +1034,7 @@ const SizeOps* size_ops_any(int n) {
                     &SizeAny::ft_magnitude,
                     &SizeAny::abs_spectrum_items,
                     &SizeAny::corr_peaks,
+                    nullptr,
                     &launch_band_table,
                     &SizeAny::one_width,
                     &SizeAny::one_width,

@@ -518,6 +518,25 @@ cudaError_t launch_rows_w(const Ctx& c, int w, float scale, float beta, Gate g) 
   return cudaErrorInvalidValue;
 }
 
+template <int N>
+cudaError_t launch_cross_rows(const Ctx& c, const CrossArgs& a, Gate g) {
+  using P = BlkCfg<N, Blocked<N>::WR, 1>;
+  auto kern = k_cross_rows<N>;
+  static std::atomic<unsigned long long> configured{0ull};
+  cudaError_t e = configure(kern, P::SMEM, configured);
+  if (e != cudaSuccess || a.count <= 0) return e;
+  return launch_pdl(kern, a.per * a.count * (N / Blocked<N>::WR), P::NT, P::SMEM, c.st, a, g, c.tw);
+}
+template <int N, bool AVG>
+cudaError_t launch_cross_cols(const Ctx& c, const CrossArgs& a) {
+  using P = BlkCfg<N, Blocked<N>::BC, 1>;
+  auto kern = k_cross_cols<N, AVG>;
+  static std::atomic<unsigned long long> configured{0ull};
+  cudaError_t e = configure(kern, P::SMEM, configured);
+  if (e != cudaSuccess || a.count <= 0) return e;
+  return launch_pdl(kern, a.count * (N / Blocked<N>::BC), P::NT, P::SMEM, c.st, a, c.At, c.tw);
+}
+
 #define SPE_TRY(x)                         \
   do {                                     \
     cudaError_t e_ = (x);                  \
@@ -727,28 +746,33 @@ struct SizeImpl {
   }
 
   // ---- generic transforms over `c.count` items starting at `data` (c.first ignored)
+  // (the Fourier-space crossover of the sides without blocked passes)
   static cudaError_t fft2(const Ctx& c, float2* data, int sign) {
-    if (sign > 0) {
-      Ctx z = c;
-      z.first = 0;
-      SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, data, data, nullptr), c.count, c.st, c.tw)));
-      OpColsTransform<+1> ct;
+    if constexpr (Blocked<N>::ok) {
+      return cudaErrorInvalidValue;
+    } else {
+      if (sign > 0) {
+        Ctx z = c;
+        z.first = 0;
+        SPE_TRY((launch_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, data, data, nullptr), c.count, c.st, c.tw)));
+        OpColsTransform<+1> ct;
+        ct.first = 0;
+          ct.src = data;
+        ct.dst = data;
+        return launch_pass<N, AX_COLS>(ct, c.count, c.st, c.tw);
+      }
+      OpColsTransform<-1> ct;
       ct.first = 0;
-        ct.src = data;
+      ct.src = data;
       ct.dst = data;
-      return launch_pass<N, AX_COLS>(ct, c.count, c.st, c.tw);
+      SPE_TRY((launch_pass<N, AX_COLS>(ct, c.count, c.st, c.tw)));
+      OpRowsFinal fin;
+      fin.first = 0;
+      fin.T = data;
+      fin.out = data;
+      fin.scale = scale();
+      return launch_pass<N, AX_ROWS>(fin, c.count, c.st, c.tw);
     }
-    OpColsTransform<-1> ct;
-    ct.first = 0;
-    ct.src = data;
-    ct.dst = data;
-    SPE_TRY((launch_pass<N, AX_COLS>(ct, c.count, c.st, c.tw)));
-    OpRowsFinal fin;
-    fin.first = 0;
-    fin.T = data;
-    fin.out = data;
-    fin.scale = scale();
-    return launch_pass<N, AX_ROWS>(fin, c.count, c.st, c.tw);
   }
 
   // M[p] = |FFT+(src[p])| (2D), tmp: scratch of count items
@@ -792,6 +816,24 @@ struct SizeImpl {
     z.first = 0;
     SPE_TRY(rows_peak(z, scratch1, part1));
     return rows_peak(z, scratch2, part2);
+  }
+
+  // parents' row transforms, column pass, children's rows
+  static cudaError_t cross_fourier(const Ctx& c, const CrossArgs& a, Gate g) {
+    if constexpr (Blocked<N>::ok) {
+      SPE_TRY(launch_cross_rows<N>(c, a, g));
+      k_cross_bits<N><<<dim3((N * Plan<N>::TPT + 127) / 128, (unsigned)a.count), 128, 0, c.st>>>(a);
+      SPE_TRY(cudaGetLastError());
+      SPE_TRY((a.per == 5 ? launch_cross_cols<N, true>(c, a) : launch_cross_cols<N, false>(c, a)));
+      OpRowsChild ch;
+      ch.a = a;
+      ch.npix = (size_t)N * N;
+      ch.scale = scale();
+      ch.g = g;
+      return run_pass<N, AX_ROWS>(ch, a.count, c.st, c.tw);
+    } else {
+      return cudaErrorInvalidValue;
+    }
   }
 
   // partials (rows of the column pass): sum_{A>=0} |FFT+(rho)|^2, sum_{A>=0} A^2
@@ -928,6 +970,7 @@ struct SizeImpl {
                               &SizeImpl<N>::ft_magnitude,
                               &SizeImpl<N>::abs_spectrum_items,
                               &SizeImpl<N>::corr_peaks,
+                              Blocked<N>::ok ? &SizeImpl<N>::cross_fourier : nullptr,
                               &SizeImpl<N>::band_table,
                               &SizeImpl<N>::col_widths,
                               &SizeImpl<N>::row_widths,
