@@ -7,6 +7,7 @@
 #include "spe_kernels.cuh"
 #include "spe_pipe.cuh"
 #include "spe_blocked.cuh"
+#include "spe_cluster.cuh"
 #include "spe_support.cuh"
 #include "spe_pairs.cuh"
 #include "spe_tma.cuh"
@@ -322,6 +323,28 @@ cudaError_t launch_rows_blocked_last(const Ctx& c, float scale) {
   return cudaGetLastError();
 }
 
+// ---- one cluster per individual (spe_cluster.cuh)
+template <int N, int UPD>
+cudaError_t launch_cluster(const Ctx& c, int iters, float scale, float beta, Gate g) {
+  using P = ClusterCfg<N>;
+  auto kern = k_cluster_iterate<N, UPD>;
+  static std::atomic<unsigned long long> configured{0ull};
+  cudaError_t e = configure(kern, P::SMEM, configured);
+  if (e != cudaSuccess || c.count <= 0) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)c.count * P::CL);
+  cfg.blockDim = dim3(P::NT);
+  cfg.dynamicSmemBytes = P::SMEM;
+  cfg.stream = c.st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim = {P::CL, 1, 1};
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, c.rho, static_cast<const int*>(c.S), c.A, c.ipp, c.first, iters, scale, beta,
+                            g, c.tw);
+}
+
 template <int N, int WP>
 cudaError_t launch_cols_pairs_st(const Ctx& c) {
   using P = PairColStCfg<N, WP>;
@@ -611,6 +634,15 @@ struct SizeImpl {
   // caller holds their operands (an engine does, the allocation-free entry
   // point does not)
   static cudaError_t iterate(const Ctx& c, int upd, int iters, float beta, Gate g, int wc, int wr) {
+    if constexpr (ClusterCfg<N>::ok) {
+      if (wc == 0 && wr <= 0 && c.count <= ClusterCfg<N>::MOST && !c.mark && c.grid_div <= 1) {
+        switch (upd) {
+          case 0: return launch_cluster<N, UPD_HIO>(c, iters, scale(), beta, g);
+          case 1: return launch_cluster<N, UPD_RAAR>(c, iters, scale(), beta, g);
+          default: return launch_cluster<N, UPD_ER>(c, iters, scale(), beta, g);
+        }
+      }
+    }
     if constexpr (Blocked<N>::ok) {
       const bool cols = wc == 0 || wc == blocked_cols_code<N>(), rows = wr <= 0 || wr == blocked_rows_code<N>();
       if (cols && rows && c.At && c.sp && c.odd) {
