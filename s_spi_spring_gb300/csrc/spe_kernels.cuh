@@ -779,17 +779,17 @@ struct OpColsKnownPower : OpKeep {
 // adjoint of FFT+; no normalisation).
 enum { LOSS_AMPLITUDE = 0, LOSS_POISSON = 1 };
 
-// (roundings spelled out, so that every kernel's loss terms have the same bits;
-// add them with loss_add)
+// adds the loss term to `sum`; *g: 2 dL/dconj(F) (roundings spelled out, so that
+// every kernel's sums have the same bits)
 template <int LOSS>
-__device__ __forceinline__ float loss_term(float2 F, float a, float eps, float2* g) {
+__device__ __forceinline__ void loss_term(float2 F, float a, float eps, float& sum, float2* g) {
   const float m2 = fmaf(F.x, F.x, __fmul_rn(F.y, F.y));
   if (LOSS == LOSS_AMPLITUDE) {
     const float m = sqrtf(m2);
     const float d = m - a;
     const float f = m > 0.f ? 2.f * d / m : 0.f;
     if (g) *g = make_float2(f * F.x, f * F.y);
-    return __fmul_rn(d, d);
+    sum = fmaf(d, d, sum);
   } else {
     // the hardware logarithm and reciprocal (a few ulp) instead of the
     // IEEE-rounded logf and division: the loss and the gradient stay within
@@ -799,10 +799,9 @@ __device__ __forceinline__ float loss_term(float2 F, float a, float eps, float2*
     const float den = __fadd_rn(m2, eps);
     const float f = 2.f * (1.f - __fdividef(i, den));
     if (g) *g = make_float2(f * F.x, f * F.y);
-    return fmaf(-i, __logf(den), m2);
+    sum = __fadd_rn(sum, fmaf(-i, __logf(den), m2));
   }
 }
-__device__ __forceinline__ void loss_add(float& sum, float term) { sum = __fadd_rn(sum, term); }
 
 // row pass: S rho -> FFT+ (x) -> T
 struct OpRowsSupportForward : OpKeep {
@@ -835,14 +834,14 @@ struct OpColsLoss : OpBase {
   __device__ float2 load(const Px& q, Acc&) const { return T[q.ti]; }
   __device__ float2 mid(float2 v, const Px& q, const Mid&, Acc& acc) const {
     float2 g = make_float2(0.f, 0.f);
-    if (q.a >= 0.f) loss_add(acc.l, loss_term<LOSS>(v, q.a, eps, &g));
+    if (q.a >= 0.f) loss_term<LOSS>(v, q.a, eps, acc.l, &g);
     return g;
   }
   __device__ void store(float2 v, const Px& q, Acc& acc) const {
     if (GRAD) {
       T[q.ti] = v;
     } else if (q.a >= 0.f) {
-      loss_add(acc.l, loss_term<LOSS>(v, q.a, eps, nullptr));
+      loss_term<LOSS>(v, q.a, eps, acc.l, nullptr);
     }
   }
 };
@@ -871,11 +870,12 @@ struct OpRowsGradOut : OpKeep {
 struct AdamParams {
   float b1, b2, step_size, inv_sqrt_bc2, eps;
   // one real component: moments mm, vv and parameter p after gradient g
+  // (roundings spelled out: every kernel's step has the same bits)
   __device__ __forceinline__ float upd(float g, float& mm, float& vv, float p) const {
-    mm = mm + (1.f - b1) * (g - mm);
-    vv = vv * b2 + (1.f - b2) * g * g;
-    const float den = sqrtf(vv) * inv_sqrt_bc2 + eps;
-    return p - step_size * (mm / den);
+    mm = fmaf(1.f - b1, __fsub_rn(g, mm), mm);
+    vv = fmaf(vv, b2, __fmul_rn(__fmul_rn(1.f - b2, g), g));
+    const float den = fmaf(sqrtf(vv), inv_sqrt_bc2, eps);
+    return fmaf(-step_size, mm / den, p);
   }
   // a complex pixel: gradient g (zeroed outside the support s)
   __device__ __forceinline__ void step(float2 g, int s, float2& mm, float2& vv, float2& p) const {

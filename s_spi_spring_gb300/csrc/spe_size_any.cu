@@ -594,10 +594,11 @@ int best_threads(const AnyPlan& pl) {
   return best;
 }
 
-// plain: the radices of the operations whose results are compared digit by
-// digit.  A far-field loss is a 64-bit sum that a few bright pixels dominate,
-// and a shrink-wrap's support is a threshold: other radices round differently,
-// which moves a loss in its ninth digit and may flip a pixel.
+// plain: the radices and threads of the operations whose results are compared
+// digit by digit.  A far-field loss is a 64-bit sum that a few bright pixels
+// dominate, and a shrink-wrap's support is a threshold: other radices round
+// differently, and so do other shares of a thread's float sum, which moves a
+// loss in its ninth digit; a rounding may flip a pixel of a support.
 bool make_plan(int n, AnyPlan& pl, bool plain) {
   if (n < 2) return false;
   pl.n = n;
@@ -642,7 +643,7 @@ bool make_plan(int n, AnyPlan& pl, bool plain) {
   const size_t budget = (table + 2 * per_line <= kAnySmem / 2) ? kAnySmem / 2 : kAnySmem;
   const size_t w = (budget - table) / per_line;
   pl.W = (int)(w < 8 ? w : 8);
-  pl.threads = best_threads(pl);
+  pl.threads = plain ? (pl.big ? kAnyThreadsBig : kAnyThreads) : best_threads(pl);
   // the bounds of fdiv: indices below W n < 2^17, divisors below 2^15
   if (n >= (1 << 15)) return false;
   while (pl.W > 1 && (size_t)pl.W * n >= (1u << 17)) --pl.W;

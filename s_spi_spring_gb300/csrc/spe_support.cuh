@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(LossCols<N>::NT, LossCols<N>::MINB)
     for (int e = 0; e < E; ++e) {
       const float a = e % 4 == 0 ? a4[e / 4].x : e % 4 == 1 ? a4[e / 4].y : e % 4 == 2 ? a4[e / 4].z : a4[e / 4].w;
       float2 d = make_float2(0.f, 0.f);
-      if (a >= 0.f) loss_add(acc, loss_term<LOSS>(v[e], a, eps, GRAD ? &d : nullptr));
+      if (a >= 0.f) loss_term<LOSS>(v[e], a, eps, acc, GRAD ? &d : nullptr);
       v[e] = d;
     }
     if (PF && nxt < ntiles) fetch(nv, nxt, nrows);
