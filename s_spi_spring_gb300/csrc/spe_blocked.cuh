@@ -159,17 +159,31 @@ struct BlkCfg {
   __host__ __device__ static constexpr int step(int e) { return (e / R0) * TPT + (e % R0) * NB; }
 };
 
-// column pass: T -> FFT+ (y) -> P_M with A -> FFT- (y) -> T
-template <int N>
+// Row tiles of an ER call.  The update multiplies by the support, so that
+// outside the row tiles that hold any the density, and its row transform, are
+// zeros, and of the projected column transform only those tiles' rows are
+// used.  A support is compact (a quarter of the rows or less, from the
+// oversampling that phase retrieval needs): the passes between the first and
+// the last column pass leave the other tiles out.  `odd` carries the tiles'
+// state, `live` the list of those with support, its length first.
+// (A tile that is not finite counts as one with support: 0 times it is not 0.
+// Not with a phase gate, which may empty the support: the projection of an
+// all-zero transform goes by the signs of its zeros.)
+enum { TILE_ODD = 1, TILE_LIVE = 2 };
+
+// column pass: T -> FFT+ (y) -> P_M with A -> FFT- (y) -> T.  IN / OUT: only
+// the rows of live tiles are read (the others are zeros) / written.
+template <int N, bool IN, bool OUT>
 __global__ void __launch_bounds__(BlkCfg<N, Blocked<N>::BC, Blocked<N>::NXC>::NT, Blocked<N>::MBC)
-    k_cols_blocked(float2* __restrict__ T, const float* __restrict__ At, int ipp, int first, int count,
-                   const float2* __restrict__ twg) {
+    k_cols_blocked(float2* __restrict__ T, const float* __restrict__ At, const unsigned char* __restrict__ odd, int ipp,
+                   int first, int count, const float2* __restrict__ twg) {
   using B = Blocked<N>;
   constexpr int W = B::BC, NX = B::NXC;
   using C = BlkCfg<N, W, NX>;
   using Lay = typename C::Lay;
   constexpr int NT = C::NT, E = C::E, TPI = N / W;
   constexpr bool PF = B::PREFETCH;
+  static_assert(C::TPT % B::WR == 0 && C::NB % B::WR == 0, "a thread's rows are tiles apart");
   extern __shared__ __align__(128) unsigned char sm[];
   float2* tw = reinterpret_cast<float2*>(sm);
   float2* xb = reinterpret_cast<float2*>(sm + C::TWB);
@@ -187,17 +201,37 @@ __global__ void __launch_bounds__(BlkCfg<N, Blocked<N>::BC, Blocked<N>::NXC>::NT
     const int tile = ntiles - 1 - k;
     return T + off + (size_t)(tile / TPI) * N * N + (size_t)(tile % TPI) * B::XS;
   };
-  float2 v[E], nx[PF ? E : 1];
-  int k = blockIdx.x;
-  if (PF && k < ntiles) {
+  // the thread's rows of live tiles, as bits
+  auto rows_of = [&](int k) {
+    if (!IN && !OUT) return 0xffffffffu;
+    const unsigned char* f = odd + (size_t)(first + (ntiles - 1 - k) / TPI) * (N / B::WR) + j / B::WR;
+    unsigned r = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) r |= (__ldcg(f + C::step(e) / B::WR) & TILE_LIVE) ? 1u << e : 0u;
+    return r;
+  };
+  auto fetch = [&](float2* v, int k, unsigned rows) {
     const float2* g = tile_ptr(k);
 #pragma unroll
-    for (int e = 0; e < E; ++e) nx[e] = __ldcg(g + (size_t)C::step(e) * B::YS);
+    for (int e = 0; e < E; ++e)
+      v[e] = !IN || ((rows >> e) & 1u) ? __ldcg(g + (size_t)C::step(e) * B::YS) : make_float2(0.f, 0.f);
+  };
+  float2 v[E], nx[PF ? E : 1];
+  int k = blockIdx.x;
+  unsigned rows = 0, nrows = 0;
+  if (k < ntiles) {
+    rows = rows_of(k);
+    if (PF) fetch(nx, k, rows);
+    nrows = k + (int)gridDim.x < ntiles ? rows_of(k + gridDim.x) : rows;
   }
   for (; k < ntiles; k += gridDim.x) {
-    float2* g = tile_ptr(k);
+    const int nk = k + gridDim.x;
+    if (PF) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) v[e] = PF ? nx[PF ? e : 0] : __ldcg(g + (size_t)C::step(e) * B::YS);
+      for (int e = 0; e < E; ++e) v[e] = nx[PF ? e : 0];
+    } else {
+      fetch(v, k, rows);
+    }
     const int tile = ntiles - 1 - k;
     const int p = first + tile / TPI;
     const float4* A4 = reinterpret_cast<const float4*>(At + (ipp > 0 ? (size_t)(p / ipp) * N * N : 0)) +
@@ -213,15 +247,14 @@ __global__ void __launch_bounds__(BlkCfg<N, Blocked<N>::BC, Blocked<N>::NXC>::NT
       v[4 * i + 2] = project(v[4 * i + 2], a[i].z);
       v[4 * i + 3] = project(v[4 * i + 3], a[i].w);
     }
-    if (PF) {
-      const int nk = k + gridDim.x;
-      const float2* gn = tile_ptr(nk < ntiles ? nk : k);
-#pragma unroll
-      for (int e = 0; e < E; ++e) nx[PF ? e : 0] = __ldcg(gn + (size_t)C::step(e) * B::YS);
-    }
+    if (PF) fetch(nx, nk < ntiles ? nk : k, nk < ntiles ? nrows : rows);
     fft_x<N, Lay, -1, NX, C::EX>(v, xb, tw, c, j);
+    float2* g = tile_ptr(k);
 #pragma unroll
-    for (int e = 0; e < E; ++e) g[(size_t)C::step(e) * B::YS] = v[e];
+    for (int e = 0; e < E; ++e)
+      if (!OUT || ((rows >> e) & 1u)) g[(size_t)C::step(e) * B::YS] = v[e];
+    rows = nrows;
+    if (nk + (int)gridDim.x < ntiles) nrows = rows_of(nk + gridDim.x);
   }
 }
 
@@ -239,11 +272,12 @@ struct BlkRowCfg : BlkCfg<N, Blocked<N>::WR, Blocked<N>::NXR> {
 };
 
 // row pass: T -> FFT- (x) -> /N^2 -> update with (rho, support) -> rho -> FFT+ (x) -> T
-template <int N, int UPD>
+template <int N, int UPD, bool LIST>
 __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
     k_rows_blocked(float2* __restrict__ T, float2* __restrict__ rho, const int* __restrict__ S,
-                   const SpBits<N>* __restrict__ sp, const unsigned char* __restrict__ odd, int first, int count,
-                   float scale, float beta, Gate g, const float2* __restrict__ twg) {
+                   const SpBits<N>* __restrict__ sp, const unsigned char* __restrict__ odd,
+                   const int* __restrict__ live, int first, int count, float scale, float beta, Gate g,
+                   const float2* __restrict__ twg) {
   using B = Blocked<N>;
   using C = BlkRowCfg<N>;
   using Lay = typename C::Lay;
@@ -260,7 +294,9 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
   pdl_wait();
   const int t = threadIdx.x;
   const int c = t % W, j = t / W;
-  const int ntiles = count * TPI;
+  // the tiles of the pass: all, or (LIST) the live ones by their list
+  const int ntiles = LIST ? __ldcg(live) : count * TPI;
+  auto tile_at = [&](int k) { return LIST ? __ldcg(live + 1 + k) : k; };
   // offset of a tile's first row in T (blocked), rho and S (row-major)
   auto t_base = [&](int tile) {
     return (size_t)(first + tile / TPI) * N * N + (size_t)(tile % TPI) * (W * B::YS);
@@ -287,22 +323,24 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
   // the thread's support bits of a tile, bit 16: the tile's support is not 0 / 1
   auto bits_of = [&](int tile) {
     const unsigned b = sp[((size_t)first * N + (size_t)tile * W + c) * TPT + j];
-    return b | ((unsigned)odd[(size_t)first * TPI + tile] << 16);
+    return b | ((unsigned)(odd[(size_t)first * TPI + tile] & TILE_ODD) << 16);
   };
-  int tile = blockIdx.x;
+  int i = blockIdx.x, tile = 0, nxt = 0;
   unsigned nbits = 0;
-  if (tile < ntiles) {
+  if (i < ntiles) {
+    tile = tile_at(i);
     stage_T(tile, 0);
     stage_R(tile, 0);
     nbits = bits_of(tile);
   }
   cp_async_commit();
-  for (int k = 0; tile < ntiles; ++k, tile += gridDim.x) {
-    const int nxt = tile + gridDim.x;
+  for (int k = 0; i < ntiles; ++k, i += gridDim.x, tile = nxt) {
+    const bool more = i + (int)gridDim.x < ntiles;
+    nxt = more ? tile_at(i + gridDim.x) : 0;
     const int s = ST == 2 ? (k & 1) : 0;
     const unsigned bits = nbits;
     if constexpr (ST == 2) {
-      if (nxt < ntiles) {
+      if (more) {
         stage_T(nxt, s ^ 1);
         stage_R(nxt, s ^ 1);
         nbits = bits_of(nxt);
@@ -322,7 +360,7 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
     for (int e = 0; e < E; ++e) v[e] = sT[C::step(e) * W];
     if constexpr (ST == 1) {
       __syncthreads();  // every thread has read its elements of T
-      if (nxt < ntiles) stage_T(nxt, 0);
+      if (more) stage_T(nxt, 0);
       cp_async_commit();
     }
     fft_x<N, Lay, -1, NX, 0>(v, xb, tw, c, j);
@@ -334,12 +372,12 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
       int m = (int)((bits >> e) & 1u);
       if (plain) m = S[rb + C::step(e)];
       const float2 r = update<UPD>(rp, prev, m, beta, g);
-      rho[rb + C::step(e)] = r;
+      if (NEED_PREV) rho[rb + C::step(e)] = r;  // (ER reads no previous iterate, and the last pass writes the result)
       v[e] = r;
     }
     if constexpr (ST == 1) {
       if (NEED_PREV) __syncthreads();  // every thread has read its elements of the previous iterate
-      if (nxt < ntiles) {
+      if (more) {
         stage_R(nxt, 0);
         nbits = bits_of(nxt);
       }
@@ -354,13 +392,14 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
   cp_async_wait_all();  // no copy outlives the CTA
 }
 
-// First pass of a call: rho -> FFT+ (x) -> T; packs the support.  One tile
-// per CTA, loads in flight over many CTAs per SM.
-template <int N>
+// First pass of a call: rho -> FFT+ (x) -> T; packs the support and, with LIST,
+// lists the live tiles (*live: 0 before).  One tile per CTA, loads in flight
+// over many CTAs per SM.
+template <int N, bool LIST>
 __global__ void __launch_bounds__(BlkRowCfg<N>::NT, BlkCfg<N, Blocked<N>::WR, 1>::E <= 8 ? 1024 / BlkRowCfg<N>::NT : 2)
     k_rows_blocked_first(const float2* __restrict__ rho, const int* __restrict__ S, float2* __restrict__ T,
-                         SpBits<N>* __restrict__ sp, unsigned char* __restrict__ odd, int first,
-                         const float2* __restrict__ twg) {
+                         SpBits<N>* __restrict__ sp, unsigned char* __restrict__ odd, int* __restrict__ live,
+                         int first, const float2* __restrict__ twg) {
   using B = Blocked<N>;
   using C = BlkCfg<N, B::WR, 1>;
   using Lay = typename C::Lay;
@@ -387,8 +426,20 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, BlkCfg<N, Blocked<N>::WR, 1>
     other |= m[e] & ~1;
   }
   sp[((size_t)first * N + (size_t)tile * W + c) * TPT + j] = (SpBits<N>)bits;
-  const int any = __syncthreads_or(other);  // (also: the twiddles are in shared memory)
-  if (t == 0) odd[(size_t)first * TPI + tile] = any ? 1 : 0;
+  int state = other != 0 ? TILE_ODD : 0;
+  if (LIST) {
+    float chk = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) chk += 0.f * v[e].x + 0.f * v[e].y;
+    if (bits != 0 || chk != 0.f) state |= TILE_LIVE;
+  }
+  // (also: the twiddles are in shared memory)
+  state = (__syncthreads_or(state & TILE_ODD) ? TILE_ODD : 0) |
+          (LIST && __syncthreads_or(state & TILE_LIVE) ? TILE_LIVE : 0);
+  if (t == 0) {
+    odd[(size_t)first * TPI + tile] = (unsigned char)state;
+    if (state & TILE_LIVE) live[1 + atomicAdd(live, 1)] = tile;
+  }
   fft_x<N, Lay, +1, 1, 0>(v, xb, tw, c, j);
   float2* gt = T + (size_t)(first + tile / TPI) * N * N + (size_t)(tile % TPI) * (W * B::YS) + B::at(c, j);
 #pragma unroll
