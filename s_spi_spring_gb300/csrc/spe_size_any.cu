@@ -35,6 +35,7 @@ namespace {
 constexpr int kAnyThreads = 512;     // most threads of a pass CTA
 constexpr int kAnyThreadsBig = 256;  // the same for plans with a prime radix of 11 or more (128 registers each)
 constexpr int kMaxRadices = 24;
+
 constexpr size_t kAnySmem = 220 * 1024;  // shared-memory budget of one CTA (two line buffers)
 
 struct AnyPlan {
@@ -321,6 +322,19 @@ __device__ __forceinline__ void any_sym_outputs(const PassArgs& a, int R) {
   }
 }
 
+// Butterflies per thread of any_sym_outputs (first: 1, 2 or 4) for nb butterflies
+// and G groups of q, by the warps each of an SM's four schedulers gets and a
+// warp's instructions per term (kSymQ table reads and their index steps, and
+// per butterfly two reads and 2 kSymQ multiply-adds), and their product (second).
+struct SymRounds {
+  int first, second;
+};
+__host__ __device__ __forceinline__ SymRounds sym_rounds(int nb, int G) {
+  const int c1 = (nb * G + 127) / 128 * 34, c2 = ((nb + 1) / 2 * G + 127) / 128 * 44,
+            c4 = ((nb + 3) / 4 * G + 127) / 128 * 64;
+  return c4 <= c2 && c4 <= c1 ? SymRounds{4, c4} : c2 <= c1 ? SymRounds{2, c2} : SymRounds{1, c1};
+}
+
 // One pass of an odd prime radix above 31, in the symmetric form of the
 // prime DFT with run-time R (H = (R-1)/2), in two steps over shared memory:
 //   1. per butterfly and pair (r, R-r), r = 1 .. H: y_r = x_r w^{k r},
@@ -362,11 +376,10 @@ __device__ __noinline__ void any_pass_sym(const PassArgs a, int R) {
     src[(R - r) * m] = csub(x, y);
   }
   __syncthreads();
-  // 2. output pairs, as many butterflies per thread as leave every thread work
-  const int G = (H + kSymQ) / kSymQ;  // groups of q in [0, H]
-  const int NT = blockDim.x;
-  if (((nl * m + 3) / 4) * G >= NT) any_sym_outputs<S, 4>(a, R);
-  else if (((nl * m + 1) / 2) * G >= NT) any_sym_outputs<S, 2>(a, R);
+  // 2. output pairs
+  const int bb = sym_rounds(nl * m, (H + kSymQ) / kSymQ).first;
+  if (bb == 4) any_sym_outputs<S, 4>(a, R);
+  else if (bb == 2) any_sym_outputs<S, 2>(a, R);
   else any_sym_outputs<S, 1>(a, R);
 }
 
@@ -459,8 +472,9 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
   };
   // a thread's elements in batches of U: the batch's memory reads are issued
   // before the first of them is used (one at a time, the waits for them were
-  // 35-45% of the iteration's passes)
-  constexpr int U = 8;
+  // 35-45% of the iteration's passes; eight at a time is 12% slower at 600 and
+  // 1000, where a thread has ten elements)
+  constexpr int U = 4;
   auto batches = [&](auto&& body) {
     for (int i0 = threadIdx.x; i0 < tot; i0 += NT * U) body(i0);
   };
@@ -570,6 +584,8 @@ int fewest_radices(int n, int* rad) {
 
 size_t smem_of(const AnyPlan& pl) { return (2 * (size_t)pl.W * pl.LS + pl.n) * sizeof(float2); }
 
+int largest_radix(const AnyPlan& pl) { return *std::max_element(pl.rad, pl.rad + pl.nrad); }
+
 // Threads of a pass CTA: those that keep the most threads of an SM (as many
 // CTAs as its shared memory and registers hold) busy in the pass with the
 // fewest butterflies (the largest radix), the larger of equals, as they have
@@ -577,9 +593,8 @@ size_t smem_of(const AnyPlan& pl) { return (2 * (size_t)pl.W * pl.LS + pl.n) * s
 // and takes them all.  512 threads at every side left five of six idle at 100
 // (935 -> 487 us for 8 iterations of 200 individuals).
 int best_threads(const AnyPlan& pl) {
-  const int top = pl.big ? kAnyThreadsBig : kAnyThreads, regs = pl.big ? 512 : 1024;
-  int rmax = 1, best = top;
-  for (int i = 0; i < pl.nrad; ++i) rmax = std::max(rmax, pl.rad[i]);
+  const int top = pl.big ? kAnyThreadsBig : kAnyThreads, regs = pl.big ? 512 : 1024, rmax = largest_radix(pl);
+  int best = top;
   if (rmax > 31) return top;
   const int fly = pl.W * (pl.n / rmax), ctas = (int)(kAnySmem / smem_of(pl));
   double most = 0.0;
@@ -642,7 +657,11 @@ bool make_plan(int n, AnyPlan& pl, bool plain) {
   // two CTAs per SM where half the budget still holds two lines
   const size_t budget = (table + 2 * per_line <= kAnySmem / 2) ? kAnySmem / 2 : kAnySmem;
   const size_t w = (budget - table) / per_line;
-  pl.W = (int)(w < 8 ? w : 8);
+  // lines per CTA: 8, and 32 with a run-time prime, whose pass has work for its
+  // threads only with many lines (8 iterations of 64 individuals of 97^2 with
+  // 8 / 16 / 32 lines 713 / 640 / 473 us, 100 of 263^2 8157 / 6821 / 5454; at
+  // smooth sides fewer or more lines than 8 are slower)
+  pl.W = (int)std::min<size_t>(w, plain || largest_radix(pl) <= 31 ? 8 : 32);
   pl.threads = plain ? (pl.big ? kAnyThreadsBig : kAnyThreads) : best_threads(pl);
   // the bounds of fdiv: indices below W n < 2^17, divisors below 2^15
   if (n >= (1 << 15)) return false;
@@ -651,7 +670,7 @@ bool make_plan(int n, AnyPlan& pl, bool plain) {
 }
 
 struct AnyEntry {
-  AnyPlan plan, plain;  // the same tiles
+  AnyPlan plan, plain, blur;  // blur: the plain radices on the plan's tiles
   SizeOps ops;
 };
 
@@ -662,9 +681,37 @@ const AnyPlan& plan_of(int n) {
   std::lock_guard<std::mutex> lock(g_any_mutex);
   return g_any.at(n)->plan;
 }
+const AnyPlan& blur_of(int n) {
+  std::lock_guard<std::mutex> lock(g_any_mutex);
+  return g_any.at(n)->blur;
+}
 const AnyPlan& plain_of(int n) {
   std::lock_guard<std::mutex> lock(g_any_mutex);
   return g_any.at(n)->plain;
+}
+
+// Lines per CTA of one launch.  With a run-time prime: the width with the least
+// rounds of its pass over the waves of CTAs (two per SM), as that pass is most
+// of the time (100 of 263^2 with 25 / 16 / 8 lines 5454 / 6821 / 8157 us).  Else the plan's, halved
+// while it would leave SMs without a CTA.
+int launch_width(const AnyPlan& pl, int count) {
+  const int R = largest_radix(pl), sms = sm_count();
+  int W = pl.W;
+  if (R <= 31) {
+    while (W > 2 && (size_t)count * ((pl.n + W - 1) / W) < (size_t)sms) W /= 2;
+    return W;
+  }
+  size_t least = ~size_t(0);
+  for (int half = pl.W; half >= std::min(pl.W, 4); half /= 2) {
+    const size_t ctas = (size_t)count * ((pl.n + half - 1) / half), waves = (ctas + 2 * sms - 1) / (2 * sms);
+    const int nb = half * (pl.n / R), G = ((R - 1) / 2 + kSymQ) / kSymQ;
+    const size_t cost = waves * sym_rounds(nb, G).second;
+    if (cost <= least) {  // (the narrower of equals: shorter reads and writes)
+      least = cost;
+      W = half;
+    }
+  }
+  return W;
 }
 
 template <int AXIS, class Op, bool BIG>
@@ -676,8 +723,7 @@ cudaError_t launch_any_k(const Op& op, AnyPlan pl, int count, cudaStream_t st, c
   if (e != cudaSuccess || count <= 0) return e;
   // narrower tiles where the plan's leave SMs without a CTA (not where the op
   // reduces: its partials are one per tile of the plan)
-  if (Op::NSUM + Op::NMAX == 0 && !Op::PEAK)
-    while (pl.W > 2 && (size_t)count * ((pl.n + pl.W - 1) / pl.W) < (size_t)sm_count()) pl.W /= 2;
+  if (Op::NSUM + Op::NMAX == 0 && !Op::PEAK) pl.W = launch_width(pl, count);
   const int tpi = (pl.n + pl.W - 1) / pl.W;
   const int grid = (int)((unsigned)count * tpi), threads = pl.threads;
   const size_t smem = smem_of(pl);
@@ -762,7 +808,7 @@ struct SizeAny {
   }
 
   static cudaError_t blur_magnitude(const Ctx& c, float sigma_ft) {
-    const AnyPlan& pl = plain_of(c.n);
+    const AnyPlan& pl = blur_of(c.n);
     SPE_TRY((launch_any<AX_ROWS>(rows_forward<SRC_RHO>(c, c.rho, c.T, nullptr), pl, c.count, c.st, c.tw)));
     SPE_TRY((launch_any<AX_COLS>(cols_project(c), pl, c.count, c.st, c.tw)));
     OpRowsModulusForward mf;
@@ -1021,7 +1067,10 @@ const SizeOps* size_ops_any(int n) {
   if (it != g_any.end()) return &it->second->ops;
   std::unique_ptr<AnyEntry> en(new AnyEntry());
   if (!make_plan(n, en->plan, false) || !make_plan(n, en->plain, true)) return nullptr;
-  const int tiles = (n + en->plan.W - 1) / en->plan.W;
+  en->blur = en->plain;
+  en->blur.W = en->plan.W;
+  en->blur.threads = best_threads(en->blur);
+  const int tiles = (n + en->plan.W - 1) / en->plan.W, loss_tiles = (n + en->plain.W - 1) / en->plain.W;
   en->ops = SizeOps{n,
                     tiles,
                     tiles,
@@ -1043,7 +1092,7 @@ const SizeOps* size_ops_any(int n) {
                     0,
                     &SizeAny::known_power,
                     &SizeAny::loss_grad,
-                    tiles,
+                    loss_tiles,
                     &SizeAny::adam_step,
                     0,
                     0,

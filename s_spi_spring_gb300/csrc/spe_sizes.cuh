@@ -660,10 +660,10 @@ struct SizeImpl {
           case 1: return iterate_blocked<UPD_RAAR, false>(c, iters, beta, g);
           default:
             // live tiles: with an open gate (reality 0), and where a pass has
-            // the work to hide the list behind (ten iterations, dense / live:
-            // 512^2 x 4 166 / 195 us, x 8 286 / 292, x 16 489 / 459; 256^2 x 8
-            // 115 / 131, x 32 274 / 242; 1024^2 x 1 226 / 215)
-            return g.hi >= 3.14159f && g.lo >= 3.14159f && (N >= 1024 || (size_t)c.count * N * N >= (1u << 21))
+            // the work to hide the list behind (us a call, dense / live:
+            // 512^2 x 1 81 / 102, x 4 207 / 190; 256^2 x 9 77 / 92; 768^2 x 1
+            // 104 / 99, x 3 312 / 234)
+            return g.hi >= 3.14159f && g.lo >= 3.14159f && (N >= 768 || (size_t)c.count * N * N >= (1u << 20))
                        ? iterate_blocked<UPD_ER, true>(c, iters, beta, g)
                        : iterate_blocked<UPD_ER, false>(c, iters, beta, g);
         }
