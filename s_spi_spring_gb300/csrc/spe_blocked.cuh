@@ -325,18 +325,20 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
     const unsigned b = sp[((size_t)first * N + (size_t)tile * W + c) * TPT + j];
     return b | ((unsigned)(odd[(size_t)first * TPI + tile] & TILE_ODD) << 16);
   };
-  int i = blockIdx.x, tile = 0, nxt = 0;
+  int i = blockIdx.x, listed = 0;
   unsigned nbits = 0;
   if (i < ntiles) {
-    tile = tile_at(i);
-    stage_T(tile, 0);
-    stage_R(tile, 0);
-    nbits = bits_of(tile);
+    listed = tile_at(i);
+    stage_T(listed, 0);
+    stage_R(listed, 0);
+    nbits = bits_of(listed);
   }
   cp_async_commit();
-  for (int k = 0; i < ntiles; ++k, i += gridDim.x, tile = nxt) {
+  for (int k = 0; i < ntiles; ++k, i += gridDim.x) {
+    const int tile = LIST ? listed : i;
     const bool more = i + (int)gridDim.x < ntiles;
-    nxt = more ? tile_at(i + gridDim.x) : 0;
+    const int nxt = LIST && !more ? 0 : tile_at(i + gridDim.x);
+    listed = nxt;
     const int s = ST == 2 ? (k & 1) : 0;
     const unsigned bits = nbits;
     if constexpr (ST == 2) {

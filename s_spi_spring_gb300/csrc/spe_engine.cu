@@ -1322,18 +1322,28 @@ int spe_autotune(spe_engine* e, int first, int count, int iterations, int* cols,
     }
     if (!rc && blocked < whole * 0.99f) best_r = blk_r, best_chunk = blk_chunk, best_lanes = blk_lanes;
   }
+  // the sides whose default is none of the codes (one cluster per individual,
+  // spe_cluster.cuh): kept where it is the fastest
+  bool by_default = false;
+  if (!rc && !blk_c && e->ops->default_cols > 0) {
+    float td = 0.f, tb = 0.f;
+    if (!(rc = trial_s(0, 0, 0, 1, &td))) rc = trial_s(col_of(best_r), best_r, best_chunk, best_lanes, &tb);
+    by_default = !rc && td < tb;
+  }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   if (rc) return rc;
   CK(cudaMemcpyAsync(e->rho + (size_t)first * e->npix, save, bytes, cudaMemcpyDeviceToDevice, e->st), "restore");
   CK(cudaStreamSynchronize(e->st), "synchronize");
   best_c = col_of(best_r);
-  e->tile_cols = best_c;
-  e->tile_rows = best_r;
-  e->chunk = best_chunk;
-  e->lanes = best_lanes;
-  if (cols) *cols = best_c;
-  if (rows) *rows = best_r;
+  e->tile_cols = by_default ? 0 : best_c;
+  e->tile_rows = by_default ? 0 : best_r;
+  e->chunk = by_default ? 0 : best_chunk;
+  e->lanes = by_default ? 1 : best_lanes;
+  int c = 0, r = 0;
+  spe_get_tiles(e, &c, &r);
+  if (cols) *cols = c;
+  if (rows) *rows = r;
   return SPE_OK;
 }
 

@@ -57,3 +57,19 @@ def test_many_individuals(n, P):
     a = run(e, (16, 8), 0, P, "raar", 2, 0.0, dens, S)
     b = run(e, (0, 0), 0, P, "raar", 2, 0.0, dens, S)
     assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+def test_autotune_may_keep_the_default():
+    """At a side whose default is a cluster per individual the tuner compares it
+    with the codes it times, and the densities come back as they were."""
+    n, P = 64, 6
+    I, _, _ = synthetic.polygon_pattern(seed=1, n=n, diameter=n * 0.3, photons=1e7, stop_radius=2)
+    dens, S = synthetic.start_population(n, P, n * 0.25, seed=5)
+    e = _lib.Engine(n, 0)
+    e.set_amplitudes(_lib.prepare_pattern(I, (-1, -1), True))
+    before = run(e, (16, 8), 0, P, "raar", 3, 0.0, dens, S)
+    e.upload(0, dens, S)
+    e.autotune(0, P)
+    assert np.array_equal(e.download(0, P)[0].view(np.uint32), dens.view(np.uint32))
+    e.raar(0, P, 3, 0.9, 0.0)
+    assert np.array_equal(e.download(0, P)[0].view(np.uint32), before.view(np.uint32))
