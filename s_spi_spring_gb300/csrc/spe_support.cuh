@@ -12,8 +12,8 @@
 // fills the field runs every tile, as the row-major kernels did.
 //
 // Measured on GB300 (row-major passes over every row before -> now): a loss and
-// its gradient at 1024^2 x 32 511 -> 341 us, ten refinement steps at 512^2 x 64
-// 3909 -> 1346 us.  The column pass transforms every
+// its gradient at 1024^2 x 32 511 -> 333 us, ten refinement steps at 512^2 x 64
+// 3909 -> 1305 us (345 and 1360 with one exchange buffer in the column pass).  The column pass transforms every
 // column twice and is bound like the iteration's (spe_blocked.cuh); the row
 // passes by the reads of the int32 support.
 #pragma once
@@ -40,8 +40,8 @@ struct LossRows : BlkCfg<N, Blocked<N>::WR, 1> {
   static constexpr int MINB = C::E <= 8 ? 1024 / C::NT : 2;
 };
 template <int N>
-struct LossCols : BlkCfg<N, Blocked<N>::BC, 1> {
-  using C = BlkCfg<N, Blocked<N>::BC, 1>;
+struct LossCols : BlkCfg<N, Blocked<N>::BC, 2> {
+  using C = BlkCfg<N, Blocked<N>::BC, 2>;
   static constexpr int MINB = C::E <= 8 ? 1024 / C::NT : 2;
 };
 
@@ -116,6 +116,9 @@ __global__ void __launch_bounds__(LossCols<N>::NT, LossCols<N>::MINB)
   using Lay = typename C::Lay;
   constexpr int E = C::E, NT = C::NT, W = Blocked<N>::BC, WR = Blocked<N>::WR, TPI = N / W;
   constexpr bool PF = E <= 8;
+  // two exchange buffers in turn (an even number of exchanges a tile), one
+  // where only the forward transform runs
+  constexpr int NX = GRAD ? 2 : 1;
   static_assert(C::TPT % WR == 0 && C::NB % WR == 0 && E <= 32, "a thread's rows are tiles apart");
   extern __shared__ __align__(128) unsigned char sm[];
   float2* tw = reinterpret_cast<float2*>(sm);
@@ -165,7 +168,7 @@ __global__ void __launch_bounds__(LossCols<N>::NT, LossCols<N>::MINB)
     float4 a4[E / 4];
 #pragma unroll
     for (int i = 0; i < E / 4; ++i) a4[i] = __ldg(A4 + i);
-    fft_x<N, Lay, +1, 1, 0>(v, xb, tw, c, j);
+    fft_x<N, Lay, +1, NX, 0>(v, xb, tw, c, j);
     float acc = 0.f;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
@@ -176,7 +179,7 @@ __global__ void __launch_bounds__(LossCols<N>::NT, LossCols<N>::MINB)
     }
     if (PF && nxt < ntiles) fetch(nv, nxt, nrows);
     if (GRAD) {
-      fft_x<N, Lay, -1, 1, 0>(v, xb, tw, c, j);
+      fft_x<N, Lay, -1, NX, C::EX>(v, xb, tw, c, j);
       float2* g = tile_ptr(tile);
 #pragma unroll
       for (int e = 0; e < E; ++e)
