@@ -481,9 +481,9 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, BlkCfg<N, Blocked<N>::WR, 1>
 // passes read and write the row-major arrays in runs of 32 / WR pixels.  An
 // op's per-pixel operand comes in the order of k_block_amplitudes.
 template <int N, int AXIS, class Op>
-struct BlkPassCfg : BlkCfg<N, AXIS == AX_ROWS ? Blocked<N>::WR : Blocked<N>::BC, 1> {
+struct BlkPassCfg : BlkCfg<N, AXIS == AX_ROWS ? Blocked<N>::WR : Blocked<N>::BC, 2> {
   static constexpr int W = AXIS == AX_ROWS ? Blocked<N>::WR : Blocked<N>::BC;
-  using C = BlkCfg<N, W, 1>;
+  using C = BlkCfg<N, W, 2>;
   // registers a thread: 64 (a pair of arrays: 80) per 8 elements
   static constexpr int REGS = C::E <= 8 ? (Op::PAIR ? 80 : 64) : 128;
   static constexpr int MINB = 65536 / (C::NT * REGS) < 1 ? 1 : 65536 / (C::NT * REGS);
@@ -528,8 +528,9 @@ __global__ void __launch_bounds__(BlkPassCfg<N, AXIS, Op>::NT, BlkPassCfg<N, AXI
     if constexpr (Op::AMP) q.a = e % 4 == 0 ? a[e / 4].x : e % 4 == 1 ? a[e / 4].y : e % 4 == 2 ? a[e / 4].z : a[e / 4].w;
     return q;
   };
-  pass_elements<N, E, Lay, Op>(op, px, acc, [&](float2* v, auto sign) {
-    fft_x<N, Lay, decltype(sign)::value, 1, 0>(v, xb, tw, c, j);
+  // (two exchange buffers in turn: one barrier per exchange)
+  pass_elements<N, E, Lay, Op>(op, px, acc, [&](float2* v, auto sign, auto nth) {
+    fft_x<N, Lay, decltype(sign)::value, 2, decltype(nth)::value * C::EX>(v, xb, tw, c, j);
   });
   if constexpr (Op::NSUM + Op::NMAX > 0) {
     float r[NRED];

@@ -240,9 +240,11 @@ struct Px {
 
 // An op over a thread's E elements held in registers: load, transform,
 // pointwise step, transform, store.  px(e): the pixel of element e; fft(v,
-// sign): the transform of the CTA's sequences (std::integral_constant sign).
+// sign, nth): the tile's first or second transform (std::integral_constants).
 template <int N, int E, class Lay, class Op, class PxF, class Fft>
 __device__ __forceinline__ void pass_elements(const Op& op, const PxF& px, typename Op::Acc& acc, const Fft& fft) {
+  using First = std::integral_constant<int, 0>;
+  using Second = std::integral_constant<int, 1>;
   float2 v[E];
   if constexpr (Op::PAIR) {
     float2 u[E];
@@ -256,10 +258,10 @@ __device__ __forceinline__ void pass_elements(const Op& op, const PxF& px, typen
 #pragma unroll
       for (int e = 0; e < E; ++e) op.load_pair(px(e), v[e], u[e], acc);
     }
-    fft(v, std::integral_constant<int, Op::FFT1>());
+    fft(v, std::integral_constant<int, Op::FFT1>(), First());
 #pragma unroll
     for (int e = 0; e < E; ++e) op.store_pair(v[e], px(e), 0);
-    fft(u, std::integral_constant<int, Op::FFT1>());
+    fft(u, std::integral_constant<int, Op::FFT1>(), Second());
 #pragma unroll
     for (int e = 0; e < E; ++e) op.store_pair(u[e], px(e), 1);
   } else {
@@ -273,11 +275,11 @@ __device__ __forceinline__ void pass_elements(const Op& op, const PxF& px, typen
 #pragma unroll
       for (int e = 0; e < E; ++e) v[e] = op.load(px(e), acc);
     }
-    if constexpr (Op::FFT1 != 0) fft(v, std::integral_constant<int, Op::FFT1>());
+    if constexpr (Op::FFT1 != 0) fft(v, std::integral_constant<int, Op::FFT1>(), First());
     if constexpr (Op::FFT2 != 0) {
 #pragma unroll
       for (int e = 0; e < E; ++e) v[e] = op.mid(v[e], px(e), op.fetch_mid(px(e)), acc);
-      fft(v, std::integral_constant<int, Op::FFT2>());
+      fft(v, std::integral_constant<int, Op::FFT2>(), Second());
     }
     if constexpr (Op::FETCH_STORE) {
       typename Op::Raw r[E];
@@ -323,7 +325,7 @@ __global__ void __launch_bounds__(PassCfg<N, AXIS>::NT, PassCfg<N, AXIS>::MINB)
     q.a = Op::AMP ? __ldg(op.amp(p, N) + (size_t)q.y * N + q.x) : 0.f;
     return q;
   };
-  pass_elements<N, E, typename C::Lay, Op>(op, px, acc, [&](float2* v, auto sign) {
+  pass_elements<N, E, typename C::Lay, Op>(op, px, acc, [&](float2* v, auto sign, auto) {
     fft_reg<N, typename C::Lay, decltype(sign)::value>(v, buf, tw, c, j);
   });
   if constexpr (Op::NSUM + Op::NMAX > 0) {
