@@ -13,9 +13,10 @@
 //
 // Measured on GB300 (row-major passes over every row before -> now): a loss and
 // its gradient at 1024^2 x 32 511 -> 333 us, ten refinement steps at 512^2 x 64
-// 3909 -> 1305 us (345 and 1360 with one exchange buffer in the column pass).  The column pass transforms every
-// column twice and is bound like the iteration's (spe_blocked.cuh); the row
-// passes by the reads of the int32 support.
+// 3909 -> 1305 us (345 and 1360 with one exchange buffer in the column pass).
+// The column pass transforms every column twice and is bound like the
+// iteration's (spe_blocked.cuh); the row passes by the reads of the int32
+// support.
 #pragma once
 #include "spe_blocked.cuh"
 
