@@ -17,6 +17,7 @@
 #include "../../include/spe_engine.h"
 #include "spe_engine_impl.h"
 #include "spe_kernels.cuh"
+#include "spe_workspace.h"
 
 using namespace spe_detail;
 
@@ -185,19 +186,7 @@ __global__ void k_gather(float2* __restrict__ rho, int* __restrict__ S, const in
 
 namespace {
 
-// grow-only scratch carved into aligned pieces
-struct Carve {
-  char* p;
-  size_t used = 0;
-  template <class T>
-  T* take(size_t n) {
-    used = (used + 255) & ~size_t(255);
-    T* r = reinterpret_cast<T*>(p + used);
-    used += n * sizeof(T);
-    return r;
-  }
-};
-
+// (the workspace only grows)
 int ensure_work(spe_engine* e, size_t bytes) {
   if (bytes <= e->work_bytes) return SPE_OK;
   CK(cudaStreamSynchronize(e->st), "synchronize");
@@ -207,6 +196,11 @@ int ensure_work(spe_engine* e, size_t bytes) {
   CK(cudaMalloc(&e->work, bytes), "population workspace");
   e->work_bytes = bytes;
   return SPE_OK;
+}
+
+// no piece of the workspace ends outside it
+int check_work(const Carve& cv) {
+  return cv.fits() ? SPE_OK : fail(SPE_ERR_STATE, "workspace of %zu bytes carved to %zu", cv.cap, cv.used);
 }
 
 // Solver's "indexes sorted by error" (src/solver.cpp:571-573, 719-721)
@@ -254,9 +248,10 @@ int average_module_dev(spe_engine* e, int first, int count, const std::vector<in
   const size_t npix = e->npix;
   float* M = cv.take<float>((size_t)count * npix);
   int* ord = cv.take<int>(count);
+  float2* tmp = cv.take<float2>((size_t)count * npix);
+  if (const int rc = check_work(cv)) return rc;
   spe::Ctx c = item_ctx(e, count, e->A);  // (transforms only; no amplitudes read)
   if (ft) {
-    float2* tmp = cv.take<float2>((size_t)count * npix);
     CK(e->ops->ft_magnitude(c, e->rho + (size_t)first * npix, tmp, M), "average module transforms");
   } else {
     spe::k_abs<<<152 * 8, 256, 0, e->st>>>(e->rho + (size_t)first * npix, M, (size_t)count * npix);
@@ -319,7 +314,7 @@ int spe_reshift(spe_engine* e, int first, int count, int ref_slot, const float* 
                       (size_t)(count + 1) * 2 * sizeof(double) +
                       (size_t)count * (sizeof(spe::ShiftItem) + 2 * sizeof(int) + 8 * sizeof(double)) + 64 * 256;
   if ((rc = ensure_work(e, need))) return rc;
-  Carve cv{(char*)e->work};
+  Carve cv{(char*)e->work, e->work_bytes};
   float2* D = cv.take<float2>((size_t)(count + 1) * npix);  // [0,count) members, count: reference
   float2* scratch = cv.take<float2>((size_t)count * npix);
   double* part = cv.take<double>((size_t)count * tr * spe::NRED);
@@ -330,6 +325,7 @@ int spe_reshift(spe_engine* e, int first, int count, int ref_slot, const float* 
   int* ri = cv.take<int>(count);
   double* peaks = cv.take<double>((size_t)count * 4);
   spe::ShiftItem* items = cv.take<spe::ShiftItem>(count);
+  if ((rc = check_work(cv))) return rc;
   // set_ref_density (gpu_context.cu:632-667): a snapshot of the reference
   if (!e->ref) CK(cudaMalloc(&e->ref, npix * sizeof(float2)), "reference buffer");
   if (ref_slot >= 0)
@@ -419,7 +415,7 @@ int spe_average_module(spe_engine* e, int first, int count, const float* errors,
   if ((rc = ensure_work(e, (size_t)count * npix * (sizeof(float) + sizeof(float2)) + count * sizeof(int) + 1024)))
     return rc;
   if (!e->avg_mod) CK(cudaMalloc(&e->avg_mod, npix * sizeof(float)), "average module buffer");
-  Carve cv{(char*)e->work};
+  Carve cv{(char*)e->work, e->work_bytes};
   if ((rc = average_module_dev(e, first, count, sorted_order(errors, count), ft != 0, fraction, e->avg_mod, cv)))
     return rc;
   if (out) CK(cudaMemcpyAsync(out, e->avg_mod, npix * sizeof(float), cudaMemcpyDeviceToHost, e->st), "download");
@@ -449,12 +445,13 @@ int spe_initialize_pop(spe_engine* e, int first, int count, int support_size, fl
                       (items.size() + 1) * sizeof(spe::InitItem) + count * (sizeof(float) + 2 * sizeof(double)) +
                       4096;
   if ((rc = ensure_work(e, need))) return rc;
-  Carve cv{(char*)e->work};
+  Carve cv{(char*)e->work, e->work_bytes};
   double* part = cv.take<double>((size_t)count * tc * spe::NRED);
   spe::InitDraw* dinds = cv.take<spe::InitDraw>(count);
   spe::InitItem* ditems = cv.take<spe::InitItem>(items.size() + 1);
   float* dscale = cv.take<float>(count);
   double* sums = cv.take<double>((size_t)count * 2);
+  if ((rc = check_work(cv))) return rc;
   CK(cudaMemcpyAsync(dinds, inds.data(), count * sizeof(spe::InitDraw), cudaMemcpyHostToDevice, e->st), "draws");
   if (!items.empty())
     CK(cudaMemcpyAsync(ditems, items.data(), items.size() * sizeof(spe::InitItem), cudaMemcpyHostToDevice, e->st),
@@ -503,9 +500,10 @@ int spe_far_field(spe_engine* e, int first, int count, float* modulus) {
   CK(cudaSetDevice(e->dev), "cudaSetDevice");
   const size_t npix = e->npix;
   if ((rc = ensure_work(e, (size_t)count * npix * (sizeof(float) + sizeof(float2)) + 512))) return rc;
-  Carve cv{(char*)e->work};
+  Carve cv{(char*)e->work, e->work_bytes};
   float* M = cv.take<float>((size_t)count * npix);
   float2* tmp = cv.take<float2>((size_t)count * npix);
+  if ((rc = check_work(cv))) return rc;
   CK(e->ops->ft_magnitude(item_ctx(e, count, e->A), e->rho + (size_t)first * npix, tmp, M), "far-field transforms");
   CK(cudaMemcpyAsync(modulus, M, (size_t)count * npix * sizeof(float), cudaMemcpyDeviceToHost, e->st), "download");
   CK(cudaStreamSynchronize(e->st), "synchronize");
@@ -561,21 +559,15 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
 
   // ---- host: order, support size, average module, draws (solver.cpp:716-801)
   const std::vector<int> order = sorted_order(errors, P);
-  size_t need = (size_t)(P + 1) * npix * sizeof(float2)        // spectra
-                + (size_t)items * npix * sizeof(float2)        // correlation scratch
-                + (size_t)5 * P * npix * sizeof(float2)        // parents per child (and correlation scratch)
-                + (size_t)P * npix * sizeof(float2)            // children
-                + (size_t)3 * P * npix * sizeof(int)           // supports per child
-                + (size_t)(2 * items + P + 1) * tr * spe::NRED * sizeof(double) + (size_t)items * 4 * sizeof(double) +
-                (size_t)(P + 1) * 2 * sizeof(double) + (size_t)items * (2 * sizeof(int) + sizeof(spe::ShiftItem)) +
-                (size_t)P * (sizeof(spe::CrossChild) + npix / 4 + 2 * sizeof(int)) + 64 * 256;
+  const size_t nred = (size_t)tr * spe::NRED;
+  const size_t need = CrossWork::bytes(P, npix, nred, pairs, per, 0);
   const size_t mod_need = (size_t)P * npix * (sizeof(float) + sizeof(float2)) + P * sizeof(int) + 1024;
   if ((rc = ensure_work(e, std::max(need, mod_need)))) return rc;
   if (!e->avg_mod) CK(cudaMalloc(&e->avg_mod, npix * sizeof(float)), "average module buffer");
 
   long long* bsum = nullptr;
   {
-    Carve cv{(char*)e->work};
+    Carve cv{(char*)e->work, e->work_bytes};
     bsum = cv.take<long long>(1);
     CK(cudaMemsetAsync(bsum, 0, sizeof(long long), e->st), "memset");
     spe::k_int_sum<<<152, 256, 0, e->st>>>(e->S + (size_t)best_slot * npix, npix, bsum);
@@ -584,7 +576,7 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
     CK(cudaMemcpyAsync(&hb, bsum, sizeof(long long), cudaMemcpyDeviceToHost, e->st), "support sum");
     CK(cudaStreamSynchronize(e->st), "synchronize");
     // GetAverageModule(rec_array, true, 0.66) (solver.cpp:731)
-    Carve cm{(char*)e->work};
+    Carve cm{(char*)e->work, e->work_bytes};
     if (averaged && (rc = average_module_dev(e, first, P, order, true, 0.66f, e->avg_mod, cm))) return rc;
     // suppdim (solver.cpp:724-729)
     float suppdim = (float)(2. * std::sqrt((double)float(hb) / M_PI));
@@ -627,35 +619,22 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
       if (!ch[i].cft) ch[i].w = wr++;
 
     // (grows only when the crossmaps need more room; synchronises first)
-    if ((rc = ensure_work(e, need + cmaps.size() * sizeof(int) + 4096))) return rc;
-    Carve cv2{(char*)e->work};
-    float2* D = cv2.take<float2>((size_t)(P + 1) * npix);
-    float2* scratch = cv2.take<float2>((size_t)items * npix);
-    float2* W = cv2.take<float2>((size_t)5 * P * npix);
-    float2* C = cv2.take<float2>((size_t)P * npix);
-    int* Ws = cv2.take<int>((size_t)3 * P * npix);
-    double* part = cv2.take<double>((size_t)items * tr * spe::NRED);
-    double* part2 = cv2.take<double>((size_t)items * tr * spe::NRED);
-    double* psum = cv2.take<double>((size_t)(P + 1) * tr * spe::NRED);
-    double* peaks = cv2.take<double>((size_t)items * 4);
-    double* sums = cv2.take<double>((size_t)(P + 1) * 2);
-    int* xi = cv2.take<int>(items);
-    int* ri = cv2.take<int>(items);
-    spe::ShiftItem* sitems = cv2.take<spe::ShiftItem>(5 * P);
-    spe::CrossChild* dch = cv2.take<spe::CrossChild>(P);
-    unsigned char* bits = cv2.take<unsigned char>((size_t)P * npix / 4);
-    int* dcm = cv2.take<int>(cmaps.size() + 1);
+    if ((rc = ensure_work(e, CrossWork::bytes(P, npix, nred, pairs, per, cmaps.size())))) return rc;
+    Carve cv2{(char*)e->work, e->work_bytes};
+    const CrossWork ws(cv2, P, npix, nred, pairs, per, cmaps.size());
+    if ((rc = check_work(cv2))) return rc;
 
     // ---- alignment of self, p2, p3 and the average to p1
     // (prepare_parents / reshift_parent, gpu_context.cu:1536-1694; spectra
     // not normalised on this path).  Spectra of the members and the average.
     spe::Ctx c = item_ctx(e, P, Apat);
-    CK(e->ops->abs_spectrum_items(c, e->rho + (size_t)first * npix, D, psum), "spectra");
+    CK(e->ops->abs_spectrum_items(c, e->rho + (size_t)first * npix, ws.D, ws.psum), "spectra");
     if (averaged)
-      CK(e->ops->abs_spectrum_items(item_ctx(e, 1, Apat), e->rho + (size_t)avg_slot * npix, D + (size_t)P * npix,
-                                    psum + (size_t)P * tr * spe::NRED),
+      CK(e->ops->abs_spectrum_items(item_ctx(e, 1, Apat), e->rho + (size_t)avg_slot * npix, ws.D + (size_t)P * npix,
+                                    ws.psum + P * nred),
          "average spectrum");
-    if ((rc = reduce(e, averaged ? P + 1 : P, {{psum, tr, 0, 0, 0}, {psum, tr, 1, 0, 1}}, sums, 2))) return rc;
+    if ((rc = reduce(e, averaged ? P + 1 : P, {{ws.psum, tr, 0, 0, 0}, {ws.psum, tr, 1, 0, 1}}, ws.sums, 2)))
+      return rc;
     if ((rc = band_weights(e, first, P, minr, maxr))) return rc;
     std::vector<int> hx(items), hr(items);
     for (int i = 0; i < P; ++i) {
@@ -665,15 +644,15 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
         hr[pairs * i + k] = p1[i];
       }
     }
-    CK(cudaMemcpyAsync(xi, hx.data(), items * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
-    CK(cudaMemcpyAsync(ri, hr.data(), items * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
+    CK(cudaMemcpyAsync(ws.xi, hx.data(), items * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
+    CK(cudaMemcpyAsync(ws.ri, hr.data(), items * sizeof(int), cudaMemcpyHostToDevice, e->st), "pairs");
     spe::Ctx ci = item_ctx(e, items, Apat);
     // (W holds nothing yet: scratch of the second product)
-    CK(e->ops->corr_peaks(ci, D, D, xi, ri, 0, 0, scratch, W, part, part2), "correlation");
-    if ((rc = reduce(e, items, {{part, tr, 0, 2, 0}, {part2, tr, 0, 2, 2}}, peaks, 4))) return rc;
+    CK(e->ops->corr_peaks(ci, ws.D, ws.D, ws.xi, ws.ri, 0, 0, ws.scratch, ws.W, ws.part, ws.part2), "correlation");
+    if ((rc = reduce(e, items, {{ws.part, tr, 0, 2, 0}, {ws.part2, tr, 0, 2, 2}}, ws.peaks, 4))) return rc;
     std::vector<double> hp((size_t)items * 4), hs((size_t)(averaged ? P + 1 : P) * 2);
-    CK(cudaMemcpyAsync(hp.data(), peaks, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "peaks");
-    CK(cudaMemcpyAsync(hs.data(), sums, hs.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "sums");
+    CK(cudaMemcpyAsync(hp.data(), ws.peaks, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "peaks");
+    CK(cudaMemcpyAsync(hs.data(), ws.sums, hs.size() * sizeof(double), cudaMemcpyDeviceToHost, e->st), "sums");
     CK(cudaStreamSynchronize(e->st), "synchronize");
 
     // ---- gathered parents per child (source pool: the population, slots absolute)
@@ -702,14 +681,16 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
       spe::ShiftItem& it = hi[per * w + 1];
       it = spe::ShiftItem{first + p1[i], per * w + 1, -1, -1, 0, 0, 1.f, 0.f, 0, 0, 1, first + p1[i]};
     }
-    CK(cudaMemcpyAsync(sitems, hi.data(), hi.size() * sizeof(spe::ShiftItem), cudaMemcpyHostToDevice, e->st),
+    CK(cudaMemcpyAsync(ws.items, hi.data(), hi.size() * sizeof(spe::ShiftItem), cudaMemcpyHostToDevice, e->st),
        "items");
-    CK(cudaMemcpyAsync(dch, hc.data(), P * sizeof(spe::CrossChild), cudaMemcpyHostToDevice, e->st), "children");
-    CK(cudaMemcpyAsync(dcm, cmaps.data(), cmaps.size() * sizeof(int), cudaMemcpyHostToDevice, e->st), "crossmaps");
+    CK(cudaMemcpyAsync(ws.children, hc.data(), P * sizeof(spe::CrossChild), cudaMemcpyHostToDevice, e->st),
+       "children");
+    CK(cudaMemcpyAsync(ws.cmaps, cmaps.data(), cmaps.size() * sizeof(int), cudaMemcpyHostToDevice, e->st),
+       "crossmaps");
     const spe::Gate g = gate_er(reality);
     // (the children's slots are no parent's: the population is read and written)
-    const spe::CrossArgs a{e->rho, e->S, e->rho, e->S, sitems, dch, W, Ws, C, bits, dcm, (int)cmaps.size(),
-                           e->avg_mod, per, ncft, crossdiff, use_average, crosssym, update_support};
+    const spe::CrossArgs a{e->rho, e->S, e->rho, e->S, ws.items, ws.children, ws.W, ws.Ws, ws.C, ws.bits, ws.cmaps,
+                           (int)cmaps.size(), e->avg_mod, per, ncft, crossdiff, use_average, crosssym, update_support};
     // Fourier-space children: their parents' transforms stay in the passes
     // where the side has blocked ones; the others' go through W
     const bool fused = e->ops->cross_fourier != nullptr;
@@ -717,13 +698,13 @@ int spe_crossover(spe_engine* e, int first, int count, const float* errors, int 
     if (fused && ncft > 0) CK(e->ops->cross_fourier(item_ctx(e, ncft, Apat), a, g), "Fourier-space children");
     if (from < P) {
       const unsigned px = (unsigned)((npix + 255) / 256);
-      spe::k_shift_gather<<<dim3(px, (unsigned)(per * (P - from))), 256, 0, e->st>>>(e->rho, e->S, W, Ws,
-                                                                                  sitems + per * from, n, g);
+      spe::k_shift_gather<<<dim3(px, (unsigned)(per * (P - from))), 256, 0, e->st>>>(e->rho, e->S, ws.W, ws.Ws,
+                                                                                  ws.items + per * from, n, g);
       CK(cudaGetLastError(), "parent gather");
-      if (!fused && ncft > 0) CK(e->ops->fft2(item_ctx(e, per * ncft, Apat), W, +1), "parent transforms");
+      if (!fused && ncft > 0) CK(e->ops->fft2(item_ctx(e, per * ncft, Apat), ws.W, +1), "parent transforms");
       spe::k_cross<<<dim3(px, (unsigned)(P - from)), 256, 0, e->st>>>(a, from, Apat, n);
       CK(cudaGetLastError(), "crossover");
-      if (!fused && ncft > 0) CK(e->ops->fft2(item_ctx(e, ncft, Apat), C, -1), "child transforms");
+      if (!fused && ncft > 0) CK(e->ops->fft2(item_ctx(e, ncft, Apat), ws.C, -1), "child transforms");
       spe::k_cross_finish<<<dim3(px, (unsigned)(P - from)), 256, 0, e->st>>>(a, from, npix, g);
       CK(cudaGetLastError(), "crossover finish");
     }
