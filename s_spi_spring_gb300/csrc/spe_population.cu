@@ -169,17 +169,25 @@ __global__ void k_scale_items(float2* __restrict__ rho, const float* __restrict_
 }
 
 // individual dst_first+blockIdx.y <- individual src[blockIdx.y] (density and
-// support, 16-byte vectors; npix is a multiple of 4)
+// support; 16-byte accesses where every individual starts on 16 bytes in both
+// arrays, as a multiple of 4 pixels does: not at odd sides)
 __global__ void k_gather(float2* __restrict__ rho, int* __restrict__ S, const int* __restrict__ src, int dst_first,
                          size_t npix) {
   const size_t from = (size_t)src[blockIdx.y] * npix, to = (size_t)(dst_first + blockIdx.y) * npix;
+  const size_t stride = (size_t)gridDim.x * blockDim.x, i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (npix % 4 != 0) {
+    for (size_t i = i0; i < npix; i += stride) {
+      rho[to + i] = rho[from + i];
+      S[to + i] = S[from + i];
+    }
+    return;
+  }
   const float4* rs = reinterpret_cast<const float4*>(rho + from);
   float4* rd = reinterpret_cast<float4*>(rho + to);
   const int4* ss = reinterpret_cast<const int4*>(S + from);
   int4* sd = reinterpret_cast<int4*>(S + to);
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < npix / 2; i += stride) rd[i] = rs[i];
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < npix / 4; i += stride) sd[i] = ss[i];
+  for (size_t i = i0; i < npix / 2; i += stride) rd[i] = rs[i];
+  for (size_t i = i0; i < npix / 4; i += stride) sd[i] = ss[i];
 }
 
 }  // namespace spe
