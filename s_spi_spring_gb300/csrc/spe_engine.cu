@@ -225,6 +225,11 @@ int have_patterns(spe_engine* e, int first, int count) {
   return SPE_OK;
 }
 
+size_t max_tiles(const spe::SizeOps* o) {
+  return (size_t)std::max(std::max(o->tiles_rows, o->tiles_cols), o->loss_tiles);
+}
+size_t region(spe_engine* e) { return (size_t)e->cap * max_tiles(e->ops) * spe::NRED; }
+
 spe::Ctx make_ctx(spe_engine* e, int first, int count) {
   spe::Ctx c;
   c.n = e->n;
@@ -249,6 +254,9 @@ spe::Ctx make_ctx(spe_engine* e, int first, int count) {
   c.band = e->band;
   c.sp = e->sp;
   c.odd = e->odd;
+  // (the loss passes may run on another stream than an iteration, so they share
+  // none of its arrays: their flags follow the region of their own partials)
+  c.flags = reinterpret_cast<unsigned char*>(e->partials + region(e));
   c.bad = e->sel_state;
   return c;
 }
@@ -349,11 +357,6 @@ int run_iterations(spe_engine* e, int first, int count, int upd, int iters, floa
   CK(cudaStreamWaitEvent(e->st, e->join, 0), "join");
   return SPE_OK;
 }
-
-size_t max_tiles(const spe::SizeOps* o) {
-  return (size_t)std::max(std::max(o->tiles_rows, o->tiles_cols), o->loss_tiles);
-}
-size_t region(spe_engine* e) { return (size_t)e->cap * max_tiles(e->ops) * spe::NRED; }
 
 int reduce(spe_engine* e, int count, std::initializer_list<spe::RedJob> jobs, double* out, int ostride) {
   spe::RedJobs j;

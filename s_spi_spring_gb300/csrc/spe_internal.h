@@ -68,8 +68,9 @@ struct Ctx {
   const float* At;
   const float* band;  // weights of the correlation ops (SizeOps::band_table)
   void* sp;
-  unsigned char* odd;  // (the loss passes: row tiles with support)
-  unsigned* bad;       // per individual: a gradient that is not finite
+  unsigned char* odd;
+  unsigned char* flags;  // the loss passes: row tiles with support
+  unsigned* bad;         // per individual: a gradient that is not finite
 };
 
 // One gathered, shifted copy of an individual (reference shift kernel,

@@ -441,7 +441,7 @@ cudaError_t launch_loss_rows_in(const Ctx& c) {
   using P = LossRows<N>;
   static std::atomic<unsigned long long> configured{0ull};
   return launch_loss(k_loss_rows_in<N>, P::SMEM, configured, c.count * (N / Blocked<N>::WR), P::NT, c.st,
-                     static_cast<const float2*>(c.rho), static_cast<const int*>(c.S), c.T, c.odd, c.first, c.tw);
+                     static_cast<const float2*>(c.rho), static_cast<const int*>(c.S), c.T, c.flags, c.first, c.tw);
 }
 template <int N, int LOSS, bool GRAD>
 cudaError_t launch_loss_cols(const Ctx& c, float eps, double* partials) {
@@ -454,7 +454,7 @@ cudaError_t launch_loss_cols(const Ctx& c, float eps, double* partials) {
   const int tiles = c.count * (N / Blocked<N>::BC);
   const int slots = resident_ctas(kern, P::NT, P::SMEM, resident);
   return launch_pdl(kern, tiles < slots ? tiles : slots, P::NT, P::SMEM, c.st, c.T, c.At, c.ipp,
-                    static_cast<const unsigned char*>(c.odd), c.first, c.count, eps, partials, c.tw);
+                    static_cast<const unsigned char*>(c.flags), c.first, c.count, eps, partials, c.tw);
 }
 template <int N>
 cudaError_t launch_loss_rows_out(const Ctx& c, float2* grad, const float* scale) {
@@ -482,7 +482,7 @@ cudaError_t launch_adam_rows(const Ctx& c, float2* m, float2* v, const AdamParam
   using P = LossRows<N>;
   static std::atomic<unsigned long long> configured{0ull};
   return launch_loss(k_adam_rows<N, OUTSIDE>, P::SMEM, configured, c.count * (N / Blocked<N>::WR), P::NT, c.st, c.T,
-                     static_cast<const unsigned char*>(c.odd), static_cast<const int*>(c.S), c.rho, m, v, ap, fresh,
+                     static_cast<const unsigned char*>(c.flags), static_cast<const int*>(c.S), c.rho, m, v, ap, fresh,
                      next, c.first, c.tw);
 }
 
