@@ -302,17 +302,30 @@ int spe_loss_grad(spe_engine* e, const void* density, const int32_t* support, in
  * reference counterpart).  spe_loss_grad_cols computes the loss into
  * loss_out (may be NULL) and the adjoint up to its column pass, leaving the
  * column-transformed gradient in `half` (device, complex64 count*n*n,
- * caller-owned, not the density; it also holds the forward transform).  Its
- * order in memory is the engine's own, and parts that the support multiplies
- * by zero may be left as they were.  spe_grad_rows then runs the adjoint's last pass
- * from `half` into grad_out times grad_scale (as in spe_loss_grad); grad_out
- * may be `half` itself.  `half` must be left unchanged between the calls.
+ * row-major, caller-owned, not the density; it also holds the forward
+ * transform).  spe_grad_rows then runs the adjoint's last pass from `half`
+ * into grad_out times grad_scale (as in spe_loss_grad); grad_out may be
+ * `half` itself.  `half` must be left unchanged between the calls.  Neither
+ * call uses engine memory other than that of the loss sums (spe_grad_rows
+ * none), so that an iteration may run on another stream meanwhile.
  * The gradient equals spe_loss_grad's bit for bit.  density, support and
  * half must start on a 16-byte boundary. */
 int spe_loss_grad_cols(spe_engine* e, const void* density, const int32_t* support, int count, int loss, float eps,
                        double* loss_out, void* half);
 int spe_grad_rows(spe_engine* e, const void* half, const int32_t* support, int count, void* grad_out,
                   const float* grad_scale);
+
+/* The same two steps for a caller that only hands the buffers on: nothing is
+ * read or written for rows without support, which is where most of the time
+ * of spe_loss_grad_cols and spe_grad_rows goes.  `kept` (device, complex64
+ * count*n*n) and `marks` (device, count * (n + 4) bytes on a 4-byte boundary)
+ * are the caller's; their contents are the engine's own and must be left
+ * unchanged, with the support, until spe_loss_backward, whose grad_out may be
+ * `kept` itself.  Otherwise as above, the gradient's bits too. */
+int spe_loss_forward(spe_engine* e, const void* density, const int32_t* support, int count, int loss, float eps,
+                     double* loss_out, void* kept, void* marks);
+int spe_loss_backward(spe_engine* e, const void* kept, const void* marks, const int32_t* support, int count,
+                      void* grad_out, const float* grad_scale);
 
 /* CUDA graphs of engine calls (no reference counterpart).  Between
  * spe_graph_begin(stream) and spe_graph_end(stream, &g), asynchronous engine

@@ -86,6 +86,8 @@ SIGNATURES = {
     "spe_loss_grad": (_i, [_vp, _vp, _vp, _i, _i, _f, _vp, _vp, _vp]),
     "spe_loss_grad_cols": (_i, [_vp, _vp, _vp, _i, _i, _f, _vp, _vp]),
     "spe_selftest_bounded_wait": (_i, [_vp]),
+    "spe_loss_forward": (_i, [_vp, _vp, _vp, _i, _i, _f, _vp, _vp, _vp]),
+    "spe_loss_backward": (_i, [_vp, _vp, _vp, _vp, _i, _vp, _vp]),
     "spe_grad_rows": (_i, [_vp, _vp, _vp, _i, _vp, _vp]),
     "spe_set_amplitudes_batch": (_i, [_vp, _fp, _i, _i]),
     "spe_adam_step": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _f, _f, _f, _f, _f, _i, _vp]),
@@ -406,6 +408,16 @@ class Engine:
     def grad_rows(self, half_ptr, support_ptr, count, grad_ptr, scale_ptr=0):
         """The adjoint's last pass from ``half`` (grad may be half)."""
         call("spe_grad_rows", self.h, _vp(half_ptr), _vp(support_ptr), int(count), _vp(grad_ptr),
+             _vp(scale_ptr or 0))
+
+    def loss_forward(self, density_ptr, support_ptr, count, kept_ptr, marks_ptr, loss=0, eps=0.0, loss_ptr=0):
+        """Loss, and what its gradient needs in ``kept`` and ``marks``."""
+        call("spe_loss_forward", self.h, _vp(density_ptr), _vp(support_ptr), int(count), int(loss), float(eps),
+             _vp(loss_ptr or 0), _vp(kept_ptr), _vp(marks_ptr))
+
+    def loss_backward(self, kept_ptr, marks_ptr, support_ptr, count, grad_ptr, scale_ptr=0):
+        """The gradient from ``kept`` and ``marks`` (grad may be kept)."""
+        call("spe_loss_backward", self.h, _vp(kept_ptr), _vp(marks_ptr), _vp(support_ptr), int(count), _vp(grad_ptr),
              _vp(scale_ptr or 0))
 
     def adam_step(self, density_ptr, support_ptr, m_ptr, v_ptr, count, loss=1, eps=0.0, lr=1e-3, beta1=0.9,

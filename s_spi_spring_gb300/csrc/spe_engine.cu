@@ -230,6 +230,12 @@ size_t max_tiles(const spe::SizeOps* o) {
 }
 size_t region(spe_engine* e) { return (size_t)e->cap * max_tiles(e->ops) * spe::NRED; }
 
+// marks of the loss passes for `items` items: spe_loss_forward's layout
+static void set_marks(spe::Ctx& c, void* marks, int items) {
+  c.bad = static_cast<unsigned*>(marks);
+  c.flags = static_cast<unsigned char*>(marks) + (size_t)items * sizeof(unsigned);
+}
+
 spe::Ctx make_ctx(spe_engine* e, int first, int count) {
   spe::Ctx c;
   c.n = e->n;
@@ -255,9 +261,8 @@ spe::Ctx make_ctx(spe_engine* e, int first, int count) {
   c.sp = e->sp;
   c.odd = e->odd;
   // (the loss passes may run on another stream than an iteration, so they share
-  // none of its arrays: their flags follow the region of their own partials)
-  c.flags = reinterpret_cast<unsigned char*>(e->partials + region(e));
-  c.bad = e->sel_state;
+  // none of its arrays: their marks follow the region of their own partials)
+  set_marks(c, e->partials + region(e), e->cap);
   return c;
 }
 
@@ -1009,6 +1014,14 @@ static int loss_args(spe_engine* e, const void* density, const int32_t* support,
   return 0;
 }
 
+// the buffers between the two halves of the gradient
+static int kept_args(const spe_engine* e, const void* kept, const void* marks) {
+  if (!kept || !marks) return fail(SPE_ERR_INVALID, "null gradient buffer or marks");
+  if (misaligned16(e, kept)) return fail(SPE_ERR_INVALID, "the gradient buffer must start on a 16-byte boundary");
+  if (reinterpret_cast<uintptr_t>(marks) & 3u) return fail(SPE_ERR_INVALID, "marks must start on a 4-byte boundary");
+  return SPE_OK;
+}
+
 // per-item losses from the column-pass partials into loss_out
 static int loss_sums(spe_engine* e, int count, double* loss_out) {
   return reduce(e, count, {{e->partials, e->ops->loss_tiles, 0, 0, 0}}, loss_out, 1);
@@ -1060,6 +1073,43 @@ int spe_grad_rows(spe_engine* e, const void* half, const int32_t* support, int c
   c.T = static_cast<float2*>(const_cast<void*>(half));
   CK(e->ops->loss_grad(c, SPE_LOSS_AMPLITUDE, 0.f, nullptr, static_cast<float2*>(grad_out), grad_scale,
                        spe::GRAD_ROWS),
+     "gradient row pass");
+  return SPE_OK;
+}
+
+int spe_loss_forward(spe_engine* e, const void* density, const int32_t* support, int count, int loss, float eps,
+                     double* loss_out, void* kept, void* marks) {
+  int rc;
+  if (loss_args(e, density, support, count, loss, eps, &rc)) return rc;
+  if ((rc = kept_args(e, kept, marks))) return rc;
+  if (kept == density) return fail(SPE_ERR_INVALID, "the gradient buffer must not be the density");
+  if ((rc = spe_reserve(e, count))) return rc;  // partials for `count` items
+  CK(cudaSetDevice(e->dev), "cudaSetDevice");
+  spe::Ctx c = make_ctx(e, 0, count);
+  c.rho = static_cast<float2*>(const_cast<void*>(density));
+  c.S = const_cast<int*>(support);
+  c.T = static_cast<float2*>(kept);
+  set_marks(c, marks, count);
+  CK(e->ops->loss_grad(c, loss, eps, e->partials, c.T, nullptr, spe::GRAD_FORWARD), "loss kernels");
+  return loss_out ? loss_sums(e, count, loss_out) : SPE_OK;
+}
+
+int spe_loss_backward(spe_engine* e, const void* kept, const void* marks, const int32_t* support, int count,
+                      void* grad_out, const float* grad_scale) {
+  if (!e) return fail(SPE_ERR_INVALID, "null engine");
+  if (count < 0) return fail(SPE_ERR_INVALID, "negative count");
+  if (count == 0) return SPE_OK;
+  int rc = kept_args(e, kept, marks);
+  if (rc) return rc;
+  if (!support || !grad_out) return fail(SPE_ERR_INVALID, "null support or output");
+  if (misaligned16(e, support)) return fail(SPE_ERR_INVALID, "the support must start on a 16-byte boundary");
+  CK(cudaSetDevice(e->dev), "cudaSetDevice");
+  spe::Ctx c = make_ctx(e, 0, count);
+  c.S = const_cast<int*>(support);
+  c.T = static_cast<float2*>(const_cast<void*>(kept));
+  set_marks(c, const_cast<void*>(marks), count);
+  CK(e->ops->loss_grad(c, SPE_LOSS_AMPLITUDE, 0.f, nullptr, static_cast<float2*>(grad_out), grad_scale,
+                       spe::GRAD_BACKWARD),
      "gradient row pass");
   return SPE_OK;
 }
@@ -1160,6 +1210,7 @@ int spe_adam_step(spe_engine* e, void* density, const int32_t* support, void* ex
   spe::Ctx c = make_ctx(e, 0, count);
   c.rho = static_cast<float2*>(density);
   c.S = const_cast<int*>(support);
+  c.bad = nullptr;
   CK(e->ops->adam_step(c, loss, eps, e->partials, static_cast<float2*>(exp_avg), static_cast<float2*>(exp_avg_sq),
                        adam_params(lr, beta1, beta2, adam_eps, step)),
      "refinement kernels");
@@ -1178,6 +1229,7 @@ int spe_adam_run(spe_engine* e, void* density, const int32_t* support, void* exp
   spe::Ctx c = make_ctx(e, 0, count);
   c.rho = static_cast<float2*>(density);
   c.S = const_cast<int*>(support);
+  c.bad = nullptr;
   const bool inside = e->ops->blocked_cols != 0;
   if (!inside) {
     const size_t bytes = (size_t)count * e->npix * sizeof(float2);

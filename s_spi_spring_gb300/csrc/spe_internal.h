@@ -9,8 +9,10 @@
 
 namespace spe {
 
-// Stages of the far-field loss gradient (SizeOps::loss_grad).
-enum { GRAD_ALL = 0, GRAD_COLS = 1, GRAD_ROWS = 2 };
+// Stages of the far-field loss gradient (SizeOps::loss_grad): all of it; up to
+// the column pass, and the row pass, through a whole row-major T; the same two
+// through T and the flags as they are (Ctx::flags, bad).
+enum { GRAD_ALL = 0, GRAD_COLS = 1, GRAD_ROWS = 2, GRAD_FORWARD = 3, GRAD_BACKWARD = 4 };
 
 // Host pattern encoding (spe_host.cpp).
 int prepare_pattern(const float* in, int n, int cx, int cy, bool use_bounds, float* out);
@@ -69,8 +71,11 @@ struct Ctx {
   const float* band;  // weights of the correlation ops (SizeOps::band_table)
   void* sp;
   unsigned char* odd;
-  unsigned char* flags;  // the loss passes: row tiles with support
-  unsigned* bad;         // per individual: a gradient that is not finite
+  // marks of the loss passes: row tiles with support, and per individual
+  // whether the column-transformed gradient is not finite (bad null: not marked,
+  // for a caller that updates nothing outside the support)
+  unsigned char* flags;
+  unsigned* bad;
 };
 
 // One gathered, shifted copy of an individual (reference shift kernel,

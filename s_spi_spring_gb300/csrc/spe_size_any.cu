@@ -975,7 +975,7 @@ struct SizeAny {
   static cudaError_t loss_grad_t(const Ctx& c, float eps, double* partials, float2* grad, const float* scale,
                                  int stage) {
     const AnyPlan& pl = plain_of(c.n);
-    if (stage == GRAD_ROWS) return grad_rows(c, pl, grad, scale);
+    if (stage == GRAD_ROWS || stage == GRAD_BACKWARD) return grad_rows(c, pl, grad, scale);
     OpRowsSupportForward rf;
     rf.first = c.first;
     rf.rho = c.rho;
@@ -1000,8 +1000,7 @@ struct SizeAny {
     cl.ipp = c.ipp;
     cl.eps = eps;
     SPE_TRY((launch_any<AX_COLS>(cl, pl, c.count, c.st, c.tw)));
-    if (stage == GRAD_COLS) return cudaSuccess;
-    return grad_rows(c, pl, grad, scale);
+    return stage == GRAD_ALL ? grad_rows(c, pl, grad, scale) : cudaSuccess;
   }
 
   static cudaError_t loss_grad(const Ctx& c, int loss, float eps, double* partials, float2* grad,

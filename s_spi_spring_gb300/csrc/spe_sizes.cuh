@@ -436,17 +436,18 @@ cudaError_t launch_loss(K kern, size_t smem, std::atomic<unsigned long long>& co
   if (e != cudaSuccess || grid <= 0) return e;
   return launch_pdl(kern, grid, threads, smem, st, args...);
 }
-template <int N>
+template <int N, class L>
 cudaError_t launch_loss_rows_in(const Ctx& c) {
   using P = LossRows<N>;
   static std::atomic<unsigned long long> configured{0ull};
-  return launch_loss(k_loss_rows_in<N>, P::SMEM, configured, c.count * (N / Blocked<N>::WR), P::NT, c.st,
-                     static_cast<const float2*>(c.rho), static_cast<const int*>(c.S), c.T, c.flags, c.first, c.tw);
+  return launch_loss(k_loss_rows_in<N, L>, P::SMEM, configured, c.count * (N / Blocked<N>::WR), P::NT, c.st,
+                     static_cast<const float2*>(c.rho), static_cast<const int*>(c.S), c.T, c.flags, c.bad, c.first,
+                     c.tw);
 }
-template <int N, int LOSS, bool GRAD>
+template <int N, int LOSS, bool GRAD, class L, bool MARK>
 cudaError_t launch_loss_cols(const Ctx& c, float eps, double* partials) {
   using P = LossCols<N>;
-  auto kern = k_loss_cols<N, LOSS, GRAD>;
+  auto kern = k_loss_cols<N, LOSS, GRAD, L, MARK>;
   static std::atomic<unsigned long long> configured{0ull};
   static std::atomic<int> resident[64] = {};
   cudaError_t e = configure(kern, P::SMEM, configured);
@@ -454,28 +455,15 @@ cudaError_t launch_loss_cols(const Ctx& c, float eps, double* partials) {
   const int tiles = c.count * (N / Blocked<N>::BC);
   const int slots = resident_ctas(kern, P::NT, P::SMEM, resident);
   return launch_pdl(kern, tiles < slots ? tiles : slots, P::NT, P::SMEM, c.st, c.T, c.At, c.ipp,
-                    static_cast<const unsigned char*>(c.flags), c.first, c.count, eps, partials, c.tw);
+                    static_cast<const unsigned char*>(c.flags), c.bad, c.first, c.count, eps, partials, c.tw);
 }
-template <int N>
+template <int N, class L>
 cudaError_t launch_loss_rows_out(const Ctx& c, float2* grad, const float* scale) {
   using P = LossRows<N>;
   static std::atomic<unsigned long long> configured{0ull};
-  cudaError_t e = cudaMemsetAsync(c.bad + c.first, 0, (size_t)c.count * sizeof(unsigned), c.st);
-  if (e != cudaSuccess) return e;
-  e = launch_loss(k_loss_rows_out<N>, P::SMEM, configured, c.count * (N / Blocked<N>::WR), P::NT, c.st,
-                  static_cast<const float2*>(c.T), static_cast<const int*>(c.S), grad, scale, c.bad, c.first, c.tw);
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)c.count, 8);
-  cfg.blockDim = dim3(256);
-  cfg.stream = c.st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_loss_rows_bad, static_cast<const int*>(c.S), grad, N, Blocked<N>::WR, c.first,
-                            static_cast<const unsigned*>(c.bad));
+  return launch_loss(k_loss_rows_out<N, L>, P::SMEM, configured, c.count * (N / Blocked<N>::WR), P::NT, c.st,
+                     static_cast<const float2*>(c.T), static_cast<const int*>(c.S), grad, scale,
+                     static_cast<const unsigned char*>(c.flags), static_cast<const unsigned*>(c.bad), c.first, c.tw);
 }
 template <int N, bool OUTSIDE>
 cudaError_t launch_adam_rows(const Ctx& c, float2* m, float2* v, const AdamParams& ap, int fresh, int next) {
@@ -900,10 +888,10 @@ struct SizeImpl {
   // grad = scale[p] * 2 S FFT-(dL/dconj F) for items [first, first+count)
   // of c.rho / c.S (c.T is scratch).  Through the support's row tiles where
   // the side has blocked passes (spe_support.cuh), else row-major.
-  // S * rho -> FFT+ (x) -> T
-  static cudaError_t support_forward(const Ctx& c) {
+  // S * rho -> FFT+ (x) -> T; whole: row-major, every row after the column pass
+  static cudaError_t support_forward(const Ctx& c, bool whole) {
     if constexpr (Blocked<N>::ok) {
-      return launch_loss_rows_in<N>(c);
+      return whole ? launch_loss_rows_in<N, LossRowMajor<N>>(c) : launch_loss_rows_in<N, LossT<N>>(c);
     } else {
       OpRowsSupportForward rf;
       rf.first = c.first;
@@ -914,9 +902,13 @@ struct SizeImpl {
     }
   }
   template <int LOSS, bool GRAD>
-  static cudaError_t loss_cols(const Ctx& c, float eps, double* partials) {
+  static cudaError_t loss_cols(const Ctx& c, float eps, double* partials, bool whole) {
     if constexpr (Blocked<N>::ok) {
-      return launch_loss_cols<N, LOSS, GRAD>(c, eps, partials);
+      if constexpr (GRAD) {
+        if (whole) return launch_loss_cols<N, LOSS, true, LossRowMajor<N>, false>(c, eps, partials);
+        if (c.bad) return launch_loss_cols<N, LOSS, true, LossT<N>, true>(c, eps, partials);
+      }
+      return launch_loss_cols<N, LOSS, GRAD, LossT<N>, false>(c, eps, partials);
     } else {
       OpColsLoss<LOSS, GRAD> cl;
       cl.first = c.first;
@@ -929,9 +921,10 @@ struct SizeImpl {
     }
   }
   // the last pass of the adjoint: T -> FFT- (x) -> grad = scale[p] * S * .
-  static cudaError_t grad_rows(const Ctx& c, float2* grad, const float* scale) {
+  static cudaError_t grad_rows(const Ctx& c, float2* grad, const float* scale, bool whole) {
     if constexpr (Blocked<N>::ok) {
-      return launch_loss_rows_out<N>(c, grad, scale);
+      return whole ? launch_loss_rows_out<N, LossRowMajor<N>>(c, grad, scale)
+                   : launch_loss_rows_out<N, LossT<N>>(c, grad, scale);
     } else {
       OpRowsGradOut go;
       go.first = c.first;
@@ -945,20 +938,20 @@ struct SizeImpl {
   template <int LOSS>
   static cudaError_t loss_grad_t(const Ctx& c, float eps, double* partials, float2* grad, const float* scale,
                                  int stage) {
-    if (stage == GRAD_ROWS) return grad_rows(c, grad, scale);
-    SPE_TRY(support_forward(c));
-    if (!grad && stage == GRAD_ALL) return loss_cols<LOSS, false>(c, eps, partials);
-    SPE_TRY((loss_cols<LOSS, true>(c, eps, partials)));
-    if (stage == GRAD_COLS) return cudaSuccess;
-    return grad_rows(c, grad, scale);
+    const bool whole = stage == GRAD_COLS || stage == GRAD_ROWS;
+    if (stage == GRAD_ROWS || stage == GRAD_BACKWARD) return grad_rows(c, grad, scale, whole);
+    SPE_TRY(support_forward(c, whole));
+    if (!grad && stage == GRAD_ALL) return loss_cols<LOSS, false>(c, eps, partials, false);
+    SPE_TRY((loss_cols<LOSS, true>(c, eps, partials, whole)));
+    return stage == GRAD_ALL ? grad_rows(c, grad, scale, false) : cudaSuccess;
   }
   // loss (partials) at the current densities, then one Adam step in place
   template <int LOSS>
   static cudaError_t adam_step_t(const Ctx& c, float eps, double* partials, float2* m, float2* v,
                                  const AdamStep& a) {
     const AdamParams ap = {a.b1, a.b2, a.step_size, a.inv_sqrt_bc2, a.eps};
-    if (!a.prepared) SPE_TRY(support_forward(c));
-    SPE_TRY((loss_cols<LOSS, true>(c, eps, partials)));
+    if (!a.prepared) SPE_TRY(support_forward(c, false));
+    SPE_TRY((loss_cols<LOSS, true>(c, eps, partials, false)));
     if constexpr (Blocked<N>::ok) {
       return a.inside ? launch_adam_rows<N, false>(c, m, v, ap, a.fresh, a.next)
                       : launch_adam_rows<N, true>(c, m, v, ap, a.fresh, a.next);

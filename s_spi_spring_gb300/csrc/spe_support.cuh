@@ -11,6 +11,10 @@
 // zeros in registers), and the last row pass transforms those.  A support that
 // fills the field runs every tile, as the row-major kernels did.
 //
+// A caller may also ask for the column-transformed gradient itself, whole and
+// row-major (LossRowMajor): the forward row pass still skips, the column pass
+// writes every row and the last row pass reads every row.
+//
 // Measured on GB300 (row-major passes over every row before -> now): a loss and
 // its gradient at 1024^2 x 32 511 -> 333 us, ten refinement steps at 512^2 x 64
 // 3909 -> 1305 us (345 and 1360 with one exchange buffer in the column pass).
@@ -28,11 +32,19 @@ namespace spe {
 // may replace the scratch in place.
 template <int N>
 struct LossT {
+  static constexpr bool WHOLE = false;  // only the flagged row tiles are written
   static constexpr int WR = Blocked<N>::WR, BC = Blocked<N>::BC;
   static constexpr int XS = WR;  // offset of a step in x that is a multiple of BC, per column
   __host__ __device__ static constexpr int at(int y, int x) {
     return (y / WR) * (WR * N) + (x / BC) * (WR * BC) + (y % WR) * BC + x % BC;
   }
+};
+
+template <int N>
+struct LossRowMajor {
+  static constexpr bool WHOLE = true;
+  static constexpr int XS = 1;
+  __host__ __device__ static constexpr int at(int y, int x) { return y * N + x; }
 };
 
 template <int N>
@@ -47,7 +59,7 @@ struct LossCols : BlkCfg<N, Blocked<N>::BC, 2> {
 };
 
 // A thread's place in a row pass: row c of the tile, position j.
-template <int N>
+template <int N, class L>
 struct RowSlot {
   int c, j, tile, p;
   size_t gi, ti;  // of element 0
@@ -58,7 +70,7 @@ struct RowSlot {
     tile = blockIdx.x;
     p = first + tile / TPI;
     gi = ((size_t)first * N + (size_t)tile * W + c) * N + j;
-    ti = ((size_t)first * N + (size_t)tile * W) * N + LossT<N>::at(c, j);
+    ti = ((size_t)first * N + (size_t)tile * W) * N + L::at(c, j);
   }
 };
 
@@ -77,11 +89,13 @@ __device__ __forceinline__ bool tile_has_support(const int* __restrict__ S, int 
   return __syncthreads_or(any) != 0;
 }
 
-// S rho -> FFT+ (x) -> T for the row tiles with support, flagged in `flags`
-template <int N>
+// S rho -> FFT+ (x) -> T for the row tiles with support, flagged in `flags`;
+// clears `bad`
+template <int N, class L>
 __global__ void __launch_bounds__(LossRows<N>::NT, LossRows<N>::MINB)
     k_loss_rows_in(const float2* __restrict__ rho, const int* __restrict__ S, float2* __restrict__ T,
-                   unsigned char* __restrict__ flags, int first, const float2* __restrict__ twg) {
+                   unsigned char* __restrict__ flags, unsigned* __restrict__ bad, int first,
+                   const float2* __restrict__ twg) {
   using C = LossRows<N>;
   constexpr int E = C::E;
   extern __shared__ __align__(128) unsigned char sm[];
@@ -89,9 +103,12 @@ __global__ void __launch_bounds__(LossRows<N>::NT, LossRows<N>::MINB)
   float2* xb = reinterpret_cast<float2*>(sm + C::TWB);
   pdl_enter();
   pdl_wait();
-  const RowSlot<N> q(first);
+  const RowSlot<N, L> q(first);
   const bool any = tile_has_support<N>(S, first, q.tile);
-  if (threadIdx.x == 0) flags[(size_t)first * (N / Blocked<N>::WR) + q.tile] = any ? 1 : 0;
+  if (threadIdx.x == 0) {
+    flags[(size_t)first * (N / Blocked<N>::WR) + q.tile] = any ? 1 : 0;
+    if (bad && q.tile % (N / Blocked<N>::WR) == 0) bad[q.p] = 0u;
+  }
   if (!any) return;
   int m[E];
 #pragma unroll
@@ -103,16 +120,19 @@ __global__ void __launch_bounds__(LossRows<N>::NT, LossRows<N>::MINB)
   __syncthreads();
   fft_x<N, typename C::Lay, +1, 1, 0>(v, xb, tw, q.c, q.j);
 #pragma unroll
-  for (int e = 0; e < E; ++e) T[q.ti + (size_t)C::step(e) * LossT<N>::XS] = v[e];
+  for (int e = 0; e < E; ++e) T[q.ti + (size_t)C::step(e) * L::XS] = v[e];
 }
 
 // T -> FFT+ (y) = F -> loss terms over the known pixels (one sum per tile); with
 // GRAD -> 2 dL/dconj(F) -> FFT- (y) -> T.  Persistent: the flags of tile k + 2
-// and the rows of tile k + 1 are read while tile k is transformed.
-template <int N, int LOSS, bool GRAD>
+// and the rows of tile k + 1 are read while tile k is transformed.  MARK: bad[p]
+// is set where an item's result is not finite in any row, written or not: the
+// row transform carries it to every pixel, and 0 times it is not a number.
+template <int N, int LOSS, bool GRAD, class L, bool MARK>
 __global__ void __launch_bounds__(LossCols<N>::NT, LossCols<N>::MINB)
     k_loss_cols(float2* __restrict__ T, const float* __restrict__ At, int ipp, const unsigned char* __restrict__ flags,
-                int first, int count, float eps, double* __restrict__ partials, const float2* __restrict__ twg) {
+                unsigned* __restrict__ bad, int first, int count, float eps, double* __restrict__ partials,
+                const float2* __restrict__ twg) {
   using C = LossCols<N>;
   using Lay = typename C::Lay;
   constexpr int E = C::E, NT = C::NT, W = Blocked<N>::BC, WR = Blocked<N>::WR, TPI = N / W;
@@ -139,7 +159,7 @@ __global__ void __launch_bounds__(LossCols<N>::NT, LossCols<N>::MINB)
     return r;
   };
   auto tile_ptr = [&](int tile) {
-    return T + (size_t)(first + tile / TPI) * N * N + LossT<N>::at(j, (tile % TPI) * W + c);
+    return T + (size_t)(first + tile / TPI) * N * N + L::at(j, (tile % TPI) * W + c);
   };
   auto fetch = [&](float2* v, int tile, unsigned rows) {
     const float2* g = tile_ptr(tile);
@@ -184,7 +204,13 @@ __global__ void __launch_bounds__(LossCols<N>::NT, LossCols<N>::MINB)
       float2* g = tile_ptr(tile);
 #pragma unroll
       for (int e = 0; e < E; ++e)
-        if ((rows >> e) & 1u) g[(size_t)C::step(e) * N] = v[e];
+        if (L::WHOLE || ((rows >> e) & 1u)) g[(size_t)C::step(e) * N] = v[e];
+      if constexpr (MARK) {
+        float chk = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) chk += 0.f * v[e].x + 0.f * v[e].y;
+        if (chk != 0.f) bad[p] = 1u;
+      }
     }
     const float r[NRED] = {acc, 0.f, 0.f, 0.f};
     block_reduce_store<NT, 1, 0>(partials, tile, r);
@@ -194,11 +220,12 @@ __global__ void __launch_bounds__(LossCols<N>::NT, LossCols<N>::MINB)
 }
 
 // T -> FFT- (x) -> G = scale[p] * S * (.) (G may be T); the row tiles without
-// support are zeros.  bad[p] is set where a result is not finite.
-template <int N>
+// support (unless T is whole) are zeros, or not a number where bad[p]
+template <int N, class L>
 __global__ void __launch_bounds__(LossRows<N>::NT, LossRows<N>::MINB)
     k_loss_rows_out(const float2* T, const int* __restrict__ S, float2* G, const float* __restrict__ scale,
-                    unsigned* __restrict__ bad, int first, const float2* __restrict__ twg) {
+                    const unsigned char* __restrict__ flags, const unsigned* __restrict__ bad, int first,
+                    const float2* __restrict__ twg) {
   using C = LossRows<N>;
   constexpr int E = C::E;
   extern __shared__ __align__(128) unsigned char sm[];
@@ -206,55 +233,43 @@ __global__ void __launch_bounds__(LossRows<N>::NT, LossRows<N>::MINB)
   float2* xb = reinterpret_cast<float2*>(sm + C::TWB);
   pdl_enter();
   pdl_wait();
-  const RowSlot<N> q(first);
-  if (!tile_has_support<N>(S, first, q.tile)) {
+  const RowSlot<N, L> q(first);
+  if (!L::WHOLE && !__ldcg(flags + (size_t)first * (N / Blocked<N>::WR) + q.tile)) {
+    const float f = __ldcg(bad + q.p) ? __int_as_float(0x7fffffff) : 0.f;
     float2* z = G + ((size_t)first * N + (size_t)q.tile * Blocked<N>::WR) * N;
     if ((reinterpret_cast<uintptr_t>(z) & 15u) == 0) {
 #pragma unroll
-      for (int i = 0; i < E / 2; ++i)
-        reinterpret_cast<float4*>(z)[threadIdx.x + i * C::NT] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < E / 2; ++i) reinterpret_cast<float4*>(z)[threadIdx.x + i * C::NT] = make_float4(f, f, f, f);
     } else {
 #pragma unroll
-      for (int i = 0; i < E; ++i) z[threadIdx.x + i * C::NT] = make_float2(0.f, 0.f);
+      for (int i = 0; i < E; ++i) z[threadIdx.x + i * C::NT] = make_float2(f, f);
     }
     return;
   }
   float2 v[E];
   int m[E];
 #pragma unroll
-  for (int e = 0; e < E; ++e) v[e] = __ldcg(T + q.ti + (size_t)C::step(e) * LossT<N>::XS);
+  for (int e = 0; e < E; ++e) v[e] = __ldcg(T + q.ti + (size_t)C::step(e) * L::XS);
 #pragma unroll
   for (int e = 0; e < E; ++e) m[e] = __ldg(S + q.gi + C::step(e));
   load_twiddles<N>(tw, twg, C::NT);
   __syncthreads();
   fft_x<N, typename C::Lay, -1, 1, 0>(v, xb, tw, q.c, q.j);  // (its barriers: the tile has been read)
   const float sc = scale ? scale[q.p - first] : 1.f;
-  float chk = 0.f;
+  if (L::WHOLE) {
+    int any = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) any |= m[e] > 0;
+    if (!__syncthreads_or(any)) {  // 0 or not a number, as above: no negative zeros
+#pragma unroll
+      for (int e = 0; e < E; ++e) G[q.gi + C::step(e)] = make_float2(fmaf(v[e].x, 0.f, 0.f), fmaf(v[e].y, 0.f, 0.f));
+      return;
+    }
+  }
 #pragma unroll
   for (int e = 0; e < E; ++e) {
-    chk += 0.f * v[e].x + 0.f * v[e].y;
     const float f = m[e] > 0 ? sc : 0.f;
     G[q.gi + C::step(e)] = make_float2(v[e].x * f, v[e].y * f);
-  }
-  if (chk != 0.f) bad[q.p] = 1u;
-}
-
-// A column transform that is not finite reaches every row, and 0 times it is
-// not a number: the rows without support of such items (bad[p]) as well.
-// One block of the y dimension takes every gridDim.y-th row tile.
-static __global__ void k_loss_rows_bad(const int* __restrict__ S, float2* __restrict__ G, int n, int rows, int first,
-                                       const unsigned* __restrict__ bad) {
-  const int p = first + blockIdx.x;
-  pdl_enter();
-  pdl_wait();
-  if (!bad[p]) return;
-  const float q = __int_as_float(0x7fffffff);
-  for (int t = blockIdx.y; t < n / rows; t += gridDim.y) {
-    const size_t base = ((size_t)p * n + (size_t)t * rows) * n;
-    int any = 0;
-    for (int i = threadIdx.x; i < rows * n; i += blockDim.x) any |= S[base + i] > 0;
-    if (!__syncthreads_or(any))
-      for (int i = threadIdx.x; i < rows * n; i += blockDim.x) G[base + i] = make_float2(q, q);
   }
 }
 
@@ -276,7 +291,7 @@ __global__ void __launch_bounds__(LossRows<N>::NT, LossRows<N>::E <= 8 ? 768 / L
   float2* xb = reinterpret_cast<float2*>(sm + C::TWB);
   pdl_enter();
   pdl_wait();
-  const RowSlot<N> q(first);
+  const RowSlot<N, LossT<N>> q(first);
   const bool any = __ldcg(flags + (size_t)first * (N / Blocked<N>::WR) + q.tile) != 0;
   if (!any && !OUTSIDE) return;
   int s[E];

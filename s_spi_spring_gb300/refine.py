@@ -69,9 +69,9 @@ class FarFieldLoss(torch.autograd.Function):
 
     With a gradient of at most STORE_GRADIENT_BYTES (or recompute=False) the
     forward pass computes the loss and the adjoint up to its column pass in
-    one set of passes (``spe_loss_grad_cols``) and keeps that half-transformed
+    one set of passes (``spe_loss_forward``) and keeps that half-transformed
     gradient; the backward pass is the adjoint's last row pass with the
-    upstream scale fused in, in place (``spe_grad_rows``).  Above that size
+    upstream scale fused in, in place (``spe_loss_backward``).  Above that size
     (or with recompute=True) nothing is kept: the backward pass recomputes the
     transform and the whole adjoint (``spe_loss_grad``).  Both run the same
     kernels on the same values, so the gradients are bit-identical."""
@@ -87,14 +87,15 @@ class FarFieldLoss(torch.autograd.Function):
         out = torch.empty(count, dtype=torch.float64, device=density.device)
         if recompute is None:
             recompute = density.numel() * density.element_size() > STORE_GRADIENT_BYTES
-        ctx.half = None
+        ctx.half = ctx.marks = None
         if recompute or not ctx.needs_input_grad[0]:
             engine.loss_grad(density.data_ptr(), support.data_ptr(), count, LOSSES[loss], eps, out.data_ptr(), 0, 0)
         else:
             half = torch.empty_like(density)
-            engine.loss_grad_cols(density.data_ptr(), support.data_ptr(), count, half.data_ptr(), LOSSES[loss], eps,
-                                  out.data_ptr())
-            ctx.half = half
+            marks = torch.empty(count * (density.shape[-1] + 4), dtype=torch.uint8, device=density.device)
+            engine.loss_forward(density.data_ptr(), support.data_ptr(), count, half.data_ptr(), marks.data_ptr(),
+                                LOSSES[loss], eps, out.data_ptr())
+            ctx.half, ctx.marks = half, marks
         ctx.save_for_backward(density, support)
         ctx.engine, ctx.loss, ctx.eps = engine, loss, eps
         return out
@@ -106,8 +107,10 @@ class FarFieldLoss(torch.autograd.Function):
         scale = grad_out.to(torch.float32).contiguous()
         _bind_stream(ctx.engine, density.device)
         if ctx.half is not None:
-            grad, ctx.half = ctx.half, None
-            ctx.engine.grad_rows(grad.data_ptr(), support.data_ptr(), count, grad.data_ptr(), scale.data_ptr())
+            grad, marks = ctx.half, ctx.marks
+            ctx.half = ctx.marks = None
+            ctx.engine.loss_backward(grad.data_ptr(), marks.data_ptr(), support.data_ptr(), count,
+                                     grad.data_ptr(), scale.data_ptr())
             return grad, None, None, None, None, None
         grad = torch.empty_like(density)
         ctx.engine.loss_grad(density.data_ptr(), support.data_ptr(), count, LOSSES[ctx.loss], ctx.eps, 0,
