@@ -165,10 +165,12 @@ struct BlkCfg {
 // used.  A support is compact (a quarter of the rows or less, from the
 // oversampling that phase retrieval needs): the passes between the first and
 // the last column pass leave the other tiles out.  `odd` carries the tiles'
-// state, `live` the list of those with support, its length first.
+// state, `live` the list of those with support: its length, a counter per
+// individual (tiles seen, and 2^16 times those with support), the tiles.
 // (A tile that is not finite counts as one with support: 0 times it is not 0.
-// Not with a phase gate, which may empty the support: the projection of an
-// all-zero transform goes by the signs of its zeros.)
+// An individual without any support has all its tiles in the list: its density
+// is zeros of either sign, and the projection of an all-zero transform goes by
+// their signs.  Not with a phase gate, which may empty a support.)
 enum { TILE_ODD = 1, TILE_LIVE = 2 };
 
 // column pass: T -> FFT+ (y) -> P_M with A -> FFT- (y) -> T.  IN / OUT: only
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
   const int c = t % W, j = t / W;
   // the tiles of the pass: all, or (LIST) the live ones by their list
   const int ntiles = LIST ? __ldcg(live) : count * TPI;
-  auto tile_at = [&](int k) { return LIST ? __ldcg(live + 1 + k) : k; };
+  auto tile_at = [&](int k) { return LIST ? __ldcg(live + 1 + count + k) : k; };
   // offset of a tile's first row in T (blocked), rho and S (row-major)
   auto t_base = [&](int tile) {
     return (size_t)(first + tile / TPI) * N * N + (size_t)(tile % TPI) * (W * B::YS);
@@ -395,13 +397,13 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
 }
 
 // First pass of a call: rho -> FFT+ (x) -> T; packs the support and, with LIST,
-// lists the live tiles (*live: 0 before).  One tile per CTA, loads in flight
-// over many CTAs per SM.
+// lists the live tiles (length and counters: 0 before).  One tile per CTA, loads
+// in flight over many CTAs per SM.
 template <int N, bool LIST>
 __global__ void __launch_bounds__(BlkRowCfg<N>::NT, BlkCfg<N, Blocked<N>::WR, 1>::E <= 8 ? 1024 / BlkRowCfg<N>::NT : 2)
     k_rows_blocked_first(const float2* __restrict__ rho, const int* __restrict__ S, float2* __restrict__ T,
                          SpBits<N>* __restrict__ sp, unsigned char* __restrict__ odd, int* __restrict__ live,
-                         int first, const float2* __restrict__ twg) {
+                         int first, int count, const float2* __restrict__ twg) {
   using B = Blocked<N>;
   using C = BlkCfg<N, B::WR, 1>;
   using Lay = typename C::Lay;
@@ -440,7 +442,22 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, BlkCfg<N, Blocked<N>::WR, 1>
           (LIST && __syncthreads_or(state & TILE_LIVE) ? TILE_LIVE : 0);
   if (t == 0) {
     odd[(size_t)first * TPI + tile] = (unsigned char)state;
-    if (state & TILE_LIVE) live[1 + atomicAdd(live, 1)] = tile;
+    if (LIST) {
+      int* list = live + 1 + count;
+      if (state & TILE_LIVE) list[atomicAdd(live, 1)] = tile;
+      // the individual's last tile sees whether it has any support
+      __threadfence();
+      const int add = 1 + (state & TILE_LIVE ? 1 << 16 : 0);
+      if (atomicAdd(live + 1 + tile / TPI, add) + add == TPI) {
+        __threadfence();
+        const int t0 = tile / TPI * TPI, at = atomicAdd(live, TPI);
+        for (int k = 0; k < TPI; ++k) {
+          unsigned char* f = odd + (size_t)first * TPI + t0 + k;
+          *f = (unsigned char)(__ldcg(f) | TILE_LIVE);
+          list[at + k] = t0 + k;
+        }
+      }
+    }
   }
   fft_x<N, Lay, +1, 1, 0>(v, xb, tw, c, j);
   float2* gt = T + (size_t)(first + tile / TPI) * N * N + (size_t)(tile % TPI) * (W * B::YS) + B::at(c, j);

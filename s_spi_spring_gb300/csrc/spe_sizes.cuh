@@ -287,7 +287,8 @@ cudaError_t launch_cols_blocked(const Ctx& c) {
                     static_cast<const unsigned char*>(c.odd), c.ipp, c.first, c.count, c.tw);
 }
 // the list of an ER call's live row tiles, in the magnitudes' memory of its
-// individuals (free during an iteration; a tile is at least two rows)
+// individuals (free during an iteration; a tile is at least two rows): length,
+// counters, tiles
 template <int N>
 int* live_tiles(const Ctx& c) {
   return reinterpret_cast<int*>(c.M + (size_t)c.first * N * N);
@@ -315,9 +316,10 @@ cudaError_t launch_rows_blocked_first(const Ctx& c) {
   cudaError_t e = configure(kern, P::SMEM, configured);
   if (e != cudaSuccess || c.count <= 0) return e;
   int* live = LIST ? live_tiles<N>(c) : nullptr;
-  if (LIST && (e = cudaMemsetAsync(live, 0, sizeof(int), c.st)) != cudaSuccess) return e;
+  if (LIST && (e = cudaMemsetAsync(live, 0, (size_t)(1 + c.count) * sizeof(int), c.st)) != cudaSuccess)
+    return e;
   kern<<<(unsigned)c.count * (N / Blocked<N>::WR), P::NT, P::SMEM, c.st>>>(
-      c.rho, c.S, c.T, static_cast<SpBits<N>*>(c.sp), c.odd, live, c.first, c.tw);
+      c.rho, c.S, c.T, static_cast<SpBits<N>*>(c.sp), c.odd, live, c.first, c.count, c.tw);
   return cudaGetLastError();
 }
 template <int N>
