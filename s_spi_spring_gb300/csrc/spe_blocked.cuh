@@ -171,14 +171,20 @@ struct BlkCfg {
 // An individual without any support has all its tiles in the list: its density
 // is zeros of either sign, and the projection of an all-zero transform goes by
 // their signs.  Not with a phase gate, which may empty a support.)
+// The flags and the list cost a dependent read each before a tile's own; from
+// 3/8 of the tiles on that is more than the rest saves, and every tile runs (20
+// iterations, us, support over 25 / 36 / 45% of the rows; no live tiles:
+// 512^2 x 64 2127 / 2342 / 3208; 3214, 1024^2 x 4 890 / 930 / 1048; 1024; live
+// tiles whatever the support, over all rows: 3607 and 1265).
 enum { TILE_ODD = 1, TILE_LIVE = 2 };
+__device__ __forceinline__ bool every_tile(const int* live, int tiles) { return __ldcg(live) > tiles / 8 * 3; }
 
 // column pass: T -> FFT+ (y) -> P_M with A -> FFT- (y) -> T.  IN / OUT: only
 // the rows of live tiles are read (the others are zeros) / written.
 template <int N, bool IN, bool OUT>
 __global__ void __launch_bounds__(BlkCfg<N, Blocked<N>::BC, Blocked<N>::NXC>::NT, Blocked<N>::MBC)
-    k_cols_blocked(float2* __restrict__ T, const float* __restrict__ At, const unsigned char* __restrict__ odd, int ipp,
-                   int first, int count, const float2* __restrict__ twg) {
+    k_cols_blocked(float2* __restrict__ T, const float* __restrict__ At, const unsigned char* __restrict__ odd,
+                   const int* __restrict__ live, int ipp, int first, int count, const float2* __restrict__ twg) {
   using B = Blocked<N>;
   constexpr int W = B::BC, NX = B::NXC;
   using C = BlkCfg<N, W, NX>;
@@ -196,6 +202,7 @@ __global__ void __launch_bounds__(BlkCfg<N, Blocked<N>::BC, Blocked<N>::NXC>::NT
   const int t = threadIdx.x;
   const int c = t % W, j = t / W;
   const int ntiles = count * TPI;
+  const bool all = (!IN && !OUT) || every_tile(live, count * (N / B::WR));
   // tiles run downward (see the head of the file); T is written by other
   // SMs between the launches: loads go to L2 (__ldcg)
   const size_t off = (size_t)first * N * N + B::at(j, c);
@@ -205,7 +212,7 @@ __global__ void __launch_bounds__(BlkCfg<N, Blocked<N>::BC, Blocked<N>::NXC>::NT
   };
   // the thread's rows of live tiles, as bits
   auto rows_of = [&](int k) {
-    if (!IN && !OUT) return 0xffffffffu;
+    if (all) return 0xffffffffu;
     const unsigned char* f = odd + (size_t)(first + (ntiles - 1 - k) / TPI) * (N / B::WR) + j / B::WR;
     unsigned r = 0;
 #pragma unroll
@@ -297,8 +304,9 @@ __global__ void __launch_bounds__(BlkRowCfg<N>::NT, Blocked<N>::MBR)
   const int t = threadIdx.x;
   const int c = t % W, j = t / W;
   // the tiles of the pass: all, or (LIST) the live ones by their list
-  const int ntiles = LIST ? __ldcg(live) : count * TPI;
-  auto tile_at = [&](int k) { return LIST ? __ldcg(live + 1 + count + k) : k; };
+  const bool all = !LIST || every_tile(live, count * TPI);
+  const int ntiles = all ? count * TPI : __ldcg(live);
+  auto tile_at = [&](int k) { return all ? k : __ldcg(live + 1 + count + k); };
   // offset of a tile's first row in T (blocked), rho and S (row-major)
   auto t_base = [&](int tile) {
     return (size_t)(first + tile / TPI) * N * N + (size_t)(tile % TPI) * (W * B::YS);

@@ -273,6 +273,13 @@ template <int N>
 constexpr int blocked_rows_code() {
   return Blocked<N>::ok ? 800 + Blocked<N>::WR : 0;
 }
+// the list of an ER call's live row tiles, in the magnitudes' memory of its
+// individuals (free during an iteration; a tile is at least two rows): length,
+// counters, tiles
+template <int N>
+int* live_tiles(const Ctx& c) {
+  return reinterpret_cast<int*>(c.M + (size_t)c.first * N * N);
+}
 template <int N, bool IN, bool OUT>
 cudaError_t launch_cols_blocked(const Ctx& c) {
   using P = BlkCfg<N, Blocked<N>::BC, Blocked<N>::NXC>;
@@ -284,14 +291,8 @@ cudaError_t launch_cols_blocked(const Ctx& c) {
   const int tiles = c.count * (N / Blocked<N>::BC);
   const int slots = share(resident_ctas(kern, P::NT, P::SMEM, resident), c.grid_div);
   return launch_pdl(kern, tiles < slots ? tiles : slots, P::NT, P::SMEM, c.st, c.T, c.At,
-                    static_cast<const unsigned char*>(c.odd), c.ipp, c.first, c.count, c.tw);
-}
-// the list of an ER call's live row tiles, in the magnitudes' memory of its
-// individuals (free during an iteration; a tile is at least two rows): length,
-// counters, tiles
-template <int N>
-int* live_tiles(const Ctx& c) {
-  return reinterpret_cast<int*>(c.M + (size_t)c.first * N * N);
+                    static_cast<const unsigned char*>(c.odd),
+                    static_cast<const int*>(IN || OUT ? live_tiles<N>(c) : nullptr), c.ipp, c.first, c.count, c.tw);
 }
 template <int N, int UPD, bool LIST>
 cudaError_t launch_rows_blocked(const Ctx& c, float scale, float beta, Gate g) {
@@ -649,11 +650,15 @@ struct SizeImpl {
           case 0: return iterate_blocked<UPD_HIO, false>(c, iters, beta, g);
           case 1: return iterate_blocked<UPD_RAAR, false>(c, iters, beta, g);
           default:
-            // live tiles: with an open gate (reality 0), and where a pass has
-            // the work to hide the list behind (us a call, dense / live:
-            // 512^2 x 1 81 / 102, x 4 207 / 190; 256^2 x 9 77 / 92; 768^2 x 1
-            // 104 / 99, x 3 312 / 234)
-            return g.hi >= 3.14159f && g.lo >= 3.14159f && (N >= 768 || (size_t)c.count * N * N >= (1u << 20))
+            // live tiles: with an open gate (reality 0), and from the
+            // population on whose passes have the work to hide the flags and
+            // the list behind (20 iterations of a support over 25% of the rows,
+            // us, live / not: 512^2 x 4 336 / 295, x 8 525 / 510, x 9 490 / 514,
+            // x 16 811 / 884; 768^2 x 2 448 / 410, x 4 655 / 690; 1024^2 x 2
+            // 612 / 635 but 5 iterations 191 / 187, x 3 758 / 866; 256^2 x 16
+            // 319 / 290, x 33 437 / 468).  Several engines' calls at once hide
+            // them sooner (512^2 x 4 190 / 207), which a call cannot know.
+            return g.hi >= 3.14159f && g.lo >= 3.14159f && (size_t)c.count * N * N > (2u << 20)
                        ? iterate_blocked<UPD_ER, true>(c, iters, beta, g)
                        : iterate_blocked<UPD_ER, false>(c, iters, beta, g);
         }
