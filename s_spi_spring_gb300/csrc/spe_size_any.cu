@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
   if constexpr (Op::NSUM + Op::NMAX > 0) {
     float r[NRED];
     acc.values(r);
-    block_reduce_store<BIG ? kAnyThreadsBig : kAnyThreads, Op::NSUM, Op::NMAX, true>(op.partials, blockIdx.x, r);
+    block_reduce_store<BIG ? kAnyThreadsBig : kAnyThreads, Op::NSUM, Op::NMAX>(op.partials, blockIdx.x, r, NT);
   }
   if constexpr (Op::PEAK) block_argmax_store<BIG ? kAnyThreadsBig : kAnyThreads, true>(op.partials, acc.mx, acc.idx);
 }
