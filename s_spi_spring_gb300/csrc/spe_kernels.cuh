@@ -113,6 +113,12 @@ __device__ __forceinline__ float cabsf2(float2 v) {
 // x 32 313 us against 323 here, ten refinement steps 512^2 x 64 1320 against
 // 1339, evaluation 512^2 x 64 473 against 476.)
 // ---------------------------------------------------------------------------
+// a += b as a pair of floats, high part and rounding error (Knuth's two-sum)
+__device__ __forceinline__ void add_pair(float& hi, float& lo, float b) {
+  const float s = __fadd_rn(hi, b), t = __fsub_rn(s, hi);
+  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(b, t)));
+  hi = s;
+}
 // digits of the sum in x, y, z, the exponent field of the largest value in w;
 // w = 255: not finite, x the float sum
 __device__ __forceinline__ int4 warp_sum(float v) {
@@ -146,18 +152,23 @@ __device__ __forceinline__ double warp_sum_value(int4 s) {
   const double v = fma(whole(s.z), 1.0 / 4194304, whole((long long)s.x * 4194304 + s.y));
   return v * __hiloint2double((s.w - 170 + 1023) << 20, 0);  // v in units of 2^(w - 170)
 }
-// nt: threads of the CTA (whole warps, at most MOST)
-template <int MOST, int NSUM, int NMAX>
+// nt: threads of the CTA (whole warps, at most MOST); low: null, or (LOW) what
+// the threads' sums v lack
+template <int MOST, int NSUM, int NMAX, bool LOW = false>
 __device__ __forceinline__ void block_reduce_store(double* __restrict__ partials, size_t slot, const float (&v)[NRED],
-                                                   int nt = MOST) {
+                                                   int nt = MOST, const float* low = nullptr) {
   static_assert(NSUM + NMAX <= NRED, "too many reduction values");
-  __shared__ int4 sums[NSUM > 0 ? NSUM : 1][MOST / 32];
+  __shared__ int4 sums[NSUM > 0 ? NSUM * (LOW ? 2 : 1) : 1][MOST / 32];
   __shared__ float top[NMAX > 0 ? NMAX : 1][MOST / 32];
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = nt / 32;
 #pragma unroll
   for (int k = 0; k < NSUM; ++k) {
     const int4 s = warp_sum(v[k]);
     if (lane == 0) sums[k][wid] = s;
+    if (LOW) {
+      const int4 l = warp_sum(low[k]);
+      if (lane == 0) sums[NSUM + k][wid] = l;
+    }
   }
 #pragma unroll
   for (int k = 0; k < NMAX; ++k) {
@@ -169,6 +180,7 @@ __device__ __forceinline__ void block_reduce_store(double* __restrict__ partials
   __syncthreads();
   for (int k = wid; k < NSUM; k += nw) {
     double a = lane < nw ? warp_sum_value(sums[k][lane]) : 0.0;
+    if (LOW && lane < nw) a += warp_sum_value(sums[NSUM + k][lane]);
 #pragma unroll
     for (int off = MOST > 512 ? 16 : MOST > 256 ? 8 : MOST > 128 ? 4 : 2; off > 0; off >>= 1)
       a += __shfl_down_sync(0xffffffffu, a, off);
@@ -381,6 +393,8 @@ struct OpBase {
   // reordered -- all are issued before the first value is formed
   static constexpr bool FETCH = false;
   static constexpr bool FETCH_STORE = false;  // likewise fetch_store, then store
+  // run-time sides: a thread's sums as pairs of floats (ThreadSums)
+  static constexpr bool PAIRS = true;
   // likewise the operands of the pointwise step: fetch_mid, then mid
   struct Mid {};
   template <class Q>
@@ -848,6 +862,7 @@ struct OpRowsSupportForward : OpKeep {
 // -> FFT- (y) -> T
 template <int LOSS, bool GRAD>
 struct OpColsLoss : OpBase {
+  static constexpr bool PAIRS = false;  // (its plan leaves a thread few terms)
   static constexpr int FFT1 = +1, FFT2 = GRAD ? -1 : 0, NSUM = 1, NMAX = 0;
   static constexpr bool AMP = true;
   float2* T;

@@ -428,6 +428,46 @@ __device__ __forceinline__ void fft_any(float2*& cur, float2*& oth, const AnyPla
   }
 }
 
+// A thread's sums and maxima.  It may have tens of terms here (a tile of up to 32
+// lines over as few as 64 threads, where the compiled passes have 4 to 16), so
+// each is added to a pair of floats: the sum does not lose by the tile's shape.
+template <class Op>
+struct ThreadSums {
+  static constexpr bool PAIRS = Op::PAIRS && Op::NSUM > 0;
+  typename Op::Acc acc;
+  float v[NRED] = {}, low[NRED] = {};
+  // f(the accumulator of one element)
+  template <class F>
+  __device__ __forceinline__ auto element(const F& f) {
+    if constexpr (PAIRS) {
+      struct Fold {
+        ThreadSums& s;
+        typename Op::Acc one;
+        __device__ __forceinline__ ~Fold() {
+          float r[NRED];
+          one.values(r);
+#pragma unroll
+          for (int k = 0; k < Op::NSUM; ++k) add_pair(s.v[k], s.low[k], r[k]);
+#pragma unroll
+          for (int k = Op::NSUM; k < Op::NSUM + Op::NMAX; ++k) s.v[k] = fmaxf(s.v[k], r[k]);
+        }
+      } fold{*this, {}};
+      return f(fold.one);
+    } else {
+      return f(acc);
+    }
+  }
+  __device__ __forceinline__ void finish() {
+    if constexpr (PAIRS) {
+#pragma unroll
+      for (int k = 0; k < Op::NSUM; ++k)
+        if (!isfinite(v[k])) low[k] = 0.f;  // (the error of an overflowed sum is not a number)
+    } else {
+      acc.values(v);
+    }
+  }
+};
+
 template <int AXIS, class Op, bool BIG>
 // BIG kernels: two 256-thread CTAs per SM, 128 registers a thread (a few
 // spilled bytes; one CTA per SM without the cap ran 30% slower at side 1054)
@@ -447,7 +487,8 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
   const size_t base = (size_t)p * n * n;
   const int tot = nl * n;
   const unsigned inv_nl = fdiv_inv(nl);
-  typename Op::Acc acc;
+  ThreadSums<Op> sums;
+  using Acc = typename Op::Acc;
   // element i of the tile: row passes walk along x (whole rows), column
   // passes across the tile's columns first (row segments of nl elements)
   const float* amp = Op::AMP ? op.amp(p, n) : nullptr;
@@ -485,8 +526,9 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
         int at;
         const Px q = px(i, at);
         float2 v1, v2;
-        typename Op::Acc once;
-        op.load_pair(q, v1, v2, second ? once : acc);
+        Acc once;
+        if (second) op.load_pair(q, v1, v2, once);
+        else sums.element([&](Acc& a) { op.load_pair(q, v1, v2, a); });
         cur[at] = second ? v2 : v1;
       }
       __syncthreads();
@@ -509,12 +551,14 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
         for (int u = 0; u < U; ++u)
           if (i0 + u * NT < tot) {
             int x;
-            cur[at[u]] = op.form(r[u], px(i0 + u * NT, x), acc);
+            cur[at[u]] = sums.element([&](Acc& a) { return op.form(r[u], px(i0 + u * NT, x), a); });
           }
       } else {
         float2 v[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) if (i0 + u * NT < tot) v[u] = op.load(px(i0 + u * NT, at[u]), acc);
+        for (int u = 0; u < U; ++u)
+          if (i0 + u * NT < tot)
+            v[u] = sums.element([&](Acc& a) { return op.load(px(i0 + u * NT, at[u]), a); });
 #pragma unroll
         for (int u = 0; u < U; ++u)
           if (i0 + u * NT < tot) cur[at[u]] = v[u];
@@ -535,7 +579,8 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
           }
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          if (i0 + u * NT < tot) cur[at[u]] = op.mid(cur[at[u]], q[u], m[u], acc);
+          if (i0 + u * NT < tot)
+            cur[at[u]] = sums.element([&](Acc& a) { return op.mid(cur[at[u]], q[u], m[u], a); });
       });
       __syncthreads();
       fft_any<Op::FFT2, BIG>(cur, oth, pl, tws, nl);
@@ -544,15 +589,15 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
     for (int i = threadIdx.x; i < tot; i += blockDim.x) {
       int at;
       const Px q = px(i, at);
-      op.store(cur[at], q, acc);
+      sums.element([&](Acc& a) { op.store(cur[at], q, a); });
     }
   }
   if constexpr (Op::NSUM + Op::NMAX > 0) {
-    float r[NRED];
-    acc.values(r);
-    block_reduce_store<BIG ? kAnyThreadsBig : kAnyThreads, Op::NSUM, Op::NMAX>(op.partials, blockIdx.x, r, NT);
+    sums.finish();
+    block_reduce_store<BIG ? kAnyThreadsBig : kAnyThreads, Op::NSUM, Op::NMAX, ThreadSums<Op>::PAIRS>(
+        op.partials, blockIdx.x, sums.v, NT, sums.low);
   }
-  if constexpr (Op::PEAK) block_argmax_store<BIG ? kAnyThreadsBig : kAnyThreads, true>(op.partials, acc.mx, acc.idx);
+  if constexpr (Op::PEAK) block_argmax_store<BIG ? kAnyThreadsBig : kAnyThreads, true>(op.partials, sums.acc.mx, sums.acc.idx);
 }
 
 // ---------------------------------------------------------------------------
