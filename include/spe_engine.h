@@ -271,8 +271,14 @@ int spe_crossover_draws(uint32_t seed, int count, const int32_t* order, float su
  * Row codes: W (exchange padding l + l/16), 100+W (padding chosen per
  * exchange), 400+W (two rows per thread in packed registers), 500+W /
  * 600+W (tiles moved by TMA, either padding), 700+W (one stage instead of
- * two).  Every code computes bit-identical results; only codes compiled for
- * the engine's pattern size are accepted (spe_autotune times them all). */
+ * two).  Codes of a pair, each only with the other or 0: 800+W (a blocked
+ * transform scratch; the default of 256, 384, 512, 768, 1024 and 2048), 900
+ * (one thread-block cluster per individual for a whole call, the default of
+ * 32, 64 and 128; calls of more than 48 individuals at 128, or in blocks on
+ * two lanes, run the passes' default widths).  Every code computes
+ * bit-identical results; only codes compiled for the engine's pattern size
+ * are accepted (spe_autotune times them all).  spe_get_tiles returns codes
+ * that spe_set_tiles takes back. */
 int spe_set_tiles(spe_engine* e, int cols, int rows);
 int spe_get_tiles(spe_engine* e, int* cols, int* rows);
 

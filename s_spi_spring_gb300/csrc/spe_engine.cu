@@ -978,6 +978,9 @@ int spe_set_tiles(spe_engine* e, int cols, int rows) {
       if (w[i] == v) return true;
     return false;
   };
+  // the cluster form is the default of its sides (tile_cols = tile_rows = 0)
+  const int cl = e->ops->cluster;
+  if (cl && ((cols == cl && (rows == cl || rows == 0)) || (cols == 0 && rows == cl))) cols = rows = 0;
   if (!ok(cols, e->ops->col_widths) || !ok(rows, e->ops->row_widths))
     return fail(SPE_ERR_INVALID, "tile widths %d/%d not compiled for size %d", cols, rows, e->n);
   // the blocked-scratch passes hand T to each other in their own layout
@@ -1270,6 +1273,10 @@ int spe_get_schedule(spe_engine* e, int* chunk, int* lanes) {
 int spe_get_tiles(spe_engine* e, int* cols, int* rows) {
   if (!e || !cols || !rows) return fail(SPE_ERR_INVALID, "null argument");
   const spe::SizeOps* o = e->ops;
+  if (o->cluster && e->tile_cols == 0 && e->tile_rows <= 0) {
+    *cols = *rows = o->cluster;
+    return SPE_OK;
+  }
   if (o->blocked_cols && (e->tile_cols == 0 || e->tile_cols == o->blocked_cols) &&
       (e->tile_rows <= 0 || e->tile_rows == o->blocked_rows)) {
     *cols = o->blocked_cols;

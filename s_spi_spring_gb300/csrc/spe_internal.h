@@ -235,6 +235,8 @@ struct SizeOps {
   int blocked_cols, blocked_rows;
   size_t sp_bytes;
   cudaError_t (*block_amplitudes)(const float* A, float* At, int npatterns, cudaStream_t st);
+  // tile code of the default where that is a cluster per individual, else 0
+  int cluster;
 };
 
 const SizeOps* size_ops(int n);

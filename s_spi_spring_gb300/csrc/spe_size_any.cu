@@ -1153,7 +1153,8 @@ const SizeOps* size_ops_any(int n) {
                     0,
                     0,
                     0,
-                    nullptr};
+                    nullptr,
+                    0};
   const SizeOps* out = &en->ops;
   g_any.emplace(n, std::move(en));
   return out;

@@ -1031,7 +1031,8 @@ struct SizeImpl {
                               blocked_cols_code<N>(),
                               blocked_rows_code<N>(),
                               Blocked<N>::ok ? (size_t)N * Plan<N>::TPT * sizeof(SpBits<N>) : 0,
-                              &SizeImpl<N>::block_amplitudes};
+                              &SizeImpl<N>::block_amplitudes,
+                              ClusterCfg<N>::ok ? 900 : 0};
     return &t;
   }
 };
