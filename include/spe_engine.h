@@ -110,7 +110,9 @@ int spe_get_amplitudes(spe_engine* e, float* amplitudes);
  * initialisation and the loss use each slot's own pattern; alignment,
  * averages and crossover act on ranges within one pattern (others are
  * rejected).  spe_set_amplitudes returns to a single shared pattern;
- * spe_get_amplitudes reads pattern 0. */
+ * spe_get_amplitudes reads pattern 0.  Device memory per pattern: 12 n^2 bytes
+ * (the amplitudes, the same in the order of the iteration's kernels, and the
+ * correlations' weights), 8 n^2 at sides without blocked passes. */
 int spe_set_amplitudes_batch(spe_engine* e, const float* amplitudes, int npatterns, int individuals_per_pattern);
 
 /* Population capacity in individuals (device memory for density, support

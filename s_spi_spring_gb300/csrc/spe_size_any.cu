@@ -47,17 +47,17 @@ struct AnyPlan {
   int threads;            // of a CTA
   int big;                // a prime radix of 11 or more (any_pass_prime, any_pass_sym: the BIG kernels)
   // divisors of the index arithmetic as fast-division constants (fdiv):
-  // the side, and per pass the butterflies per line n / R, the stride NS of
-  // the pass's outputs and the span NS * R of its sub-transforms
+  // the side, and per pass the butterflies per line n / R and the stride NS of
+  // the pass's outputs
   unsigned inv_n;
   int ns[kMaxRadices];
-  unsigned inv_m[kMaxRadices], inv_ns[kMaxRadices], inv_span[kMaxRadices];
+  unsigned inv_m[kMaxRadices], inv_ns[kMaxRadices];
 };
 
 // x / d as one multiply-high, inv = ceil(2^32 / d) (0 encodes d = 1).  Exact
 // for x < 2^17 and d < 2^15: with x = q d + s and inv d = 2^32 + r, r < d,
 // x inv / 2^32 = q + (s + x r / 2^32) / d, and s + x r / 2^32 < d.  Every
-// index divided here is below W n <= 8 * 9386 < 2^17 (make_plan checks).
+// index divided here is below W n < 2^17 (make_plan narrows W to that).
 __host__ __device__ constexpr unsigned fdiv_inv(int d) { return d <= 1 ? 0u : 0xFFFFFFFFu / (unsigned)d + 1u; }
 __device__ __forceinline__ int fdiv(int x, unsigned inv) { return inv ? (int)__umulhi((unsigned)x, inv) : x; }
 
@@ -666,11 +666,12 @@ int best_threads(const AnyPlan& pl) {
   return best;
 }
 
-// plain: the radices and threads of the operations whose results are compared
-// digit by digit.  A far-field loss is a 64-bit sum that a few bright pixels
-// dominate, and a shrink-wrap's support is a threshold: other radices round
-// differently, and so do other shares of a thread's float sum, which moves a
-// loss in its ninth digit; a rounding may flip a pixel of a support.
+// plain: radices 8, 4 and the primes, 8 lines and the most threads.  A
+// shrink-wrap takes these radices because its support is a threshold of what
+// they transform: other radices round differently, and that may flip a pixel.
+// The loss and the refinement take all three: their threads' float sums (one
+// to a few terms, without ThreadSums' pairs) depend on which pixels share a
+// thread.
 bool make_plan(int n, AnyPlan& pl, bool plain) {
   if (n < 2) return false;
   pl.n = n;
@@ -705,7 +706,6 @@ bool make_plan(int n, AnyPlan& pl, bool plain) {
     pl.ns[i] = ns;
     pl.inv_m[i] = fdiv_inv(n / pl.rad[i]);
     pl.inv_ns[i] = fdiv_inv(ns);
-    pl.inv_span[i] = fdiv_inv(ns * pl.rad[i]);
   }
   pl.LS = n | 1;
   const size_t table = (size_t)n * sizeof(float2);
@@ -1111,11 +1111,6 @@ void fill_any(float2* out, int n) {
 }
 
 }  // namespace
-
-bool any_side_supported(int n) {
-  AnyPlan pl;
-  return make_plan(n, pl, false);
-}
 
 const SizeOps* size_ops_any(int n) {
   std::lock_guard<std::mutex> lock(g_any_mutex);
