@@ -862,7 +862,7 @@ struct OpRowsSupportForward : OpKeep {
 // -> FFT- (y) -> T
 template <int LOSS, bool GRAD>
 struct OpColsLoss : OpBase {
-  static constexpr bool PAIRS = false;  // (its plan leaves a thread few terms)
+  static constexpr bool PAIRS = false;  // (on the plain plan a thread's share does not change)
   static constexpr int FFT1 = +1, FFT2 = GRAD ? -1 : 0, NSUM = 1, NMAX = 0;
   static constexpr bool AMP = true;
   float2* T;

@@ -669,9 +669,9 @@ int best_threads(const AnyPlan& pl) {
 // plain: radices 8, 4 and the primes, 8 lines and the most threads.  A
 // shrink-wrap takes these radices because its support is a threshold of what
 // they transform: other radices round differently, and that may flip a pixel.
-// The loss and the refinement take all three: their threads' float sums (one
-// to a few terms, without ThreadSums' pairs) depend on which pixels share a
-// thread.
+// The loss and the refinement take all three: they add a thread's terms in
+// floats, without ThreadSums' pairs, so that another share of the pixels would
+// move a loss in its ninth digit.
 bool make_plan(int n, AnyPlan& pl, bool plain) {
   if (n < 2) return false;
   pl.n = n;
