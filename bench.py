@@ -44,6 +44,7 @@ B_PER_PIXEL_ITER = 24  # rho read+write 16 B, amplitude 4 B, support 4 B
 # summed over one column and one row launch of every lane.  A configuration
 # without a capture reports no traffic.
 ITER_DRAM_BYTES = {
+    (804, 804, 0, 1): 680_100_000,  # 135.3 + 69.3 + 270.6 + 204.9 MB, the blocked-scratch pair, one whole-range lane
     (8, 104, 0, 1): 757_700_000,   # 135.3 + 78.4 + 335.6 + 208.4 MB, one whole-range lane
     (8, 104, 32, 2): 634_000_000,  # 2 x (68.2 + 8.9 + 167.8 + 72.1) MB, two 32-individual lanes
     (8, 702, 32, 2): 631_000_000,  # 2 x (68.2 + 8.8 + 167.8 + 70.7) MB, one-stage 2-row tiles, two lanes
@@ -1034,8 +1035,8 @@ def run_profile_memetic():
     st = MemeticSettings(generations=10, popsize=POP, alg="RAAR", it=100, beta=BETA, it_ER=20, it_eval=20,
                          sigma=3.0, threshold=0.1)
     sol = Solver(I, gpus=[0], seed=42)
-    sol.engine.set_tiles(8, 104)
-    sol.engine.set_schedule(32, 2)
+    sol.engine.set_tiles(804, 804)
+    sol.engine.set_schedule(0, 1)
     recs = sol.InitializePop(POP, 128, itemsize=[128 * 0.2, 128 * 0.9], nitems=[2, 8], exponent=[0.5, 0.5],
                              scaling=[0.5, 1.5], phaserange=0)
     run = MemeticRun(sol, recs, st)

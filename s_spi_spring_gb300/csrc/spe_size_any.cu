@@ -27,6 +27,7 @@
 #include <memory>
 #include <mutex>
 
+#include "spe_radices.h"
 #include "spe_sizes.cuh"
 
 namespace spe {
@@ -34,7 +35,6 @@ namespace {
 
 constexpr int kAnyThreads = 512;     // most threads of a pass CTA
 constexpr int kAnyThreadsBig = 256;  // the same for plans with a prime radix of 11 or more (128 registers each)
-constexpr int kMaxRadices = 24;
 
 constexpr size_t kAnySmem = 220 * 1024;  // shared-memory budget of one CTA (two line buffers)
 
@@ -615,30 +615,6 @@ __global__ void __launch_bounds__(BIG ? kAnyThreadsBig : kAnyThreads, 2)
 // ---------------------------------------------------------------------------
 // plans
 // ---------------------------------------------------------------------------
-// n (primes up to 7) as a product of the fewest factors in [2, 10], the
-// largest first; fewest factors, then the smallest sum (equal factors).
-int fewest_radices(int n, int* rad) {
-  int best = kMaxRadices + 1, best_sum = 0, cur[kMaxRadices];
-  auto search = [&](auto&& self, int rest, int top, int k, int sum) -> void {
-    if (rest == 1) {
-      if (k < best || (k == best && sum < best_sum)) {
-        best = k;
-        best_sum = sum;
-        std::copy(cur, cur + k, rad);
-      }
-      return;
-    }
-    if (k + 1 > best || k >= kMaxRadices) return;
-    for (int f = top; f >= 2; --f)
-      if (rest % f == 0) {
-        cur[k] = f;
-        self(self, rest / f, f, k + 1, sum + f);
-      }
-  };
-  search(search, n, 10, 0, 0);
-  return best > kMaxRadices ? 0 : best;
-}
-
 size_t smem_of(const AnyPlan& pl) { return (2 * (size_t)pl.W * pl.LS + pl.n) * sizeof(float2); }
 
 int largest_radix(const AnyPlan& pl) { return *std::max_element(pl.rad, pl.rad + pl.nrad); }
@@ -676,9 +652,8 @@ bool make_plan(int n, AnyPlan& pl, bool plain) {
   if (n < 2) return false;
   pl.n = n;
   pl.nrad = 0;
-  // the part of the side without prime factors above 7: in as few passes of
-  // radix 2 .. 10 as it can be, or (`plain`) by 8, 4 and its primes; then the
-  // larger primes
+  // the part of the side without prime factors above 7: by the radices 2 .. 10
+  // that suit it, or (`plain`) by 8, 4 and its primes; then the larger primes
   int smooth = 1, m = n;
   for (int f : {2, 3, 5, 7})
     for (; m % f == 0; m /= f) smooth *= f;
@@ -686,7 +661,7 @@ bool make_plan(int n, AnyPlan& pl, bool plain) {
     for (int f : {8, 4, 2, 3, 5, 7})
       for (; smooth % f == 0; smooth /= f) pl.rad[pl.nrad++] = f;
   } else {
-    pl.nrad = fewest_radices(smooth, pl.rad);
+    pl.nrad = choose_radices(n, smooth, pl.rad);
   }
   for (int f = 11; m > 1 && pl.nrad < kMaxRadices;) {
     if (m % f == 0) {
