@@ -820,14 +820,23 @@ struct SizeImpl {
   }
 
   // M[p] = |FFT+(src[p])| (2D), tmp: scratch of count items
+  // (row-major where a blocked column pass has two columns: it would write the
+  // magnitudes in 8-byte pieces; an average modulus of 24 of 2048^2 1328 us against
+  // 1028)
   static cudaError_t ft_magnitude(const Ctx& c, const float2* src, float2* tmp, float* M) {
     Ctx z = c;
     z.first = 0;
-    SPE_TRY((run_pass<N, AX_ROWS>(rows_forward<SRC_RHO>(z, src, tmp, nullptr), c.count, c.st, c.tw)));
+    const auto forward = rows_forward<SRC_RHO>(z, src, tmp, nullptr);
     OpColsMagnitude cm;
     cm.src = tmp;
     cm.M = M;
-    return run_pass<N, AX_COLS>(cm, c.count, c.st, c.tw);
+    if constexpr (Blocked<N>::ok && Blocked<N>::BC < 4) {
+      SPE_TRY((launch_pass<N, AX_ROWS>(forward, c.count, c.st, c.tw)));
+      return launch_pass<N, AX_COLS>(cm, c.count, c.st, c.tw);
+    } else {
+      SPE_TRY((run_pass<N, AX_ROWS>(forward, c.count, c.st, c.tw)));
+      return run_pass<N, AX_COLS>(cm, c.count, c.st, c.tw);
+    }
   }
 
   // dst[p] = FFT+(|src[p]|) (2D)
