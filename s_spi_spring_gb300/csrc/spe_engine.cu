@@ -178,6 +178,7 @@ int fail(int code, const char* fmt, ...) {
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();  // (a refused call's status is not the next launch's)
   return fail(e == cudaErrorMemoryAllocation ? SPE_ERR_NOMEM : SPE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
