@@ -424,7 +424,9 @@ int spe_get_schedule(spe_engine* e, int* chunk, int* lanes);
  * iteration kernels on the resident population [first, first+count) with
  * `iterations` RAAR steps per trial -- the column width first, then row
  * widths jointly with the schedule (spe_set_schedule) -- keeps the fastest
- * and restores the densities.
+ * and restores the densities.  Error reduction has the support's row tiles
+ * only with codes of 800 + W: where RAAR steps prefer others, a population
+ * that runs much of it is better left at the default.
  * cols / rows (may be NULL) receive the widths; spe_get_schedule the
  * schedule. */
 int spe_autotune(spe_engine* e, int first, int count, int iterations, int* cols, int* rows);
